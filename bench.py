@@ -54,7 +54,7 @@ def parse():
     p.add_argument("--no-e2e", action="store_true")
     p.add_argument("--no-fp64", action="store_true")
     p.add_argument("--no-clocks", action="store_true", help="do not sample nvidia-smi (profiler runs)")
-    p.add_argument("--roofline-kernels", default="assemble,colupd,refl,hemv,dots,wcorr,wfin,her2k,bisect,invit,vhx,btred,applyV,vel,xhz")
+    p.add_argument("--roofline-kernels", default="assemble,hemv,colstep,her2k,bisect,invit,vhx,btred,applyV,vel,xhz")
     p.add_argument("--no-configs", action="store_true", help="skip the samples of the other configurations")
     p.add_argument("--large-cell", type=int, default=0, metavar="NQ",
                    help="instead of the headline bench: NQ q-points around K of the N=11164 cell, range I 1..256 "
@@ -391,7 +391,7 @@ def roofline_for(kclass, rec, n, nq):
             "frac": None, "launches": launches, "avg_launch_ms": ms / launches}
 
 
-ALL_KERNELS = "assemble,colupd,refl,hemv,dots,wcorr,wfin,her2k,bisect,invit,vhx,btred,applyV,vel,xhz"
+ALL_KERNELS = "assemble,hemv,colstep,her2k,bisect,invit,vhx,btred,applyV,vel,xhz"
 
 
 def timed(fn, nq, n, kclasses=ALL_KERNELS):

@@ -45,8 +45,8 @@ int device_sms() {
 }
 
 unsigned kt_mask = 0;
-static const char *kt_names[KT_N] = {"assemble", "colupd", "refl", "hemv", "dots", "wcorr", "wfin", "her2k",
-                                     "bisect", "invit", "vhx", "btred", "applyV", "vel", "xhz"};
+static const char *kt_names[KT_N] = {"assemble", "hemv", "colstep", "her2k", "bisect", "invit", "vhx", "btred",
+                                     "applyV", "vel", "xhz"};
 struct KtPending {
   int k;
   cudaEvent_t a, b;
@@ -219,8 +219,8 @@ int ensure_ws_sized(pp_ctx *c, int B, int mcap, int64_t n, int64_t nbnd_max, int
   free_ws(c);
   const int nb = 32;
   const int64_t lda = (n + 7) / 8 * 8;
-  const int nchunk = (int)((n + 31) / 32);
-  const int nrb = (int)((n + 31) / 32) + 1;  // partial sums per column kernel block
+  // mat-vec partial slots: n/32 (FP64 form), 3 ceil(n/64) (double-float form)
+  const int nchunk = (int)(3 * ((n + 63) / 64));
   const int64_t T = std::min<int64_t>(((int64_t)mcap + 63) / 64 * 64, 2048);
   const int nbr = (int)nbr_max;
   const int ldwp = std::max(std::max(mcap, nbr), 64);
@@ -240,7 +240,6 @@ int ensure_ws_sized(pp_ctx *c, int B, int mcap, int64_t n, int64_t nbnd_max, int
   w.lde = lda;
   w.sE = lda * mcap;
   w.nchunk = nchunk;
-  w.nrb = nrb;
   w.scratch_threads = T;
   w.ldwp = ldwp;
   w.ksplit = ksplit;
@@ -255,12 +254,12 @@ int ensure_ws_sized(pp_ctx *c, int B, int mcap, int64_t n, int64_t nbnd_max, int
   add(&w.W, 16 * (size_t)B * lda * nb);
   add(&w.P, 16 * (size_t)B * nchunk * lda);
   add(&w.X, 16 * (size_t)B * 2 * nb);
-  add((void **)&w.nrm, 8 * (size_t)B * nrb);
-  add((void **)&w.wv, 16 * (size_t)B * nrb);
+  w.spart = (n + 15) / 16 + 1;
+  add(&w.part, 16 * (size_t)B * w.spart);
   add((void **)&w.d, 8 * (size_t)B * n);
   add((void **)&w.e, 8 * (size_t)B * n);
   add((void **)&w.tau, 16 * (size_t)B * n);
-  add((void **)&w.scal, 16 * (size_t)B * 4);
+  add(&w.scal, 16 * (size_t)B);
   add((void **)&w.w, 8 * (size_t)B * n);
   add((void **)&w.rng, 8 * (size_t)B * 8);
   add((void **)&w.tinfo, 8 * (size_t)B * 8);
@@ -356,12 +355,11 @@ EigWork view_of(const EigWork &w, int off, int cnt) {
   v.W = sh(w.W, 16 * (size_t)w.lda * w.nb);
   v.P = sh(w.P, 16 * (size_t)w.nchunk * w.lda);
   v.X = sh(w.X, 16 * 2 * (size_t)w.nb);
-  v.nrm = (double *)sh(w.nrm, 8 * (size_t)w.nrb);
-  v.wv = (z64 *)sh(w.wv, 16 * (size_t)w.nrb);
+  v.part = sh(w.part, 16 * (size_t)w.spart);
   v.d = (double *)sh(w.d, 8 * nmax);
   v.e = (double *)sh(w.e, 8 * nmax);
   v.tau = (z64 *)sh(w.tau, 16 * nmax);
-  v.scal = (z64 *)sh(w.scal, 16 * 4);
+  v.scal = sh(w.scal, 16);
   v.w = (double *)sh(w.w, 8 * nmax);
   v.rng = (int64_t *)sh(w.rng, 8 * 8);
   v.tinfo = (double *)sh(w.tinfo, 8 * 8);
@@ -585,10 +583,10 @@ int run_batch_graph(pp_ctx *c, int B, const pp_eig_opts *o, int mcap, bool want_
         const float ms = time_config(c, B, o, mcap, want_z, spc, 6);
         if (ms > 0.f && ms < best.ms) best = Tuned{spc, 6, ms};
       }
-      // then fewer persistent mat-vec blocks per SM (6 -> 4 -> 3 -> 2) while that helps:
+      // then, FP64 form, fewer persistent mat-vec blocks per SM (6 -> 4 -> 3 -> 2) while that helps:
       // with several streams the mat-vecs of different parts share the SMs
       for (int bps : {4, 3, 2}) {
-        if (best.ms > 1e29f) break;
+        if (best.ms > 1e29f || o->precision == PP_PREC_MIXED) break;
         const float ms = time_config(c, B, o, mcap, want_z, best.split, bps);
         if (!(ms > 0.f && ms < best.ms)) break;
         best = Tuned{best.split, bps, ms};

@@ -9,8 +9,8 @@
 //     panel corrections) follows the zlatrd recurrence; after each panel the
 //     trailing matrix gets the rank-2nb update A -= V W^H + W V^H.  The full
 //     Hermitian square is kept so that every matrix-vector pass reads
-//     coalesced columns (only its lower triangle is read after assembly).  A = Q T Q^H with Q = H(0) H(1) ... H(n-2),
-//     H(i) = I - tau_i v_i v_i^H.
+//     coalesced columns (only its lower triangle is read after assembly).
+//     A = Q T Q^H with Q = H(0) H(1) ... H(n-2), H(i) = I - tau_i v_i v_i^H.
 //  2. Eigenvalues of T by Sturm-count bisection, one thread per eigenvalue
 //     index, with the dstebz tolerance rule max(abstol, pivmin,
 //     2 ulp max(|lo|,|hi|)).  Always FP64.
@@ -65,193 +65,215 @@ __device__ double block_sum(double v, double *sh) {
   __syncthreads();
   return r;
 }
-template <int NT>
-__device__ z64 block_sum_z(z64 v, double *sh) {
-  z64 r;
-  r.re = block_sum<NT>(v.re, sh);
-  r.im = block_sum<NT>(v.im, sh);
-  return r;
-}
-
 // ===========================================================================
 // Stage 1: reduction to tridiagonal form
 // ===========================================================================
 constexpr int TR_NT = 256;   // threads of the column kernels
-constexpr int HV_CC = 32;    // hemv tile width = rows per partial-sum slot
 
-// Sum of a value over groups of TPR consecutive lanes (every lane of the
-// warp takes part; the group's sum ends up in each of its lanes).
-template <class R, int TPR>
-__device__ __forceinline__ C<R> row_reduce(C<R> y) {
-#pragma unroll
-  for (int o = TPR / 2; o > 0; o >>= 1) {
-    C<R> other;
-    float *dst = (float *)&other;
-    const float *src = (const float *)&y;
-#pragma unroll
-    for (int f = 0; f < (int)(sizeof(C<R>) / sizeof(float)); ++f) dst[f] = __shfl_xor_sync(0xffffffffu, src[f], o);
-    y = cadd(y, other);
+// Sums over threads.  Double: plain FP64 adds.  Double-float: an unevaluated
+// sum of three floats, whose additions lose nothing above ~2^-70 of the
+// largest term -- no less than an FP64 sum, without the FP64 pipe (a
+// dependent FP64 add waits 64-150 cycles on this chip, and a division or a
+// square root 560-690; such chains were most of a column's time).
+struct tf {
+  float a, b, c;
+};
+template <class R>
+struct Sum;
+template <>
+struct Sum<double> {
+  typedef double T;
+  PP_D static T zero() { return 0.0; }
+  PP_D static T from(double x) { return x; }
+  PP_D static T add(T x, T y) { return x + y; }
+  PP_D static T sub(T x, T y) { return x - y; }
+  PP_D static T mul(double x, double y) { return x * y; }
+  PP_D static T shfl_xor(T x, int o) { return __shfl_xor_sync(0xffffffffu, x, o); }
+  PP_D static double to(T x) { return x; }
+  PP_D static double toR(T x) { return x; }
+};
+template <>
+struct Sum<df> {
+  typedef tf T;
+  PP_D static T zero() { return tf{0.f, 0.f, 0.f}; }
+  PP_D static T from(df x) { return tf{x.hi, x.lo, 0.f}; }
+  PP_D static T add(T x, T y) {
+    float s, e0, t, e1, u, e2;
+    two_sum(x.a, y.a, s, e0);
+    two_sum(x.b, y.b, t, e1);
+    two_sum(t, e0, u, e2);
+    return tf{s, u, __fadd_rn(__fadd_rn(x.c, y.c), __fadd_rn(e1, e2))};
   }
+  PP_D static T sub(T x, T y) { return add(x, tf{-y.a, -y.b, -y.c}); }
+  // the product of two double-floats with every partial product kept
+  PP_D static T mul(df x, df y) {
+    const float p = __fmul_rn(x.hi, y.hi), pe = __fmaf_rn(x.hi, y.hi, -p);
+    const float q = __fmul_rn(x.hi, y.lo), qe = __fmaf_rn(x.hi, y.lo, -q);
+    const float r = __fmul_rn(x.lo, y.hi), re = __fmaf_rn(x.lo, y.hi, -r);
+    float s, e1, u, e2;
+    two_sum(pe, q, s, e1);
+    two_sum(s, r, u, e2);
+    return tf{p, u, __fadd_rn(__fmaf_rn(x.lo, y.lo, __fadd_rn(qe, re)), __fadd_rn(e1, e2))};
+  }
+  PP_D static T shfl_xor(T x, int o) {
+    return tf{__shfl_xor_sync(0xffffffffu, x.a, o), __shfl_xor_sync(0xffffffffu, x.b, o),
+              __shfl_xor_sync(0xffffffffu, x.c, o)};
+  }
+  PP_D static double to(T x) { return (double)x.a + ((double)x.b + (double)x.c); }
+  PP_D static df toR(T x) {
+    float s, e;
+    two_sum(x.a, x.b, s, e);
+    df r;
+    fast_two_sum(s, __fadd_rn(e, x.c), r.hi, r.lo);
+    return r;
+  }
+};
+// complex value of R from another lane
+template <class R>
+__device__ __forceinline__ R shfl_real(R x, int src) {
+  R y;
+  float *dst = (float *)&y;
+  const float *p = (const float *)&x;
+#pragma unroll
+  for (int f = 0; f < (int)(sizeof(R) / sizeof(float)); ++f) dst[f] = __shfl_sync(0xffffffffu, p[f], src);
   return y;
 }
-constexpr int CU_TPR = 1;                // threads per row of k_colupd (one panel column left to apply)
-constexpr int CU_ROWS = TR_NT / CU_TPR;  // rows per k_colupd block
-
-// A(i:n,i) -= V(i:n,cb:jj) conj(W(i,cb:jj))^T + W(i:n,cb:jj) conj(V(i,cb:jj))^T ;
-// d[i] = Re A(i,i) ; partial sums of |A(r,i)|^2 for r >= i+2.  The panel
-// columns below cb = c_begin were applied already by the previous column's
-// k_wcorr (which reads the same rows of V and W); here c_begin = jj - 1.
-// With fin != 0 it first completes the previous panel column jj-1 (the
-// zlatrd step w += alpha v, alpha = -1/2 tau (w^H v), from the partial sums
-// of k_wcorr): rows >= i+1 are written back by the block that owns them;
-// row i, which every block reads, is completed locally and not written (no
-// later kernel reads it).
 template <class R>
-__global__ void __launch_bounds__(TR_NT) k_colupd(C<R> *Ab, int64_t lda, int64_t sA, C<R> *Wb, int64_t sW,
-                                                  const int *nvec, int i, int k0, int jj, double *dd, int64_t sd,
-                                                  double *nrm, int nrb, int fin, int nprev, z64 *scal,
-                                                  const z64 *wv, int c_begin) {
-  __shared__ C<R> sv[64], sw[64];
-  __shared__ double red[32];
-  __shared__ z64 s_alpha;
-  const int b = blockIdx.y;
-  const int n = nvec[b];
-  if (i >= n) return;
-  C<R> *A = Ab + b * sA;
-  C<R> *W = Wb + b * sW;
-  const int64_t ldw = lda;
-  if (fin && threadIdx.x < 32) {  // warp 0 sums the previous column's partials
-    z64 sacc{0.0, 0.0};
-    for (int k = threadIdx.x; k < nprev; k += 32) {
-      sacc.re += wv[b * nrb + k].re;
-      sacc.im += wv[b * nrb + k].im;
-    }
+__device__ __forceinline__ R shfl_xor_real(R x, int o) {
+  R y;
+  float *dst = (float *)&y;
+  const float *p = (const float *)&x;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      sacc.re += __shfl_xor_sync(0xffffffffu, sacc.re, o);
-      sacc.im += __shfl_xor_sync(0xffffffffu, sacc.im, o);
-    }
-    if (threadIdx.x == 0) {
-      const z64 ts = zmul(scal[b * 4 + 1], sacc);
-      s_alpha = z64{-0.5 * ts.re, -0.5 * ts.im};
-    }
-  }
-  __syncthreads();
-  const C<R> alpha = fin ? cfrom64<R>(s_alpha) : cz<R>();
-  for (int c = c_begin + threadIdx.x; c < jj; c += blockDim.x) {
-    sv[c] = A[i + lda * (k0 + c)];
-    C<R> wc = W[i + ldw * c];
-    if (fin && c == jj - 1) {
-      cmac(wc, alpha, A[i + lda * (i - 1)]);
-      wc = cfin(wc);
-    }
-    sw[c] = wc;
-  }
-  __syncthreads();
-  // CU_TPR threads share one row, each taking the panel columns c = sub mod
-  // CU_TPR, so that the loads of a row are spread over independent threads.
-  const int sub = threadIdx.x % CU_TPR;
-  const int r = i + blockIdx.x * CU_ROWS + threadIdx.x / CU_TPR;
-  double part = 0.0;
-  C<R> acc = cz<R>();
-  if (r < n) {
-#pragma unroll 4
-    for (int c = c_begin + sub; c < jj; c += CU_TPR) {
-      C<R> wrc = W[r + ldw * c];
-      if (fin && c == jj - 1) {
-        cmac(wrc, alpha, A[r + lda * (i - 1)]);
-        wrc = cfin(wrc);
-        if (r > i) W[r + ldw * c] = wrc;
-      }
-      cmac(acc, A[r + lda * (k0 + c)], cconj(sw[c]));
-      cmac(acc, wrc, cconj(sv[c]));
-    }
-  }
-  acc = cfin(acc);
-  acc = row_reduce<R, CU_TPR>(acc);
-  if (r < n && sub == 0) {
-    C<R> a = A[r + lda * i];
-    if (jj > 0) a = csub(a, acc);
-    if (r == i) {
-      a.im = RT<R>::zero();
-      dd[b * sd + i] = RT<R>::to(a.re);
-    }
-    A[r + lda * i] = a;
-    if (r == i + 1) scal[b * 4 + 2] = cto64(a);  // alpha of k_reflector
-    if (r >= i + 2) {
-      z64 t = cto64(a);
-      part = t.re * t.re + t.im * t.im;
-    }
-  }
-  double sn = block_sum<TR_NT>(part, red);
-  if (threadIdx.x == 0) nrm[b * nrb + blockIdx.x] = sn;
+  for (int f = 0; f < (int)(sizeof(R) / sizeof(float)); ++f) dst[f] = __shfl_xor_sync(0xffffffffu, p[f], o);
+  return y;
 }
 
-// zlarfg on A(i+1:n, i); v := [1, x/(alpha-beta)] written back in place.
-// Every block forms the same scalars (alpha = A(i+1, i) as saved by
-// k_colupd, the norm from the same partial sums in the same order) and
-// scales RF_ROWS rows; block 0 writes the scalars and v(i+1) = 1.
-constexpr int RF_ROWS = 4 * TR_NT;
+// Sums of y and of z over each group of 8 consecutive lanes, in every lane of
+// the group.  Halving: after the first exchange half of the lanes carry y and
+// half z, after the second one component each, so a lane makes 4 additions
+// instead of the 12 of two plain butterflies (an FP64 addition holds the pipe
+// for 16 cycles per warp).
 template <class R>
-__global__ void __launch_bounds__(TR_NT) k_reflector(C<R> *Ab, int64_t lda, int64_t sA, const int *nvec, int i,
-                                                     int nparts, const double *nrm, int nrb, double *ee, z64 *tau,
-                                                     int64_t sd, z64 *scal) {
-  __shared__ double red[32];
-  __shared__ z64 s_scale;
-  __shared__ int s_skip;
-  const int b = blockIdx.y;
-  const int n = nvec[b];
-  if (i >= n - 1) {
-    if (blockIdx.x == 0 && threadIdx.x == 0 && i < n) {
-      tau[b * sd + i] = z64{0.0, 0.0};
-      ee[b * sd + i] = 0.0;
-      scal[b * 4 + 0] = z64{0.0, 0.0};
-      scal[b * 4 + 1] = z64{0.0, 0.0};
-    }
-    return;
-  }
-  C<R> *A = Ab + b * sA;
-  double p = 0.0;
-  for (int k = threadIdx.x; k < nparts; k += blockDim.x) p += nrm[b * nrb + k];
-  double xn2 = block_sum<TR_NT>(p, red);
-  if (threadIdx.x == 0) {
-    const z64 alpha = scal[b * 4 + 2];
-    double xnorm = sqrt(xn2);
-    z64 t, sc;
-    double beta;
-    int skip = 0;
-    if (xnorm == 0.0 && alpha.im == 0.0) {
-      t = z64{0.0, 0.0};
-      beta = alpha.re;
-      sc = z64{1.0, 0.0};
-      skip = 1;
-    } else {
-      double nrm3 = sqrt(alpha.re * alpha.re + alpha.im * alpha.im + xn2);
-      beta = -copysign(nrm3, alpha.re);
-      t = z64{(beta - alpha.re) / beta, -alpha.im / beta};
-      // 1/(alpha - beta)
-      double dr = alpha.re - beta, di = alpha.im;
-      double den = dr * dr + di * di;
-      sc = z64{dr / den, -di / den};
-    }
-    if (blockIdx.x == 0) {
-      ee[b * sd + i] = beta;
-      tau[b * sd + i] = t;
-      scal[b * 4 + 0] = sc;
-      scal[b * 4 + 1] = t;
-    }
-    s_scale = sc;
-    s_skip = skip;
-  }
-  __syncthreads();
-  const C<R> scR = cfrom64<R>(s_scale);
-  if (!s_skip) {
-    const int rb = i + 2 + blockIdx.x * RF_ROWS, re = min(n, rb + RF_ROWS);
-#pragma unroll
-    for (int r = rb + threadIdx.x; r < re; r += TR_NT) A[r + lda * i] = cmul(A[r + lda * i], scR);
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) A[(i + 1) + lda * i] = cfrom64<R>(1.0, 0.0);
+__device__ __forceinline__ void group8_sum(C<R> &y, C<R> &z) {
+  const int lane = threadIdx.x & 31;
+  const bool hz = (lane & 4) != 0, him = (lane & 2) != 0;
+  const C<R> keep = hz ? z : y, send = hz ? y : z;
+  const C<R> got{shfl_xor_real(send.re, 4), shfl_xor_real(send.im, 4)};
+  const C<R> m = cadd(keep, got);
+  const R k1 = him ? m.im : m.re, s1 = him ? m.re : m.im;
+  R v = RT<R>::add(k1, shfl_xor_real(s1, 2));
+  v = RT<R>::add(v, shfl_xor_real(v, 1));
+  const int g = lane & ~7;
+  y = C<R>{shfl_real(v, g), shfl_real(v, g + 2)};
+  z = C<R>{shfl_real(v, g + 4), shfl_real(v, g + 6)};
 }
+
+// ---- the reflector's scalars (zlarfg): from |x|^2 and alpha, beta =
+// -copysign(sqrt(|alpha|^2 + |x|^2), Re alpha), tau = ((beta - Re alpha) /
+// beta, -Im alpha / beta) and 1 / (alpha - beta).  All lanes of a warp take
+// part; the four quotients run in lanes 0-3 (one division in time).
+// A sum of x values scaled by 2^-e per value (squares by 2^-2e) keeps the
+// double-float form clear of the float range.
+template <class R>
+struct Reflector {
+  C<R> tau, scale;  // scale belongs to values multiplied by prescale()
+  typename Sum<R>::T beta, t_re, t_im;
+  int e;  // beta is to be multiplied by 2^e
+  int skip;
+};
+__device__ __forceinline__ float pow2_clamped(int e) {  // 2^e, |e| <= 126
+  return __int_as_float((e + 127) << 23);
+}
+__device__ __forceinline__ Reflector<double> reflector_scalars(double xn2, int, C<double> al) {
+  Reflector<double> f;
+  const int lane = threadIdx.x & 31;
+  f.e = 0;
+  f.skip = xn2 == 0.0 && al.im == 0.0;
+  const double nrm = sqrt(al.re * al.re + al.im * al.im + xn2);
+  f.beta = f.skip ? al.re : -copysign(nrm, al.re);
+  const double dr = al.re - f.beta, di = al.im;
+  const double num = lane == 0 ? -dr : (lane == 2 ? dr : -di);
+  const double den = lane < 2 ? f.beta : dr * dr + di * di;
+  const double quo = f.skip ? 0.0 : num / den;
+  f.t_re = __shfl_sync(0xffffffffu, quo, 0);
+  f.t_im = __shfl_sync(0xffffffffu, quo, 1);
+  f.tau = C<double>{f.t_re, f.t_im};
+  f.scale = C<double>{__shfl_sync(0xffffffffu, quo, 2), __shfl_sync(0xffffffffu, quo, 3)};
+  return f;
+}
+__device__ __forceinline__ tf tf_norm(tf x) {
+  float s, e, t, u;
+  two_sum(x.a, x.b, s, e);
+  two_sum(e, x.c, t, u);
+  tf r;
+  fast_two_sum(s, t, r.a, r.b);
+  r.c = u;
+  return r;
+}
+__device__ __forceinline__ tf tf_scale(tf x, float f) {  // f a power of two
+  return tf{__fmul_rn(x.a, f), __fmul_rn(x.b, f), __fmul_rn(x.c, f)};
+}
+__device__ __forceinline__ tf tf_mulf(float q, tf x) {
+  const float p = __fmul_rn(q, x.a), pe = __fmaf_rn(q, x.a, -p);
+  const float r = __fmul_rn(q, x.b), re = __fmaf_rn(q, x.b, -r);
+  float s, e;
+  two_sum(pe, r, s, e);
+  return tf{p, s, __fadd_rn(__fmaf_rn(q, x.c, re), e)};
+}
+// The same in expansions of three floats: square root and quotients from a
+// float estimate and two exact-remainder corrections (Newton / long division),
+// about 2^-66 relative -- more than the FP64 forms, at float latency.
+__device__ __forceinline__ Reflector<df> reflector_scalars(tf xn2, int ex, C<df> al) {
+  typedef Sum<df> S;
+  Reflector<df> f;
+  const int lane = threadIdx.x & 31;
+  const int ea = (int)(__float_as_uint(fmaxf(fabsf(al.re.hi), fabsf(al.im.hi))) >> 23) - 127;
+  const int E = max(ex, min(max(ea, -120), 120));
+  const float fa = pow2_clamped(-E);
+  const int d2 = 2 * (ex - E);
+  const df ar{__fmul_rn(al.re.hi, fa), __fmul_rn(al.re.lo, fa)}, ai{__fmul_rn(al.im.hi, fa), __fmul_rn(al.im.lo, fa)};
+  f.e = E;
+  f.skip = xn2.a == 0.f && al.im.hi == 0.f;
+  const tf s = tf_norm(S::add(tf_scale(xn2, d2 < -126 ? 0.f : pow2_clamped(d2)), S::add(S::mul(ar, ar), S::mul(ai, ai))));
+  // sqrt
+  const float y = rsqrtf(s.a), r = __fmul_rn(s.a, y), hy = 0.5f * y;
+  const float p = __fmul_rn(r, r), pe = __fmaf_rn(r, r, -p);
+  const float c1 = __fmul_rn(__fadd_rn(__fsub_rn(__fsub_rn(s.a, p), pe), s.b), hy);
+  df h;
+  fast_two_sum(r, c1, h.hi, h.lo);
+  const tf rem = S::sub(s, S::mul(h, h));
+  tf beta{h.hi, h.lo, __fmul_rn(__fadd_rn(rem.a, __fadd_rn(rem.b, rem.c)), hy)};
+  if (!signbit(ar.hi)) beta = tf{-beta.a, -beta.b, -beta.c};
+  if (f.skip) beta = S::from(ar);
+  f.beta = beta;
+  // quotients
+  const tf dr = tf_norm(S::sub(S::from(ar), beta));  // alpha_r - beta: no cancellation
+  const df dh{dr.a, dr.b};
+  tf dd = S::mul(dh, dh);
+  dd.c = __fmaf_rn(2.f * dr.a, dr.c, dd.c);
+  const tf den = tf_norm(lane < 2 ? beta : S::add(dd, S::mul(ai, ai)));
+  const tf num = lane == 0 ? tf{-dr.a, -dr.b, -dr.c} : (lane == 2 ? dr : tf{-ai.hi, -ai.lo, 0.f});
+  const float rc = __frcp_rn(den.a);
+  const float q0 = __fmul_rn(num.a, rc);
+  const tf m1 = tf_norm(S::sub(num, tf_mulf(q0, den)));
+  const float q1 = __fmul_rn(m1.a, rc);
+  const tf m2 = tf_norm(S::sub(m1, tf_mulf(q1, den)));
+  tf q = tf_norm(tf{q0, q1, __fmul_rn(m2.a, rc)});
+  if (f.skip) q = S::zero();
+  const df qd = S::toR(q);
+  f.tau = C<df>{shfl_real(qd, 0), shfl_real(qd, 1)};
+  f.scale = C<df>{shfl_real(qd, 2), shfl_real(qd, 3)};
+  f.t_re = tf{__shfl_sync(0xffffffffu, q.a, 0), __shfl_sync(0xffffffffu, q.b, 0), __shfl_sync(0xffffffffu, q.c, 0)};
+  f.t_im = tf{__shfl_sync(0xffffffffu, q.a, 1), __shfl_sync(0xffffffffu, q.b, 1), __shfl_sync(0xffffffffu, q.c, 1)};
+  return f;
+}
+__device__ __forceinline__ C<double> prescale(C<double> x, int) { return x; }
+__device__ __forceinline__ C<df> prescale(C<df> x, int e) {
+  const float f = pow2_clamped(-e);
+  return C<df>{df{__fmul_rn(x.re.hi, f), __fmul_rn(x.re.lo, f)}, df{__fmul_rn(x.im.hi, f), __fmul_rn(x.im.lo, f)}};
+}
+__device__ __forceinline__ float magnitude(C<double>) { return 0.f; }
+__device__ __forceinline__ float magnitude(C<df> x) { return fmaxf(fabsf(x.re.hi), fabsf(x.im.hi)); }
 
 // Lower-triangle Hermitian mat-vec y = A v on the trailing block [i+1, n),
 // over the lower tile pairs (R >= C) of HL_T x HL_T: a tile is read once and
@@ -270,6 +292,10 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src, bool vali
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
+__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait0() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
@@ -279,10 +305,61 @@ __device__ __forceinline__ void tile_pair(int p, int &Rt, int &Ct) {
   while (Rt * (Rt + 1) / 2 > p) --Rt;
   Ct = p - Rt * (Rt + 1) / 2;
 }
+// One of the panel products of column i, by HL_NT threads (t) of one block of
+// the mat-vec's launch: X[c] = V(:,c)^H v (c < jj), X[jj+c] = W(:,c)^H v over rows [i+1, n).
+// They need only v, so they run beside the mat-vec instead of in a launch of
+// their own.  Each thread's sum is renormalised every 4 rows.
+template <class R>
+__device__ __forceinline__ void panel_dot(const C<R> *A, const C<R> *W, int64_t lda, int n, int i, int k0, int jj,
+                                          int c2, int t, typename Sum<R>::T (*red)[HL_NT / 32], C<R> *X) {
+  typedef Sum<R> S;
+  typedef typename S::T T;
+  const bool some = c2 < 2 * jj;  // (the last block's spare groups only pass the barrier)
+  const bool useW = c2 >= jj;
+  const int c = useW ? c2 - jj : c2;
+  const C<R> *Xc = useW ? (W + lda * c) : (A + lda * (k0 + c));
+  const C<R> *v = A + lda * i;
+  C<R> acc = cz<R>();
+  int r = some ? i + 1 + t : n;
+  for (; r + 3 * HL_NT < n; r += 4 * HL_NT) {
+    C<R> x[4], y[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      x[u] = Xc[r + u * HL_NT];
+      y[u] = v[r + u * HL_NT];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) cmacc(acc, x[u], y[u]);
+    acc = cfin(acc);
+  }
+  for (; r < n; r += HL_NT) cmacc(acc, Xc[r], v[r]);
+  acc = cfin(acc);
+  T sr = S::from(acc.re), si = S::from(acc.im);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    sr = S::add(sr, S::shfl_xor(sr, o));
+    si = S::add(si, S::shfl_xor(si, o));
+  }
+  if ((t & 31) == 0) {
+    red[0][t >> 5] = sr;
+    red[1][t >> 5] = si;
+  }
+  __syncthreads();
+  if (t == 0 && some) {
+#pragma unroll
+    for (int k = 1; k < HL_NT / 32; ++k) {
+      sr = S::add(sr, red[0][k]);
+      si = S::add(si, red[1][k]);
+    }
+    X[c2] = C<R>{S::toR(sr), S::toR(si)};
+  }
+}
+
 template <class R>
 __global__ void __launch_bounds__(HL_NT, HL_BPS) k_hemv_lower(const C<R> *Ab, int64_t lda, int64_t sA,
                                                               const int *nvec, int i, C<R> *Pb, int64_t sP,
-                                                              int64_t ldp) {
+                                                              int64_t ldp, const C<R> *Wb, int64_t sW, int k0,
+                                                              int jj, C<R> *X, int ldx) {
   __shared__ __align__(16) C<R> tile[2][HL_T * HL_LD];  // tile[buf][c * HL_LD + r]
   __shared__ __align__(16) C<R> vR[2][HL_T], vC[2][HL_T];
   __shared__ C<R> red[2][2][HL_T];
@@ -290,9 +367,15 @@ __global__ void __launch_bounds__(HL_NT, HL_BPS) k_hemv_lower(const C<R> *Ab, in
   const int n = nvec[b];
   const int r0 = i + 1;
   if (r0 >= n) return;
+  if ((int)blockIdx.x < 2 * jj) {
+    __shared__ typename Sum<R>::T dred[2][HL_NT / 32];
+    panel_dot<R>(Ab + b * sA, Wb + b * sW, lda, n, i, k0, jj, blockIdx.x, threadIdx.x, dred, X + b * ldx);
+    return;
+  }
+  const int bx = blockIdx.x - 2 * jj, gx = gridDim.x - 2 * jj;  // among the mat-vec's blocks
   const int nt = (n - r0 + HL_T - 1) / HL_T;
   const int npairs = nt * (nt + 1) / 2;
-  if ((int)blockIdx.x >= npairs) return;
+  if (bx >= npairs) return;
   const C<R> *A = Ab + b * sA;
   const int tid = threadIdx.x;
   // copies of tile pair p into buffer buf (zero outside the matrix)
@@ -325,11 +408,11 @@ __global__ void __launch_bounds__(HL_NT, HL_BPS) k_hemv_lower(const C<R> *Ab, in
   const int lane = tid & (HL_T - 1), wid = tid / HL_T;
   const int prod = wid >> 1, half = wid & 1;
   constexpr int SPAN = HL_T / 2;
-  issue(blockIdx.x, 0);
+  issue(bx, 0);
   int buf = 0;
-  for (int p = blockIdx.x; p < npairs; p += gridDim.x) {
-    if (p + (int)gridDim.x < npairs)
-      issue(p + gridDim.x, buf ^ 1);
+  for (int p = bx; p < npairs; p += gx) {
+    if (p + gx < npairs)
+      issue(p + gx, buf ^ 1);
     else
       cp_async_commit();  // an empty group keeps "all but the newest" meaning this tile
     cp_async_wait1();
@@ -371,122 +454,595 @@ __global__ void __launch_bounds__(HL_NT, HL_BPS) k_hemv_lower(const C<R> *Ab, in
   cp_async_wait0();
 }
 
-// X[c] = V(:,c)^H v (c < jj), X[jj+c] = W(:,c)^H v, over rows [i+1, n).
-template <class R>
-__global__ void __launch_bounds__(TR_NT) k_dots(const C<R> *Ab, int64_t lda, int64_t sA, const C<R> *Wb, int64_t sW,
-                                                const int *nvec, int i, int k0, int jj, z64 *X, int ldx) {
-  __shared__ double red[32];
-  const int b = blockIdx.y;
-  const int n = nvec[b];
-  if (i >= n - 1) return;
-  const C<R> *A = Ab + b * sA;
-  const C<R> *W = Wb + b * sW;
-  const int c2 = blockIdx.x;
-  const bool useW = c2 >= jj;
-  const int c = useW ? c2 - jj : c2;
-  const C<R> *Xc = useW ? (W + lda * c) : (A + lda * (k0 + c));
-  C<R> acc = cz<R>();
-#pragma unroll 4
-  for (int r = i + 1 + threadIdx.x; r < n; r += blockDim.x) cmacc(acc, Xc[r], A[r + lda * i]);
-  z64 s = block_sum_z<TR_NT>(cto64(cfin(acc)), red);
-  if (threadIdx.x == 0) X[b * ldx + c2] = s;
+// ---- the mat-vec of the double-float form
+// Lower-triangle Hermitian mat-vec on tiles of 64 rows x 32 columns of the
+// trailing block.  Warps 0-3 form A_RC v_C (16 rows each; a lane: one row,
+// half of the columns), warps 4-7 A_RC^H v_R (8 columns each; a lane: one
+// column, 16 rows): every sum ends inside one warp, so that the only barrier
+// per tile is the one that hands over its buffer.  In the two tiles on the
+// diagonal the entries above it are masked in both products and the diagonal
+// itself in the second.  Each CTA walks a run of consecutive tiles of the
+// row-major tile list and keeps the row sums in registers along a tile row,
+// so a row gets one partial per run that crosses its tile row and one per
+// tile row from its own on (hv_slots) instead of one per 32 columns.  The
+// runs depend on the order of the trailing block, the column of the panel and
+// the number of SMs only.  The first CTAs of the grid form the panel products
+// (panel_dot), 2 per CTA.
+// Bound by instruction issue: 96 double-float lane operations per stored
+// element (two complex multiply-adds), 122 instructions in all where the
+// 32 x 32 tiles of the earlier kernel took 152.  One matrix of order 4764,
+// first columns: 66.5 us -> 53.5 us (3.4 TB/s); four of them 196 us.  Measured
+// and not kept: packed f32x2 arithmetic (30% fewer instructions, but three
+// shared-memory reads per vector entry: 57 us); bulk copies by a fetching warp
+// with mbarriers (61 us: 1 KB copies are issued too slowly); tiles of 64 x 64.
+constexpr int HV_R = 64, HV_C = 32, HV_LD = HV_R + 1;
+constexpr int HV_NT = 256;
+constexpr int HV_BPS = 3;  // resident CTAs per SM
+constexpr int HV_TILE = HV_C * HV_LD * 16;
+constexpr int HV_SMEM = 2 * HV_TILE + 2 * (HV_R + HV_C) * 16;
+// CTAs of the panel products, CTAs left for the runs, tiles per run
+__host__ __device__ __forceinline__ int hv_dots(int jj) { return jj; }
+__host__ __device__ __forceinline__ int hv_ctas(int jj, int sms) {
+  return HV_BPS * sms - hv_dots(jj) > 1 ? HV_BPS * sms - hv_dots(jj) : 1;
+}
+__host__ __device__ __forceinline__ int hv_run(int rows, int jj, int sms) {
+  const int nt = (rows + HV_R - 1) / HV_R, tiles = nt * (nt + 1), g = hv_ctas(jj, sms);
+  return (tiles + g - 1) / g;
+}
+// Partial slots of a row in tile row R of nt: runs first .. first + nseg - 1
+// cross it (slots 0 .. nseg-1), tile rows R .. nt-1 hold its column (slots
+// 2 nt + R .. 3 nt - 1).
+__device__ __forceinline__ void hv_slots(int R, int run, int &first, int &nseg) {
+  const int s = R * (R + 1);
+  first = s / run;
+  nseg = (s + 2 * R + 1) / run - first + 1;
 }
 
-// w = tau (y - W x1 - V x2) with y = sum of hemv partials; partial w^H v.
-// WC_TPR threads share one row: each sums a strided subset of the partial
-// slots, then a shuffle reduction; this keeps many independent loads in
-// flight per row (the slots are the latency-bound part).
-constexpr int WC_TPR = 8;
-constexpr int WC_ROWS = TR_NT / WC_TPR;  // rows per block
-template <class R>
-__global__ void __launch_bounds__(TR_NT) k_wcorr(C<R> *Ab, int64_t lda, int64_t sA, C<R> *Wb, int64_t sW,
-                                                 const C<R> *Pb, int64_t sP, int64_t ldp, const int *nvec, int i,
-                                                 int k0, int jj, const z64 *X, int ldx, const z64 *scal, z64 *wv,
-                                                 int nrb, int fuse) {
-  __shared__ C<R> x1[64], x2[64], nv[64], nw[64];
-  __shared__ double red[32];
+__global__ void __launch_bounds__(HV_NT, HV_BPS) k_hemv_df(const zdf *Ab, int64_t lda, int64_t sA, const int *nvec,
+                                                           int i, zdf *Pb, int64_t sP, int64_t ldp, const zdf *Wb,
+                                                           int64_t sW, int k0, int jj, zdf *X, int ldx, int sms) {
+  extern __shared__ __align__(16) unsigned char hv_smem[];
+  zdf *tiles = (zdf *)hv_smem;              // [2][32 columns][HV_LD]
+  zdf *vecs = tiles + 2 * HV_C * HV_LD;     // [2][v_R 64, v_C 32]
   const int b = blockIdx.y;
   const int n = nvec[b];
-  if (i >= n - 1) return;
-  C<R> *A = Ab + b * sA;
-  C<R> *W = Wb + b * sW;
-  for (int c = threadIdx.x; c < jj; c += blockDim.x) {
-    x1[c] = cfrom64<R>(X[b * ldx + c]);       // V^H v
-    x2[c] = cfrom64<R>(X[b * ldx + jj + c]);  // W^H v
-    if (fuse) {                               // row i+1 of V and W
-      nv[c] = cconj(A[(i + 1) + lda * (k0 + c)]);
-      nw[c] = cconj(W[(i + 1) + lda * c]);
+  const int r0 = i + 1;
+  if (r0 >= n) return;
+  const zdf *A = Ab + b * sA;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nd = hv_dots(jj);
+  if ((int)blockIdx.x < nd) {
+    const int g = warp >> 2;
+    panel_dot<df>(A, Wb + b * sW, lda, n, i, k0, jj, blockIdx.x * 2 + g, tid & (HL_NT - 1),
+                  (Sum<df>::T(*)[4])hv_smem + 2 * g,
+                  X + b * ldx);
+    return;
+  }
+  const int nt = (n - r0 + HV_R - 1) / HV_R;
+  const int run = hv_run(n - r0, jj, sms);
+  const int x = blockIdx.x - nd;
+  int t = x * run;
+  const int tend = min(t + run, nt * (nt + 1));
+  if (t >= tend) return;
+  int R = (int)((sqrtf(4.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+  while ((R + 1) * (R + 2) <= t) ++R;
+  while (R * (R + 1) > t) --R;
+  int Cc = t - R * (R + 1);
+  int Ri = R, Ci = Cc, ti = t;  // the next tile to request
+  // this thread's part of a tile: row tr, columns tc, tc + 4, ...
+  const int tr = tid & (HV_R - 1), tc = tid / HV_R;
+  // copies of the next tile and its vector pieces into buffer buf (zero
+  // outside the matrix); an empty group past the run's end
+  auto issue = [&](int buf) {
+    if (ti < tend) {
+      const int rt0 = r0 + Ri * HV_R, ct0 = r0 + Ci * HV_C;
+      const zdf *src = A + rt0 + tr + lda * (ct0 + tc);
+      zdf *dst = tiles + buf * (HV_C * HV_LD) + tc * HV_LD + tr;
+      zdf *vdst = vecs + buf * (HV_R + HV_C) + tid;
+      const int k = tid < HV_R ? rt0 + tid : ct0 + tid - HV_R;
+      if (rt0 + HV_R <= n) {  // (every column of a full tile row exists)
+#pragma unroll
+        for (int j = 0; j < HV_C / 4; ++j) cp_async16(dst + 4 * j * HV_LD, src + 4 * j * lda);
+        if (tid < HV_R + HV_C) cp_async16(vdst, A + k + lda * i);
+      } else {
+#pragma unroll
+        for (int j = 0; j < HV_C / 4; ++j) {
+          const bool ok = rt0 + tr < n && ct0 + tc + 4 * j < n;
+          cp_async16(dst + 4 * j * HV_LD, ok ? (const void *)(src + 4 * j * lda) : (const void *)A, ok);
+        }
+        if (tid < HV_R + HV_C) cp_async16(vdst, k < n ? (const void *)(A + k + lda * i) : (const void *)A, k < n);
+      }
+      ++ti;
+      if (++Ci > 2 * Ri + 1) {
+        ++Ri;
+        Ci = 0;
+      }
+    }
+    cp_async_commit();
+  };
+  issue(0);
+  zdf y = cz<df>();  // row sum (warps 0-3)
+  zdf *Pm = Pb + b * sP;
+  for (int buf = 0; t < tend; ++t, buf ^= 1) {
+    cp_async_wait0();
+    __syncthreads();  // this tile has landed, the other buffer is free
+    issue(buf ^ 1);
+    const zdf *tl = tiles + buf * (HV_C * HV_LD);
+    const zdf *vl = vecs + buf * (HV_R + HV_C);
+    const int off = HV_C * (Cc - 2 * R);  // >= 0 on the diagonal: entry (r, c) is below it for r > c + off
+    if (warp < 4) {
+      const int r = warp * 16 + (lane & 15), cb = lane & 16;
+      const zdf *vc = vl + HV_R + cb, *ta = tl + cb * HV_LD + r;
+      if (off < 0) {
+#pragma unroll 4
+        for (int k = 0; k < 16; ++k) cmac(y, ta[k * HV_LD], vc[k]);
+      } else {
+        for (int k = 0; k < 16; ++k) cmac(y, r >= cb + k + off ? ta[k * HV_LD] : cz<df>(), vc[k]);
+      }
+      y = cfin(y);
+      if (off == HV_C || t + 1 == tend) {  // the row sums end here
+        y = cadd(y, zdf{shfl_xor_real(y.re, 16), shfl_xor_real(y.im, 16)});
+        int first, nseg;
+        hv_slots(R, run, first, nseg);
+        const int row = r0 + R * HV_R + r;
+        if (lane < 16 && row < n) Pm[(int64_t)(x - first) * ldp + row] = y;
+        y = cz<df>();
+      }
+    } else {
+      const int c = (warp - 4) * 8 + (lane & 7), rb = (lane >> 3) * 16;
+      const zdf *vr = vl + rb, *ta = tl + c * HV_LD + rb;
+      zdf s = cz<df>();
+      if (off < 0) {
+#pragma unroll 4
+        for (int k = 0; k < 16; ++k) cmacc(s, ta[k], vr[k]);
+      } else {
+        for (int k = 0; k < 16; ++k) cmacc(s, rb + k > c + off ? ta[k] : cz<df>(), vr[k]);
+      }
+      s = cfin(s);
+      // over the four row groups: lanes below 16 end up with the real part, the others with the imaginary part
+      const bool im = lane >= 16;
+      df q = df_add(im ? s.im : s.re, shfl_xor_real(im ? s.re : s.im, 16));
+      q = df_add(q, shfl_xor_real(q, 8));
+      const df qi = shfl_xor_real(q, 16);
+      const int col = r0 + Cc * HV_C + c;
+      if (lane < 8 && col < n) Pm[(int64_t)(2 * nt + R) * ldp + col] = zdf{q, qi};
+    }
+    if (++Cc > 2 * R + 1) {
+      ++R;
+      Cc = 0;
     }
   }
-  __syncthreads();
-  const int sub = threadIdx.x % WC_TPR;
-  const int r = i + 1 + blockIdx.x * WC_ROWS + threadIdx.x / WC_TPR;
-  z64 part{0.0, 0.0};
-  const int nch = cdiv_dev(n - i - 1, HV_CC);
-  C<R> y = cz<R>(), nxt = cz<R>();
-  if (r < n) {
-    const C<R> *Pr = Pb + b * sP + r;
-#pragma unroll 4
-    for (int ch = sub; ch < nch; ch += WC_TPR) y = cadd(y, Pr[(int64_t)ch * ldp]);
-    // this thread's share of the panel corrections, columns c = sub mod
-    // WC_TPR; with fuse also the same columns' update of column i+1
+  cp_async_wait0();
+}
+
+// ---- the work between two mat-vecs
+// What the row work of panel column i reads.  Rows r >= col = i + 1; the
+// mat-vec's partials of row r lie in `slots` slots of P: one per tile row /
+// column of 32 (k_hemv_lower), or (double-float form) the runs of its tile row
+// and the tile rows from its own on.
+template <class R>
+struct PanelCol {
+  const C<R> *A, *W, *P;
+  int64_t lda, ldp;
+  int n, i, k0, jj, next, nt, run;  // next: column i + 1 belongs to the same panel
+  __device__ __forceinline__ PanelCol(const C<R> *A_, const C<R> *W_, const C<R> *P_, int64_t lda_, int64_t ldp_, int n_,
+                                      int i_, int k0_, int jj_, int next_, int sms)
+      : A(A_), W(W_), P(P_), lda(lda_), ldp(ldp_), n(n_), i(i_), k0(k0_), jj(jj_), next(next_) {
+    nt = cdiv_dev(n - i - 1, std::is_same<R, double>::value ? HL_T : HV_R);
+    run = std::is_same<R, double>::value ? 1 : hv_run(n - i - 1, jj, sms);
+  }
+  // the number of slots of row r: 0 .. nseg-1, then from nseg + skip on
+  __device__ __forceinline__ int slots(int r, int &nseg, int &skip) const {
+    if constexpr (std::is_same<R, double>::value) {
+      nseg = nt;
+      skip = 0;
+      return nt;
+    } else {
+      int first;
+      const int Rt = (r - i - 1) / HV_R;
+      hv_slots(Rt, run, first, nseg);
+      skip = 2 * nt + Rt - nseg;
+      return nseg + nt - Rt;
+    }
+  }
+};
+// What one lane (sub = 0 .. 7 of the row's eight) reads of row r: its slots
+// and panel columns sub, sub + 8, ..., and, in lane 0, v and column i + 1.
+constexpr int CT_TPR = 8;
+template <class R>
+struct PanelRow {
+  C<R> p[4], w[4], v[4], vi, a;
+  __device__ __forceinline__ void load(const PanelCol<R> &c, int r, int sub) {
+    const bool in = r < c.n;
+    int nseg, skip;
+    const int nch = c.slots(in ? r : c.i + 1, nseg, skip);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int k = sub + CT_TPR * u;
+      p[u] = in && k < nch ? c.P[r + (int64_t)(k + (k >= nseg ? skip : 0)) * c.ldp] : cz<R>();
+      w[u] = in && k < c.jj ? c.W[r + c.lda * k] : cz<R>();
+      v[u] = in && k < c.jj ? c.A[r + c.lda * (c.k0 + k)] : cz<R>();
+    }
+    const bool own = in && sub == 0;
+    vi = own ? c.A[r + c.lda * c.i] : cz<R>();
+    a = own && c.next ? c.A[r + c.lda * (c.i + 1)] : cz<R>();
+  }
+  // y = (mat-vec) - W x1 - V x2 and nxt = the panel columns' part of column
+  // i + 1's update (x1, x2, row i + 1 of V and W conjugated in shared memory),
+  // summed over the row's eight lanes
+  __device__ __forceinline__ void sums(const PanelCol<R> &c, int r, int sub, const C<R> *x1, const C<R> *x2,
+                                       const C<R> *nv, const C<R> *nw, C<R> &y, C<R> &nxt) const {
+    y = cadd(cadd(p[0], p[1]), cadd(p[2], p[3]));
+    nxt = cz<R>();
+    int nseg, skip;
+    const int nch = c.slots(r < c.n ? r : c.i + 1, nseg, skip);
+    for (int ch = sub + 4 * CT_TPR; ch < nch; ch += 4 * CT_TPR) {
+      C<R> t[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int k = ch + CT_TPR * u;
+        t[u] = r < c.n && k < nch ? c.P[r + (int64_t)(k + (k >= nseg ? skip : 0)) * c.ldp] : cz<R>();
+      }
+      y = cadd(y, cadd(cadd(t[0], t[1]), cadd(t[2], t[3])));
+    }
     C<R> acc = cz<R>();
-#pragma unroll 4
-    for (int c = sub; c < jj; c += WC_TPR) {
-      const C<R> wrc = W[r + lda * c], vrc = A[r + lda * (k0 + c)];
-      cmac(acc, wrc, x1[c]);
-      cmac(acc, vrc, x2[c]);
-      if (fuse) {
-        cmac(nxt, vrc, nw[c]);
-        cmac(nxt, wrc, nv[c]);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int k = sub + CT_TPR * u;
+      if (CT_TPR * u >= c.jj) break;
+      if (k < c.jj) {
+        cmac(acc, w[u], x1[k]);
+        cmac(acc, v[u], x2[k]);
+        if (c.next) {
+          cmac(nxt, v[u], nw[k]);
+          cmac(nxt, w[u], nv[k]);
+        }
       }
     }
     y = csub(y, cfin(acc));
+    nxt = cfin(nxt);
+    group8_sum(y, nxt);
   }
-  y = row_reduce<R, WC_TPR>(y);
-  if (fuse) {
-    // A(r, i+1) -= V(r, 0:jj) conj(W(i+1, 0:jj))^T + W(r, 0:jj) conj(V(i+1, 0:jj))^T
-    nxt = row_reduce<R, WC_TPR>(cfin(nxt));
-    if (r < n && sub == 0) A[r + lda * (i + 1)] = csub(A[r + lda * (i + 1)], nxt);
+};
+// x1 = V^H v, x2 = W^H v and row i + 1 of V and W (conjugated) into shared memory
+template <class R>
+__device__ __forceinline__ void panel_small(const PanelCol<R> &c, const C<R> *X, C<R> *x1, C<R> *x2, C<R> *nv, C<R> *nw) {
+  for (int k = threadIdx.x; k < c.jj; k += blockDim.x) {
+    x1[k] = X[k];
+    x2[k] = X[c.jj + k];
+    if (c.next) {
+      nv[k] = cconj(c.A[c.i + 1 + c.lda * (c.k0 + k)]);
+      nw[k] = cconj(c.W[c.i + 1 + c.lda * k]);
+    }
   }
-  if (r < n && sub == 0) {
-    const C<R> t = cfrom64<R>(scal[b * 4 + 1]);
-    C<R> w = cmul(t, y);
-    W[r + lda * jj] = w;
-    z64 w64 = cto64(w), v64 = cto64(A[r + lda * i]);
-    part = z64{w64.re * v64.re + w64.im * v64.im, w64.re * v64.im - w64.im * v64.re};
-  }
-  z64 s = block_sum_z<TR_NT>(part, red);
-  if (threadIdx.x == 0) wv[b * nrb + blockIdx.x] = s;
+}
+// sum over lanes 0, 8, 16, 24 (the rows of a warp), in every one of them
+template <class R>
+__device__ __forceinline__ C<R> rows4_sum(C<R> x) {
+#pragma unroll
+  for (int o = 16; o >= 8; o >>= 1) x = cadd(x, C<R>{shfl_xor_real(x.re, o), shfl_xor_real(x.im, o)});
+  return x;
 }
 
-// alpha = -1/2 tau (w^H v) ; w += alpha v
+// Large trailing blocks: the row work of column i on the whole chip.
+//   w0 = tau (y - W x1 - V x2) into column jj of W, column i + 1 less the panel
+//   columns' part, and one partial of w0^H v per block.
+// k_colstep then only completes w and forms the next reflector.
 template <class R>
-__global__ void __launch_bounds__(TR_NT) k_wfin(const C<R> *Ab, int64_t lda, int64_t sA, C<R> *Wb, int64_t sW,
-                                                const int *nvec, int i, int jj, int nparts, const z64 *scal,
-                                                const z64 *wv, int nrb) {
-  __shared__ z64 s_alpha;
+constexpr int wp_threads = std::is_same<R, double>::value ? 128 : 256;  // FP64: spread over more SMs' FP64 pipes
+template <class R>
+__global__ void __launch_bounds__(wp_threads<R>) k_wpart(C<R> *Ab, int64_t lda, int64_t sA, C<R> *Wb, int64_t sW,
+                                                         const C<R> *Pb, int64_t sP, int64_t ldp, const int *nvec, int i,
+                                                         int k0, int jj, int next, int sms, const C<R> *X, int ldx,
+                                                         const C<R> *taub, C<R> *partb, int64_t spart) {
+  constexpr int NW = wp_threads<R> / 32;
+  __shared__ C<R> x1[32], x2[32], nv[32], nw[32], red[NW];
   const int b = blockIdx.y;
   const int n = nvec[b];
-  if (i >= n - 1) return;
-  if (threadIdx.x == 0) {
-    z64 s{0.0, 0.0};
-    for (int k = 0; k < nparts; ++k) {
-      s.re += wv[b * nrb + k].re;
-      s.im += wv[b * nrb + k].im;
+  const int col = i + 1;
+  const int rb = col + blockIdx.x * NW * 4;
+  if (rb >= n) return;
+  C<R> *A = Ab + b * sA;
+  C<R> *W = Wb + b * sW;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sub = tid % CT_TPR;
+  const PanelCol<R> pc(A, W, Pb + b * sP, lda, ldp, n, i, k0, jj, next, sms);
+  const int r = rb + tid / CT_TPR;
+  PanelRow<R> q;
+  q.load(pc, r, sub);
+  const C<R> tau = taub[b];
+  panel_small(pc, X + b * ldx, x1, x2, nv, nw);
+  __syncthreads();
+  C<R> y, nxt, dot = cz<R>();
+  q.sums(pc, r, sub, x1, x2, nv, nw, y, nxt);
+  C<R> *part = partb + b * spart;
+  if (sub == 0 && r < n) {
+    const C<R> w = cmul(tau, y);
+    W[r + lda * jj] = w;
+    if (next) A[r + lda * col] = csub(q.a, nxt);
+    cmacc(dot, w, q.vi);
+    if (r == col) part[0] = w;  // w0(i+1)
+  }
+  dot = rows4_sum(cfin(dot));
+  if (lane == 0) red[warp] = dot;
+  __syncthreads();
+  if (tid == 0) {
+#pragma unroll
+    for (int k = 1; k < NW; ++k) dot = cadd(dot, red[k]);
+    part[1 + blockIdx.x] = dot;
+  }
+}
+
+// One panel column's scalar and row work, one cluster of CTAs per matrix (rows
+// are dealt to the CTAs' warps in groups of 4).  With do_w != 0, for column i
+// (its mat-vec partials in P, the products x1 = V^H v and x2 = W^H v in X):
+//   w0 = tau (y - W x1 - V x2),  alpha = -1/2 tau (w0^H v),  w = w0 + alpha v
+//   (column jj of W); do_w = 2: w0, the panel columns' part of column i + 1
+//   and the nparts partials of w0^H v were formed by k_wpart;
+// with do_next, for column i + 1 = col of the same panel (do_w = 0: the
+// panel's first column):
+//   A(col:n, col) -= V W(col,:)^H + W V(col,:)^H over the panel columns 0..jj,
+//   d, the reflector (zlarfg: beta, tau, v = [1; x / (alpha - beta)]) and v
+//   written back in place.
+// The two global sums (w0^H v and |x|^2) cross the CTAs through distributed
+// shared memory: each warp writes its part into every CTA of the cluster and
+// passes the cluster barrier (0.2-0.3 us).  Bound by latency: the loads of a
+// row (partial slots, panel columns, v, the next column) are all issued at
+// once, ahead of the first barrier; a row's w, v and next-column entry stay in
+// shared memory between the phases (rows past CT_CAP of a CTA: in global
+// memory).  Eight threads share a row, each summing every eighth partial slot
+// and panel column.  Measured, one matrix, 16 panel columns, a column's launches
+// besides the mat-vec: four before (column update, reflector, panel products,
+// corrections; 7-12 us each, mostly FP64 reductions, divisions and square
+// roots), now 9.3 us at n = 84 (one launch), 11.5 us at n = 1092 and 13.3 us at
+// n = 4764 (with k_wpart).
+constexpr int CT_CLUSTER = 16;           // largest cluster (non-portable size)
+constexpr int CT_CAP = 512;              // rows of a CTA kept in shared memory
+constexpr int CT_NW = TR_NT / 32;        // warps
+__device__ __forceinline__ void cluster_arrive() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the address of a shared variable of this CTA in CTA `rank` of the cluster
+template <class T>
+__device__ __forceinline__ T *cluster_ptr(T *p, int rank) {
+  uint64_t out;
+  asm("mapa.u64 %0, %1, %2;" : "=l"(out) : "l"((uint64_t)p), "r"(rank));
+  return (T *)out;
+}
+
+template <class R>
+__global__ void __launch_bounds__(TR_NT) k_colstep(C<R> *Ab, int64_t lda, int64_t sA, C<R> *Wb, int64_t sW,
+                                                   const C<R> *Pb, int64_t sP, int64_t ldp, const int *nvec, int i,
+                                                   int k0, int jj, int do_w, int do_next, int sms, const C<R> *X,
+                                                   int ldx, const C<R> *partb, int64_t spart, C<R> *taub, double *dd,
+                                                   double *ee, z64 *tau64, int64_t sd) {
+  typedef Sum<R> S;
+  typedef typename S::T T;
+  __shared__ C<R> cw[CT_CAP], cv[CT_CAP], ca[CT_CAP];
+  __shared__ C<R> x1[32], x2[32], nv[32], nw[32];
+  // written by the warps of the whole cluster
+  __shared__ C<R> in_wv[CT_CLUSTER * CT_NW];
+  __shared__ T in_sq[CT_CLUSTER * CT_NW];
+  __shared__ int in_e[CT_CLUSTER * CT_NW];
+  __shared__ C<R> in_w, in_alpha;
+  // results of the CTA's first warp
+  __shared__ C<R> s_alpha, s_wn, s_scale;
+  __shared__ int s_skip, s_e;
+  const int rank = blockIdx.x, CS = gridDim.x;  // the cluster spans gridDim.x
+  const int b = blockIdx.y;
+  const int n = nvec[b];
+  const int col = i + 1;
+  if (col >= n) return;
+  cluster_arrive();  // distributed shared memory may be written once every CTA has started
+  bool started = false;
+  C<R> *A = Ab + b * sA;
+  C<R> *W = Wb + b * sW;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // row of local index l (groups of 4 rows dealt to the CTAs in turn)
+  auto row_of = [&](int l) { return col + ((l >> 2) * CS + rank) * 4 + (l & 3); };
+  const bool cached = do_w == 1;  // w0, v and column col are in shared memory
+  C<R> alpha = cz<R>(), wn = cz<R>();
+  // alpha from the lanes' parts of w0^H v (summed here over the first warp)
+  auto finish_alpha = [&](C<R> part, C<R> w0, C<R> tau) {
+    const T sr = S::from(part.re), si = S::from(part.im);
+    // lanes 0-15 the real parts, 16-31 the imaginary parts
+    const bool im = lane >= 16;
+    T v = S::add(im ? si : sr, S::shfl_xor(im ? sr : si, 16));
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v = S::add(v, S::shfl_xor(v, o));
+    const R mine = S::toR(v);
+    const C<R> s{shfl_real(mine, 0), shfl_real(mine, 16)};
+    const C<R> ts = cmul(tau, s);
+    const R h = RT<R>::from(-0.5);
+    const C<R> al{RT<R>::mul(h, ts.re), RT<R>::mul(h, ts.im)};
+    if (lane == 0) {
+      s_alpha = al;
+      s_wn = cadd(w0, al);  // w(i+1): v(i+1) = 1
     }
-    z64 t = scal[b * 4 + 1];
-    z64 ts = zmul(t, s);
-    s_alpha = z64{-0.5 * ts.re, -0.5 * ts.im};
+  };
+  if (do_w == 1) {
+    const PanelCol<R> pc(A, W, Pb + b * sP, lda, ldp, n, i, k0, jj, do_next, sms);
+    const int sub = lane % CT_TPR;
+    PanelRow<R> q;
+    int l = warp * 4 + lane / CT_TPR;
+    q.load(pc, row_of(l), sub);
+    const C<R> tau = taub[b];
+    panel_small(pc, X + b * ldx, x1, x2, nv, nw);
+    __syncthreads();
+    C<R> dot = cz<R>(), wfirst = cz<R>();
+    while (row_of(l & ~3) < n) {  // (uniform over the warp)
+      const int r = row_of(l);
+      C<R> y, nxt;
+      q.sums(pc, r, sub, x1, x2, nv, nw, y, nxt);
+      if (sub == 0 && r < n) {
+        const C<R> w = cmul(tau, y);
+        const C<R> a = csub(q.a, nxt);
+        if (l < CT_CAP) {
+          cw[l] = w;
+          cv[l] = q.vi;
+          ca[l] = a;
+        } else {
+          W[r + lda * jj] = w;
+          if (do_next) A[r + lda * col] = a;
+        }
+        cmacc(dot, w, q.vi);
+        dot = cfin(dot);
+        if (l == 0) wfirst = w;
+      }
+      l += 4 * CT_NW;
+      if (row_of(l & ~3) < n) q.load(pc, row_of(l), sub);
+    }
+    // w0^H v: lanes 0, 8, 16, 24 of each warp, then all warps of the cluster
+    dot = rows4_sum(dot);
+    const C<R> part{shfl_real(dot.re, 0), shfl_real(dot.im, 0)};
+    const C<R> wf{shfl_real(wfirst.re, 0), shfl_real(wfirst.im, 0)};
+    cluster_wait();
+    started = true;
+    if (lane < CS) {
+      *cluster_ptr(&in_wv[rank * CT_NW + warp], lane) = part;
+      if (rank == 0 && warp == 0) *cluster_ptr(&in_w, lane) = wf;
+    }
+    cluster_arrive();
+    cluster_wait();
+    if (warp == 0) {
+      C<R> mine = cz<R>();
+      for (int k = lane; k < CS * CT_NW; k += 32) mine = cadd(mine, in_wv[k]);
+      finish_alpha(mine, in_w, tau);
+    }
+    __syncthreads();
+  } else if (do_w == 2) {
+    if (warp == 0) {
+      const C<R> *part = partb + b * spart;
+      const C<R> tau = taub[b];
+      const int nparts = cdiv_dev(n - col, wp_threads<R> / CT_TPR);
+      C<R> mine = cz<R>();
+      for (int k = lane; k < nparts; k += 32) mine = cadd(mine, part[1 + k]);
+      finish_alpha(mine, part[0], tau);
+    }
+    __syncthreads();
+  }
+  if (do_w) {
+    alpha = s_alpha;
+    wn = cconj(s_wn);
+  }
+  // ---- one thread per row: w completed, column `col` updated
+  float big = 0.f;
+  for (int l = tid; row_of(l) < n; l += TR_NT) {
+    const int r = row_of(l);
+    const bool held = l < CT_CAP;
+    C<R> a = cz<R>();
+    if (do_next) a = held && cached ? ca[l] : A[r + lda * col];
+    if (do_w) {
+      const C<R> v = held && cached ? cv[l] : A[r + lda * i];
+      C<R> w = held && cached ? cw[l] : W[r + lda * jj];
+      cmac(w, alpha, v);
+      w = cfin(w);
+      W[r + lda * jj] = w;
+      if (do_next) {
+        C<R> acc = w;  // conj(v(i+1)) = 1
+        cmac(acc, v, wn);
+        a = csub(a, cfin(acc));
+      }
+    }
+    if (do_next) {
+      if (r == col) a.im = RT<R>::zero();
+      if (r == col + 1) s_scale = a;  // alpha of the reflector (rank 0; read below, before it is reused)
+      if (r >= col + 2) big = fmaxf(big, magnitude(a));
+      if (held)
+        ca[l] = a;
+      else
+        A[r + lda * col] = a;
+    }
+  }
+  if (!do_next || col == n - 1) {  // the panel's last column, or no reflector: the matrix ends here
+    if (do_next && rank == 0 && tid == 0) {
+      A[col + lda * col] = ca[0];
+      dd[b * sd + col] = RT<R>::to(ca[0].re);
+      tau64[b * sd + col] = z64{0.0, 0.0};
+      ee[b * sd + col] = 0.0;
+      taub[b] = cz<R>();
+    }
+    if (!started) cluster_wait();
+    return;
+  }
+  // |x|^2.  Double-float: of the values scaled by the warp's largest exponent
+  // (the float square of a small entry would underflow)
+  __syncwarp();
+  int e = 0;
+  if constexpr (!std::is_same<R, double>::value)
+    e = min(max((int)(__reduce_max_sync(0xffffffffu, __float_as_uint(big)) >> 23) - 127, -120), 120);
+  T sq = S::zero();
+  for (int l = tid; row_of(l) < n; l += TR_NT) {
+    const int r = row_of(l);
+    if (r < col + 2) continue;
+    const C<R> a = prescale(l < CT_CAP ? ca[l] : A[r + lda * col], e);
+    sq = S::add(sq, S::add(S::mul(a.re, a.re), S::mul(a.im, a.im)));
+  }
+  __syncwarp();
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sq = S::add(sq, S::shfl_xor(sq, o));
+  if (!started) cluster_wait();
+  if (lane < CS) {
+    *cluster_ptr(&in_sq[rank * CT_NW + warp], lane) = sq;
+    *cluster_ptr(&in_e[rank * CT_NW + warp], lane) = e;
+    // (row col + 1 is the second thread's of rank 0)
+    if (rank == 0 && warp == 0) *cluster_ptr(&in_alpha, lane) = s_scale;
+  }
+  cluster_arrive();
+  cluster_wait();
+  Reflector<R> f;
+  if (warp == 0) {
+    int emax = 0;
+    if constexpr (!std::is_same<R, double>::value) {
+      int el = -120;
+      for (int k = lane; k < CS * CT_NW; k += 32) el = max(el, in_e[k]);
+      emax = __reduce_max_sync(0xffffffffu, el);
+    }
+    T v = S::zero();
+    for (int k = lane; k < CS * CT_NW; k += 32) {
+      if constexpr (!std::is_same<R, double>::value) {
+        const int d2 = 2 * (in_e[k] - emax);
+        v = S::add(v, tf_scale(in_sq[k], d2 < -126 ? 0.f : pow2_clamped(d2)));
+      } else {
+        v = S::add(v, in_sq[k]);
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = S::add(v, S::shfl_xor(v, o));
+    f = reflector_scalars(v, emax, in_alpha);
+    if (lane == 0) {
+      s_scale = f.scale;
+      s_skip = f.skip;
+      s_e = f.e;
+    }
   }
   __syncthreads();
-  const int r = i + 1 + blockIdx.x * TR_NT + threadIdx.x;
-  if (r >= n) return;
-  const C<R> *A = Ab + b * sA;
-  C<R> *W = Wb + b * sW;
-  C<R> acc = W[r + lda * jj];
-  cmac(acc, cfrom64<R>(s_alpha), A[r + lda * i]);
-  W[r + lda * jj] = cfin(acc);
+  const C<R> sc = s_scale;
+  const int skip = s_skip, pe = s_e;
+  for (int l = tid; row_of(l) < n; l += TR_NT) {
+    const int r = row_of(l);
+    C<R> a = l < CT_CAP ? ca[l] : A[r + lda * col];
+    if (r == col + 1) a = C<R>{RT<R>::from(1.0), RT<R>::zero()};
+    if (r >= col + 2 && !skip) a = cmul(prescale(a, pe), sc);
+    A[r + lda * col] = a;
+  }
+  if (rank == 0 && warp == 0) {
+    // four conversions to FP64, one per lane
+    const T q = lane == 0 ? S::from(ca[0].re) : lane == 1 ? f.beta : lane == 2 ? f.t_re : f.t_im;
+    const double x = S::to(q) * __hiloint2double((1023 + (lane == 1 ? f.e : 0)) << 20, 0);
+    if (lane == 0) {
+      dd[b * sd + col] = x;
+      taub[b] = f.tau;
+    }
+    if (lane == 1) ee[b * sd + col] = x;
+    if (lane == 2) tau64[b * sd + col].re = x;
+    if (lane == 3) tau64[b * sd + col].im = x;
+  }
 }
 
 // Trailing update A(k1:n, k1:n) -= V W^H + W V^H (full square), K = jb.
@@ -558,6 +1114,63 @@ __global__ void __launch_bounds__(256) k_her2k(C<R> *Ab, int64_t lda, int64_t sA
 // the residency the kernel is compiled for).
 static int hemv_blocks(int bps) { return device_sms() * std::max(1, std::min(bps, HL_BPS)); }
 
+// Clusters of 16 CTAs are beyond the portable size, the mat-vec's tiles beyond
+// 48 KB of shared memory: opted in once per device.
+template <class R>
+static cudaError_t prepare_colstep() {
+  static std::mutex mu;
+  static bool done[PP_MAX_DEVICES] = {};
+  const int dev = device_index();
+  std::lock_guard<std::mutex> g(mu);
+  if (dev >= 0 && done[dev]) return cudaSuccess;
+  cudaError_t e = cudaFuncSetAttribute(k_colstep<R>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (std::is_same<R, df>::value && e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_hemv_df, cudaFuncAttributeMaxDynamicSharedMemorySize, HV_SMEM);
+  if (e == cudaSuccess && dev >= 0) done[dev] = true;
+  return e;
+}
+
+// One column step; the cluster has a CTA per 8 rows, at most CT_CLUSTER (a
+// function of the batch's largest order only).  Past CT_SPLIT rows the row work
+// goes to the whole chip first (k_wpart): one cluster works through CT_SPLIT
+// rows in one pass, and more passes cost more than the extra launch (both
+// launches against one: 11.5 us / 13.3 us at n = 1092, 13.2 us / 34.9 us at
+// n = 4764; FP64 form 12.4 us / 22.4 us at n = 1092).
+constexpr int CT_SPLIT = CT_CLUSTER * CT_NW * 4;
+template <class R>
+static cudaError_t launch_colstep(EigWork &w, int i, int k0, int jj, int do_w, int do_next, cudaStream_t s) {
+  const int rows = w.nmax - i - 1;
+  const int64_t sW = (int64_t)w.lda * w.nb, sP = (int64_t)w.nchunk * w.lda;
+  if (do_w && rows > CT_SPLIT) {
+    do_w = 2;
+    PP_KT(KT_COLSTEP, s, (k_wpart<R><<<dim3(cdiv(rows, wp_threads<R> / CT_TPR), w.B), wp_threads<R>, 0, s>>>(
+                             (C<R> *)w.A, w.lda, w.sA, (C<R> *)w.W, sW, (const C<R> *)w.P, sP, w.lda, w.nvec, i, k0, jj,
+                             do_next, device_sms(), (const C<R> *)w.X, 2 * w.nb, (const C<R> *)w.scal, (C<R> *)w.part,
+                             w.spart)));
+    count_launch(1);
+  }
+  int cs = 1;
+  while (cs < CT_CLUSTER && cs * 8 < rows) cs *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cs, w.B);
+  cfg.blockDim = dim3(TR_NT);
+  cfg.stream = s;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = cs;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaError_t e = cudaSuccess;
+  PP_KT(KT_COLSTEP, s, (e = cudaLaunchKernelEx(&cfg, k_colstep<R>, (C<R> *)w.A, w.lda, w.sA, (C<R> *)w.W, sW,
+                                               (const C<R> *)w.P, sP, w.lda, (const int *)w.nvec, i, k0, jj, do_w,
+                                               do_next, device_sms(), (const C<R> *)w.X, 2 * w.nb,
+                                               (const C<R> *)w.part, w.spart, (C<R> *)w.scal, w.d, w.e, w.tau,
+                                               (int64_t)w.nmax)));
+  count_launch(1);
+  return e;
+}
+
 template <class R>
 cudaError_t tridiagonalize(EigWork &w, cudaStream_t s) {
   C<R> *A = (C<R> *)w.A;
@@ -565,43 +1178,28 @@ cudaError_t tridiagonalize(EigWork &w, cudaStream_t s) {
   C<R> *P = (C<R> *)w.P;
   const int B = w.B, nmax = w.nmax, nb = w.nb;
   const int64_t lda = w.lda, sA = w.sA, sW = (int64_t)w.lda * nb, sP = (int64_t)w.nchunk * w.lda;
-  const int64_t sd = w.nmax;
+  PP_CUDA_TRY(prepare_colstep<R>());
   if (w.tcErr) PP_CUDA_TRY(cudaMemsetAsync(w.tcErr, 0, sizeof(int) * B, s));
   for (int k0 = 0; k0 < nmax; k0 += nb) {
     const int jb = min(nb, nmax - k0);
-    int nprev = 0;  // k_wcorr blocks of the previous column, when its w is still to be completed
+    PP_CUDA_TRY(launch_colstep<R>(w, k0 - 1, k0, 0, 0, 1, s));  // the panel's first column
     for (int jj = 0; jj < jb; ++jj) {
       const int i = k0 + jj;
-      const int nparts = cdiv(nmax - i, CU_ROWS);
-      const int fin = (jj > 0 && nprev > 0) ? 1 : 0;
-      PP_KT(KT_COLUPD, s, (k_colupd<R><<<dim3(nparts, B), TR_NT, 0, s>>>(A, lda, sA, W, sW, w.nvec, i, k0, jj, w.d, sd,
-                                                                         w.nrm, w.nrb, fin, nprev, w.scal,
-                                                                         (z64 *)w.wv, jj > 0 ? jj - 1 : 0)));
-      nprev = 0;
-      if (i >= nmax - 1) {
-        count_launch(1);
-        continue;
-      }
-      PP_KT(KT_REFL, s, (k_reflector<R><<<dim3(std::max(1, cdiv(nmax - i - 2, RF_ROWS)), B), TR_NT, 0, s>>>(
-                            A, lda, sA, w.nvec, i, nparts, w.nrm, w.nrb, w.e, w.tau, sd, w.scal)));
-      const int m = nmax - i - 1;
-      const int nt = cdiv(m, HL_T);
-      PP_KT(KT_HEMV, s, (k_hemv_lower<R><<<dim3(std::min(nt * (nt + 1) / 2, hemv_blocks(w.hemv_bps)), 1, B), HL_NT, 0, s>>>(
-                            A, lda, sA, w.nvec, i, P, sP, lda)));
-      if (jj > 0) PP_KT(KT_DOTS, s, (k_dots<R><<<dim3(2 * jj, B), TR_NT, 0, s>>>(A, lda, sA, W, sW, w.nvec, i, k0, jj, (z64 *)w.X, 2 * nb)));
-      const int nr = cdiv(m, TR_NT);
-      const int nrw = cdiv(m, WC_ROWS);
-      // within a panel, k_wcorr also applies columns 0 .. jj-1 to column i+1
-      PP_KT(KT_WCORR, s, (k_wcorr<R><<<dim3(nrw, B), TR_NT, 0, s>>>(A, lda, sA, W, sW, P, sP, lda, w.nvec, i, k0, jj, (z64 *)w.X, 2 * nb,
-                                               w.scal, (z64 *)w.wv, w.nrb, jj + 1 < jb ? 1 : 0)));
-      if (jj == jb - 1 || i == nmax - 2) {
-        // last column of the panel: the trailing update reads W next
-        PP_KT(KT_WFIN, s, (k_wfin<R><<<dim3(nr, B), TR_NT, 0, s>>>(A, lda, sA, W, sW, w.nvec, i, jj, nrw, w.scal, (z64 *)w.wv, w.nrb)));
-        count_launch(jj > 0 ? 7 : 6);
+      if (i >= nmax - 1) break;
+      if constexpr (std::is_same<R, df>::value) {
+        // (a smaller matrix of the batch may have more, shorter runs)
+        const int nt = cdiv(nmax - i - 1, HV_R);
+        const int gx = hv_dots(jj) + std::min(nt * (nt + 1), hv_ctas(jj, device_sms()));
+        PP_KT(KT_HEMV, s, (k_hemv_df<<<dim3(gx, B), HV_NT, HV_SMEM, s>>>(A, lda, sA, w.nvec, i, P, sP, lda, W, sW, k0,
+                                                                        jj, (C<R> *)w.X, 2 * nb, device_sms())));
       } else {
-        nprev = nrw;  // completed by the next column's k_colupd
-        count_launch(jj > 0 ? 6 : 5);
+        const int nt = cdiv(nmax - i - 1, HL_T);
+        const int gx = 2 * jj + std::min(nt * (nt + 1) / 2, hemv_blocks(w.hemv_bps));
+        PP_KT(KT_HEMV, s, (k_hemv_lower<R><<<dim3(gx, 1, B), HL_NT, 0, s>>>(A, lda, sA, w.nvec, i, P, sP, lda, W, sW, k0,
+                                                                            jj, (C<R> *)w.X, 2 * nb)));
       }
+      count_launch(1);
+      PP_CUDA_TRY(launch_colstep<R>(w, i, k0, jj, 1, jj + 1 < jb ? 1 : 0, s));
     }
     const int k1 = k0 + jb;
     if (k1 < nmax) {

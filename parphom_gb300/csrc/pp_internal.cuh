@@ -23,8 +23,7 @@ int device_sms();
 // Optional per-launch CUDA-event timing of selected kernel classes
 // (pp_ktimer_enable / pp_ktimer_report).
 enum KClass {
-  KT_ASSEMBLE = 0, KT_COLUPD, KT_REFL, KT_HEMV, KT_DOTS, KT_WCORR, KT_WFIN, KT_HER2K, KT_BISECT, KT_INVIT,
-  KT_VHX, KT_BTRED, KT_APPLYV, KT_VEL, KT_XHZ, KT_N
+  KT_ASSEMBLE = 0, KT_HEMV, KT_COLSTEP, KT_HER2K, KT_BISECT, KT_INVIT, KT_VHX, KT_BTRED, KT_APPLYV, KT_VEL, KT_XHZ, KT_N
 };
 extern unsigned kt_mask;
 void kt_begin(int k, cudaStream_t s);
@@ -58,13 +57,12 @@ struct EigWork {
   void *P = nullptr;   // [B][nchunk*nmax] hemv partial sums
   int nchunk = 0;
   void *X = nullptr;   // [B][2*nb]       V^H v and W^H v
-  double *nrm = nullptr;  // [B][nrb]     partial column norms
-  z64 *wv = nullptr;      // [B][nrb]     partial w^H v
-  int nrb = 0;            // partial-sum slots per matrix (>= row blocks of any column kernel)
+  void *part = nullptr;   // [B][spart]   partial sums of a column's row work (16-byte complex)
+  int64_t spart = 0;
   double *d = nullptr;    // [B][nmax] tridiagonal diagonal
   double *e = nullptr;    // [B][nmax] off-diagonal (real)
   z64 *tau = nullptr;     // [B][nmax] reflector scalars
-  z64 *scal = nullptr;    // [B][4]    per-column scalars (scale, tau, alpha)
+  void *scal = nullptr;   // [B]       tau of the current column (16-byte complex)
 
   // tridiagonal eigen stage
   double *w = nullptr;    // [B][nmax] eigenvalues (ascending)
@@ -125,7 +123,8 @@ cudaError_t geom_build_masks(Geometry &g, cudaStream_t s);
 cudaError_t geom_symmetrize_fc(Geometry &g, int enforce_asr, cudaStream_t s);
 cudaError_t geom_block_nonzero(const Geometry &g, uint8_t *d_flags, cudaStream_t s);
 
-// D(q) for B q-points into 16-byte complex storage (z64 if dfmt==0, zdf if 1).
+// D(q) for B q-points into 16-byte complex storage (z64 if dfmt==0, double-float
+// in the trailing matrix's order zpk if 1).
 cudaError_t assemble_batch(const Geometry &g, const double *d_q, int B, void *A, int64_t lda, int64_t sA,
                            int dfmt, cudaStream_t s);
 // dD/dq_k (derivative 1..3, method 'A' or 'C') or D (derivative 0), FP64.

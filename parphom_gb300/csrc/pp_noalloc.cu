@@ -23,7 +23,6 @@ constexpr int64_t NOALLOC_MAX_N = PP_NOALLOC_MAX_N;
 constexpr int64_t NB = 32;
 constexpr int64_t LDA_MAX = (NOALLOC_MAX_N + 7) / 8 * 8;
 constexpr int64_t NCHUNK_MAX = (NOALLOC_MAX_N + 31) / 32;
-constexpr int64_t NRB_MAX = (NOALLOC_MAX_N + 31) / 32 + 1;
 
 constexpr size_t al(size_t x) { return (x + 255) & ~(size_t)255; }
 // byte offsets of the scratch buffers inside the array
@@ -31,13 +30,13 @@ constexpr size_t OFF_NVEC = 0;
 constexpr size_t OFF_W = al(OFF_NVEC + sizeof(int));
 constexpr size_t OFF_P = al(OFF_W + 16 * (size_t)LDA_MAX * NB);
 constexpr size_t OFF_X = al(OFF_P + 16 * (size_t)NCHUNK_MAX * LDA_MAX);
-constexpr size_t OFF_NRM = al(OFF_X + 16 * 2 * NB);
-constexpr size_t OFF_WV = al(OFF_NRM + 8 * (size_t)NRB_MAX);
-constexpr size_t OFF_D = al(OFF_WV + 16 * (size_t)NRB_MAX);
+constexpr int64_t PART_MAX = (NOALLOC_MAX_N + 15) / 16 + 1;
+constexpr size_t OFF_PART = al(OFF_X + 16 * 2 * NB);
+constexpr size_t OFF_D = al(OFF_PART + 16 * (size_t)PART_MAX);
 constexpr size_t OFF_E = al(OFF_D + 8 * (size_t)NOALLOC_MAX_N);
 constexpr size_t OFF_TAU = al(OFF_E + 8 * (size_t)NOALLOC_MAX_N);
 constexpr size_t OFF_SCAL = al(OFF_TAU + 16 * (size_t)NOALLOC_MAX_N);
-constexpr size_t OFF_WW = al(OFF_SCAL + 16 * 4);
+constexpr size_t OFF_WW = al(OFF_SCAL + 16);
 constexpr size_t OFF_RNG = al(OFF_WW + 8 * (size_t)NOALLOC_MAX_N);
 constexpr size_t OFF_TINFO = al(OFF_RNG + 8 * 8);
 constexpr size_t OFF_INFO = al(OFF_TINFO + 8 * 8);
@@ -152,13 +151,12 @@ extern "C" PP_API int pp_heevx_values_noalloc(double *a_dev, int64_t lda, int64_
   w.P = base + OFF_P;
   w.nchunk = (int)((n + 31) / 32);
   w.X = base + OFF_X;
-  w.nrm = (double *)(base + OFF_NRM);
-  w.wv = (z64 *)(base + OFF_WV);
-  w.nrb = (int)NRB_MAX;
+  w.part = base + OFF_PART;
+  w.spart = PART_MAX;
   w.d = (double *)(base + OFF_D);
   w.e = (double *)(base + OFF_E);
   w.tau = (z64 *)(base + OFF_TAU);
-  w.scal = (z64 *)(base + OFF_SCAL);
+  w.scal = base + OFF_SCAL;
   w.w = (double *)(base + OFF_WW);
   w.rng = (int64_t *)(base + OFF_RNG);
   w.tinfo = (double *)(base + OFF_TINFO);
