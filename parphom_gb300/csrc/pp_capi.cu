@@ -255,7 +255,7 @@ int ensure_ws_sized(pp_ctx *c, int B, int mcap, int64_t n, int64_t nbnd_max, int
   add(&w.P, 16 * (size_t)B * nchunk * lda);
   add(&w.X, 16 * (size_t)B * 2 * nb);
   w.spart = (n + 15) / 16 + 1;
-  add(&w.part, 16 * (size_t)B * w.spart);
+  add(&w.part, 32 * (size_t)B * w.spart);
   add((void **)&w.d, 8 * (size_t)B * n);
   add((void **)&w.e, 8 * (size_t)B * n);
   add((void **)&w.tau, 16 * (size_t)B * n);
@@ -355,7 +355,7 @@ EigWork view_of(const EigWork &w, int off, int cnt) {
   v.W = sh(w.W, 16 * (size_t)w.lda * w.nb);
   v.P = sh(w.P, 16 * (size_t)w.nchunk * w.lda);
   v.X = sh(w.X, 16 * 2 * (size_t)w.nb);
-  v.part = sh(w.part, 16 * (size_t)w.spart);
+  v.part = sh(w.part, 32 * (size_t)w.spart);
   v.d = (double *)sh(w.d, 8 * nmax);
   v.e = (double *)sh(w.e, 8 * nmax);
   v.tau = (z64 *)sh(w.tau, 16 * nmax);

@@ -716,13 +716,37 @@ __device__ __forceinline__ void panel_small(const PanelCol<R> &c, const C<R> *X,
     }
   }
 }
-// sum over lanes 0, 8, 16, 24 (the rows of a warp), in every one of them
+// A complex sum over rows of products rounded to R row by row: the three-float
+// sums of the double-float form do not depend on how the rows are dealt to
+// lanes and CTAs (beyond ~2^-70), so a matrix gives the same result in a batch
+// of any largest order.
 template <class R>
-__device__ __forceinline__ C<R> rows4_sum(C<R> x) {
+struct __align__(16) RowSum {
+  typename Sum<R>::T re, im;
+  __device__ __forceinline__ void zero() { re = im = Sum<R>::zero(); }
+  // += conj(w) v
+  __device__ __forceinline__ void add_product(C<R> w, C<R> v) {
+    C<R> p = cz<R>();
+    cmacc(p, w, v);
+    p = cfin(p);
+    re = Sum<R>::add(re, Sum<R>::from(p.re));
+    im = Sum<R>::add(im, Sum<R>::from(p.im));
+  }
+  __device__ __forceinline__ void add(const RowSum &o) {
+    re = Sum<R>::add(re, o.re);
+    im = Sum<R>::add(im, o.im);
+  }
+  // over lanes 0, 8, 16, 24 (the rows of a warp), in every one of them
+  __device__ __forceinline__ void rows4() {
 #pragma unroll
-  for (int o = 16; o >= 8; o >>= 1) x = cadd(x, C<R>{shfl_xor_real(x.re, o), shfl_xor_real(x.im, o)});
-  return x;
-}
+    for (int o = 16; o >= 8; o >>= 1) {
+      re = Sum<R>::add(re, Sum<R>::shfl_xor(re, o));
+      im = Sum<R>::add(im, Sum<R>::shfl_xor(im, o));
+    }
+  }
+};
+constexpr int ROWSUM_BYTES = 32;  // the larger of the two forms
+static_assert(sizeof(RowSum<df>) == ROWSUM_BYTES && sizeof(RowSum<double>) <= ROWSUM_BYTES, "partial-sum slots");
 
 // Large trailing blocks: the row work of column i on the whole chip.
 //   w0 = tau (y - W x1 - V x2) into column jj of W, column i + 1 less the panel
@@ -734,9 +758,10 @@ template <class R>
 __global__ void __launch_bounds__(wp_threads<R>) k_wpart(C<R> *Ab, int64_t lda, int64_t sA, C<R> *Wb, int64_t sW,
                                                          const C<R> *Pb, int64_t sP, int64_t ldp, const int *nvec, int i,
                                                          int k0, int jj, int next, int sms, const C<R> *X, int ldx,
-                                                         const C<R> *taub, C<R> *partb, int64_t spart) {
+                                                         const C<R> *taub, RowSum<R> *partb, int64_t spart) {
   constexpr int NW = wp_threads<R> / 32;
-  __shared__ C<R> x1[32], x2[32], nv[32], nw[32], red[NW];
+  __shared__ C<R> x1[32], x2[32], nv[32], nw[32];
+  __shared__ RowSum<R> red[NW];
   const int b = blockIdx.y;
   const int n = nvec[b];
   const int col = i + 1;
@@ -752,22 +777,24 @@ __global__ void __launch_bounds__(wp_threads<R>) k_wpart(C<R> *Ab, int64_t lda, 
   const C<R> tau = taub[b];
   panel_small(pc, X + b * ldx, x1, x2, nv, nw);
   __syncthreads();
-  C<R> y, nxt, dot = cz<R>();
+  C<R> y, nxt;
+  RowSum<R> dot;
+  dot.zero();
   q.sums(pc, r, sub, x1, x2, nv, nw, y, nxt);
-  C<R> *part = partb + b * spart;
+  RowSum<R> *part = partb + b * spart;
   if (sub == 0 && r < n) {
     const C<R> w = cmul(tau, y);
     W[r + lda * jj] = w;
     if (next) A[r + lda * col] = csub(q.a, nxt);
-    cmacc(dot, w, q.vi);
-    if (r == col) part[0] = w;  // w0(i+1)
+    dot.add_product(w, q.vi);
+    if (r == col) *(C<R> *)&part[0] = w;  // w0(i+1)
   }
-  dot = rows4_sum(cfin(dot));
+  dot.rows4();
   if (lane == 0) red[warp] = dot;
   __syncthreads();
   if (tid == 0) {
 #pragma unroll
-    for (int k = 1; k < NW; ++k) dot = cadd(dot, red[k]);
+    for (int k = 1; k < NW; ++k) dot.add(red[k]);
     part[1 + blockIdx.x] = dot;
   }
 }
@@ -818,14 +845,14 @@ template <class R>
 __global__ void __launch_bounds__(TR_NT) k_colstep(C<R> *Ab, int64_t lda, int64_t sA, C<R> *Wb, int64_t sW,
                                                    const C<R> *Pb, int64_t sP, int64_t ldp, const int *nvec, int i,
                                                    int k0, int jj, int do_w, int do_next, int sms, const C<R> *X,
-                                                   int ldx, const C<R> *partb, int64_t spart, C<R> *taub, double *dd,
+                                                   int ldx, const RowSum<R> *partb, int64_t spart, C<R> *taub, double *dd,
                                                    double *ee, z64 *tau64, int64_t sd) {
   typedef Sum<R> S;
   typedef typename S::T T;
   __shared__ C<R> cw[CT_CAP], cv[CT_CAP], ca[CT_CAP];
   __shared__ C<R> x1[32], x2[32], nv[32], nw[32];
   // written by the warps of the whole cluster
-  __shared__ C<R> in_wv[CT_CLUSTER * CT_NW];
+  __shared__ RowSum<R> in_wv[CT_CLUSTER * CT_NW];
   __shared__ T in_sq[CT_CLUSTER * CT_NW];
   __shared__ int in_e[CT_CLUSTER * CT_NW];
   __shared__ C<R> in_w, in_alpha;
@@ -847,8 +874,8 @@ __global__ void __launch_bounds__(TR_NT) k_colstep(C<R> *Ab, int64_t lda, int64_
   const bool cached = do_w == 1;  // w0, v and column col are in shared memory
   C<R> alpha = cz<R>(), wn = cz<R>();
   // alpha from the lanes' parts of w0^H v (summed here over the first warp)
-  auto finish_alpha = [&](C<R> part, C<R> w0, C<R> tau) {
-    const T sr = S::from(part.re), si = S::from(part.im);
+  auto finish_alpha = [&](const RowSum<R> &part, C<R> w0, C<R> tau) {
+    const T sr = part.re, si = part.im;
     // lanes 0-15 the real parts, 16-31 the imaginary parts
     const bool im = lane >= 16;
     T v = S::add(im ? si : sr, S::shfl_xor(im ? sr : si, 16));
@@ -873,7 +900,9 @@ __global__ void __launch_bounds__(TR_NT) k_colstep(C<R> *Ab, int64_t lda, int64_
     const C<R> tau = taub[b];
     panel_small(pc, X + b * ldx, x1, x2, nv, nw);
     __syncthreads();
-    C<R> dot = cz<R>(), wfirst = cz<R>();
+    RowSum<R> dot;
+    dot.zero();
+    C<R> wfirst = cz<R>();
     while (row_of(l & ~3) < n) {  // (uniform over the warp)
       const int r = row_of(l);
       C<R> y, nxt;
@@ -889,16 +918,17 @@ __global__ void __launch_bounds__(TR_NT) k_colstep(C<R> *Ab, int64_t lda, int64_
           W[r + lda * jj] = w;
           if (do_next) A[r + lda * col] = a;
         }
-        cmacc(dot, w, q.vi);
-        dot = cfin(dot);
+        dot.add_product(w, q.vi);
         if (l == 0) wfirst = w;
       }
       l += 4 * CT_NW;
       if (row_of(l & ~3) < n) q.load(pc, row_of(l), sub);
     }
     // w0^H v: lanes 0, 8, 16, 24 of each warp, then all warps of the cluster
-    dot = rows4_sum(dot);
-    const C<R> part{shfl_real(dot.re, 0), shfl_real(dot.im, 0)};
+    dot.rows4();
+    RowSum<R> part;
+    part.re = shfl_real(dot.re, 0);
+    part.im = shfl_real(dot.im, 0);
     const C<R> wf{shfl_real(wfirst.re, 0), shfl_real(wfirst.im, 0)};
     cluster_wait();
     started = true;
@@ -909,19 +939,21 @@ __global__ void __launch_bounds__(TR_NT) k_colstep(C<R> *Ab, int64_t lda, int64_
     cluster_arrive();
     cluster_wait();
     if (warp == 0) {
-      C<R> mine = cz<R>();
-      for (int k = lane; k < CS * CT_NW; k += 32) mine = cadd(mine, in_wv[k]);
+      RowSum<R> mine;
+      mine.zero();
+      for (int k = lane; k < CS * CT_NW; k += 32) mine.add(in_wv[k]);
       finish_alpha(mine, in_w, tau);
     }
     __syncthreads();
   } else if (do_w == 2) {
     if (warp == 0) {
-      const C<R> *part = partb + b * spart;
+      const RowSum<R> *part = partb + b * spart;
       const C<R> tau = taub[b];
       const int nparts = cdiv_dev(n - col, wp_threads<R> / CT_TPR);
-      C<R> mine = cz<R>();
-      for (int k = lane; k < nparts; k += 32) mine = cadd(mine, part[1 + k]);
-      finish_alpha(mine, part[0], tau);
+      RowSum<R> mine;
+      mine.zero();
+      for (int k = lane; k < nparts; k += 32) mine.add(part[1 + k]);
+      finish_alpha(mine, *(const C<R> *)&part[0], tau);
     }
     __syncthreads();
   }
@@ -1145,8 +1177,8 @@ static cudaError_t launch_colstep(EigWork &w, int i, int k0, int jj, int do_w, i
     do_w = 2;
     PP_KT(KT_COLSTEP, s, (k_wpart<R><<<dim3(cdiv(rows, wp_threads<R> / CT_TPR), w.B), wp_threads<R>, 0, s>>>(
                              (C<R> *)w.A, w.lda, w.sA, (C<R> *)w.W, sW, (const C<R> *)w.P, sP, w.lda, w.nvec, i, k0, jj,
-                             do_next, device_sms(), (const C<R> *)w.X, 2 * w.nb, (const C<R> *)w.scal, (C<R> *)w.part,
-                             w.spart)));
+                             do_next, device_sms(), (const C<R> *)w.X, 2 * w.nb, (const C<R> *)w.scal,
+                             (RowSum<R> *)w.part, w.spart * ROWSUM_BYTES / (int)sizeof(RowSum<R>))));
     count_launch(1);
   }
   int cs = 1;
@@ -1165,7 +1197,8 @@ static cudaError_t launch_colstep(EigWork &w, int i, int k0, int jj, int do_w, i
   PP_KT(KT_COLSTEP, s, (e = cudaLaunchKernelEx(&cfg, k_colstep<R>, (C<R> *)w.A, w.lda, w.sA, (C<R> *)w.W, sW,
                                                (const C<R> *)w.P, sP, w.lda, (const int *)w.nvec, i, k0, jj, do_w,
                                                do_next, device_sms(), (const C<R> *)w.X, 2 * w.nb,
-                                               (const C<R> *)w.part, w.spart, (C<R> *)w.scal, w.d, w.e, w.tau,
+                                               (const RowSum<R> *)w.part,
+                                               w.spart * ROWSUM_BYTES / (int)sizeof(RowSum<R>), (C<R> *)w.scal, w.d, w.e, w.tau,
                                                (int64_t)w.nmax)));
   count_launch(1);
   return e;
@@ -1219,18 +1252,6 @@ cudaError_t tridiagonalize(EigWork &w, cudaStream_t s) {
 // ===========================================================================
 // Stage 2: eigenvalues of the tridiagonal matrix (FP64 bisection)
 // ===========================================================================
-__device__ __forceinline__ int sturm_count(const double *d, const double *e2, int n, double x, double pivmin) {
-  double q = d[0] - x;
-  if (fabs(q) <= pivmin) q = -pivmin;
-  int c = q < 0.0;
-  for (int k = 1; k < n; ++k) {
-    q = d[k] - e2[k - 1] / q - x;
-    if (fabs(q) <= pivmin) q = -pivmin;
-    c += q < 0.0;
-  }
-  return c;
-}
-
 // Gerschgorin interval, pivmin and the index range of the wanted eigenvalues.
 __global__ void k_tdprep(const double *dd, const double *ee, int64_t sd, const int *nvec, char range, double vl,
                          double vu, int64_t il, int64_t iu, int64_t *rng, double *tinfo, int64_t *info,
@@ -1293,6 +1314,91 @@ __global__ void k_tdprep(const double *dd, const double *ee, int64_t sd, const i
   info[b] = (tcerr && tcerr[b]) ? PP_INFO_TIMEOUT : 0;
 }
 
+// FP64 Sturm count (the number of eigenvalues below x) of the tridiagonal
+// scaled by a power of two to norm 1/2 .. 1, by the recurrence of the leading
+// principal minors
+//   p_{k+1} = (d_k - x) p_k - e_{k-1}^2 p_{k-1},
+// a sign change per eigenvalue below x.  Like the quotient form q = p_{k+1} /
+// p_k it is exact for entries perturbed by a few units in the last place, but
+// a row costs one dependent multiply-add instead of a division (85 instead of
+// 600 cycles of latency, 3 instead of ~20 operations on a pipe that takes 16
+// cycles per warp operation).  Rows are taken MC_NB at a time, the pair (p_k,
+// p_{k+1}) rescaled by a power of two after each block.  If a minor of the
+// block falls below 2^-MC_LIM, the block is repeated row by row with a
+// rescaling after each, and a vanishing minor replaced by -2^-MC_PIV p_k (a
+// quotient of -2^-MC_PIV, as the quotient form does).  (The float and
+// double-float counts keep the quotient form: their reciprocals take 40
+// cycles, and the minors' checks cost more than that saves.)
+constexpr int MC_NB = 8, MC_LIM = 700, MC_PIV = 400;
+struct MinorCount {
+  const double2 *t;     // d, e^2 in shared memory, or null:
+  const double *d, *e;  // from global memory, to be scaled by sc
+  double sc;
+  __device__ __forceinline__ double step(int k, double x, double p0, double p1) const {
+    double dk, e2;
+    if (t) {
+      dk = t[k].x;
+      e2 = t[k - 1].y;
+    } else {
+      const double ek = e[k - 1] * sc;
+      dk = d[k] * sc;
+      e2 = ek * ek;
+    }
+    return fma(dk - x, p1, -(e2 * p0));
+  }
+  __device__ static __forceinline__ int expo(double p) { return ((__double2hiint(p) >> 20) & 2047) - 1023; }
+  __device__ static __forceinline__ double scale(double p, int e) { return p * __hiloint2double((1023 + e) << 20, 0); }
+  // the larger of the pair brought to exponent 0
+  __device__ static __forceinline__ void rescale(double &p0, double &p1) {
+    const int e = max(expo(p0), expo(p1));
+    p0 = scale(p0, -e);
+    p1 = scale(p1, -e);
+  }
+  __device__ static __forceinline__ void guard(double &p0, double &p1) {
+    if (expo(p1) < expo(p0) - MC_PIV) p1 = -scale(p0, -MC_PIV);  // (zero: exponent -1023)
+    rescale(p0, p1);
+  }
+  __device__ __forceinline__ int operator()(int n, double x) const {
+    double p0 = 1.0, p1 = (t ? t[0].x : d[0] * sc) - x;
+    guard(p0, p1);
+    unsigned cnt = (unsigned)__double2hiint(p1) >> 31;
+    auto rows = [&](int k, int k1) {
+      for (; k < k1; ++k) {
+        const double q = step(k, x, p0, p1);
+        p0 = p1;
+        p1 = q;
+        guard(p0, p1);
+        cnt += (unsigned)(__double2hiint(p0) ^ __double2hiint(p1)) >> 31;
+      }
+    };
+    int k = 1;
+    for (; k + MC_NB <= n; k += MC_NB) {
+      double q[MC_NB];
+      int least = 0x7ff00000;
+      unsigned c = 0;
+      int s = __double2hiint(p1);
+#pragma unroll
+      for (int u = 0; u < MC_NB; ++u) {
+        q[u] = step(k + u, x, u < 2 ? (u == 0 ? p0 : p1) : q[u - 2], u == 0 ? p1 : q[u - 1]);
+        const int h = __double2hiint(q[u]);
+        least = min(least, h & 0x7fffffff);
+        c += (unsigned)(s ^ h) >> 31;
+        s = h;
+      }
+      if (least >= (1023 - MC_LIM) << 20) {
+        cnt += c;
+        p0 = q[MC_NB - 2];
+        p1 = q[MC_NB - 1];
+        rescale(p0, p1);
+      } else {
+        rows(k, k + MC_NB);
+      }
+    }
+    rows(k, n);
+    return (int)cnt;
+  }
+};
+
 __device__ __forceinline__ int sturm_count32(const float *d, const float *e2, int n, float x, float pivmin) {
   float q = d[0] - x;
   if (fabsf(q) <= pivmin) q = -pivmin;
@@ -1350,85 +1456,80 @@ __device__ __forceinline__ int sturm_count_df(const float *dh, const float *dl, 
   return c;
 }
 
-// One thread per wanted eigenvalue.  mode 0: FP64 counts from global memory;
-// mode 1: the tridiagonal in shared memory, the interval first narrowed with
-// FP32 Sturm counts (cheap on the FP32 pipes), then widened by a margin far
-// above the FP32 backward error of the count (64 eps32 (||T|| + |x|)),
-// checked with two counts (falling back to the Gerschgorin interval if the
-// check fails) and finished in FP64; mode 2 (mixed form): as mode 1 but
-// checked and finished with double-float counts, whose accuracy floor
-// (a few 2^-44 ||T||) ends the bisection.
+// One thread per wanted eigenvalue: bisection on Sturm counts of the
+// tridiagonal scaled by a power of two to norm 1/2 .. 1.  mode 0: FP64 counts
+// from global memory; mode 1 (FP64 form): the tridiagonal in shared memory, the
+// interval first narrowed with FP32 Sturm counts, then widened by a margin far
+// above the FP32 backward error of the count (64 eps32 (||T|| + |x|)), checked
+// with two counts (falling back to the Gerschgorin interval if the check
+// fails) and finished in FP64; mode 2 (mixed form): as mode 1 but checked and
+// finished with double-float counts, whose accuracy floor (a few 2^-44 ||T||)
+// ends the bisection.
 __global__ void __launch_bounds__(128) k_bisect(const double *dd, const double *ee, int64_t sd, const int *nvec,
                                                 const int64_t *rng, const double *tinfo, double abstol, double *wout,
                                                 int64_t *info, int mode) {
-  extern __shared__ double sm[];
+  extern __shared__ __align__(16) unsigned char bs_smem[];
   const int b = blockIdx.y;
   const int n = nvec[b];
   const double *d = dd + b * sd;
   const double *e = ee + b * sd;
-  double *sd_ = sm;
-  double *se2 = sm + n;
-  float *fd = (float *)(sm + 2 * n);
-  float *fe2 = fd + n;
-  // mode 2 layout: d.hi, d.lo, e2.hi, e2.lo
-  float *gdh = (float *)sm, *gdl = gdh + n, *ge2h = gdl + n, *ge2l = ge2h + n;
-  if (mode == 1) {
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-      const double e2 = (k < n - 1) ? e[k] * e[k] : 0.0;
-      sd_[k] = d[k];
-      se2[k] = e2;
-      fd[k] = (float)d[k];
-      fe2[k] = (float)e2;
-    }
-    __syncthreads();
-  } else if (mode == 2) {
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-      const double e2 = (k < n - 1) ? e[k] * e[k] : 0.0;
-      const df dk = df_from(d[k]), ek = df_from(e2);
-      gdh[k] = dk.hi;
-      gdl[k] = dk.lo;
-      ge2h[k] = ek.hi;
-      ge2l[k] = ek.lo;
-    }
-    __syncthreads();
-    fd = gdh;
-    fe2 = ge2h;
-  }
+  const double tnorm = tinfo[b * 8 + 2];
   const int64_t lo_idx = rng[b * 8 + 0];
   const int64_t m = rng[b * 8 + 2];
+  if ((int64_t)blockIdx.x * blockDim.x >= m) return;
+  // shared memory: (d, e^2) in FP64 (mode 1); then d.hi, e^2.hi (modes 1, 2), d.lo, e^2.lo (mode 2) in float
+  double2 *td = (double2 *)bs_smem;
+  float *gdh = (float *)(mode == 1 ? (void *)(td + n) : (void *)bs_smem), *ge2h = gdh + n, *gdl = ge2h + n, *ge2l = gdl + n;
+  // power of two with sc ||T|| in [1/2, 1); mode 2 keeps the caller's units
+  int te = 0;
+  if (mode != 2) frexp(tnorm, &te);
+  te = max(min(te, 1000), -1000);
+  const double sc = ldexp(1.0, -te), isc = ldexp(1.0, te);
+  if (mode != 0) {
+    for (int k = threadIdx.x; k < n; k += blockDim.x) {
+      const double es = (k < n - 1) ? e[k] * sc : 0.0, ds = d[k] * sc, e2 = es * es;
+      if (mode == 1) {
+        td[k] = make_double2(ds, e2);
+        gdh[k] = (float)ds;
+        ge2h[k] = (float)e2;
+      } else {
+        const df dk = df_from(ds), ek = df_from(e2);
+        gdh[k] = dk.hi;
+        gdl[k] = dk.lo;
+        ge2h[k] = ek.hi;
+        ge2l[k] = ek.lo;
+      }
+    }
+    __syncthreads();
+  }
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= m) return;
+  if (tnorm == 0.0) {  // the zero matrix
+    wout[b * sd + j] = 0.0;
+    return;
+  }
   const int64_t idx = lo_idx + j;
-  const double gl = tinfo[b * 8 + 0], gu = tinfo[b * 8 + 1], tnorm = tinfo[b * 8 + 2];
-  const double pivmin = tinfo[b * 8 + 3];
+  // everything below in units of 1 / sc
+  const double gl = tinfo[b * 8 + 0] * sc, gu = tinfo[b * 8 + 1] * sc, tn = tnorm * sc;
+  const double pivmin = tinfo[b * 8 + 3] * sc, atol = abstol * sc;
   double lo = gl, hi = gu;
   const double ulp = DBL_EPSILON;
-  const float pivdf = fmaxf(1e-30f, (float)pivmin);
+  const float piv32 = fmaxf(1e-30f, (float)pivmin);
+  const MinorCount minors{mode == 1 ? td : nullptr, d, e, sc};
   auto count64 = [&](double x) -> int {
-    if (mode == 2) return sturm_count_df(gdh, gdl, ge2h, ge2l, n, df_from(x), pivdf);
-    if (mode == 1) return sturm_count(sd_, se2, n, x, pivmin);
-    double q = d[0] - x;
-    if (fabs(q) <= pivmin) q = -pivmin;
-    int c = q < 0.0;
-    for (int k = 1; k < n; ++k) {
-      q = d[k] - (e[k - 1] * e[k - 1]) / q - x;
-      if (fabs(q) <= pivmin) q = -pivmin;
-      c += q < 0.0;
-    }
-    return c;
+    return mode == 2 ? sturm_count_df(gdh, gdl, ge2h, ge2l, n, df_from(x), piv32) : minors(n, x);
   };
-  if (mode != 0 && tnorm > 0.0 && tnorm < 1e30) {
+  if (mode != 0 && tnorm < 1e30) {
     float lo32 = (float)lo, hi32 = (float)hi;
-    const float piv32 = fmaxf(1e-30f, (float)pivmin);
-    const float stop = 16.0f * FLT_EPSILON * (float)tnorm;
+    const float stop = 16.0f * FLT_EPSILON * (float)tn;
     for (int it = 0; it < 48 && hi32 - lo32 > stop; ++it) {
       const float mid = 0.5f * (lo32 + hi32);
-      if (sturm_count32(fd, fe2, n, mid, piv32) >= idx)
+      if (sturm_count32(gdh, ge2h, n, mid, piv32) >= idx)
         hi32 = mid;
       else
         lo32 = mid;
     }
-    const double marg = 64.0 * FLT_EPSILON * (tnorm + fmax(fabs((double)lo32), fabs((double)hi32)));
+    const double marg = 64.0 * FLT_EPSILON * (tn + fmax(fabs((double)lo32), fabs((double)hi32)));
     const double l2 = fmax(gl, (double)lo32 - marg), h2 = fmin(gu, (double)hi32 + marg);
     if (count64(l2) < idx && count64(h2) >= idx) {
       lo = l2;
@@ -1436,10 +1537,10 @@ __global__ void __launch_bounds__(128) k_bisect(const double *dd, const double *
     }
   }
   // accuracy floor of the double-float count (mode 2)
-  const double floor_df = (mode == 2) ? 4.0 * 0x1p-44 * tnorm : 0.0;
+  const double floor_df = (mode == 2) ? 4.0 * 0x1p-44 * tn : 0.0;
   bool conv = false;
   for (int it = 0; it < 256; ++it) {
-    double tol = fmax(fmax(fmax(abstol, pivmin), 2.0 * ulp * fmax(fabs(lo), fabs(hi))), floor_df);
+    double tol = fmax(fmax(fmax(atol, pivmin), 2.0 * ulp * fmax(fabs(lo), fabs(hi))), floor_df);
     if (hi - lo <= tol) {
       conv = true;
       break;
@@ -1451,13 +1552,13 @@ __global__ void __launch_bounds__(128) k_bisect(const double *dd, const double *
       lo = mid;
   }
   if (!conv) atomicOr((unsigned long long *)&info[b], (unsigned long long)PP_INFO_NOCONV);
-  wout[b * sd + j] = 0.5 * (lo + hi);
+  wout[b * sd + j] = 0.5 * (lo + hi) * isc;
 }
 
 // Opt the bisection kernel into the dynamic shared memory it needs for order
 // n (done once per size outside any stream capture).
 size_t bisect_smem(int64_t n, int mixed) {
-  const size_t b = mixed ? 4 * (size_t)n * sizeof(float) : 2 * (size_t)n * (sizeof(double) + sizeof(float));
+  const size_t b = (size_t)n * (mixed ? 4 * sizeof(float) : sizeof(double2) + 2 * sizeof(float));
   return b <= 200 * 1024 ? b : 0;
 }
 
@@ -1486,8 +1587,13 @@ cudaError_t tridiag_eigenvalues(EigWork &w, char range, double vl, double vu, in
     mode = mixed ? 2 : 1;
     PP_CUDA_TRY(prepare_bisect(smem));
   }
-  dim3 g(cdiv(w.nmax, 128), w.B);
-  PP_KT(KT_BISECT, s, (k_bisect<<<g, 128, smem, s>>>(w.d, w.e, sd, w.nvec, w.rng, w.tinfo, abstol, w.w, w.info, mode)));
+  // 128 threads a block, or fewer while that leaves SMs idle (a thread's
+  // bisection is one dependent chain, so few eigenvalues want many SMs)
+  const int mmax = range == 'I' ? (int)(iu - il + 1) : w.nmax;
+  int nt = 128;
+  while (nt > 32 && cdiv(mmax, nt) * (int64_t)w.B < device_sms()) nt /= 2;
+  dim3 g(cdiv(mmax, nt), w.B);
+  PP_KT(KT_BISECT, s, (k_bisect<<<g, nt, smem, s>>>(w.d, w.e, sd, w.nvec, w.rng, w.tinfo, abstol, w.w, w.info, mode)));
   count_launch(2);
   return cudaGetLastError();
 }

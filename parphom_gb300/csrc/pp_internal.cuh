@@ -57,7 +57,7 @@ struct EigWork {
   void *P = nullptr;   // [B][nchunk*nmax] hemv partial sums
   int nchunk = 0;
   void *X = nullptr;   // [B][2*nb]       V^H v and W^H v
-  void *part = nullptr;   // [B][spart]   partial sums of a column's row work (16-byte complex)
+  void *part = nullptr;   // [B][spart]   partial sums of a column's row work (32 bytes)
   int64_t spart = 0;
   double *d = nullptr;    // [B][nmax] tridiagonal diagonal
   double *e = nullptr;    // [B][nmax] off-diagonal (real)

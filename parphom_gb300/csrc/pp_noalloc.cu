@@ -32,7 +32,7 @@ constexpr size_t OFF_P = al(OFF_W + 16 * (size_t)LDA_MAX * NB);
 constexpr size_t OFF_X = al(OFF_P + 16 * (size_t)NCHUNK_MAX * LDA_MAX);
 constexpr int64_t PART_MAX = (NOALLOC_MAX_N + 15) / 16 + 1;
 constexpr size_t OFF_PART = al(OFF_X + 16 * 2 * NB);
-constexpr size_t OFF_D = al(OFF_PART + 16 * (size_t)PART_MAX);
+constexpr size_t OFF_D = al(OFF_PART + 32 * (size_t)PART_MAX);
 constexpr size_t OFF_E = al(OFF_D + 8 * (size_t)NOALLOC_MAX_N);
 constexpr size_t OFF_TAU = al(OFF_E + 8 * (size_t)NOALLOC_MAX_N);
 constexpr size_t OFF_SCAL = al(OFF_TAU + 16 * (size_t)NOALLOC_MAX_N);
