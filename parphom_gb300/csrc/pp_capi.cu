@@ -219,20 +219,19 @@ int ensure_ws_sized(pp_ctx *c, int B, int mcap, int64_t n, int64_t nbnd_max, int
   free_ws(c);
   const int nb = 32;
   const int64_t lda = (n + 7) / 8 * 8;
-  // mat-vec partial slots: n/32 (FP64 form), 3 ceil(n/64) (double-float form)
-  const int nchunk = (int)(3 * ((n + 63) / 64));
+  // mat-vec partial slots: n/32, n/16 up to 128 rows (FP64 form), 3 ceil(n/64) (double-float form)
+  const int nchunk = (int)std::max<int64_t>(3 * ((n + 63) / 64), 8);
   const int64_t T = std::min<int64_t>(((int64_t)mcap + 63) / 64 * 64, 2048);
   const int nbr = (int)nbr_max;
   const int ldwp = std::max(std::max(mcap, nbr), 64);
-  // split-K partials: ceil(n/512) chunks of 32 x ldwp, or the Gram product's
-  // ceil(n/64) chunks of 32 x 32, whichever is larger
-  const int ksplit = (int)std::max<int64_t>((n + 511) / 512, ((n + 63) / 64 * 32 + ldwp - 1) / ldwp);
+  // split-K partials: 8 chunks of 32 x ldwp, or one per 256 rows
+  const int ksplit = (int)std::max<int64_t>((n + 255) / 256, 8);
   const int64_t nbnd = nbnd_max;
   std::vector<std::pair<void **, size_t>> parts;
   EigWork &w = c->w;
   w = EigWork();
   w.B = B;
-  w.nmax = (int)n;
+  w.nmax = w.nmin = (int)n;
   w.mcap = mcap;
   w.nb = nb;
   w.lda = lda;
@@ -318,7 +317,8 @@ int ensure_ws(pp_ctx *c, int B, int mcap) { return ensure_ws_sized(c, B, mcap, c
 size_t ws_bytes_estimate(int64_t n, int B, int mcap, int64_t nbnd, int64_t nbr) {
   const int64_t T = std::min<int64_t>(((int64_t)mcap + 63) / 64 * 64, 2048);
   size_t per = 16 * (size_t)n * n + 16 * (size_t)n * mcap + 8 * (size_t)5 * n * T + (size_t)n * T +
-               16 * (size_t)n * 64 * 2 + 16 * (size_t)((n + 511) / 512) * 32 * std::max(mcap, 64) +
+               16 * (size_t)n * 64 * 2 + 16 * (size_t)std::max<int64_t>((n + 255) / 256, 8) * 32 * std::max(mcap, 64) +
+               16 * (size_t)n * std::max<int64_t>(3 * ((n + 63) / 64), 8) +  // mat-vec partials
                16 * (size_t)((n + 63) / 64) * 32 * 32 + her2k_tc_bytes(n) + 8 * (size_t)(n + 128) +
                8 * 8 * 3 * (size_t)mcap + 16 * 3 * (size_t)nbnd + 16 * (size_t)nbr * (n + mcap) +
                16 * 1024 * (size_t)std::max<int64_t>(1, (n + 30) / 32);  // compact-WY factors of all panels
@@ -439,7 +439,7 @@ int split_ways() {
 // stream.)
 int run_batch(pp_ctx *c, int B, const pp_eig_opts *o, int mcap, bool want_z) {
   EigWork &w = c->w;
-  w.B = B;
+  w.B = w.batch = B;
   cudaStream_t s = c->stream;
   const int prec = o->precision;
   TRY_CUDA(assemble_batch(c->g, c->d_q, B, w.A, w.lda, w.sA, prec == PP_PREC_MIXED ? 1 : 0, s));
@@ -1252,7 +1252,8 @@ int pp_solve_multi(pp_ctx *const *ctxs, int64_t nctx, const int64_t *cell, const
     }
     TRY_CUDA(cudaMemcpyAsync(h->d_q, qh.data(), sizeof(double) * 3 * Bb, cudaMemcpyHostToDevice, s));
     TRY_CUDA(cudaMemcpyAsync(w.nvec, nv.data(), sizeof(int) * Bb, cudaMemcpyHostToDevice, s));
-    w.B = Bb;
+    w.B = w.batch = Bb;
+    w.nmin = *std::min_element(nv.begin(), nv.begin() + Bb);
     for (auto &g : segs) {
       EigWork v = view_of(w, g.off, g.cnt);
       TRY_CUDA(assemble_batch(g.c->g, h->d_q + 3 * g.off, g.cnt, v.A, w.lda, w.sA, fmt, s));

@@ -283,11 +283,13 @@ __device__ __forceinline__ float magnitude(C<df> x) { return fmaxf(fabsf(x.re.hi
 // strided set of tile pairs with two shared-memory buffers: the next tile
 // (and its two vector pieces) is copied by cp.async while the double-float
 // arithmetic of the current one runs.
-constexpr int HL_T = 32;
-constexpr int HL_LD = HL_T + 1;  // padded column stride of the shared tile
-constexpr int HL_NT = 128;
+constexpr int HL_T = 32;         // tile of large trailing blocks
+constexpr int HL_TS = 16;        // tile of trailing blocks up to HL_SMALL rows: four times the tiles, so that
+constexpr int HL_SMALL = 128;    // more SMs' FP64 pipes take part (n = 84: 9.1 -> 7.9 us between events)
+constexpr int HL_NT = 128;       // threads for a tile of 32 (4 T)
 constexpr int HL_BPS = 6;        // resident blocks per SM
 constexpr int HL_UNROLL = 4;     // inner-loop unrolling (keeps the kernel's code small)
+__host__ __device__ __forceinline__ int hl_tile(int rows) { return rows <= HL_SMALL ? HL_TS : HL_T; }
 __device__ __forceinline__ void cp_async16(void *dst, const void *src, bool valid) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(valid ? 16 : 0) : "memory");
@@ -305,34 +307,34 @@ __device__ __forceinline__ void tile_pair(int p, int &Rt, int &Ct) {
   while (Rt * (Rt + 1) / 2 > p) --Rt;
   Ct = p - Rt * (Rt + 1) / 2;
 }
-// One of the panel products of column i, by HL_NT threads (t) of one block of
-// the mat-vec's launch: X[c] = V(:,c)^H v (c < jj), X[jj+c] = W(:,c)^H v over rows [i+1, n).
-// They need only v, so they run beside the mat-vec instead of in a launch of
+// One of the panel products of column i, by 128 threads (t) of one block of
+// the double-float mat-vec's launch: X[c] = V(:,c)^H v (c < jj), X[jj+c] =
+// W(:,c)^H v over rows [i+1, n).  They need only v, so they run beside the mat-vec instead of in a launch of
 // their own.  Each thread's sum is renormalised every 4 rows.
-template <class R>
-__device__ __forceinline__ void panel_dot(const C<R> *A, const C<R> *W, int64_t lda, int n, int i, int k0, int jj,
-                                          int c2, int t, typename Sum<R>::T (*red)[HL_NT / 32], C<R> *X) {
-  typedef Sum<R> S;
-  typedef typename S::T T;
+__device__ __forceinline__ void panel_dot(const zdf *A, const zdf *W, int64_t lda, int n, int i, int k0, int jj,
+                                          int c2, int t, Sum<df>::T (*red)[4], zdf *X) {
+  typedef Sum<df> S;
+  typedef S::T T;
+  constexpr int NT = 128;
   const bool some = c2 < 2 * jj;  // (the last block's spare groups only pass the barrier)
   const bool useW = c2 >= jj;
   const int c = useW ? c2 - jj : c2;
-  const C<R> *Xc = useW ? (W + lda * c) : (A + lda * (k0 + c));
-  const C<R> *v = A + lda * i;
-  C<R> acc = cz<R>();
+  const zdf *Xc = useW ? (W + lda * c) : (A + lda * (k0 + c));
+  const zdf *v = A + lda * i;
+  zdf acc = cz<df>();
   int r = some ? i + 1 + t : n;
-  for (; r + 3 * HL_NT < n; r += 4 * HL_NT) {
-    C<R> x[4], y[4];
+  for (; r + 3 * NT < n; r += 4 * NT) {
+    zdf x[4], y[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      x[u] = Xc[r + u * HL_NT];
-      y[u] = v[r + u * HL_NT];
+      x[u] = Xc[r + u * NT];
+      y[u] = v[r + u * NT];
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) cmacc(acc, x[u], y[u]);
     acc = cfin(acc);
   }
-  for (; r < n; r += HL_NT) cmacc(acc, Xc[r], v[r]);
+  for (; r < n; r += NT) cmacc(acc, Xc[r], v[r]);
   acc = cfin(acc);
   T sr = S::from(acc.re), si = S::from(acc.im);
 #pragma unroll
@@ -347,36 +349,67 @@ __device__ __forceinline__ void panel_dot(const C<R> *A, const C<R> *W, int64_t 
   __syncthreads();
   if (t == 0 && some) {
 #pragma unroll
-    for (int k = 1; k < HL_NT / 32; ++k) {
+    for (int k = 1; k < NT / 32; ++k) {
       sr = S::add(sr, red[0][k]);
       si = S::add(si, red[1][k]);
     }
-    X[c2] = C<R>{S::toR(sr), S::toR(si)};
+    X[c2] = zdf{S::toR(sr), S::toR(si)};
   }
 }
 
-template <class R>
-__global__ void __launch_bounds__(HL_NT, HL_BPS) k_hemv_lower(const C<R> *Ab, int64_t lda, int64_t sA,
-                                                              const int *nvec, int i, C<R> *Pb, int64_t sP,
-                                                              int64_t ldp, const C<R> *Wb, int64_t sW, int k0,
-                                                              int jj, C<R> *X, int ldx) {
-  __shared__ __align__(16) C<R> tile[2][HL_T * HL_LD];  // tile[buf][c * HL_LD + r]
-  __shared__ __align__(16) C<R> vR[2][HL_T], vC[2][HL_T];
-  __shared__ C<R> red[2][2][HL_T];
+// The same in FP64, one product per warp: a warp's sum takes 10 additions
+// across lanes, a block's 40 and a barrier, and an FP64 addition holds the pipe
+// for 16 cycles.
+__device__ __forceinline__ void panel_dot_warp(const z64 *A, const z64 *W, int64_t lda, int n, int i, int k0, int jj,
+                                               int c2, z64 *X) {
+  if (c2 >= 2 * jj) return;
+  const int lane = threadIdx.x & 31;
+  const z64 *Xc = c2 >= jj ? W + lda * (c2 - jj) : A + lda * (k0 + c2);
+  const z64 *v = A + lda * i;
+  z64 acc{0.0, 0.0};
+  int r = i + 1 + lane;
+  for (; r + 3 * 32 < n; r += 4 * 32) {
+    z64 x[4], y[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      x[u] = Xc[r + u * 32];
+      y[u] = v[r + u * 32];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) cmacc(acc, x[u], y[u]);
+  }
+  for (; r < n; r += 32) cmacc(acc, Xc[r], v[r]);
+  acc.re = warp_sum(acc.re);
+  acc.im = warp_sum(acc.im);
+  if (lane == 0) X[c2] = acc;
+}
+
+// blocks of the panel products: a warp each
+__host__ __device__ __forceinline__ int hl_dots(int jj, int tile) { return (2 * jj + tile / 8 - 1) / (tile / 8); }
+template <int HL_T>
+__global__ void __launch_bounds__(4 * HL_T, HL_BPS * 32 / HL_T) k_hemv_lower(const z64 *Ab, int64_t lda, int64_t sA,
+                                                              const int *nvec, int i, z64 *Pb, int64_t sP,
+                                                              int64_t ldp, const z64 *Wb, int64_t sW, int k0,
+                                                              int jj, z64 *X, int ldx) {
+  constexpr int HL_LD = HL_T + 1;  // padded column stride of the shared tile
+  constexpr int HL_NT = 4 * HL_T;
+  __shared__ __align__(16) z64 tile[2][HL_T * HL_LD];  // tile[buf][c * HL_LD + r]
+  __shared__ __align__(16) z64 vR[2][HL_T], vC[2][HL_T];
+  __shared__ z64 red[2][2][HL_T];
   const int b = blockIdx.z;
   const int n = nvec[b];
   const int r0 = i + 1;
-  if (r0 >= n) return;
-  if ((int)blockIdx.x < 2 * jj) {
-    __shared__ typename Sum<R>::T dred[2][HL_NT / 32];
-    panel_dot<R>(Ab + b * sA, Wb + b * sW, lda, n, i, k0, jj, blockIdx.x, threadIdx.x, dred, X + b * ldx);
+  if (r0 >= n || hl_tile(n - r0) != HL_T) return;
+  const int nd = hl_dots(jj, HL_T);
+  if ((int)blockIdx.x < nd) {
+    panel_dot_warp(Ab + b * sA, Wb + b * sW, lda, n, i, k0, jj, blockIdx.x * (HL_NT / 32) + threadIdx.x / 32, X + b * ldx);
     return;
   }
-  const int bx = blockIdx.x - 2 * jj, gx = gridDim.x - 2 * jj;  // among the mat-vec's blocks
+  const int bx = blockIdx.x - nd, gx = gridDim.x - nd;  // among the mat-vec's blocks
   const int nt = (n - r0 + HL_T - 1) / HL_T;
   const int npairs = nt * (nt + 1) / 2;
   if (bx >= npairs) return;
-  const C<R> *A = Ab + b * sA;
+  const z64 *A = Ab + b * sA;
   const int tid = threadIdx.x;
   // copies of tile pair p into buffer buf (zero outside the matrix)
   auto issue = [&](int p, int buf) {
@@ -387,8 +420,8 @@ __global__ void __launch_bounds__(HL_NT, HL_BPS) k_hemv_lower(const C<R> *Ab, in
     constexpr int CS = HL_NT / HL_T;
     const int r = tid % HL_T, cb = tid / HL_T;
     const int rr = rt0 + r;
-    const C<R> *src = A + rr + lda * (ct0 + cb);
-    C<R> *dst = &tile[buf][cb * HL_LD + r];
+    const z64 *src = A + rr + lda * (ct0 + cb);
+    z64 *dst = &tile[buf][cb * HL_LD + r];
 #pragma unroll
     for (int j = 0; j < HL_T / CS; ++j) {
       const bool ok = rr < n && ct0 + cb + CS * j < n;
@@ -421,9 +454,9 @@ __global__ void __launch_bounds__(HL_NT, HL_BPS) k_hemv_lower(const C<R> *Ab, in
     tile_pair(p, Rt, Ct);
     const int rt0 = r0 + Rt * HL_T, ct0 = r0 + Ct * HL_T;
     const bool diag = (Rt == Ct);
-    const C<R> *tl = tile[buf];
+    const z64 *tl = tile[buf];
     if (prod == 0) {
-      C<R> acc = cz<R>();
+      z64 acc = z64{0.0, 0.0};
       const int r = lane;
       if (!diag) {
 #pragma unroll HL_UNROLL
@@ -431,13 +464,13 @@ __global__ void __launch_bounds__(HL_NT, HL_BPS) k_hemv_lower(const C<R> *Ab, in
       } else {  // diagonal tile: the upper part is the conjugate of the mirrored element
 #pragma unroll HL_UNROLL
         for (int c = half * SPAN; c < half * SPAN + SPAN; ++c) {
-          const C<R> a = (r >= c) ? tl[c * HL_LD + r] : cconj(tl[r * HL_LD + c]);
+          const z64 a = (r >= c) ? tl[c * HL_LD + r] : cconj(tl[r * HL_LD + c]);
           cmac(acc, a, vC[buf][c]);
         }
       }
       red[0][half][r] = cfin(acc);
     } else if (!diag) {
-      C<R> acc = cz<R>();
+      z64 acc = z64{0.0, 0.0};
       const int c = lane;
 #pragma unroll HL_UNROLL
       for (int r = half * SPAN; r < half * SPAN + SPAN; ++r) cmacc(acc, tl[c * HL_LD + r], vR[buf][r]);
@@ -513,7 +546,7 @@ __global__ void __launch_bounds__(HV_NT, HV_BPS) k_hemv_df(const zdf *Ab, int64_
   const int nd = hv_dots(jj);
   if ((int)blockIdx.x < nd) {
     const int g = warp >> 2;
-    panel_dot<df>(A, Wb + b * sW, lda, n, i, k0, jj, blockIdx.x * 2 + g, tid & (HL_NT - 1),
+    panel_dot(A, Wb + b * sW, lda, n, i, k0, jj, blockIdx.x * 2 + g, tid & 127,
                   (Sum<df>::T(*)[4])hv_smem + 2 * g,
                   X + b * ldx);
     return;
@@ -628,7 +661,7 @@ struct PanelCol {
   __device__ __forceinline__ PanelCol(const C<R> *A_, const C<R> *W_, const C<R> *P_, int64_t lda_, int64_t ldp_, int n_,
                                       int i_, int k0_, int jj_, int next_, int sms)
       : A(A_), W(W_), P(P_), lda(lda_), ldp(ldp_), n(n_), i(i_), k0(k0_), jj(jj_), next(next_) {
-    nt = cdiv_dev(n - i - 1, std::is_same<R, double>::value ? HL_T : HV_R);
+    nt = cdiv_dev(n - i - 1, std::is_same<R, double>::value ? hl_tile(n - i - 1) : HV_R);
     run = std::is_same<R, double>::value ? 1 : hv_run(n - i - 1, jj, sms);
   }
   // the number of slots of row r: 0 .. nseg-1, then from nseg + skip on
@@ -1078,7 +1111,11 @@ __global__ void __launch_bounds__(TR_NT) k_colstep(C<R> *Ab, int64_t lda, int64_
 }
 
 // Trailing update A(k1:n, k1:n) -= V W^H + W V^H (full square), K = jb.
-constexpr int HK_T = 64, HK_K = 8;
+// Tiles of 32 x 32 (2 x 2 per thread): with 64 x 64 a trailing block of a few
+// hundred rows had fewer tiles than SMs, and one of order 52 a single one
+// (FP64 pipe: 2 multiply-adds per SM and clock; n = 84 265 -> 72 us a launch,
+// n = 1092 343 -> 167 us, two of n = 2604 1169 -> 1017 us).
+constexpr int HK_T = 32, HK_K = 16, HK_P = HK_T / 16;
 template <class R>
 __global__ void __launch_bounds__(256) k_her2k(C<R> *Ab, int64_t lda, int64_t sA, const C<R> *Wb, int64_t sW,
                                                const int *nvec, int k0, int jb) {
@@ -1092,11 +1129,11 @@ __global__ void __launch_bounds__(256) k_her2k(C<R> *Ab, int64_t lda, int64_t sA
   C<R> *A = Ab + b * sA;
   const C<R> *W = Wb + b * sW;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  C<R> acc[4][4];
+  C<R> acc[HK_P][HK_P];
 #pragma unroll
-  for (int p = 0; p < 4; ++p)
+  for (int p = 0; p < HK_P; ++p)
 #pragma unroll
-    for (int q = 0; q < 4; ++q) acc[p][q] = cz<R>();
+    for (int q = 0; q < HK_P; ++q) acc[p][q] = cz<R>();
   const int jmax = min(jb, n - 1 - k0);  // reflectors that exist in this matrix
   for (int kc = 0; kc < jmax; kc += HK_K) {
     for (int e = threadIdx.x; e < HK_K * HK_T; e += 256) {
@@ -1112,18 +1149,18 @@ __global__ void __launch_bounds__(256) k_her2k(C<R> *Ab, int64_t lda, int64_t sA
     __syncthreads();
 #pragma unroll 2
     for (int k = 0; k < HK_K; ++k) {
-      C<R> vr[4], wr[4], vc[4], wc[4];
+      C<R> vr[HK_P], wr[HK_P], vc[HK_P], wc[HK_P];
 #pragma unroll
-      for (int p = 0; p < 4; ++p) {
+      for (int p = 0; p < HK_P; ++p) {
         vr[p] = sVr[k][tx + 16 * p];
         wr[p] = sWr[k][tx + 16 * p];
         vc[p] = sVc[k][ty + 16 * p];
         wc[p] = sWc[k][ty + 16 * p];
       }
 #pragma unroll
-      for (int p = 0; p < 4; ++p)
+      for (int p = 0; p < HK_P; ++p)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
+        for (int q = 0; q < HK_P; ++q) {
           cmac(acc[p][q], vr[p], wc[q]);
           cmac(acc[p][q], wr[p], vc[q]);
         }
@@ -1131,9 +1168,9 @@ __global__ void __launch_bounds__(256) k_her2k(C<R> *Ab, int64_t lda, int64_t sA
     __syncthreads();
   }
 #pragma unroll
-  for (int p = 0; p < 4; ++p)
+  for (int p = 0; p < HK_P; ++p)
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < HK_P; ++q) {
       int rr = r0 + tx + 16 * p, cc = c0 + ty + 16 * q;
       if (rr < n && cc < n) {
         C<R> *x = &A[rr + lda * cc];
@@ -1162,8 +1199,10 @@ static cudaError_t prepare_colstep() {
   return e;
 }
 
-// One column step; the cluster has a CTA per 8 rows, at most CT_CLUSTER (a
-// function of the batch's largest order only).  Past CT_SPLIT rows the row work
+// One column step; the cluster has a CTA per 8 rows, at most CT_CLUSTER, and
+// fewer where the whole batch would not run at once (two CTAs fit an SM; 64
+// matrices of order 444, FP64: 48 us a column with clusters of 16, 29 us with
+// clusters of 4).  Past CT_SPLIT rows the row work
 // goes to the whole chip first (k_wpart): one cluster works through CT_SPLIT
 // rows in one pass, and more passes cost more than the extra launch (both
 // launches against one: 11.5 us / 13.3 us at n = 1092, 13.2 us / 34.9 us at
@@ -1182,7 +1221,7 @@ static cudaError_t launch_colstep(EigWork &w, int i, int k0, int jj, int do_w, i
     count_launch(1);
   }
   int cs = 1;
-  while (cs < CT_CLUSTER && cs * 8 < rows) cs *= 2;
+  while (cs < CT_CLUSTER && cs * 8 < rows && cs * std::max(w.batch, w.B) <= device_sms()) cs *= 2;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(cs, w.B);
   cfg.blockDim = dim3(TR_NT);
@@ -1225,13 +1264,25 @@ cudaError_t tridiagonalize(EigWork &w, cudaStream_t s) {
         const int gx = hv_dots(jj) + std::min(nt * (nt + 1), hv_ctas(jj, device_sms()));
         PP_KT(KT_HEMV, s, (k_hemv_df<<<dim3(gx, B), HV_NT, HV_SMEM, s>>>(A, lda, sA, w.nvec, i, P, sP, lda, W, sW, k0,
                                                                         jj, (C<R> *)w.X, 2 * nb, device_sms())));
+        count_launch(1);
       } else {
-        const int nt = cdiv(nmax - i - 1, HL_T);
-        const int gx = 2 * jj + std::min(nt * (nt + 1) / 2, hemv_blocks(w.hemv_bps));
-        PP_KT(KT_HEMV, s, (k_hemv_lower<R><<<dim3(gx, 1, B), HL_NT, 0, s>>>(A, lda, sA, w.nvec, i, P, sP, lda, W, sW, k0,
-                                                                            jj, (C<R> *)w.X, 2 * nb)));
+        // (the tile follows each matrix's own order: a batch that has both kinds runs both kernels)
+        const int rows = nmax - i - 1;
+        if (rows > HL_SMALL) {
+          const int nt = cdiv(rows, HL_T);
+          const int gx = hl_dots(jj, HL_T) + std::min(nt * (nt + 1) / 2, hemv_blocks(w.hemv_bps));
+          PP_KT(KT_HEMV, s, (k_hemv_lower<HL_T><<<dim3(gx, 1, B), 4 * HL_T, 0, s>>>(A, lda, sA, w.nvec, i, P, sP, lda, W,
+                                                                                    sW, k0, jj, (C<R> *)w.X, 2 * nb)));
+          count_launch(1);
+        }
+        if (w.nmin - i - 1 <= HL_SMALL) {
+          const int nt = cdiv(std::min(rows, HL_SMALL), HL_TS);
+          const int gx = hl_dots(jj, HL_TS) + nt * (nt + 1) / 2;
+          PP_KT(KT_HEMV, s, (k_hemv_lower<HL_TS><<<dim3(gx, 1, B), 4 * HL_TS, 0, s>>>(A, lda, sA, w.nvec, i, P, sP, lda, W,
+                                                                                      sW, k0, jj, (C<R> *)w.X, 2 * nb)));
+          count_launch(1);
+        }
       }
-      count_launch(1);
       PP_CUDA_TRY(launch_colstep<R>(w, i, k0, jj, 1, jj + 1 < jb ? 1 : 0, s));
     }
     const int k1 = k0 + jb;
@@ -1252,21 +1303,40 @@ cudaError_t tridiagonalize(EigWork &w, cudaStream_t s) {
 // ===========================================================================
 // Stage 2: eigenvalues of the tridiagonal matrix (FP64 bisection)
 // ===========================================================================
-// Gerschgorin interval, pivmin and the index range of the wanted eigenvalues.
-__global__ void k_tdprep(const double *dd, const double *ee, int64_t sd, const int *nvec, char range, double vl,
-                         double vu, int64_t il, int64_t iu, int64_t *rng, double *tinfo, int64_t *info,
-                         const int *tcerr) {
+// Gerschgorin interval, pivmin and the index range of the wanted eigenvalues
+// (one block per matrix; the extrema do not depend on the order of the rows).
+constexpr int TD_NT = 256;
+__global__ void __launch_bounds__(TD_NT) k_tdprep(const double *dd, const double *ee, int64_t sd, const int *nvec,
+                                                  char range, double vl, double vu, int64_t il, int64_t iu, int64_t *rng,
+                                                  double *tinfo, int64_t *info, const int *tcerr) {
+  __shared__ double sgl[TD_NT / 32], sgu[TD_NT / 32], se2[TD_NT / 32];
+  __shared__ int scount[2];
   const int b = blockIdx.x;
-  if (threadIdx.x != 0) return;
   const int n = nvec[b];
   const double *d = dd + b * sd;
   const double *e = ee + b * sd;
   double gl = d[0], gu = d[0], emax2 = 0.0;
-  for (int k = 0; k < n; ++k) {
-    double off = (k > 0 ? fabs(e[k - 1]) : 0.0) + (k < n - 1 ? fabs(e[k]) : 0.0);
+  for (int k = threadIdx.x; k < n; k += TD_NT) {
+    const double off = (k > 0 ? fabs(e[k - 1]) : 0.0) + (k < n - 1 ? fabs(e[k]) : 0.0);
     gl = fmin(gl, d[k] - off);
     gu = fmax(gu, d[k] + off);
     if (k < n - 1) emax2 = fmax(emax2, e[k] * e[k]);
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    gl = fmin(gl, __shfl_xor_sync(0xffffffffu, gl, o));
+    gu = fmax(gu, __shfl_xor_sync(0xffffffffu, gu, o));
+    emax2 = fmax(emax2, __shfl_xor_sync(0xffffffffu, emax2, o));
+  }
+  if ((threadIdx.x & 31) == 0) {
+    sgl[threadIdx.x >> 5] = gl;
+    sgu[threadIdx.x >> 5] = gu;
+    se2[threadIdx.x >> 5] = emax2;
+  }
+  __syncthreads();
+  for (int k = 0; k < TD_NT / 32; ++k) {
+    gl = fmin(gl, sgl[k]);
+    gu = fmax(gu, sgu[k]);
+    emax2 = fmax(emax2, se2[k]);
   }
   const double ulp = DBL_EPSILON;
   const double safmin = DBL_MIN;
@@ -1280,13 +1350,11 @@ __global__ void k_tdprep(const double *dd, const double *ee, int64_t sd, const i
     lo = il;
     hi = iu;
   } else if (range == 'V') {
-    // eigenvalues in the half-open interval (vl, vu]
+    // eigenvalues in the half-open interval (vl, vu]: a count each in the first threads of two warps
     // local e^2 recomputed on the fly
-    double q;
-    int cl = 0, cu = 0;
-    for (int pass = 0; pass < 2; ++pass) {
-      double x = pass == 0 ? vl : vu;
-      q = d[0] - x;
+    if (threadIdx.x == 0 || threadIdx.x == 32) {
+      const double x = threadIdx.x == 0 ? vl : vu;
+      double q = d[0] - x;
       if (fabs(q) <= pivmin) q = -pivmin;
       int c = q < 0.0;
       for (int k = 1; k < n; ++k) {
@@ -1294,14 +1362,13 @@ __global__ void k_tdprep(const double *dd, const double *ee, int64_t sd, const i
         if (fabs(q) <= pivmin) q = -pivmin;
         c += q < 0.0;
       }
-      if (pass == 0)
-        cl = c;
-      else
-        cu = c;
+      scount[threadIdx.x / 32] = c;
     }
-    lo = cl + 1;
-    hi = cu;
+    __syncthreads();
+    lo = scount[0] + 1;
+    hi = scount[1];
   }
+  if (threadIdx.x != 0) return;
   int64_t m = hi - lo + 1;
   if (m < 0) m = 0;
   rng[b * 8 + 0] = lo;
@@ -1580,7 +1647,7 @@ cudaError_t prepare_bisect(size_t bytes) {
 cudaError_t tridiag_eigenvalues(EigWork &w, char range, double vl, double vu, int64_t il, int64_t iu, double abstol,
                                 cudaStream_t s, int mixed) {
   const int64_t sd = w.nmax;
-  k_tdprep<<<w.B, 32, 0, s>>>(w.d, w.e, sd, w.nvec, range, vl, vu, il, iu, w.rng, w.tinfo, w.info, w.tcErr);
+  k_tdprep<<<w.B, TD_NT, 0, s>>>(w.d, w.e, sd, w.nvec, range, vl, vu, il, iu, w.rng, w.tinfo, w.info, w.tcErr);
   const size_t smem = bisect_smem(w.nmax, mixed);
   int mode = 0;
   if (smem) {
@@ -1603,20 +1670,35 @@ cudaError_t tridiag_eigenvalues(EigWork &w, char range, double vl, double vu, in
 // Stage 3: eigenvectors of T by inverse iteration
 // ===========================================================================
 // Clusters of consecutive eigenvalues closer than rel * ||T||.
-__global__ void k_clusters(const double *ww, int64_t sd, const int64_t *rng, const double *tinfo, int *cls,
-                           int64_t scl, int *ncl, double rel) {
+constexpr int CL_NT = 256;
+__global__ void __launch_bounds__(CL_NT) k_clusters(const double *ww, int64_t sd, const int64_t *rng, const double *tinfo,
+                                                    int *cls, int64_t scl, int *ncl, double rel) {
+  __shared__ int wsum[CL_NT / 32];
   const int b = blockIdx.x;
-  if (threadIdx.x != 0) return;
   const int64_t m = rng[b * 8 + 2];
-  const double tnorm = tinfo[b * 8 + 2];
-  const double ortol = rel * tnorm;
+  const double ortol = rel * tinfo[b * 8 + 2];
   const double *w = ww + b * sd;
-  int c = 0;
-  for (int64_t j = 0; j < m; ++j) {
-    if (j == 0 || w[j] - w[j - 1] > ortol) cls[b * scl + c++] = (int)j;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int c = 0;  // cluster starts before this stretch of CL_NT eigenvalues
+  for (int64_t j0 = 0; j0 < m; j0 += CL_NT) {
+    const int64_t j = j0 + threadIdx.x;
+    const bool start = j < m && (j == 0 || w[j] - w[j - 1] > ortol);
+    const unsigned bits = __ballot_sync(0xffffffffu, start);
+    if (lane == 0) wsum[warp] = __popc(bits);
+    __syncthreads();
+    int before = c + __popc(bits & ((1u << lane) - 1u)), all = 0;
+    for (int k = 0; k < CL_NT / 32; ++k) {
+      if (k < warp) before += wsum[k];
+      all += wsum[k];
+    }
+    if (start) cls[b * scl + before] = (int)j;
+    c += all;
+    __syncthreads();
   }
-  cls[b * scl + c] = (int)m;
-  ncl[b] = c;
+  if (threadIdx.x == 0) {
+    cls[b * scl + c] = (int)m;
+    ncl[b] = c;
+  }
 }
 
 // Inverse iteration orthogonalises only inside tight clusters (where the
@@ -1936,7 +2018,7 @@ template <class R>
 cudaError_t tridiag_eigenvectors(EigWork &w, cudaStream_t s) {
   const int64_t sd = w.nmax;
   const int64_t scl = w.nmax + 1;
-  k_clusters<<<w.B, 32, 0, s>>>(w.w, sd, w.rng, w.tinfo, w.cls, scl, w.ncl, 1e-7);
+  k_clusters<<<w.B, CL_NT, 0, s>>>(w.w, sd, w.rng, w.tinfo, w.cls, scl, w.ncl, 1e-7);
   count_launch(1);
   const int64_t T = w.scratch_threads;
   const int64_t sS = (int64_t)IV_F * w.nmax * T;
@@ -1948,7 +2030,7 @@ cudaError_t tridiag_eigenvectors(EigWork &w, cudaStream_t s) {
                                                     w.info)));
     count_launch(1);
   }
-  k_clusters<<<w.B, 32, 0, s>>>(w.w, sd, w.rng, w.tinfo, w.cls, scl, w.ncl, 1e-5);
+  k_clusters<<<w.B, CL_NT, 0, s>>>(w.w, sd, w.rng, w.tinfo, w.cls, scl, w.ncl, 1e-5);
   PP_KT(KT_INVIT, s, (k_reorth<R><<<dim3(RO_BLOCKS, w.B), 256, 0, s>>>((C<R> *)w.E, w.lde, w.sE, w.nvec, w.cls, scl, w.ncl)));
   count_launch(2);
   return cudaGetLastError();
@@ -1957,15 +2039,20 @@ cudaError_t tridiag_eigenvectors(EigWork &w, cudaStream_t s) {
 // ===========================================================================
 // Stage 4: back-transform E = Q Z
 // ===========================================================================
-constexpr int BT_J = 64;     // columns per block
+constexpr int BT_J = 32;     // columns per block
+constexpr int BT_NT = 128;   // threads: a column and 8 of the 32 panel columns each
 constexpr int BT_RK = 16;    // rows per k-step
-constexpr int BT_RCH = 512;  // rows per split-K chunk
+// Rows per split-K chunk of `rows`: 8 chunks, 32 to 256 rows.  (64 columns and
+// 512 rows per block left half of the SMs without work: 4 matrices of order
+// 1092 with 1092 columns 935 us -> 606 us per panel.)
+constexpr int BT_CHUNKS = 8, BT_RMIN = 32, BT_RMAX = 256;
+static int bt_chunk(int rows) { return std::max(BT_RMIN, std::min(BT_RMAX, cdiv(cdiv(rows, BT_CHUNKS), BT_RK) * BT_RK)); }
 
 // Wp[ks][a][j] = sum_{r in chunk ks} conj(V(r,a)) X(r,j) for a < jb.
 // V(r,a) = A(r, k0+a) for r >= k0+a+1 (zero above); j < the matrix's m, or
 // ncol_fixed.
 template <class R>
-__global__ void __launch_bounds__(256) k_vhx(const C<R> *Ab, int64_t lda, int64_t sA, const C<R> *Xb, int64_t ldx,
+__global__ void __launch_bounds__(BT_NT) k_vhx(const C<R> *Ab, int64_t lda, int64_t sA, const C<R> *Xb, int64_t ldx,
                                              int64_t sX, const int *nvec, const int64_t *rng, int k0, int jb,
                                              C<R> *Wp, int64_t ldwp, int64_t sWp, int ncol_fixed, int rch) {
   __shared__ C<R> sV[BT_RK][32];
@@ -1980,19 +2067,19 @@ __global__ void __launch_bounds__(256) k_vhx(const C<R> *Ab, int64_t lda, int64_
   const C<R> *A = Ab + b * sA;
   const C<R> *X = Xb + b * sX;
   const int64_t ldX = ldx;
-  const int tj = threadIdx.x & 63, ta = threadIdx.x >> 6;
+  const int tj = threadIdx.x & 31, ta = threadIdx.x >> 5;
   C<R> acc[8];
 #pragma unroll
   for (int p = 0; p < 8; ++p) acc[p] = cz<R>();
   const int rend = min(n, rbeg + rch);
   for (int r0 = rbeg; r0 < rend; r0 += BT_RK) {
-    for (int e = threadIdx.x; e < BT_RK * 32; e += 256) {
+    for (int e = threadIdx.x; e < BT_RK * 32; e += BT_NT) {
       const int a = e & 31, rr = e >> 5;
       const int r = r0 + rr;
       sV[rr][a] = (a < jb && r < rend && r >= k0 + a + 1) ? cconj(A[r + lda * (k0 + a)]) : cz<R>();
     }
-    for (int e = threadIdx.x; e < BT_RK * BT_J; e += 256) {
-      const int jx = e & 63, rr = e >> 6;
+    for (int e = threadIdx.x; e < BT_RK * BT_J; e += BT_NT) {
+      const int jx = e & 31, rr = e >> 5;
       const int r = r0 + rr, j = j0 + jx;
       const bool ok = r < rend && j < ncol;
       sXt[rr][jx] = ok ? X[r + ldX * j] : cz<R>();
@@ -2026,14 +2113,14 @@ constexpr int BR_NT = 256;
 template <class R>
 __global__ void __launch_bounds__(BR_NT) k_btred(const C<R> *Wp, int64_t ldwp, int64_t sWp, const int *nvec,
                                                  const int64_t *rng, int k0, int jb, int mode, const z64 *Tf,
-                                                 C<R> *Wb, int64_t sWb, int ncol_fixed, int nks_fixed = 0) {
+                                                 C<R> *Wb, int64_t sWb, int ncol_fixed, int rch, int nks_fixed = 0) {
   __shared__ C<R> col[32][33];
   __shared__ z64 sT[32][33];
   const int b = blockIdx.y;
   const int n = nvec[b];
   const int ncol = ncol_fixed > 0 ? ncol_fixed : (int)rng[b * 8 + 2];
-  // split-K partials to sum: one per BT_RCH rows, or nks_fixed
-  const int nks = nks_fixed > 0 ? (n - k0 - 1 > 0 ? nks_fixed : 0) : (n - k0 - 1 + BT_RCH - 1) / BT_RCH;
+  // split-K partials to sum: one per rch rows, or nks_fixed
+  const int nks = nks_fixed > 0 ? (n - k0 - 1 > 0 ? nks_fixed : 0) : (n - k0 - 1 + rch - 1) / rch;
   const int j0 = blockIdx.x * 32;
   if (j0 >= ncol || nks <= 0) return;
   for (int e = threadIdx.x; e < 32 * 32; e += BR_NT) sT[e / 32][e % 32] = Tf[b * 1024 + e];
@@ -2061,7 +2148,7 @@ __global__ void __launch_bounds__(BR_NT) k_btred(const C<R> *Wp, int64_t ldwp, i
 // Compact-WY factors of every panel in one launch, one block per (panel,
 // matrix): the Gram matrix G = V^H V of the panel's Householder vectors
 // (products in the arithmetic R, rows staged WY_RK at a time and the sums
-// renormalised after each stage, each thread four entries), then Tf by
+// renormalised after each stage, each thread two entries above the diagonal), then Tf by
 // zlarft's forward columnwise recurrence in FP64: Tf(a,a) = tau_a,
 // Tf(0:a, a) = -tau_a Tf(0:a, 0:a) G(0:a, a).  Tf of panel P for matrix b
 // goes to Tf + P sTfp + 1024 b (row-major 32 x 32).  Panel widths follow the
@@ -2081,10 +2168,20 @@ __global__ void __launch_bounds__(256) k_wy_factors(const C<R> *Ab, int64_t lda,
   const int jb = min(nb, nref - k0);
   const C<R> *A = Ab + b * sA;
   const int tid = threadIdx.x;
-  const int ga = tid >> 3, gj = (tid & 7) * 4;  // G(ga, gj .. gj+3)
-  C<R> acc[4];
+  // the 496 entries G(a, j), a < j, that the recurrence reads: two per thread
+  int ga[2], gj[2];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) acc[q] = cz<R>();
+  for (int q = 0; q < 2; ++q) {
+    const int t = min(tid + 256 * q, 495);
+    int j = (int)((1.0f + sqrtf(1.0f + 8.0f * (float)t)) * 0.5f);
+    while (j * (j - 1) / 2 > t) --j;
+    while (j * (j + 1) / 2 <= t) ++j;
+    gj[q] = j;
+    ga[q] = t - j * (j - 1) / 2;
+  }
+  C<R> acc[2];
+#pragma unroll
+  for (int q = 0; q < 2; ++q) acc[q] = cz<R>();
   for (int r0 = k0 + 1; r0 < n; r0 += WY_RK) {
     for (int e = tid; e < WY_RK * 32; e += 256) {
       const int a = e & 31, rr = e >> 5, r = r0 + rr;
@@ -2093,18 +2190,17 @@ __global__ void __launch_bounds__(256) k_wy_factors(const C<R> *Ab, int64_t lda,
     __syncthreads();
 #pragma unroll 4
     for (int rr = 0; rr < WY_RK; ++rr) {
-      const C<R> va = sV[rr][ga];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) cmacc(acc[q], va, sV[rr][gj + q]);
+      for (int q = 0; q < 2; ++q) cmacc(acc[q], sV[rr][ga[q]], sV[rr][gj[q]]);
     }
     // renormalise after every WY_RK rows: the unnormalised low word of the
     // multiply-add is meant for short sums, the panel runs over all n rows
 #pragma unroll
-    for (int q = 0; q < 4; ++q) acc[q] = cfin(acc[q]);
+    for (int q = 0; q < 2; ++q) acc[q] = cfin(acc[q]);
     __syncthreads();
   }
 #pragma unroll
-  for (int q = 0; q < 4; ++q) G[ga][gj + q] = cto64(cfin(acc[q]));
+  for (int q = 0; q < 2; ++q) G[ga[q]][gj[q]] = cto64(cfin(acc[q]));
   for (int e = tid; e < 1024; e += 256) sT[e / 32][e % 32] = z64{0.0, 0.0};
   __syncthreads();
   if (tid < 32) {
@@ -2134,7 +2230,7 @@ __global__ void __launch_bounds__(256) k_wy_factors(const C<R> *Ab, int64_t lda,
 }
 
 // E(r, j) -= sum_a V(r, a) Y(a, j), r in [k0+1, n), j < m.
-constexpr int AV_T = 64, AV_K = 16;
+constexpr int AV_T = 32, AV_K = 16, AV_P = AV_T / 16;  // (64 x 64 tiles: too few blocks for orders of a few hundred)
 template <class R>
 __global__ void __launch_bounds__(256) k_applyV(const C<R> *Ab, int64_t lda, int64_t sA, const C<R> *Wb,
                                                 int64_t ldwp, int64_t sWb, C<R> *Eb, int64_t lde, int64_t sE,
@@ -2150,11 +2246,11 @@ __global__ void __launch_bounds__(256) k_applyV(const C<R> *Ab, int64_t lda, int
   const C<R> *Y = Wb + b * sWb;
   C<R> *E = Eb + b * sE;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  C<R> acc[4][4];
+  C<R> acc[AV_P][AV_P];
 #pragma unroll
-  for (int p = 0; p < 4; ++p)
+  for (int p = 0; p < AV_P; ++p)
 #pragma unroll
-    for (int q = 0; q < 4; ++q) acc[p][q] = cz<R>();
+    for (int q = 0; q < AV_P; ++q) acc[p][q] = cz<R>();
   for (int kc = 0; kc < jb; kc += AV_K) {
     for (int e = threadIdx.x; e < AV_K * AV_T; e += 256) {
       const int x = e % AV_T, y = e / AV_T;
@@ -2166,23 +2262,23 @@ __global__ void __launch_bounds__(256) k_applyV(const C<R> *Ab, int64_t lda, int
     __syncthreads();
 #pragma unroll 4
     for (int k = 0; k < AV_K; ++k) {
-      C<R> v[4], y[4];
+      C<R> v[AV_P], y[AV_P];
 #pragma unroll
-      for (int p = 0; p < 4; ++p) {
+      for (int p = 0; p < AV_P; ++p) {
         v[p] = sV[k][tx + 16 * p];
         y[p] = sY[k][ty + 16 * p];
       }
 #pragma unroll
-      for (int p = 0; p < 4; ++p)
+      for (int p = 0; p < AV_P; ++p)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) cmac(acc[p][q], v[p], y[q]);
+        for (int q = 0; q < AV_P; ++q) cmac(acc[p][q], v[p], y[q]);
     }
     __syncthreads();
   }
 #pragma unroll
-  for (int p = 0; p < 4; ++p)
+  for (int p = 0; p < AV_P; ++p)
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < AV_P; ++q) {
       const int r = r0 + tx + 16 * p, c = c0 + ty + 16 * q;
       if (r < n && c < m) {
         C<R> *x = &E[r + lde * c];
@@ -2211,20 +2307,20 @@ cudaError_t back_transform(EigWork &w, cudaStream_t s) {
   const int kstart = ((nref - 1) / nb) * nb;
   for (int k0 = kstart; k0 >= 0; k0 -= nb) {
     const int jb = min(nb, nref - k0);
-    const int ks = cdiv(nmax - k0 - 1, BT_RCH);
+    const int rch = bt_chunk(nmax - k0 - 1), ks = cdiv(nmax - k0 - 1, rch);
     const z64 *Tf = w.Tf + (int64_t)(k0 / nb) * w.sTfp;
     // Y = Tf V^H E ; E -= V Y (on the tensor cores in the double-float form,
     // over all mcap columns)
     const bool tc = std::is_same<R, df>::value && w.tcS && tc_enabled();
     if (tc) {
       PP_CUDA_TRY(vhx_tc(w, k0, jb, (const zdf *)E, w.lde, w.sE, w.mcap, (zdf *)Wp, ldwp, sWp, s));
-      PP_KT(KT_BTRED, s, (k_btred<R><<<dim3(cdiv(w.mcap, 32), B), BR_NT, 0, s>>>(Wp, ldwp, sWp, w.nvec, w.rng, k0, jb, 1, Tf, Wb, sWb, w.mcap, vhx_tc_splits(w))));
+      PP_KT(KT_BTRED, s, (k_btred<R><<<dim3(cdiv(w.mcap, 32), B), BR_NT, 0, s>>>(Wp, ldwp, sWp, w.nvec, w.rng, k0, jb, 1, Tf, Wb, sWb, w.mcap, rch, vhx_tc_splits(w))));
       PP_CUDA_TRY(applyV_tc(w, k0, jb, (zdf *)E, w.lde, w.sE, (const zdf *)Wb, ldwp, sWb, w.mcap, s));
       count_launch(1);
     } else {
-      PP_KT(KT_VHX, s, (k_vhx<R><<<dim3(cdiv(w.mcap, BT_J), ks, B), 256, 0, s>>>(A, w.lda, w.sA, E, w.lde, w.sE, w.nvec, w.rng, k0,
-                                                               jb, Wp, ldwp, sWp, 0, BT_RCH)));
-      PP_KT(KT_BTRED, s, (k_btred<R><<<dim3(cdiv(w.mcap, 32), B), BR_NT, 0, s>>>(Wp, ldwp, sWp, w.nvec, w.rng, k0, jb, 1, Tf, Wb, sWb, 0)));
+      PP_KT(KT_VHX, s, (k_vhx<R><<<dim3(cdiv(w.mcap, BT_J), ks, B), BT_NT, 0, s>>>(A, w.lda, w.sA, E, w.lde, w.sE, w.nvec, w.rng, k0,
+                                                               jb, Wp, ldwp, sWp, 0, rch)));
+      PP_KT(KT_BTRED, s, (k_btred<R><<<dim3(cdiv(w.mcap, 32), B), BR_NT, 0, s>>>(Wp, ldwp, sWp, w.nvec, w.rng, k0, jb, 1, Tf, Wb, sWb, 0, rch)));
       PP_KT(KT_APPLYV, s, (k_applyV<R><<<dim3(cdiv(nmax - k0 - 1, AV_T), cdiv(w.mcap, AV_T), B), 256, 0, s>>>(
           A, w.lda, w.sA, Wb, ldwp, sWb, E, w.lde, w.sE, w.nvec, w.rng, k0, jb, 0)));
       count_launch(3);
@@ -2324,18 +2420,18 @@ cudaError_t back_transform_rows(EigWork &w, const int *d_rows, int nrows, cudaSt
   count_launch(1);
   for (int k0 = 0; k0 < nref; k0 += nb) {
     const int jb = min(nb, nref - k0);
-    const int ks = cdiv(nmax - k0 - 1, BT_RCH);
+    const int rch = bt_chunk(nmax - k0 - 1), ks = cdiv(nmax - k0 - 1, rch);
     const z64 *Tf = w.Tf + (int64_t)(k0 / nb) * w.sTfp;
     const bool tc = std::is_same<R, df>::value && w.tcS && tc_enabled();
     if (tc) {
       PP_CUDA_TRY(vhx_tc(w, k0, jb, (const zdf *)X, ldx, sX, nrows, (zdf *)Wp, ldwp, sWp, s));
     } else {
-      PP_KT(KT_VHX, s, (k_vhx<R><<<dim3(cdiv(nrows, BT_J), ks, B), 256, 0, s>>>(A, w.lda, w.sA, X, ldx, sX, w.nvec,
+      PP_KT(KT_VHX, s, (k_vhx<R><<<dim3(cdiv(nrows, BT_J), ks, B), BT_NT, 0, s>>>(A, w.lda, w.sA, X, ldx, sX, w.nvec,
                                                                                w.rng, k0, jb, Wp, ldwp, sWp, nrows,
-                                                                               BT_RCH)));
+                                                                               rch)));
     }
     PP_KT(KT_BTRED, s, (k_btred<R><<<dim3(cdiv(nrows, 32), B), BR_NT, 0, s>>>(Wp, ldwp, sWp, w.nvec, w.rng, k0, jb, 2,
-                                                                          Tf, Wb, sWb, nrows,
+                                                                          Tf, Wb, sWb, nrows, rch,
                                                                           tc ? vhx_tc_splits(w) : 0)));
     if (tc) {
       PP_CUDA_TRY(applyV_tc(w, k0, jb, (zdf *)X, ldx, sX, (const zdf *)Wb, ldwp, sWb, nrows, s));

@@ -44,6 +44,8 @@ struct EigWork {
   int B = 0;           // matrices in the batch
   int boff = 0;        // index of the first matrix in the whole batch (views)
   int nmax = 0;        // largest order
+  int nmin = 0;        // smallest order
+  int batch = 0;       // matrices in the whole batch (views)
   int mcap = 0;        // eigenvector columns allocated per matrix
   int nb = 32;         // panel width
   int hemv_bps = 6;    // persistent blocks per SM of the Hermitian mat-vec (autotuned)
