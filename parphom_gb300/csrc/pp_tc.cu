@@ -15,17 +15,14 @@
 // the real part pairs k-step j of the row operand with k-step j of the
 // column operand and the imaginary part with k-step j ^ 2 (negated for the
 // Re X half, by the instruction's negate-B bit).  The 28 slice pairs with
-// s + t <= 6 go into 7 accumulators per real/imaginary part (14 x 32 TMEM
-// columns); the epilogue sums them in double-float, scales by
+// s + t <= 6 go into 7 accumulators per real/imaginary part; the fold sums
+// them in double-float, scales by
 // 2^(E_r + E_c - 16) and subtracts from A.  Separate grids for V and W keep
 // both at full relative resolution; the dropped pairs and the residual bound
 // the error by about 2^-55 |X_r| |Y_c| per product, the double-float level.
 //
-// CTA (512 threads) = 128 rows x (up to 8) column blocks of 32, both
-// products in turn.  The 112 KB row operand stays in shared memory while the
-// 28 KB column operands are streamed in by bulk copies, double-buffered so
-// that the next block's copy overlaps this block's MMAs.  One CTA per SM
-// (168 KB of shared memory, 448 tensor-memory columns).
+// The tile kernel (k_cupd_tc) takes 128 rows x a few column blocks of 64, one
+// CTA per SM: see there.
 #include <algorithm>
 #include <cfloat>
 #include <cstdint>
@@ -45,11 +42,9 @@ constexpr int TC_KS = 4;                         // k-steps of 16 (K = 64 reals)
 constexpr int TC_TILE = 4096;                    // one (slice, k-step) tile of 128 rows
 constexpr int TC_OP = TC_S * TC_KS * TC_TILE;    // one operand of a 128-row block (114688)
 constexpr int TC_RBLK = 2 * TC_OP;               // V and W operands of a 128-row block
-constexpr int TC_BBYTES = TC_S * TC_KS * 1024;   // one 32-row column block of one operand (28672)
-constexpr int TC_CB = 8;                         // column blocks per CTA
-constexpr int TC_NT = 512;                       // threads: 16 warps = 4 lane groups x 4 column quarters
-constexpr int TC_CQ = 32 / (TC_NT / 128);        // columns per thread in the epilogue (8)
-constexpr int TC_SMEM = TC_OP + 2 * TC_BBYTES + 2 * 256 + 64;  // + 2 x 32 exponent pairs, mbarriers, TMEM slot
+constexpr int TC_BBYTES = TC_S * TC_KS * 1024;   // 32 rows of one operand (28672): the long-K kernel's column operand
+constexpr int TC_NT = 512;                       // threads of the long-K kernel: 16 warps = 4 lane groups x 4 column quarters
+constexpr int TC_CQ = 32 / (TC_NT / 128);        // columns per thread in its fold (8)
 constexpr int TC_NACC = 2 * TC_S;                // accumulators: (re, im) x slice-sum group
 constexpr uint32_t TC_ID = tc::idesc_bf16(128, 32, 0);
 constexpr uint32_t TC_IDN = tc::idesc_bf16(128, 32, 1);
@@ -122,28 +117,42 @@ __global__ void __launch_bounds__(128) k_tc_slices(TcSliceSrc src, const int *nv
   if (lane == 0) E[b * sE + (int64_t)rl * es + eo] = e;
 }
 
-__device__ __forceinline__ df df_add_f(df a, float b) {
-  float s, e;
-  two_sum(a.hi, b, s, e);
-  e = __fadd_rn(e, a.lo);
+// s += a 2^-8U for one group of the sum over u of a_u 2^-8u, in the order
+// u = 6, 5, 4, 0, 1, 2, 3.  The a_u are integers of at most 2^24 in magnitude.
+// Groups 4-6 add up in float (rounding error below 2^-32 of the unit of group
+// 0).  In groups 1-3 s.hi is a multiple of 2^-8(U-1) and so of ulp(a 2^-8U),
+// which makes the three-operation sum exact without an ordering by magnitude.
+template <int U>
+__device__ __forceinline__ void fold_group(df &s, float a) {
+  constexpr float w = 1.f / (float)((uint64_t)1 << (8 * U));
+  if (U == 6)
+    s.lo = __fmul_rn(a, w);
+  else if (U >= 4)
+    s.lo = __fmaf_rn(a, w, s.lo);
+  else if (U == 0)
+    s.hi = a;
+  else {
+    const float h = __fmaf_rn(a, w, s.hi);
+    s.lo = __fadd_rn(s.lo, __fmaf_rn(a, w, __fsub_rn(s.hi, h)));
+    s.hi = h;
+  }
+}
+__device__ __forceinline__ df fold_done(df s) {
   df r;
-  fast_two_sum(s, e, r.hi, r.lo);
+  two_sum(s.hi, s.lo, r.hi, r.lo);
   return r;
 }
-
-// sum_u acc[u] 2^-8u in double-float.  acc[u] are integers below 2^24; the
-// three smallest groups are summed in float (rounding error below 2^-32 of
-// the unit of acc[0]), the rest with error-free additions.
+// all groups at once
 __device__ __forceinline__ df combine7(const float *acc) {
-  float t = __fmul_rn(acc[6], 0x1p-48f);
-  t = __fmaf_rn(acc[5], 0x1p-40f, t);
-  t = __fmaf_rn(acc[4], 0x1p-32f, t);
-  df s{acc[0], 0.f};
-  s = df_add_f(s, __fmul_rn(acc[1], 0x1p-8f));
-  s = df_add_f(s, __fmul_rn(acc[2], 0x1p-16f));
-  s = df_add_f(s, __fmul_rn(acc[3], 0x1p-24f));
-  s = df_add_f(s, t);
-  return s;
+  df s;
+  fold_group<6>(s, acc[6]);
+  fold_group<5>(s, acc[5]);
+  fold_group<4>(s, acc[4]);
+  fold_group<0>(s, acc[0]);
+  fold_group<1>(s, acc[1]);
+  fold_group<2>(s, acc[2]);
+  fold_group<3>(s, acc[3]);
+  return fold_done(s);
 }
 
 // MMAs of one column block: re acc pairs row k-step j with column k-step j,
@@ -181,7 +190,7 @@ struct TcOperand {
   int es, eo;
 };
 // C(rbase + r, cbase + c) -= sum_p X_p(r, :) Y_p(c, :)^H over the tiles of
-// 128 rows x 32 columns of rows [0, nrows_b) and columns [0, ncols_b): all of
+// 128 rows x 64 columns of rows [0, nrows_b) and columns [0, ncols_b): all of
 // them, or (tri) the lower triangle of a square trailing block.
 struct TcUpdate {
   zdf *C;
@@ -189,6 +198,7 @@ struct TcUpdate {
   int rbase, cbase;
   int ncols_fixed;  // columns: ncols_fixed, or n_b - cbase when 0; rows: n_b - rbase
   int tri, nprod;
+  int cbs;  // column blocks per CTA
   TcOperand x[2], y[2];
   // test hook (pp_debug_stall_tc_wait): matrix stall_b's first CTA waits,
   // before its first row-operand wait, on an mbarrier that nothing arrives
@@ -196,177 +206,303 @@ struct TcUpdate {
   int stall_b;
   long long stall_cycles;
 };
+// CTA = 128 rows x up to cbs column blocks of 64, both products in turn.  One
+// warp issues the MMAs, one copies, 16 fold:
+//  * the seven groups of equal slice-index sum are formed one after the other,
+//    each in one of two tensor-memory buffers (64 real + 64 imaginary columns),
+//    so that the MMAs of the next groups, and of the next column block, run
+//    while the warps add a finished group to their double-float sums (a
+//    thread: one row, 16 columns).  Order 6, 5, 4, 0, 1, 2, 3 (fold_group):
+//    long groups first, so that the end of a tile runs under them;
+//  * the row operand goes through the column buffers to tensor memory once per
+//    product (tcgen05.cp), which halves the shared-memory reads of an MMA:
+//    32.4 cycles per 128 x 64 x 16 against 48.5 with both operands in shared
+//    memory (the tensor cores' own rate: 32);
+//  * the tile of C arrives in shared memory (cp.async, a thread's own elements)
+//    during the MMAs.
+// Per tile and product: 7.2k cycles of MMA, 8k of fold, 6.5k for the update of
+// C, of which the last two are not overlapped: L2 traffic (256 KB of C, 56 KB
+// of operand) and the fold's issue slots bound it now.  The earlier kernel (128
+// x 32 tiles, all 14 accumulators at once, MMAs issued by lane 0, then the
+// fold): n = 4764, 8 matrices, 196 ms of trailing updates and 78 ms of X -= V Y;
+// now 95 and 43 ms.  (Four accumulator buffers and the row operand in shared
+// memory: 167 and 68, of which the issue by lane 0 cost 62 and 26.)
+constexpr int CU_N = 64;                            // columns of a block
+constexpr int CU_BB = TC_S * TC_KS * CU_N * 32;     // its operand (57344 bytes)
+constexpr int CU_EW = 16;                           // folding warps
+constexpr int CU_NT = 32 * CU_EW + 128;             // and the issuing warpgroup (one warp works)
+constexpr int CU_Q = CU_N / (CU_EW / 4);            // columns per thread (16)
+constexpr int CU_ACC = 2;                           // accumulator buffers
+constexpr int CU_TA = CU_ACC * 2 * CU_N;            // tensor-memory column of the row operand
+constexpr int CU_CS = 14;                           // its columns of C staged in shared memory
+constexpr int CU_STC = CU_CS * 32 * CU_EW * 16;     // (114688 bytes)
+constexpr int CU_SMEM = TC_OP + CU_STC + 256;
+static_assert(2 * CU_BB == TC_OP, "the row operand passes through the column buffers");
+constexpr uint32_t CU_ID = tc::idesc_bf16(128, CU_N, 0);
+constexpr uint32_t CU_IDN = tc::idesc_bf16(128, CU_N, 1);
+static_assert(CU_TA + TC_S * TC_KS * 8 <= 512, "accumulators and row operand exceed tensor memory");
 
-__global__ void __launch_bounds__(TC_NT, 1) k_cupd_tc(TcUpdate u, const int *nvec, int *err) {
+// Wait for a phase, giving up after `cycles` SM clocks or when another warp of
+// the CTA has given up.
+__device__ __forceinline__ bool wait_phase(uint64_t *bar, uint32_t parity, volatile int *abort,
+                                           long long cycles = 1000000000LL) {
+  const long long t0 = clock64();
+  while (!tc::mbar_try(bar, parity)) {
+    if (*abort || clock64() - t0 > cycles) return false;
+  }
+  return true;
+}
+
+// MMAs of the group u: re acc pairs row k-step j with column k-step j, im acc
+// with column k-step j ^ 2, negated for j < 2 (Re X . Im Y).  A descriptor
+// differs from the operand's first only in its start address (bits 0-13, in
+// 16-byte units).
+template <int U>
+__device__ __forceinline__ void cu_issue(uint32_t tm, uint32_t ta, uint64_t b0) {
+#pragma unroll
+  for (int s = 0; s <= U; ++s) {
+    const int t = U - s;
+#pragma unroll
+    for (int j = 0; j < TC_KS; ++j) {
+      const uint32_t acc = (s == 0 && j == 0) ? 0u : 1u;
+      const uint32_t ad = ta + (s * TC_KS + j) * 8;
+      const uint64_t br = b0 + (uint64_t)((t * TC_KS + j) * (CU_N * 32 >> 4));
+      const uint64_t bi = b0 + (uint64_t)((t * TC_KS + (j ^ 2)) * (CU_N * 32 >> 4));
+      tc::mma_bf16_ta(tm, ad, br, CU_ID, acc);
+      tc::mma_bf16_ta(tm + CU_N, ad, bi, j < 2 ? CU_IDN : CU_ID, acc);
+    }
+  }
+}
+
+__device__ __forceinline__ void cp_async16(void *dst, const void *src, bool valid) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+
+struct CuBars {
+  uint64_t row, row_free, col[2], col_free[2], acc[CU_ACC], acc_free[CU_ACC], never, drain;
+  uint32_t tmem;
+  int abort;
+};
+static_assert(sizeof(CuBars) <= 256, "barriers fit the shared memory set aside");
+
+__global__ void __launch_bounds__(CU_NT, 1) k_cupd_tc(TcUpdate u, const int *nvec, int *err) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  uint8_t *sAop = smem;                                  // row operand
-  uint8_t *sBop = smem + TC_OP;                          // two column-operand buffers
-  int *sEc = (int *)(smem + TC_OP + 2 * TC_BBYTES);      // two x 64 column exponents
-  // mbarriers: [0] row operand landed (waited by thread 0), [1], [2] column
-  // buffer 0 / 1 landed, [3] MMAs of the block done, [4] never arrived on
-  // (the test hook's wait).
-  // Each barrier a thread waits on completes exactly once between two of
-  // its waits, so parity waits cannot skip a phase.
-  uint64_t *bars = (uint64_t *)(smem + TC_OP + 2 * TC_BBYTES + 512);
-  uint32_t *tslot = (uint32_t *)(bars + 5);
+  uint8_t *sBop = smem;                // two column-operand buffers
+  zdf *stC = (zdf *)(smem + TC_OP);    // tile of C: 16 B per fold thread and column
+  CuBars &bar = *(CuBars *)(smem + TC_OP + CU_STC);
   const int b = blockIdx.z, R = blockIdx.y, q = blockIdx.x;
   const int n = nvec[b];
   const int nrows = n - u.rbase;
   const int ncols = u.ncols_fixed > 0 ? u.ncols_fixed : n - u.cbase;
   if (nrows <= 0 || ncols <= 0) return;
-  const int nrb = (nrows + 127) / 128, ncb = (ncols + 31) / 32;
+  const int nrb = (nrows + 127) / 128, ncb = (ncols + CU_N - 1) / CU_N;
   if (R >= nrb) return;
-  const int cb_beg = q * TC_CB;
-  int cb_end = min(cb_beg + TC_CB, ncb);
-  if (u.tri) cb_end = min(cb_end, 4 * (R + 1));
+  const int cb_beg = q * u.cbs;
+  int cb_end = min(cb_beg + u.cbs, ncb);
+  if (u.tri) cb_end = min(cb_end, 128 / CU_N * (R + 1));
   if (cb_beg >= cb_end) return;
   // an earlier wait of this matrix gave up: its results are already invalid
   if (*(volatile int *)&err[b]) return;
   const int ncbw = cb_end - cb_beg;
   const int nblk = u.nprod * ncbw;  // (product, column block) steps
 
-  const int tid = threadIdx.x, warp = tid >> 5;
-  if (warp == 0) tc::tmem_alloc(tslot, 512);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (warp == CU_EW) tc::tmem_alloc(&bar.tmem, 512);
   if (tid == 0) {
-    for (int i = 0; i < 5; ++i) tc::mbar_init(&bars[i], 1);
+    tc::mbar_init(&bar.row, 1);
+    tc::mbar_init(&bar.row_free, 1);
+    for (int k = 0; k < 2; ++k) {
+      tc::mbar_init(&bar.col[k], 1);
+      tc::mbar_init(&bar.col_free[k], 1);
+    }
+    for (int k = 0; k < CU_ACC; ++k) {
+      tc::mbar_init(&bar.acc[k], 1);
+      tc::mbar_init(&bar.acc_free[k], CU_EW);
+    }
+    tc::mbar_init(&bar.never, 1);
+    tc::mbar_init(&bar.drain, 1);
+    bar.abort = 0;
     tc::mbar_init_fence();
   }
   tc::fence_before();
   __syncthreads();
   tc::fence_after();
-  const uint32_t tm = *tslot;
-  const bool stall = b == u.stall_b && R == 0 && q == 0;
-  zdf *C = u.C + b * u.sC;
-  const int r0 = u.rbase + 128 * R;  // first global row of this row block
-  const int nr = min(128, nrows - 128 * R);
-  // column operand of step i (product i / ncbw, column block cb)
-  auto issue_cols = [&](int i) {
-    const TcOperand &y = u.y[i / ncbw];
-    const int cb = cb_beg + i % ncbw;
-    const int buf = i & 1;
-    uint64_t *bar = &bars[1 + buf];
-    const uint32_t ebytes = 32u * 4u * (uint32_t)y.es;
-    tc::mbar_expect_tx(bar, TC_BBYTES + ebytes);
-    const uint8_t *src = y.S + b * y.sS + (int64_t)(cb >> 2) * y.blk + (cb & 3) * 1024;
-    uint8_t *dst = sBop + buf * TC_BBYTES;
-    for (int sj = 0; sj < TC_S * TC_KS; ++sj) tc::bulk_g2s(dst + sj * 1024, src + sj * TC_TILE, 1024, bar);
-    tc::bulk_g2s(sEc + buf * 64, y.E + b * y.sE + (int64_t)32 * cb * y.es, ebytes, bar);
-  };
-  const int lg = warp & 3, cqt = warp >> 2;
-  const int rl = 128 * R + 32 * lg + (tid & 31);  // row within the block of rows = TMEM lane
-  const int r = u.rbase + rl;
-  int erow[2] = {0, 0};
-  for (int p = 0; p < u.nprod; ++p) erow[p] = u.x[p].E[b * u.x[p].sE + (int64_t)rl * u.x[p].es + u.x[p].eo];
-  const uint32_t lane_addr = tm + ((uint32_t)(32 * lg) << 16) + TC_CQ * cqt;
-  const uint32_t sa = tc::smem_u32(sAop);
-  int ok = 1, failed_i = -1;
-  for (int i = 0; i < nblk; ++i) {
-    const int p = i / ncbw, cb = cb_beg + i % ncbw;
-    const uint32_t par3 = (uint32_t)(i & 1);
-    bool good = true;  // thread 0: every copy landed and every MMA was issued
-    if (tid == 0) {
-      if (i % ncbw == 0) {
-        // row operand of product p (the previous product's MMAs are done)
-        const TcOperand &x = u.x[p];
-        tc::mbar_expect_tx(&bars[0], TC_OP);
-        const uint8_t *src = x.S + b * x.sS + (int64_t)R * x.blk;
-        for (int s = 0; s < TC_S; ++s)
-          tc::bulk_g2s(sAop + s * (TC_KS * TC_TILE), src + s * (TC_KS * TC_TILE), TC_KS * TC_TILE, &bars[0]);
-      }
-      if (i == 0) issue_cols(0);
-      if (i + 1 < nblk) issue_cols(i + 1);
-      if (p == 0 && i + 1 < ncbw) {  // the next tile of C towards L2
-        const int c0 = u.cbase + 32 * (cb + 1);
-        for (int c = c0; c < min(c0 + 32, u.cbase + ncols); ++c)
-          tc::prefetch_l2(C + r0 + u.ldc * c, (uint32_t)nr * 16u);
-      }
-      if (i == 0 && stall) good = tc::mbar_wait(&bars[4], 0u, u.stall_cycles);
-      if (i % ncbw == 0) good = good && tc::mbar_wait(&bars[0], (uint32_t)p);
-      good = good && tc::mbar_wait(&bars[1 + (i & 1)], (uint32_t)((i >> 1) & 1));
-      if (good) {
-        tc::fence_after();
-        tc_issue(tm, sa, tc::smem_u32(sBop + (i & 1) * TC_BBYTES));
-      }
-      tc::mma_commit(&bars[3]);
-      if (!good) atomicExch(&err[b], 1);
-    }
-    // this thread's entries of C, loaded while the MMAs run
-    zdf cv[TC_CQ];
-    const int cl0 = 32 * cb + TC_CQ * cqt;  // first column (local) of this thread
-#pragma unroll
-    for (int qq = 0; qq < TC_CQ; ++qq) {
-      const int cl = cl0 + qq, c = u.cbase + cl;
-      if (rl < nrows && cl < ncols && (!u.tri || r >= c)) cv[qq] = C[r + u.ldc * c];
-    }
-    bool done = tc::mbar_wait(&bars[3], par3);
-    // (already complete: makes the copied column exponents visible here)
-    done = done && tc::mbar_wait(&bars[1 + (i & 1)], (uint32_t)((i >> 1) & 1));
-    ok = __syncthreads_and(done && ok && good);
-    if (!ok) {
-      failed_i = i;
-      break;
-    }
-    tc::fence_after();
-    const int er = erow[p];
-    const TcOperand &y = u.y[p];
-    const int *ec = sEc + (i & 1) * 64;
-#pragma unroll
-    for (int cc = 0; cc < TC_CQ / 4; ++cc) {
-      float are[TC_S][4], aim[TC_S][4];
-#pragma unroll
-      for (int uu = 0; uu < TC_S; ++uu) {
-        tc::tmem_ld4(lane_addr + uu * 32 + cc * 4, are[uu]);
-        tc::tmem_ld4(lane_addr + (TC_S + uu) * 32 + cc * 4, aim[uu]);
-      }
-      tc::tmem_ld_wait();
-#pragma unroll
-      for (int qq = 0; qq < 4; ++qq) {
-        const int q16 = 4 * cc + qq;
-        const int cl = cl0 + q16, c = u.cbase + cl;
-        if (rl < nrows && cl < ncols && (!u.tri || r >= c)) {
-          float vr[TC_S], vi[TC_S];
-#pragma unroll
-          for (int uu = 0; uu < TC_S; ++uu) {
-            vr[uu] = are[uu][qq];
-            vi[uu] = aim[uu][qq];
+  const uint32_t tm = __shfl_sync(0xffffffffu, bar.tmem, 0);
+  volatile int *abort = &bar.abort;
+  // launched with 96 registers a thread (61440): 512 x 104 + 128 x 56 = 60416
+  if (warp >= CU_EW) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    const bool one = tc::elect_one();
+    bool ok = true;
+    auto wait = [&](uint64_t *w, int phase, long long cycles = 1000000000LL) {
+      ok = __all_sync(0xffffffffu, ok && wait_phase(w, (uint32_t)(phase & 1), abort, cycles));
+    };
+    if (warp == CU_EW) {
+      // ---- MMAs
+      const uint64_t a0 = tc::sdesc(tc::smem_u32(sBop), 128, 256);
+      if (b == u.stall_b && R == 0 && q == 0) wait(&bar.never, 0, u.stall_cycles);
+      for (int i = 0; i < nblk && ok; ++i) {
+        const int buf = i & 1;
+        if (i % ncbw == 0) {  // (the last product's MMAs have ended: the copy waited for them)
+          wait(&bar.row, i / ncbw);
+          if (!ok) break;
+          tc::fence_after();
+          if (one) {
+            for (int sj = 0; sj < TC_S * TC_KS; ++sj)
+              tc::tmem_cp_kstep(tm + CU_TA + sj * 8, a0 + (uint64_t)(sj * (TC_TILE >> 4)));
+            tc::mma_commit(&bar.row_free);
           }
-          const int ecol = ec[(TC_CQ * cqt + q16) * y.es + y.eo];
-          const float sc = pow2f(er + ecol - 16);
-          df pr = combine7(vr), pi = combine7(vi);
-          pr.hi = __fmul_rn(pr.hi, sc);
-          pr.lo = __fmul_rn(pr.lo, sc);
-          pi.hi = __fmul_rn(pi.hi, sc);
-          pi.lo = __fmul_rn(pi.lo, sc);
-          zdf a = cv[q16];
-          a.re = df_sub(a.re, pr);
-          a.im = df_sub(a.im, pi);
-          C[r + u.ldc * c] = a;
+          __syncwarp();
         }
+        wait(&bar.col[buf], i >> 1);
+        const uint64_t b0 = tc::sdesc(tc::smem_u32(sBop + buf * CU_BB), 128, 256);
+        int g = i * TC_S;
+        auto group = [&](auto issue) {
+          const int slot = g & (CU_ACC - 1);
+          if (g >= CU_ACC) wait(&bar.acc_free[slot], g / CU_ACC - 1);
+          tc::fence_after();
+          if (ok && one) {
+            issue(tm + slot * (2 * CU_N));
+            tc::mma_commit(&bar.acc[slot]);
+          }
+          __syncwarp();
+          ++g;
+        };
+        group([&](uint32_t d) { cu_issue<6>(d, tm + CU_TA, b0); });
+        group([&](uint32_t d) { cu_issue<5>(d, tm + CU_TA, b0); });
+        group([&](uint32_t d) { cu_issue<4>(d, tm + CU_TA, b0); });
+        group([&](uint32_t d) { cu_issue<0>(d, tm + CU_TA, b0); });
+        group([&](uint32_t d) { cu_issue<1>(d, tm + CU_TA, b0); });
+        group([&](uint32_t d) { cu_issue<2>(d, tm + CU_TA, b0); });
+        group([&](uint32_t d) { cu_issue<3>(d, tm + CU_TA, b0); });
+        if (ok && one) tc::mma_commit(&bar.col_free[buf]);
+        __syncwarp();
+      }
+      // every MMA has ended before the tensor memory is released
+      if (ok) wait(&bar.col_free[(nblk - 1) & 1], (nblk - 1) >> 1);
+      if (!ok) {
+        // give up: tell the other warps, then let the MMAs in flight finish
+        // (bounded) before the memory is released
+        if (one) {
+          *abort = 1;
+          atomicExch(&err[b], 1);
+          tc::mma_commit(&bar.drain);
+          tc::mbar_wait(&bar.drain, 0u, 200000000LL);
+        }
+        __syncwarp();
+      }
+    } else if (warp == CU_EW + 1) {
+      // ---- copies: the row operand through both column buffers, then its columns
+      int nrow = 0, ncol = 0;  // operands requested
+      auto copy_col = [&](int i) {  // column operand of step i (product i / ncbw)
+        if (one) {
+          const TcOperand &y = u.y[i / ncbw];
+          const int cb = cb_beg + i % ncbw, buf = i & 1;
+          tc::mbar_expect_tx(&bar.col[buf], CU_BB);
+          const uint8_t *src = y.S + b * y.sS + (int64_t)(cb / 2) * y.blk + (cb & 1) * (CU_N * 32);
+          for (int sj = 0; sj < TC_S * TC_KS; ++sj)
+            tc::bulk_g2s(sBop + buf * CU_BB + sj * (CU_N * 32), src + sj * TC_TILE, CU_N * 32, &bar.col[buf]);
+        }
+        ++ncol;
+      };
+      for (int i = 0; i < nblk && ok; ++i) {
+        const bool first = i % ncbw == 0, next = (i + 1) % ncbw != 0;
+        if (i > 0 && (first || next)) wait(&bar.col_free[(i - 1) & 1], (i - 1) >> 1);  // step i - 1's MMAs have ended
+        if (first && ok) {
+          if (one) {
+            const TcOperand &x = u.x[i / ncbw];
+            tc::mbar_expect_tx(&bar.row, TC_OP);
+            tc::bulk_g2s(sBop, x.S + b * x.sS + (int64_t)R * x.blk, TC_OP, &bar.row);
+          }
+          ++nrow;
+          wait(&bar.row_free, i / ncbw);
+          if (ok) copy_col(i);
+        }
+        if (next && ok) copy_col(i + 1);
+        __syncwarp();
+      }
+      // no copy may land after the block's end
+      if (nrow > 0) tc::mbar_wait(&bar.row, (uint32_t)((nrow - 1) & 1), 200000000LL);
+      for (int k = max(0, ncol - 2); k < ncol; ++k) tc::mbar_wait(&bar.col[k & 1], (uint32_t)((k >> 1) & 1), 200000000LL);
+    }
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+    // ---- fold: this thread's row (= TMEM lane) and CU_Q columns of each block
+    zdf *C = u.C + b * u.sC;
+    const int lg = warp & 3, c0q = (warp >> 2) * CU_Q;
+    const int rl = 128 * R + 32 * lg + lane;  // row within the block of rows
+    const int r = u.rbase + rl;
+    const uint32_t lane_addr = tm + ((uint32_t)(32 * lg) << 16) + c0q;
+    bool ok = true;
+    for (int i = 0; i < nblk && ok; ++i) {
+      const int p = i / ncbw, cb = cb_beg + i % ncbw;
+      const int cl0 = CU_N * cb + c0q;  // first column (local) of this thread
+      zdf *Cr = C + r + u.ldc * (u.cbase + cl0);
+      const int left = rl < nrows ? min(ncols, u.tri ? r - u.cbase + 1 : ncols) - cl0 : 0;  // columns of this thread
+      if (p > 0 && i % ncbw == 0) __threadfence();  // the previous product's sums are read back below
+#pragma unroll
+      for (int k = 0; k < CU_CS; ++k)
+        if (k < left) cp_async16(&stC[k * (32 * CU_EW) + tid], Cr + u.ldc * k, true);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      const TcOperand &x = u.x[p], &y = u.y[p];
+      const int er = x.E[b * x.sE + (int64_t)rl * x.es + x.eo] - 16;
+      const int ecl = y.E[b * y.sE + (int64_t)(cl0 + (lane & (CU_Q - 1))) * y.es + y.eo];  // of column lane & 15
+      df sr[CU_Q], si[CU_Q];
+      int g = i * TC_S;
+      auto fold = [&](auto add) {
+        const int slot = g & (CU_ACC - 1);
+        ok = __all_sync(0xffffffffu, ok && wait_phase(&bar.acc[slot], (uint32_t)((g / CU_ACC) & 1), abort));
+        if (ok) {
+          tc::fence_after();
+#pragma unroll
+          for (int c4 = 0; c4 < CU_Q; c4 += 4) {
+            float re[4], im[4];
+            tc::tmem_ld4(lane_addr + slot * (2 * CU_N) + c4, re);
+            tc::tmem_ld4(lane_addr + slot * (2 * CU_N) + CU_N + c4, im);
+            tc::tmem_ld_wait();
+#pragma unroll
+            for (int k = 0; k < 4; ++k) add(c4 + k, re[k], im[k]);
+          }
+          tc::fence_before();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(&bar.acc_free[slot]);
+        }
+        ++g;
+      };
+      fold([&](int k, float x, float y) { fold_group<6>(sr[k], x); fold_group<6>(si[k], y); });
+      fold([&](int k, float x, float y) { fold_group<5>(sr[k], x); fold_group<5>(si[k], y); });
+      fold([&](int k, float x, float y) { fold_group<4>(sr[k], x); fold_group<4>(si[k], y); });
+      fold([&](int k, float x, float y) { fold_group<0>(sr[k], x); fold_group<0>(si[k], y); });
+      fold([&](int k, float x, float y) { fold_group<1>(sr[k], x); fold_group<1>(si[k], y); });
+      fold([&](int k, float x, float y) { fold_group<2>(sr[k], x); fold_group<2>(si[k], y); });
+      fold([&](int k, float x, float y) { fold_group<3>(sr[k], x); fold_group<3>(si[k], y); });
+      if (!ok) break;
+      zdf cd[CU_Q - CU_CS];
+#pragma unroll
+      for (int k = CU_CS; k < CU_Q; ++k)
+        if (k < left) cd[k - CU_CS] = Cr[u.ldc * k];
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+      for (int k = 0; k < CU_Q; ++k) {
+        const float sc = pow2f(er + __shfl_sync(0xffffffffu, ecl, k));
+        if (k >= left) continue;
+        const zdf cv = k < CU_CS ? stC[k * (32 * CU_EW) + tid] : cd[max(k - CU_CS, 0)];
+        const df pr = fold_done(sr[k]), pi = fold_done(si[k]);
+        Cr[u.ldc * k] = zdf{df_sub(cv.re, df{__fmul_rn(pr.hi, sc), __fmul_rn(pr.lo, sc)}),
+                            df_sub(cv.im, df{__fmul_rn(pi.hi, sc), __fmul_rn(pi.lo, sc)})};
       }
     }
-    tc::fence_before();
-    __syncthreads();
-    tc::fence_after();
-  }
-  if (!ok) {
-    // let the copies and MMAs still in flight finish (bounded waits) before
-    // the shared and tensor memory are released: the row operand of the
-    // failed step's product, the failed step's MMAs and column copy, and the
-    // column copy issued for the step after it
-    if (tid == 0 && failed_i >= 0) {
-      const int fp = failed_i / ncbw;
-      tc::mbar_wait(&bars[0], (uint32_t)(fp & 1), 200000000LL);
-      tc::mbar_wait(&bars[3], (uint32_t)(failed_i & 1), 200000000LL);
-      tc::mbar_wait(&bars[1 + (failed_i & 1)], (uint32_t)((failed_i >> 1) & 1), 200000000LL);
-      const int nx = failed_i + 1;
-      if (nx < nblk) tc::mbar_wait(&bars[1 + (nx & 1)], (uint32_t)((nx >> 1) & 1), 200000000LL);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (!ok && lane == 0) {
+      *abort = 1;
+      atomicExch(&err[b], 1);
     }
-    if (tid == 0) atomicExch(&err[b], 1);
-    tc::fence_before();
-    __syncthreads();
-    tc::fence_after();
   }
-  if (warp == 0) tc::tmem_dealloc(tm, 512);
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+  if (warp == CU_EW) tc::tmem_dealloc(tm, 512);
 }
 
 // Long-K products on the tensor cores over column-major DF matrices read
@@ -409,10 +545,6 @@ constexpr int VX_LD = 33;              // staging row stride (16-byte elements)
 constexpr int VX_STX = 128 * VX_LD * 16;
 constexpr int VX_STV = 32 * VX_LD * 16;
 constexpr int VX_SMEM = TC_OP + TC_BBYTES + VX_STX + VX_STV + 128 * 4 + 32 * 4 + 64;
-__device__ __forceinline__ void cp_async16(void *dst, const void *src, bool valid) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(valid ? 16 : 0) : "memory");
-}
 
 // Slices of one k-step (16 reals) of an operand row staged in shared memory
 // (strow[r], r < 32: the real parts are K = r, the imaginary parts K = 32 + r),
@@ -543,7 +675,7 @@ __global__ void __launch_bounds__(TC_NT, 1) k_longk_tc(LongK p, const int *nvec,
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
-    tm = *tslot;
+    tm = __shfl_sync(0xffffffffu, *tslot, 0);
   }
   const zdf *A = p.A + b * p.sA;
   const zdf *Bm = p.Bm + b * p.sB;
@@ -598,12 +730,15 @@ __global__ void __launch_bounds__(TC_NT, 1) k_longk_tc(LongK p, const int *nvec,
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
-    if (tid == 0) {
-      if (p.real_a)
-        tc_issue_reala(tm, tc::smem_u32(sAop), tc::smem_u32(sBop));
-      else
-        tc_issue(tm, tc::smem_u32(sAop), tc::smem_u32(sBop));
-      tc::mma_commit(bar);
+    if (warp == 0) {
+      if (tc::elect_one()) {
+        if (p.real_a)
+          tc_issue_reala(tm, tc::smem_u32(sAop), tc::smem_u32(sBop));
+        else
+          tc_issue(tm, tc::smem_u32(sAop), tc::smem_u32(sBop));
+        tc::mma_commit(bar);
+      }
+      __syncwarp();
     }
     if (kc + 1 < kc_end) load(kc + 1);  // in flight while the MMAs run
     const bool done = tc::mbar_wait(bar, (uint32_t)((kc - kc_beg) & 1));
@@ -699,7 +834,7 @@ cudaError_t prepare_her2k_tc() {
   const int dev = device_index();
   std::lock_guard<std::mutex> g(mu);
   if (dev >= 0 && done[dev]) return cudaSuccess;
-  cudaError_t e = cudaFuncSetAttribute(k_cupd_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM);
+  cudaError_t e = cudaFuncSetAttribute(k_cupd_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, CU_SMEM);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_longk_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, VX_SMEM);
   if (e == cudaSuccess && dev >= 0) done[dev] = true;
   return e;
@@ -743,6 +878,15 @@ static int take_stall(const EigWork &w, long long *cycles) {
   return b;
 }
 
+// Column blocks per CTA for `tiles` tiles of 128 x 64 per matrix: up to 4 (the
+// 112 KB row operand is fetched once per CTA and product), fewer while that
+// leaves SMs without a CTA.
+static int cu_blocks(int64_t tiles, int B) {
+  int k = 4;
+  while (k > 1 && tiles * B < (int64_t)k * device_sms()) k /= 2;
+  return k;
+}
+
 // A(k1:n, k1:n) -= V W^H + W V^H, lower triangle (panel k0 of width jb).
 cudaError_t her2k_tc(EigWork &w, int k0, int jb, cudaStream_t s) {
   const int k1 = k0 + jb;
@@ -771,8 +915,9 @@ cudaError_t her2k_tc(EigWork &w, int k0, int jb, cudaStream_t s) {
   u.y[1] = V;
   u.stall_b = take_stall(w, &u.stall_cycles);
   const int nrb = (mmax + 127) / 128;
-  const int nq = (4 * nrb + TC_CB - 1) / TC_CB;
-  PP_KT(KT_HER2K, s, (k_cupd_tc<<<dim3(nq, nrb, w.B), TC_NT, TC_SMEM, s>>>(u, w.nvec, w.tcErr)));
+  u.cbs = cu_blocks(nrb * (nrb + 1) / 2 * (128 / CU_N), w.B);
+  const int nq = (128 / CU_N * nrb + u.cbs - 1) / u.cbs;
+  PP_KT(KT_HER2K, s, (k_cupd_tc<<<dim3(nq, nrb, w.B), CU_NT, CU_SMEM, s>>>(u, w.nvec, w.tcErr)));
   count_launch(1);
   return cudaGetLastError();
 }
@@ -806,9 +951,10 @@ cudaError_t applyV_tc(EigWork &w, int k0, int jb, zdf *X, int64_t ldx, int64_t s
   u.y[0] = TcOperand{w.tcS + vbl, w.sTcS, TC_OP, w.tcE + yexp, w.sTcE, 1, 0};
   u.x[1] = u.x[0];
   u.y[1] = u.y[0];
-  const int nrb = (mmax + 127) / 128;
-  const int nq = ((ncols + 31) / 32 + TC_CB - 1) / TC_CB;
-  PP_KT(KT_APPLYV, s, (k_cupd_tc<<<dim3(nq, nrb, w.B), TC_NT, TC_SMEM, s>>>(u, w.nvec, w.tcErr)));
+  const int nrb = (mmax + 127) / 128, ncb = (ncols + CU_N - 1) / CU_N;
+  u.cbs = cu_blocks(nrb * ncb, w.B);
+  const int nq = (ncb + u.cbs - 1) / u.cbs;
+  PP_KT(KT_APPLYV, s, (k_cupd_tc<<<dim3(nq, nrb, w.B), CU_NT, CU_SMEM, s>>>(u, w.nvec, w.tcErr)));
   count_launch(1);
   return cudaGetLastError();
 }
