@@ -29,6 +29,7 @@
 #include <cstdlib>
 #include <mutex>
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
 #include "pp_internal.cuh"
 #include "pp_tc.cuh"
@@ -42,14 +43,6 @@ constexpr int TC_KS = 4;                         // k-steps of 16 (K = 64 reals)
 constexpr int TC_TILE = 4096;                    // one (slice, k-step) tile of 128 rows
 constexpr int TC_OP = TC_S * TC_KS * TC_TILE;    // one operand of a 128-row block (114688)
 constexpr int TC_RBLK = 2 * TC_OP;               // V and W operands of a 128-row block
-constexpr int TC_BBYTES = TC_S * TC_KS * 1024;   // 32 rows of one operand (28672): the long-K kernel's column operand
-constexpr int TC_NT = 512;                       // threads of the long-K kernel: 16 warps = 4 lane groups x 4 column quarters
-constexpr int TC_CQ = 32 / (TC_NT / 128);        // columns per thread in its fold (8)
-constexpr int TC_NACC = 2 * TC_S;                // accumulators: (re, im) x slice-sum group
-constexpr uint32_t TC_ID = tc::idesc_bf16(128, 32, 0);
-constexpr uint32_t TC_IDN = tc::idesc_bf16(128, 32, 1);
-static_assert(TC_NACC * 32 <= 512, "accumulators exceed tensor memory");
-static_assert(TC_NT == 4 * 128, "long-K slicing maps one thread to each (row, k-step) of 128 rows");
 
 // 2^e as a float (exact for -126 <= e <= 127)
 __device__ __forceinline__ float pow2f(int e) {
@@ -142,43 +135,6 @@ __device__ __forceinline__ df fold_done(df s) {
   two_sum(s.hi, s.lo, r.hi, r.lo);
   return r;
 }
-// all groups at once
-__device__ __forceinline__ df combine7(const float *acc) {
-  df s;
-  fold_group<6>(s, acc[6]);
-  fold_group<5>(s, acc[5]);
-  fold_group<4>(s, acc[4]);
-  fold_group<0>(s, acc[0]);
-  fold_group<1>(s, acc[1]);
-  fold_group<2>(s, acc[2]);
-  fold_group<3>(s, acc[3]);
-  return fold_done(s);
-}
-
-// MMAs of one column block: re acc pairs row k-step j with column k-step j,
-// im acc with column k-step j ^ 2, negated for j < 2 (Re X . Im Y).  Fully
-// unrolled: a descriptor differs from the block's first only in its start
-// address (bits 0-13, in 16-byte units), so each MMA costs one add.
-__device__ __forceinline__ void tc_issue(uint32_t tm, uint32_t sa, uint32_t sb) {
-  const uint64_t a0 = tc::sdesc(sa, 128, 256), b0 = tc::sdesc(sb, 128, 256);
-#pragma unroll
-  for (int u = 0; u < TC_S; ++u) {
-#pragma unroll
-    for (int s = 0; s <= u; ++s) {
-      const int t = u - s;
-#pragma unroll
-      for (int j = 0; j < TC_KS; ++j) {
-        const uint32_t acc = (s == 0 && j == 0) ? 0u : 1u;
-        const uint64_t ad = a0 + (uint64_t)((s * TC_KS + j) * (TC_TILE >> 4));
-        const uint64_t br = b0 + (uint64_t)((t * TC_KS + j) * (1024 >> 4));
-        const uint64_t bi = b0 + (uint64_t)((t * TC_KS + (j ^ 2)) * (1024 >> 4));
-        tc::mma_bf16(tm + u * 32, ad, br, TC_ID, acc);
-        tc::mma_bf16(tm + (TC_S + u) * 32, ad, bi, j < 2 ? TC_IDN : TC_ID, acc);
-      }
-    }
-  }
-}
-
 // One operand of a product C -= X Y^H: slices in 128-row blocks of TC_OP
 // bytes placed blk bytes apart (matrix b at S + b sS), and the exponent of
 // row r at E[b sE + r es + eo].
@@ -278,6 +234,10 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src, bool vali
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
+__device__ __forceinline__ void cp_async8(void *dst, const void *src, bool valid) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(valid ? 8 : 0) : "memory");
+}
 
 struct CuBars {
   uint64_t row, row_free, col[2], col_free[2], acc[CU_ACC], acc_free[CU_ACC], never, drain;
@@ -303,7 +263,7 @@ __global__ void __launch_bounds__(CU_NT, 1) k_cupd_tc(TcUpdate u, const int *nve
   if (u.tri) cb_end = min(cb_end, 128 / CU_N * (R + 1));
   if (cb_beg >= cb_end) return;
   // an earlier wait of this matrix gave up: its results are already invalid
-  if (*(volatile int *)&err[b]) return;
+  if (__syncthreads_or(*(volatile int *)&err[b])) return;
   const int ncbw = cb_end - cb_beg;
   const int nblk = u.nprod * ncbw;  // (product, column block) steps
 
@@ -506,307 +466,534 @@ __global__ void __launch_bounds__(CU_NT, 1) k_cupd_tc(TcUpdate u, const int *nve
 }
 
 // Long-K products on the tensor cores over column-major DF matrices read
-// row-wise: element (c, r) of A at A[r + lda c] (conjugated with conj_a),
-// element (j, r) of B at Bm[r + ldb j] (conjugated with conj_b, zero above a
-// Householder panel's unit diagonal with vmask).  A complex A gives
-// C(c, j) = sum_r A(c, r) conj(B(j, r)) (tc_issue forms the conjugate
-// product); a real A (real_a) gives C(c, j) = sum_r A(c, r) B(j, r).
-// Exact slice products need K <= 64 reals, so the rows r are taken in
-// chunks of 32: per chunk both operands are sliced in
-// shared memory on the grid of the chunk, the MMAs accumulate in tensor
-// memory, and the 14 accumulators are folded into double-float registers;
-// the next chunk's rows are copied (cp.async) while the MMAs run.
-// CTA = 128 rows c x 32 rows j.
-//   mode 0 (V^H X of the back-transform): j = the 32 panel columns, the rows
-//     split over gridDim.y ranges, written to split-K slots of out
+// row-wise: element (c, r) of A at A[r + lda c], element (j, r) of B at
+// Bm[r + ldb j].
+//   mode 0 (V^H X of the back-transform): C(c, j) = sum_r A(c, r) conj(B(j, r)),
+//     j = the 32 panel columns (zero above the Householder unit diagonals), the
+//     rows split over gridDim.y ranges, written to split-K slots of out
 //     (out[(y 32 + j) ldo + c]);
-//   mode 1 (E_b = X^H Z): A = Z (real, rows c < m_b: the eigenvector
-//     index), B = X (conjugated, rows j < nrows_b: the boundary row),
-//     written to out[j + ldo c].  A real A operand needs only its two real
-//     k-steps sliced, so a chunk's slicing (128 x 2 + 32 x 4 k-steps) runs in
-//     one pass of the CTA's threads.
+//   mode 1 (E_b = X^H Z): A = Z (real, rows c < m_b: the eigenvector index),
+//     C(c, j) = sum_r A(c, r) conj(B(j, r)), B = X (rows j < nrows_b: the
+//     boundary row), written to out[j + ldo c].
+// Exact slice products need K <= 64 reals, so the rows r are taken in chunks:
+// 32 rows (re and im) in mode 0, 64 rows of the real A in mode 1.
 struct LongK {
   const zdf *A;
   int64_t lda, sA;
-  int conj_a, real_a;
   const zdf *Bm;
   int64_t ldb, sB;
-  int vmask, conj_b;
   int nrows_b;         // mode 1: valid B rows
-  int k0, jb;          // vmask: panel k0 of width jb
+  int k0, jb;          // mode 0: panel k0 of width jb
+  const uint8_t *S;    // mode 0: slices of B, LK_BOP bytes per chunk, and their exponents (32 per chunk)
+  int64_t sS;
+  const int *Ex;
+  int64_t sEx;
   int rbeg;            // rows [rbeg, n_b)
-  int ncols_a;         // rows c < ncols_a
+  int ncols_a;         // mode 0: rows c < ncols_a
   const int64_t *rng;  // mode 1: rows c < rng[8 b + 2]
   zdf *out;
   int64_t ldo, sO;
-  int mode;
 };
-constexpr int VX_LD = 33;              // staging row stride (16-byte elements)
-constexpr int VX_STX = 128 * VX_LD * 16;
-constexpr int VX_STV = 32 * VX_LD * 16;
-constexpr int VX_SMEM = TC_OP + TC_BBYTES + VX_STX + VX_STV + 128 * 4 + 32 * 4 + 64;
 
-// Slices of one k-step (16 reals) of an operand row staged in shared memory
-// (strow[r], r < 32: the real parts are K = r, the imaginary parts K = 32 + r),
-// on the same grid as slice_row.  The NKS threads of a row are adjacent lanes
-// (lane % NKS = k-step) and share the row's exponent E (largest magnitude
-// below 2^E).  Each digit is rounded onto its fixed grid without scaling:
-// m = (t + 1.5 2^(23-8(s+1))) - 1.5 2^(23-8(s+1)) is t rounded to a multiple
-// of 2^-8(s+1); t - m is exact, and is either 0 or at least ulp(t) > 2 |tl|,
-// so Fast2Sum keeps the residual pair exact and normalised.  Every thread
-// writes two 16-byte core-matrix rows per slice.
-template <int TILE, int NKS>
-__device__ __forceinline__ int slice_kstep(const zdf *strow, bool neg_im, uint8_t *blk, int row, int ks) {
-  const int part = ks >> 1, rb = (ks & 1) * 16;
-  float th[16], tl[16];
+// Digits of the long-K operands.  v = x 2^-E, |v| < 1/4, as the 56-bit integer
+// rint(2^56 v) + 0x80...80: byte 6 - s, less 128, is the digit m_s of
+//   v = sum_{s=0..6} 2^-8(s+1) m_s,  |m_s| <= 128,  residual below 2^-57.
+// Three exact extractions (24, 22 and 10 bits) by adding constants; the bits
+// of the three sums are the three integers up to constants.
+struct Fixed56 {
+  uint32_t lo, hi;
+};
+__device__ __forceinline__ Fixed56 to_fixed(float hi, float lo) {
+  constexpr float M0 = 0.75f, M1 = 1.5f * 0x1p-23f, M2 = 1.5f * 0x1p-33f;  // ulps 2^-24, 2^-46, 2^-56
+  constexpr uint64_t off = 0x0080808080808080ull - ((uint64_t)0x3f400000u << 32) - ((uint64_t)0x34400000u << 10) -
+                           0x2f400000u;
+  const float t0 = __fadd_rn(hi, M0);
+  float r = __fsub_rn(hi, __fsub_rn(t0, M0)), e;
+  fast_two_sum(r, lo, r, e);  // |r| >= |lo| or r = 0
+  const float t1 = __fadd_rn(r, M1);
+  r = __fadd_rn(__fsub_rn(r, __fsub_rn(t1, M1)), e);
+  const float t2 = __fadd_rn(r, M2);
+  const uint64_t n = (uint64_t)__float_as_uint(t1) * 1024u +
+                     (((uint64_t)__float_as_uint(t0) << 32) | __float_as_uint(t2)) + off;
+  return Fixed56{(uint32_t)n, (uint32_t)(n >> 32)};
+}
+// digit S of two numbers in half precision (low half: a): 1024 + byte by its
+// bits, less 1152 (exact).  bf16 has no room for an 8-bit byte below its
+// leading bit, and costs five instructions here instead of three.
+template <int S>
+__device__ __forceinline__ uint32_t digit2(Fixed56 a, Fixed56 b) {
+  constexpr uint32_t k = S <= 2 ? 2 - S : 6 - S;  // byte of the word
+  const uint32_t w = __byte_perm(S <= 2 ? a.hi : a.lo, S <= 2 ? b.hi : b.lo, (k + 4) << 8 | k);
+  const uint32_t x = (w & 0x00ff00ffu) | 0x64006400u;
+  const __half2 h = __hsub2(*(const __half2 *)&x, __half2{__ushort_as_half(0x6480), __ushort_as_half(0x6480)});
+  return *(const uint32_t *)&h;
+}
+
+// Exponent E of a row's grid from its largest magnitude (its elements are below
+// 2^(E-2)), and the scaling by 2^-E in up to two exact steps (2^-E exceeds the
+// float range for subnormal rows, e.g. the far tail of a localised
+// eigenvector).  A row with an infinity or NaN gets an exponent that makes every
+// product of it non-finite.
+constexpr int LK_NONFINITE = 1 << 20;
+__device__ __forceinline__ float max_abs(float m, float x) {  // NaN if one is
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(m), "f"(fabsf(x)));
+  return r;
+}
+__device__ __forceinline__ int grid_exp(float amax) {
+  if (!(amax <= FLT_MAX)) return LK_NONFINITE;
+  int E = 0;
+  if (amax > 0.f) frexpf(amax, &E);
+  return E + 2;
+}
+__device__ __forceinline__ float grid_scale(int E) { return E == LK_NONFINITE ? 0.f : pow2f(E < -100 ? -E - 100 : -E); }
+// x[0..N) to grid integers (warp-wide call)
+template <int N>
+__device__ __forceinline__ void to_fixed(const df *x, int E, bool neg, Fixed56 *f) {
+  const float sc = neg ? -grid_scale(E) : grid_scale(E);
+  if (__any_sync(0xffffffffu, E < -100)) {
+    const float pre = E < -100 ? 0x1p100f : 1.f;
+#pragma unroll
+    for (int t = 0; t < N; ++t)
+      f[t] = to_fixed(__fmul_rn(__fmul_rn(x[t].hi, pre), sc), __fmul_rn(__fmul_rn(x[t].lo, pre), sc));
+  } else {
+#pragma unroll
+    for (int t = 0; t < N; ++t) f[t] = to_fixed(__fmul_rn(x[t].hi, sc), __fmul_rn(x[t].lo, sc));
+  }
+}
+
+constexpr int LK_BOP = TC_S * TC_KS * 1024;  // 32 rows of one operand (28672 bytes)
+constexpr int LK_LD = 33;                    // staging row stride (16-byte elements)
+constexpr int LK_LDB = 65;                   // and of B in mode 1
+constexpr int LK_CW = 16;                    // computing warps
+constexpr int LK_LW = 3;                     // loading warps
+constexpr int LK_NT = 32 * (LK_CW + 1 + LK_LW);  // and the issuing one
+constexpr int LK_ACC = 4;                    // accumulator buffers of 64 columns
+constexpr int LK_TA = LK_ACC * 64;           // tensor-memory column of A
+constexpr uint32_t LK_ID = tc::idesc_f16(128, 32, 0);
+constexpr uint32_t LK_IDN = tc::idesc_f16(128, 32, 1);
+static_assert(LK_TA + TC_S * TC_KS * 8 <= 512, "accumulators and A exceed tensor memory");
+template <int MODE>
+constexpr int lk_smem() {
+  return (MODE ? 4 : 2) * LK_BOP + 128 * LK_LD * 16 + (MODE ? 32 * LK_LDB * 16 : 0) + 1024;
+}
+// Slices of the 32 panel columns for mode 0: chunk x (rows rbeg + 32 x ...) of
+// matrix y, once per panel instead of once per 128 rows of A.
+__global__ void __launch_bounds__(128) k_longk_bslice(LongK p, const int *nvec, uint8_t *S, int *Ex) {
+  __shared__ zdf st[32 * LK_LD];
+  const int b = blockIdx.y, n = nvec[b], tid = threadIdx.x, lane = tid & 31;
+  const int r0 = p.rbeg + 32 * blockIdx.x;
+  if (r0 >= n) return;
+  const int nj = min(p.jb, n - 1 - p.k0);
+  for (int j = tid >> 5; j < 32; j += 4) {
+    const int r = r0 + lane;
+    st[j * LK_LD + lane] = r < n && j < nj && r >= p.k0 + j + 1 ? p.Bm[b * p.sB + r + p.ldb * j]
+                                                                 : zdf{{0.f, 0.f}, {0.f, 0.f}};
+  }
+  __syncthreads();
+  const int j = tid >> 2, ks = tid & 3, part = ks >> 1, rb = 16 * (ks & 1);
+  df x[16];
   float amax = 0.f;
 #pragma unroll
   for (int t = 0; t < 16; ++t) {
-    const df v = ((const df *)&strow[rb + t])[part];
-    th[t] = v.hi;
-    tl[t] = v.lo;
-    amax = fmaxf(amax, fabsf(v.hi));
+    x[t] = ((const df *)&st[j * LK_LD + rb + t])[part];
+    amax = max_abs(amax, x[t].hi);
   }
-  amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-  if (NKS == 4) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-  int E = 0;
-  if (amax > 0.f) frexpf(amax, &E);
-  // 2^-E exceeds the float range when the largest magnitude is subnormal
-  // (E <= -128, e.g. the far tail of a localised eigenvector): such rows are
-  // scaled in two exact power-of-two steps
-  const int e1 = E < -100 ? 100 : 0;
-  const float sc = (part && neg_im) ? -pow2f(-E - e1) : pow2f(-E - e1);
-  if (e1) {
-#pragma unroll
-    for (int t = 0; t < 16; ++t) {
-      th[t] = __fmul_rn(th[t], 0x1p100f);
-      tl[t] = __fmul_rn(tl[t], 0x1p100f);
-    }
-  }
-#pragma unroll
-  for (int t = 0; t < 16; ++t) {
-    th[t] = __fmul_rn(th[t], sc);
-    tl[t] = __fmul_rn(tl[t], sc);
-  }
-  uint8_t *base = blk + ks * TILE + tc::core_off(row, 0);
-#pragma unroll
-  for (int sl = 0; sl < TC_S; ++sl) {
-    const float mag = 1.5f * (float)(1 << 15) * pow2f(-8 * sl);  // 1.5 2^(23 - 8(sl+1))
-    const float up = pow2f(8 * (sl + 1));
+  amax = max_abs(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+  amax = max_abs(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+  const int E = grid_exp(amax);
+  Fixed56 f[16];
+  to_fixed<16>(x, E, false, f);
+  uint8_t *dst = S + b * p.sS + (int64_t)blockIdx.x * LK_BOP + ks * 1024 + tc::core_off(j, 0);
+  auto put = [&](auto dig, int s) {
     uint32_t w[8];
 #pragma unroll
-    for (int t = 0; t < 16; t += 2) {
-      const float m0 = __fsub_rn(__fadd_rn(th[t], mag), mag);
-      const float m1 = __fsub_rn(__fadd_rn(th[t + 1], mag), mag);
-      fast_two_sum(__fsub_rn(th[t], m0), tl[t], th[t], tl[t]);
-      fast_two_sum(__fsub_rn(th[t + 1], m1), tl[t + 1], th[t + 1], tl[t + 1]);
-      const __nv_bfloat162 h = __floats2bfloat162_rn(__fmul_rn(m0, up), __fmul_rn(m1, up));
-      w[t >> 1] = *(const uint32_t *)&h;
-    }
-    uint8_t *dst = base + sl * TC_KS * TILE;
-    *(uint4 *)dst = make_uint4(w[0], w[1], w[2], w[3]);
-    *(uint4 *)(dst + 128) = make_uint4(w[4], w[5], w[6], w[7]);
-  }
-  return E;
+    for (int t = 0; t < 8; ++t) w[t] = dig(f[2 * t], f[2 * t + 1]);
+    *(uint4 *)(dst + s * TC_KS * 1024) = make_uint4(w[0], w[1], w[2], w[3]);
+    *(uint4 *)(dst + s * TC_KS * 1024 + 128) = make_uint4(w[4], w[5], w[6], w[7]);
+  };
+  put([](Fixed56 a, Fixed56 c) { return digit2<0>(a, c); }, 0);
+  put([](Fixed56 a, Fixed56 c) { return digit2<1>(a, c); }, 1);
+  put([](Fixed56 a, Fixed56 c) { return digit2<2>(a, c); }, 2);
+  put([](Fixed56 a, Fixed56 c) { return digit2<3>(a, c); }, 3);
+  put([](Fixed56 a, Fixed56 c) { return digit2<4>(a, c); }, 4);
+  put([](Fixed56 a, Fixed56 c) { return digit2<5>(a, c); }, 5);
+  put([](Fixed56 a, Fixed56 c) { return digit2<6>(a, c); }, 6);
+  if (ks == 0) Ex[b * p.sEx + 32 * (int)blockIdx.x + j] = E;
 }
 
-// tc_issue for a real row operand: re acc pairs row k-step j (j < 2) with
-// column k-step j, im acc the same row k-step with column k-step j + 2.
-__device__ __forceinline__ void tc_issue_reala(uint32_t tm, uint32_t sa, uint32_t sb) {
-  const uint64_t a0 = tc::sdesc(sa, 128, 256), b0 = tc::sdesc(sb, 128, 256);
+// MMAs of the group U.  Mode 0: as cu_issue, N = 32.  Mode 1: the real A's
+// k-step with the same k-step of Re B and of Im B (an operand each).
+template <int U, int MODE>
+__device__ __forceinline__ void lk_issue(uint32_t d, uint32_t ta, uint64_t b0) {
 #pragma unroll
-  for (int u = 0; u < TC_S; ++u) {
+  for (int s = 0; s <= U; ++s) {
+    const int t = U - s;
 #pragma unroll
-    for (int s = 0; s <= u; ++s) {
-      const int t = u - s;
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const uint32_t acc = (s == 0 && j == 0) ? 0u : 1u;
-        const uint64_t ar = a0 + (uint64_t)((s * TC_KS + j) * (TC_TILE >> 4));
-        const uint64_t br = b0 + (uint64_t)((t * TC_KS + j) * (1024 >> 4));
-        const uint64_t bi = b0 + (uint64_t)((t * TC_KS + j + 2) * (1024 >> 4));
-        tc::mma_bf16(tm + u * 32, ar, br, TC_ID, acc);
-        tc::mma_bf16(tm + (TC_S + u) * 32, ar, bi, TC_ID, acc);
-      }
+    for (int j = 0; j < TC_KS; ++j) {
+      const uint32_t acc = (s == 0 && j == 0) ? 0u : 1u;
+      const uint32_t ad = ta + (s * TC_KS + j) * 8;
+      const uint64_t br = b0 + (uint64_t)((t * TC_KS + j) * (1024 >> 4));
+      const uint64_t bi = b0 + (uint64_t)(MODE ? ((TC_S + t) * TC_KS + j) * (1024 >> 4) : (t * TC_KS + (j ^ 2)) * (1024 >> 4));
+      tc::mma_bf16_ta(d, ad, br, LK_ID, acc);
+      tc::mma_bf16_ta(d + 32, ad, bi, MODE == 0 && j < 2 ? LK_IDN : LK_ID, acc);
     }
   }
 }
 
-__global__ void __launch_bounds__(TC_NT, 1) k_longk_tc(LongK p, const int *nvec, int *err) {
+// s += a 2^-8U in the order 6, 5, ..., 0 (see fold_group): here s.hi is a
+// multiple of 2^-8(U+1) below 2^(24-8(U+1)), so that a 2^-8U is a multiple of
+// ulp(s.hi) and the three-operation sum is exact as well.
+template <int U>
+__device__ __forceinline__ void fold_up(df &s, float a) {
+  constexpr float w = 1.f / (float)((uint64_t)1 << (8 * U));
+  if (U == 6)
+    s.lo = __fmul_rn(a, w);
+  else if (U >= 4)
+    s.lo = __fmaf_rn(a, w, s.lo);
+  else if (U == 3)
+    s.hi = __fmul_rn(a, w);
+  else {
+    const float h = __fmaf_rn(a, w, s.hi);
+    s.lo = __fadd_rn(s.lo, __fsub_rn(s.hi, __fmaf_rn(a, -w, h)));
+    s.hi = h;
+  }
+}
+
+struct LkBars {
+  uint64_t b[2], done, a_ready, acc[LK_ACC], acc_free[LK_ACC], drain, st_full, st_free;
+  uint32_t tmem;
+  int abort;
+};
+static_assert(sizeof(LkBars) <= 128, "barriers fit the shared memory set aside");
+
+// CTA = 128 rows c x 32 columns j (re and im: 64 accumulator columns).  16
+// warps compute, one issues the MMAs, three load; per chunk, for the groups of
+// equal slice-index sum u = 6 ... 0: a computing warp adds the finished group
+// of chunk k to its double-float sums and then writes slice u of chunk k + 1 to
+// tensor memory (slice u of A is read by the groups >= u only, so it is free by
+// then).  The MMAs of chunk k + 1 run while the warps scale and add chunk k to
+// the result and cut the grid integers of chunk k + 2.  A thread has one row
+// c, 16 of its 64 reals of a chunk as 56-bit integers, and 8 columns j of the
+// sums.  Instruction issue bounds it: 1440 instructions per warp and chunk, 60%
+// of the issue slots (tensor cores 30%); 10.7k cycles per chunk in mode 0 and
+// 15k (twice the rows) in mode 1.  The earlier kernel cut the panel anew for
+// every 128 rows, with a float per digit, kept the slices of A in shared memory
+// and alternated slicing, MMAs and fold: 21.6k cycles per chunk.  n = 4764, 8
+// matrices: V^H X 94 -> 52 ms, X^H Z 80 -> 47 ms; n = 2604 with all vectors:
+// V^H X 29.7 -> 17.3 ms.
+template <int MODE>
+__global__ void __launch_bounds__(LK_NT, 1) k_longk_tc(LongK p, const int *nvec, int *err) {
+  constexpr int CR = MODE ? 64 : 32;  // rows r per chunk
+  constexpr int BOP = (MODE ? 2 : 1) * LK_BOP;
   extern __shared__ __align__(1024) uint8_t smem[];
-  uint8_t *sAop = smem;                                         // A rows (c), one chunk, sliced
-  uint8_t *sBop = smem + TC_OP;                                 // B rows (j), one chunk, sliced
-  zdf *stX = (zdf *)(smem + TC_OP + TC_BBYTES);                 // stX[c * VX_LD + row]
-  zdf *stV = (zdf *)(smem + TC_OP + TC_BBYTES + VX_STX);        // stV[j * VX_LD + row]
-  int *sEc = (int *)(smem + TC_OP + TC_BBYTES + VX_STX + VX_STV);
-  int *sEa = sEc + 128;
-  uint64_t *bar = (uint64_t *)(sEa + 32);
-  uint32_t *tslot = (uint32_t *)(bar + 1);
+  uint8_t *sBop = smem;                                   // two buffers: B of a chunk, sliced
+  zdf *stA = (zdf *)(smem + 2 * BOP);                     // chunk of A: row c at stA + c LK_LD
+  zdf *stB = stA + 128 * LK_LD;                           // mode 1: chunk of B, row j at stB + j LK_LDB
+  __shared__ float sRow[2][4 * 128];                      // largest magnitudes, [chunk & 1][k-step][row]
+  __shared__ float sCol[2][16 * 32];                      // mode 1: of B, [chunk & 1][rows r][column]
+  LkBars &bar = *(LkBars *)(stB + (MODE ? 32 * LK_LDB : 0));
   const int b = blockIdx.z;
   const int n = nvec[b];
   // mode 1 walks the 32-row B tiles fastest (blockIdx.x), so that the CTAs
   // sharing one 128-row tile of Z run together and read it once from DRAM
-  const int ta = p.mode == 1 ? blockIdx.y : blockIdx.x, tb = p.mode == 1 ? blockIdx.x : blockIdx.y;
+  const int ta = MODE ? blockIdx.y : blockIdx.x, tb = MODE ? blockIdx.x : 0;
   const int c0 = ta * 128;
-  const int na = p.mode == 1 ? (int)p.rng[b * 8 + 2] : p.ncols_a;  // valid rows c
+  const int na = MODE ? (int)p.rng[b * 8 + 2] : p.ncols_a;  // valid rows c
   if (c0 >= na) return;
-  const int j0 = p.mode >= 1 ? 32 * tb : 0;
-  const int nj = p.mode == 1 ? p.nrows_b : min(p.jb, n - 1 - p.k0);  // valid rows j
-  if (p.mode >= 1 && j0 >= nj) return;
+  const int j0 = 32 * tb;
+  const int nj = MODE ? p.nrows_b : min(p.jb, n - 1 - p.k0);  // valid rows j
+  if (MODE && j0 >= nj) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int lg = warp & 3, cqt = warp >> 2;
-  const int cl = 32 * lg + lane;  // row c of this thread (TMEM lane)
-  // chunks of 32 rows r: [kc_beg, kc_end)
-  const int nck = n > p.rbeg ? (n - p.rbeg + 31) / 32 : 0;
-  const int ns = p.mode == 0 ? gridDim.y : 1, si = p.mode == 0 ? blockIdx.y : 0;
+  // chunks of CR rows r: [kc_beg, kc_beg + nk)
+  const int nck = n > p.rbeg ? (n - p.rbeg + CR - 1) / CR : 0;
+  const int ns = MODE ? 1 : gridDim.y, si = MODE ? 0 : blockIdx.y;
   const int kc_beg = (int)((int64_t)nck * si / ns);
-  const int kc_end = (int)((int64_t)nck * (si + 1) / ns);
-  df accr[TC_CQ], acci[TC_CQ];
+  // nothing once a wait of this matrix has given up: its results are invalid
+  const int nk = __syncthreads_or(*(volatile int *)&err[b]) ? 0 : (int)((int64_t)nck * (si + 1) / ns) - kc_beg;
+  const int lg = warp & 3, ks = warp >> 2;
+  const int cl = 32 * lg + lane;  // row c of this thread (TMEM lane)
+  auto write = [&](const df *v) {  // this thread's row c and its 8 columns j
+    if (c0 + cl >= na) return;
+    zdf *out = p.out + b * p.sO;
 #pragma unroll
-  for (int q = 0; q < TC_CQ; ++q) accr[q] = acci[q] = df{0.f, 0.f};
-  const bool any = kc_beg < kc_end && !*(volatile int *)&err[b];
-  uint32_t tm = 0;
-  if (any) {
-    if (warp == 0) tc::tmem_alloc(tslot, 512);
+    for (int t = 0; t < 8; ++t) {
+      const int j = 8 * ks + t;
+      if (MODE == 0)
+        out[((int64_t)blockIdx.y * 32 + j) * p.ldo + c0 + cl] = zdf{v[t], v[8 + t]};
+      else if (j0 + j < nj)
+        out[j0 + j + p.ldo * (int64_t)(c0 + cl)] = zdf{v[t], v[8 + t]};
+    }
+  };
+  if (nk > 0) {
+    if (warp == LK_CW) tc::tmem_alloc(&bar.tmem, 512);
     if (tid == 0) {
-      tc::mbar_init(bar, 1);
+      for (int k = 0; k < 2; ++k) tc::mbar_init(&bar.b[k], 1);
+      tc::mbar_init(&bar.done, 1);
+      tc::mbar_init(&bar.a_ready, LK_CW);
+      for (int k = 0; k < LK_ACC; ++k) {
+        tc::mbar_init(&bar.acc[k], 1);
+        tc::mbar_init(&bar.acc_free[k], LK_CW);
+      }
+      tc::mbar_init(&bar.drain, 1);
+      tc::mbar_init(&bar.st_full, 32 * LK_LW);
+      tc::mbar_init(&bar.st_free, LK_CW);
+      bar.abort = 0;
       tc::mbar_init_fence();
     }
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
-    tm = __shfl_sync(0xffffffffu, *tslot, 0);
-  }
-  const zdf *A = p.A + b * p.sA;
-  const zdf *Bm = p.Bm + b * p.sB;
-  const uint32_t lane_addr = tm + ((uint32_t)(32 * lg) << 16) + TC_CQ * cqt;
-  // copies of a chunk into the staging buffers: lane = row r, 8 A rows and 2
-  // B rows per warp (zero outside the operands)
-  auto load = [&](int kc) {
-    const int r = p.rbeg + 32 * kc + lane;
-#pragma unroll
-    for (int jj = 0; jj < 8; ++jj) {
-      const int c = 8 * warp + jj;
-      const bool v = r < n && c0 + c < na;
-      cp_async16(&stX[c * VX_LD + lane], v ? (const void *)&A[r + p.lda * (c0 + c)] : (const void *)A, v);
-    }
-#pragma unroll
-    for (int jj = 0; jj < 2; ++jj) {
-      const int j = 2 * warp + jj;
-      bool v = r < n && j0 + j < nj;
-      if (p.vmask) v = v && r >= p.k0 + j + 1;
-      cp_async16(&stV[j * VX_LD + lane], v ? (const void *)&Bm[r + p.ldb * (j0 + j)] : (const void *)Bm, v);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  int ok = 1, failed_par = -1;
-  if (any) load(kc_beg);
-  for (int kc = kc_beg; any && kc < kc_end; ++kc) {
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
-    if (p.real_a) {  // A real: threads 0-255 slice its real k-steps, 256-383 slice B
-      if (tid < 256) {
-        const int c = tid >> 1, ks = tid & 1;
-        const int e = slice_kstep<TC_TILE, 2>(&stX[c * VX_LD], false, sAop, c, ks);
-        if (ks == 0) sEc[c] = e;
-      } else if (tid < 384) {
-        const int j = (tid - 256) >> 2, ks = tid & 3;
-        const int e = slice_kstep<1024, 4>(&stV[j * VX_LD], p.conj_b != 0, sBop, j, ks);
-        if (ks == 0) sEa[j] = e;
+    const uint32_t tm = __shfl_sync(0xffffffffu, bar.tmem, 0);
+    volatile int *abort = &bar.abort;
+    bool ok = true;
+    // launched with 96 registers a thread (61440): 512 x 104 + 128 x 56 = 60416
+    if (warp >= LK_CW) {
+      asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+      const bool one = tc::elect_one();
+      auto wait = [&](uint64_t *w, int phase) {
+        ok = __all_sync(0xffffffffu, ok && wait_phase(w, (uint32_t)(phase & 1), abort));
+      };
+      int ncopy = 0;
+      auto copy_b = [&](int k) {
+        if (MODE == 0 && one) {
+          tc::mbar_expect_tx(&bar.b[k & 1], LK_BOP);
+          tc::bulk_g2s(sBop + (k & 1) * LK_BOP, p.S + b * p.sS + (int64_t)(kc_beg + k) * LK_BOP, LK_BOP, &bar.b[k & 1]);
+        }
+        ++ncopy;
+      };
+      const int nkw = warp == LK_CW ? nk : 0;
+      if (nkw > 0) copy_b(0);
+      if (nkw > 1) copy_b(1);
+      for (int k = 0; k < nkw && ok; ++k) {
+        if (MODE == 0) wait(&bar.b[k & 1], k >> 1);
+        wait(&bar.a_ready, k);
+        const uint64_t b0 = tc::sdesc(tc::smem_u32(sBop + (k & 1) * BOP), 128, 256);
+        int g = k * TC_S;
+        auto group = [&](auto issue) {
+          const int slot = g & (LK_ACC - 1);
+          if (g >= LK_ACC) wait(&bar.acc_free[slot], g / LK_ACC - 1);
+          tc::fence_after();
+          if (ok && one) {
+            issue(tm + slot * 64);
+            tc::mma_commit(&bar.acc[slot]);
+          }
+          __syncwarp();
+          ++g;
+        };
+        group([&](uint32_t d) { lk_issue<6, MODE>(d, tm + LK_TA, b0); });
+        if (k >= 1) {  // chunk k - 1's MMAs have ended: its buffer takes chunk k + 1
+          wait(&bar.done, k - 1);
+          if (ok && k + 1 < nk) copy_b(k + 1);
+          __syncwarp();
+        }
+        group([&](uint32_t d) { lk_issue<5, MODE>(d, tm + LK_TA, b0); });
+        group([&](uint32_t d) { lk_issue<4, MODE>(d, tm + LK_TA, b0); });
+        group([&](uint32_t d) { lk_issue<3, MODE>(d, tm + LK_TA, b0); });
+        group([&](uint32_t d) { lk_issue<2, MODE>(d, tm + LK_TA, b0); });
+        group([&](uint32_t d) { lk_issue<1, MODE>(d, tm + LK_TA, b0); });
+        group([&](uint32_t d) { lk_issue<0, MODE>(d, tm + LK_TA, b0); });
+        if (ok && one) tc::mma_commit(&bar.done);
+        __syncwarp();
       }
-    } else {
-      {  // A: thread = (row c, k-step)
-        const int c = tid >> 2, ks = tid & 3;
-        const int e = slice_kstep<TC_TILE, 4>(&stX[c * VX_LD], p.conj_a != 0, sAop, c, ks);
-        if (ks == 0) sEc[c] = e;
-      }
-      if (tid < 128) {
-        const int j = tid >> 2, ks = tid & 3;
-        const int e = slice_kstep<1024, 4>(&stV[j * VX_LD], p.conj_b != 0, sBop, j, ks);
-        if (ks == 0) sEa[j] = e;
-      }
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    tc::fence_before();
-    __syncthreads();
-    tc::fence_after();
-    if (warp == 0) {
-      if (tc::elect_one()) {
-        if (p.real_a)
-          tc_issue_reala(tm, tc::smem_u32(sAop), tc::smem_u32(sBop));
-        else
-          tc_issue(tm, tc::smem_u32(sAop), tc::smem_u32(sBop));
-        tc::mma_commit(bar);
+      // every MMA has ended before the tensor memory is released, no copy lands
+      // after the block's end
+      if (nkw > 0 && ok) wait(&bar.done, nk - 1);
+      if (!ok && one) {
+        *abort = 1;
+        atomicExch(&err[b], 1);
+        tc::mma_commit(&bar.drain);
+        tc::mbar_wait(&bar.drain, 0u, 200000000LL);
       }
       __syncwarp();
-    }
-    if (kc + 1 < kc_end) load(kc + 1);  // in flight while the MMAs run
-    const bool done = tc::mbar_wait(bar, (uint32_t)((kc - kc_beg) & 1));
-    ok = __syncthreads_and(done && ok);
-    if (!ok) {
-      failed_par = (kc - kc_beg) & 1;
-      break;
-    }
-    tc::fence_after();
-    const int ec = sEc[cl];
+      if (MODE == 0)
+        for (int k = max(0, ncopy - 2); k < ncopy; ++k)
+          tc::mbar_wait(&bar.b[k & 1], (uint32_t)((k >> 1) & 1), 200000000LL);
+      if (warp > LK_CW) {
+        // copies of chunk k into the staging buffers, zero outside the operands:
+        // lane = row r (mode 1: the real parts, two rows r of 8 bytes per
+        // 16-byte element)
+        const zdf *A = p.A + b * p.sA;
+        const zdf *Bm = p.Bm + b * p.sB;
+        for (int k = 0; k < nk && ok; ++k) {
+          if (k > 0) wait(&bar.st_free, k - 1);
+          if (!ok) break;
+          const int r0 = p.rbeg + CR * (kc_beg + k) + lane;
+#pragma unroll 4
+          for (int c = warp - LK_CW - 1; c < 128; c += LK_LW) {
+            const zdf *src = A + p.lda * (c0 + c);
+            if (MODE == 0) {
+              const bool v = r0 < n && c0 + c < na;
+              cp_async16(&stA[c * LK_LD + lane], v ? src + r0 : A, v);
+            } else {
 #pragma unroll
-    for (int cc = 0; cc < TC_CQ / 4; ++cc) {
-      float are[TC_S][4], aim[TC_S][4];
-#pragma unroll
-      for (int uu = 0; uu < TC_S; ++uu) {
-        tc::tmem_ld4(lane_addr + uu * 32 + cc * 4, are[uu]);
-        tc::tmem_ld4(lane_addr + (TC_S + uu) * 32 + cc * 4, aim[uu]);
-      }
-      tc::tmem_ld_wait();
-#pragma unroll
-      for (int qq = 0; qq < 4; ++qq) {
-        const int q = 4 * cc + qq;
-        float vr[TC_S], vi[TC_S];
-#pragma unroll
-        for (int uu = 0; uu < TC_S; ++uu) {
-          vr[uu] = are[uu][qq];
-          vi[uu] = aim[uu][qq];
+              for (int h = 0; h < 2; ++h) {
+                const bool v = r0 + 32 * h < n && c0 + c < na;
+                cp_async8((df *)(stA + c * LK_LD) + lane + 32 * h, v ? src + r0 + 32 * h : A, v);
+              }
+            }
+          }
+          if (MODE == 1) {
+#pragma unroll 4
+            for (int jj = warp - LK_CW - 1; jj < 64; jj += LK_LW) {
+              const int j = jj >> 1, rr = 32 * (jj & 1);
+              const bool v = r0 + rr < n && j0 + j < nj;
+              cp_async16(&stB[j * LK_LDB + lane + rr], v ? Bm + r0 + rr + p.ldb * (j0 + j) : Bm, v);
+            }
+          }
+          tc::mbar_arrive_cp(&bar.st_full);
         }
-        const float sc = pow2f(ec + sEa[TC_CQ * cqt + q] - 16);
-        df pr = combine7(vr), pi = combine7(vi);
-        pr.hi = __fmul_rn(pr.hi, sc);
-        pr.lo = __fmul_rn(pr.lo, sc);
-        pi.hi = __fmul_rn(pi.hi, sc);
-        pi.lo = __fmul_rn(pi.lo, sc);
-        accr[q] = df_add(accr[q], pr);
-        acci[q] = df_add(acci[q], pi);
+        if (!ok && lane == 0) {
+          *abort = 1;
+          atomicExch(&err[b], 1);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");  // no copy may land after the block's end
       }
+    } else {
+      asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+      df acc[16];  // re and im of this thread's 8 columns
+#pragma unroll
+      for (int k = 0; k < 16; ++k) acc[k] = df{0.f, 0.f};
+      auto sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(32 * LK_CW) : "memory"); };
+      Fixed56 f[16];  // K = 16 ks ... of row cl
+      int En = 0;     // and the row's exponent
+      int eb = 0;     // mode 1: exponent of column lane
+      // the integers of chunk k from the staging buffers (mode 1: also B's
+      // slices of it), which then take chunk k + 1
+      auto prep = [&](int k) {
+        ok = __all_sync(0xffffffffu, ok && wait_phase(&bar.st_full, (uint32_t)(k & 1), abort));
+        df x[16];
+        if (MODE == 0) {
+#pragma unroll
+          for (int t = 0; t < 16; ++t) x[t] = ((const df *)&stA[cl * LK_LD + 16 * (ks & 1) + t])[ks >> 1];
+        } else {
+#pragma unroll
+          for (int t = 0; t < 16; t += 2) {
+            const zdf two = stA[cl * LK_LD + 8 * ks + t / 2];
+            x[t] = two.re;
+            x[t + 1] = two.im;
+          }
+        }
+        float amax = 0.f;
+#pragma unroll
+        for (int t = 0; t < 16; ++t) amax = max_abs(amax, x[t].hi);
+        float *row = sRow[k & 1], *col = sCol[k & 1];
+        row[ks * 128 + cl] = amax;
+        df yr[4], yi[4];  // mode 1: B column lane, rows r = 4 warp ... of the chunk
+        if (MODE == 1) {
+          float bmax = 0.f;
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            const zdf y = stB[lane * LK_LDB + 4 * warp + t];
+            yr[t] = y.re;
+            yi[t] = y.im;
+            bmax = max_abs(max_abs(bmax, y.re.hi), y.im.hi);
+          }
+          col[warp * 32 + lane] = bmax;
+        }
+        sync();  // the maxima are there (two sets: the next chunk's may come while these are read)
+        if (lane == 0) tc::mbar_arrive(&bar.st_free);
+        if (MODE == 1) {
+          float bmax = 0.f;
+#pragma unroll
+          for (int q = 0; q < 16; ++q) bmax = max_abs(bmax, col[q * 32 + lane]);
+          const int E = grid_exp(bmax);
+          Fixed56 fr[4], fi[4];
+          to_fixed<4>(yr, E, false, fr);
+          to_fixed<4>(yi, E, true, fi);
+          uint8_t *dst = sBop + (k & 1) * BOP + (warp >> 2) * 1024 + tc::core_off(lane, 4 * (warp & 3));
+          auto put = [&](auto dig, int s) {
+            *(uint2 *)(dst + s * TC_KS * 1024) = make_uint2(dig(fr[0], fr[1]), dig(fr[2], fr[3]));
+            *(uint2 *)(dst + (TC_S + s) * TC_KS * 1024) = make_uint2(dig(fi[0], fi[1]), dig(fi[2], fi[3]));
+          };
+          put([](Fixed56 a, Fixed56 c) { return digit2<0>(a, c); }, 0);
+          put([](Fixed56 a, Fixed56 c) { return digit2<1>(a, c); }, 1);
+          put([](Fixed56 a, Fixed56 c) { return digit2<2>(a, c); }, 2);
+          put([](Fixed56 a, Fixed56 c) { return digit2<3>(a, c); }, 3);
+          put([](Fixed56 a, Fixed56 c) { return digit2<4>(a, c); }, 4);
+          put([](Fixed56 a, Fixed56 c) { return digit2<5>(a, c); }, 5);
+          put([](Fixed56 a, Fixed56 c) { return digit2<6>(a, c); }, 6);
+          eb = E;  // of column lane
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        }
+        En = grid_exp(max_abs(max_abs(row[cl], row[128 + cl]), max_abs(row[256 + cl], row[384 + cl])));
+        to_fixed<16>(x, En, false, f);
+      };
+      const uint32_t lane_base = tm + ((uint32_t)(32 * lg) << 16);
+      auto store = [&](auto dig, int s) {
+        uint32_t w[8];
+#pragma unroll
+        for (int t = 0; t < 8; ++t) w[t] = dig(f[2 * t], f[2 * t + 1]);
+        tc::tmem_st8(lane_base + LK_TA + (s * TC_KS + ks) * 8, w);
+      };
+      auto ready = [&] {
+        tc::tmem_st_wait();
+        tc::fence_before();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&bar.a_ready);
+      };
+      prep(0);
+      store([](Fixed56 a, Fixed56 c) { return digit2<6>(a, c); }, 6);
+      store([](Fixed56 a, Fixed56 c) { return digit2<5>(a, c); }, 5);
+      store([](Fixed56 a, Fixed56 c) { return digit2<4>(a, c); }, 4);
+      store([](Fixed56 a, Fixed56 c) { return digit2<3>(a, c); }, 3);
+      store([](Fixed56 a, Fixed56 c) { return digit2<2>(a, c); }, 2);
+      store([](Fixed56 a, Fixed56 c) { return digit2<1>(a, c); }, 1);
+      store([](Fixed56 a, Fixed56 c) { return digit2<0>(a, c); }, 0);
+      ready();
+      for (int k = 0; k < nk; ++k) {
+        const int Ec = En;
+        const int ebc = MODE ? eb : p.Ex[b * p.sEx + 32 * (kc_beg + k) + lane];  // of column lane
+        const bool more = k + 1 < nk;
+        if (more) prep(k + 1);
+        df s[16];
+        int g = k * TC_S;
+        auto stage = [&](auto fold, auto dig, int u) {
+          const int slot = g & (LK_ACC - 1);
+          ok = __all_sync(0xffffffffu, ok && wait_phase(&bar.acc[slot], (uint32_t)((g / LK_ACC) & 1), abort));
+          tc::fence_after();
+          float a[16];
+          tc::tmem_ld8(lane_base + slot * 64 + 8 * ks, a);
+          tc::tmem_ld8(lane_base + slot * 64 + 32 + 8 * ks, a + 8);
+          tc::tmem_ld_wait();
+#pragma unroll
+          for (int t = 0; t < 16; ++t) fold(s[t], a[t]);
+          if (more) store(dig, u);
+          tc::fence_before();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(&bar.acc_free[slot]);
+          ++g;
+        };
+        stage([](df &v, float a) { fold_up<6>(v, a); }, [](Fixed56 a, Fixed56 c) { return digit2<6>(a, c); }, 6);
+        stage([](df &v, float a) { fold_up<5>(v, a); }, [](Fixed56 a, Fixed56 c) { return digit2<5>(a, c); }, 5);
+        stage([](df &v, float a) { fold_up<4>(v, a); }, [](Fixed56 a, Fixed56 c) { return digit2<4>(a, c); }, 4);
+        stage([](df &v, float a) { fold_up<3>(v, a); }, [](Fixed56 a, Fixed56 c) { return digit2<3>(a, c); }, 3);
+        stage([](df &v, float a) { fold_up<2>(v, a); }, [](Fixed56 a, Fixed56 c) { return digit2<2>(a, c); }, 2);
+        stage([](df &v, float a) { fold_up<1>(v, a); }, [](Fixed56 a, Fixed56 c) { return digit2<1>(a, c); }, 1);
+        stage([](df &v, float a) { fold_up<0>(v, a); }, [](Fixed56 a, Fixed56 c) { return digit2<0>(a, c); }, 0);
+        if (more) ready();
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+          const float sc = pow2f(Ec + __shfl_sync(0xffffffffu, ebc, 8 * ks + t) - 16);
+          acc[t] = df_add(acc[t], df{__fmul_rn(s[t].hi, sc), __fmul_rn(s[t].lo, sc)});
+          acc[8 + t] = df_add(acc[8 + t], df{__fmul_rn(s[8 + t].hi, sc), __fmul_rn(s[8 + t].lo, sc)});
+        }
+      }
+      if (!ok && lane == 0) {
+        *abort = 1;
+        atomicExch(&err[b], 1);
+      }
+      write(acc);
     }
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
-  }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");  // no copy may land after exit
-  if (any) {
-    if (!ok) {
-      // the MMAs whose wait gave up may still be running: give them (a
-      // bounded) time to finish before their tensor memory is released
-      if (tid == 0) {
-        atomicExch(&err[b], 1);
-        if (failed_par >= 0) tc::mbar_wait(bar, (uint32_t)failed_par, 200000000LL);
-      }
-      tc::fence_before();
-      __syncthreads();
-      tc::fence_after();
-    }
-    if (warp == 0) tc::tmem_dealloc(tm, 512);
-  }
-  // this thread's row c and its 8 rows j
-  if (c0 + cl < na) {
-    zdf *out = p.out + b * p.sO;
+    if (warp == LK_CW) tc::tmem_dealloc(tm, 512);
+  } else if (warp < LK_CW) {
+    df zero[16];
 #pragma unroll
-    for (int q = 0; q < TC_CQ; ++q) {
-      const int j = TC_CQ * cqt + q;
-      if (p.mode == 0)
-        out[((int64_t)blockIdx.y * 32 + j) * p.ldo + c0 + cl] = zdf{accr[q], acci[q]};
-      else if (j0 + j < nj)
-        out[j0 + j + p.ldo * (int64_t)(c0 + cl)] = zdf{accr[q], acci[q]};
-    }
+    for (int k = 0; k < 16; ++k) zero[k] = df{0.f, 0.f};
+    write(zero);
   }
 }
 
@@ -835,7 +1022,10 @@ cudaError_t prepare_her2k_tc() {
   std::lock_guard<std::mutex> g(mu);
   if (dev >= 0 && done[dev]) return cudaSuccess;
   cudaError_t e = cudaFuncSetAttribute(k_cupd_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, CU_SMEM);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_longk_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, VX_SMEM);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_longk_tc<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, lk_smem<0>());
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_longk_tc<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, lk_smem<1>());
   if (e == cudaSuccess && dev >= 0) done[dev] = true;
   return e;
 }
@@ -973,7 +1163,6 @@ cudaError_t vhx_tc(EigWork &w, int k0, int jb, const zdf *X, int64_t ldx, int64_
   p.Bm = (const zdf *)w.A + w.lda * k0;
   p.ldb = w.lda;
   p.sB = w.sA;
-  p.vmask = 1;
   p.k0 = k0;
   p.jb = jb;
   p.rbeg = k0 + 1;
@@ -981,8 +1170,17 @@ cudaError_t vhx_tc(EigWork &w, int k0, int jb, const zdf *X, int64_t ldx, int64_
   p.out = Wp;
   p.ldo = ldwp;
   p.sO = sWp;
-  p.mode = 0;
-  PP_KT(KT_VHX, s, (k_longk_tc<<<dim3((ncols + 127) / 128, vhx_tc_splits(w), w.B), TC_NT, VX_SMEM, s>>>(
+  // the slices of the panel and their exponents: the scratch that the update X -= V Y takes after this
+  p.S = w.tcS;
+  p.sS = w.sTcS;
+  p.Ex = w.tcE;
+  p.sEx = w.sTcE;
+  const int nck = (w.nmax - p.rbeg + 31) / 32;
+  if (nck > 0) {
+    PP_KT(KT_VHX, s, (k_longk_bslice<<<dim3(nck, w.B), 128, 0, s>>>(p, w.nvec, w.tcS, w.tcE)));
+    count_launch(1);
+  }
+  PP_KT(KT_VHX, s, (k_longk_tc<0><<<dim3((ncols + 127) / 128, vhx_tc_splits(w), w.B), LK_NT, lk_smem<0>(), s>>>(
                        p, w.nvec, w.tcErr)));
   count_launch(1);
   return cudaGetLastError();
@@ -995,19 +1193,16 @@ cudaError_t xhz_tc(EigWork &w, const zdf *X, int64_t ldx, int64_t sX, int nrows,
   p.A = Z;
   p.lda = ldz;
   p.sA = sZ;
-  p.real_a = 1;
   p.Bm = X;
   p.ldb = ldx;
   p.sB = sX;
-  p.conj_b = 1;
   p.nrows_b = nrows;
   p.rbeg = 0;
   p.rng = w.rng;
   p.out = Eb;
   p.ldo = lde;
   p.sO = sE;
-  p.mode = 1;
-  PP_KT(KT_XHZ, s, (k_longk_tc<<<dim3((nrows + 31) / 32, (w.mcap + 127) / 128, w.B), TC_NT, VX_SMEM, s>>>(
+  PP_KT(KT_XHZ, s, (k_longk_tc<1><<<dim3((nrows + 31) / 32, (w.mcap + 127) / 128, w.B), LK_NT, lk_smem<1>(), s>>>(
                        p, w.nvec, w.tcErr)));
   count_launch(1);
   return cudaGetLastError();

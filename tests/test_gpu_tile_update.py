@@ -41,3 +41,24 @@ def test_eigenpairs_over_column_block_splits(natom, nq):
             assert r.m[t] == n and r.nz[t] == n and r.info[t] == 0
             assert np.linalg.norm(D @ Z - Z * lam, axis=0).max() <= 1e-11 * norm
             assert np.abs(Z.conj().T @ Z - np.eye(n)).max() <= 1e-10
+
+
+@pytest.mark.parametrize("natom", [1, 11, 21, 22, 43, 64, 65, 86])
+def test_velocities_without_and_with_vectors(natom):
+    """The product X^H Z of the velocities without eigenvectors, at chunks of 64
+    rows, tiles of 128 eigenvectors and their remainders, against the velocities
+    formed from the eigenvectors of the same tridiagonal problem.  v w is linear
+    in products of vector pairs that differ by the two transforms' rounding, at
+    most about sqrt(n) 2^-44 each with ||dD/dq|| = max |v w| up to a small factor:
+    64 sqrt(n) 2^-44."""
+    lat, pos, phi = _random_cell(natom, natom)
+    crys = geometry.crys_from_positions(lat, pos)
+    qs = np.array([[0.11, 0.23, 0.0], [0.37, -0.19, 0.0]])
+    n = 3 * natom
+    with api.PhononContext(lat, crys, pos, np.array([1.0]), np.ones(natom, np.int64), phi) as ctx:
+        a = ctx.solve(qs, api.EigOpts(jobz="N", vel=True, precision=api.PP_PREC_MIXED), want_z=False)
+        z = ctx.solve(qs, api.EigOpts(jobz="V", vel=True, precision=api.PP_PREC_MIXED))
+        for t in range(len(qs)):
+            va, vz = (r.vel[t, :n] * np.abs(r.w[t, :n, None]) for r in (a, z))
+            assert np.isfinite(va).all()
+            assert np.abs(va - vz).max() <= 64 * np.sqrt(n) * 2.0 ** -44 * np.abs(vz).max()
