@@ -123,10 +123,21 @@ struct pp_ctx {
   cudaEvent_t ev_fork = nullptr, ev_join[MAX_SPLIT - 1] = {};
   // launch configuration of the current batch (autotuned or from the switches)
   int cur_split = 8, cur_bps = 6;
-  // captured CUDA graph of the last batch configuration
-  cudaGraphExec_t gexec = nullptr;
-  char gkey[192] = {0};
-  int64_t glaunches = 0;  // kernels in the captured graph
+  // captured CUDA graphs of the last batch configurations: a pass that
+  // alternates between configurations (forward and backward of a fit, the full
+  // and the last batch of a long list) replays them instead of capturing each
+  // anew
+  struct Graph {
+    cudaGraphExec_t exec = nullptr;
+    char key[192] = {0};
+    int64_t launches = 0;  // kernels in the graph
+    uint64_t used = 0;
+  };
+  static constexpr int MAX_GRAPHS = 4;
+  Graph graphs[MAX_GRAPHS];
+  Graph *graph = nullptr;  // of the current configuration
+  std::vector<int64_t> bnd_blocks;  // boundary blocks (I + N J) of the tables in g
+  uint64_t graph_uses = 0;
 };
 
 namespace {
@@ -193,14 +204,17 @@ void linsolve(const double *x, const double *A, double *u) {
   }
 }
 
-void drop_graph(pp_ctx *c) {
-  if (c->gexec) cudaGraphExecDestroy(c->gexec);
-  c->gexec = nullptr;
-  c->gkey[0] = 0;
+void drop_graph(pp_ctx::Graph &g) {
+  if (g.exec) cudaGraphExecDestroy(g.exec);
+  g = pp_ctx::Graph();
+}
+void drop_graphs(pp_ctx *c) {
+  for (auto &g : c->graphs) drop_graph(g);
+  c->graph = nullptr;
 }
 
 void free_ws(pp_ctx *c) {
-  drop_graph(c);
+  drop_graphs(c);
   if (c->ws) cudaFree(c->ws);
   c->ws = nullptr;
   c->ws_bytes = 0;
@@ -535,7 +549,7 @@ float time_config(pp_ctx *c, int B, const pp_eig_opts *o, int mcap, bool want_z,
   c->cur_split = split;
   c->cur_bps = bps;
   cudaStream_t s = c->stream;
-  if (run_batch_graph_cfg(c, B, o, mcap, want_z, false) != PP_OK || !c->gexec) return -1.f;
+  if (run_batch_graph_cfg(c, B, o, mcap, want_z, false) != PP_OK || !c->graph) return -1.f;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) {
     cudaGetLastError();
@@ -544,8 +558,8 @@ float time_config(pp_ctx *c, int B, const pp_eig_opts *o, int mcap, bool want_z,
   }
   float ms = -1.f;
   cudaEventRecord(e0, s);
-  const cudaError_t r = cudaGraphLaunch(c->gexec, s);
-  pp::count_launch(c->glaunches);
+  const cudaError_t r = cudaGraphLaunch(c->graph->exec, s);
+  pp::count_launch(c->graph->launches);
   cudaEventRecord(e1, s);
   if (r == cudaSuccess && cudaEventSynchronize(e1) == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
   cudaGetLastError();
@@ -613,13 +627,21 @@ int run_batch_graph_cfg(pp_ctx *c, int B, const pp_eig_opts *o, int mcap, bool w
            o->jobz, o->range, o->vel_method, o->vel, (long long)o->il, (long long)o->iu, o->vl, o->vu, o->abstol,
            want_z ? 1 : 0, c->cur_split, c->cur_bps, o->want_resid ? 1 : 0);
   cudaStream_t s = c->stream;
-  if (c->gexec && strcmp(key, c->gkey) == 0) {
-    if (!launch) return PP_OK;
-    TRY_CUDA(cudaGraphLaunch(c->gexec, s));
-    pp::count_launch(c->glaunches);
-    return PP_OK;
+  c->w.B = c->w.batch = B;  // (what follows the graph reads it)
+  c->graph = nullptr;
+  pp_ctx::Graph *slot = &c->graphs[0];  // this configuration's, or the one unused for longest
+  for (auto &g : c->graphs) {
+    if (g.exec && strcmp(key, g.key) == 0) {
+      g.used = ++c->graph_uses;
+      c->graph = &g;
+      if (!launch) return PP_OK;
+      TRY_CUDA(cudaGraphLaunch(g.exec, s));
+      pp::count_launch(g.launches);
+      return PP_OK;
+    }
+    if (g.used < slot->used) slot = &g;
   }
-  drop_graph(c);
+  drop_graph(*slot);
   TRY_CUDA(prepare_bisect(bisect_smem(c->w.nmax, o->precision == PP_PREC_MIXED)));
   if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
     cudaGetLastError();
@@ -627,7 +649,7 @@ int run_batch_graph_cfg(pp_ctx *c, int B, const pp_eig_opts *o, int mcap, bool w
   }
   const int64_t l0 = pp::g_launches.load();
   const int r = run_batch(c, B, o, mcap, want_z);
-  c->glaunches = pp::g_launches.load() - l0;
+  slot->launches = pp::g_launches.load() - l0;
   cudaGraph_t g = nullptr;
   cudaError_t e = cudaStreamEndCapture(s, &g);
   if (r != PP_OK || e != cudaSuccess || !g) {
@@ -635,19 +657,21 @@ int run_batch_graph_cfg(pp_ctx *c, int B, const pp_eig_opts *o, int mcap, bool w
     cudaGetLastError();
     return launch ? run_batch(c, B, o, mcap, want_z) : 1;
   }
-  e = cudaGraphInstantiate(&c->gexec, g, 0);
+  e = cudaGraphInstantiate(&slot->exec, g, 0);
   cudaGraphDestroy(g);
   if (e != cudaSuccess) {
-    c->gexec = nullptr;
+    slot->exec = nullptr;
     cudaGetLastError();
     return launch ? run_batch(c, B, o, mcap, want_z) : 1;
   }
-  snprintf(c->gkey, sizeof(c->gkey), "%s", key);
+  snprintf(slot->key, sizeof(slot->key), "%s", key);
+  slot->used = ++c->graph_uses;
+  c->graph = slot;
   if (!launch) {
-    pp::g_launches.fetch_sub(c->glaunches);  // captured, not launched
+    pp::g_launches.fetch_sub(slot->launches);  // captured, not launched
     return PP_OK;
   }
-  TRY_CUDA(cudaGraphLaunch(c->gexec, s));
+  TRY_CUDA(cudaGraphLaunch(slot->exec, s));
   return PP_OK;
 }
 
@@ -674,18 +698,13 @@ int pick_batch(pp_ctx *c, int64_t nq, int mcap) {
 
 // Boundary blocks (I < J, tie set with a non-home image, Phi block
 // non-zero) and the rows of their atoms, from the current Phi and tie sets;
-// replaces any earlier tables.
+// replaces any earlier tables, with the captured graphs that hold their
+// addresses and counts (all kept when the blocks are the same as before: a
+// tie set belongs to its block, so the tables are then the same too).
 int build_boundary_tables(pp_ctx *c) {
   Geometry &g = c->g;
   const int64_t N = g.natom, n = g.n;
   cudaStream_t s = c->stream;
-  for (void *p : {(void *)g.d_bnd, (void *)g.d_bndmask, (void *)g.d_brows, (void *)g.d_rowmap})
-    if (p) cudaFree(p);
-  g.d_bnd = nullptr;
-  g.d_bndmask = nullptr;
-  g.d_brows = nullptr;
-  g.d_rowmap = nullptr;
-  g.nbnd = g.nbrows = 0;
   uint8_t *d_flags = nullptr;
   if (cudaMalloc(&d_flags, (size_t)N * N) != cudaSuccess) return PP_ERR_NOMEM;
   geom_block_nonzero(g, d_flags, s);
@@ -697,15 +716,27 @@ int build_boundary_tables(pp_ctx *c) {
   cudaFree(d_flags);
   if (e != cudaSuccess) return cuda_err(e);
   std::vector<int2> bnd;
+  std::vector<int64_t> blocks;
   std::vector<uint16_t> bmask;
   for (int64_t I = 0; I < N; ++I)
     for (int64_t J = I + 1; J < N; ++J) {
       const uint16_t m = mask_h[I + N * J];
       if ((m & ~(1u << 4)) && flags_h[I + N * J]) {
         bnd.push_back(make_int2((int)I, (int)J));
+        blocks.push_back(I + N * J);
         bmask.push_back(m);
       }
     }
+  if (g.d_rowmap && blocks == c->bnd_blocks) return PP_OK;
+  drop_graphs(c);
+  c->bnd_blocks.clear();
+  for (void *p : {(void *)g.d_bnd, (void *)g.d_bndmask, (void *)g.d_brows, (void *)g.d_rowmap})
+    if (p) cudaFree(p);
+  g.d_bnd = nullptr;
+  g.d_bndmask = nullptr;
+  g.d_brows = nullptr;
+  g.d_rowmap = nullptr;
+  g.nbnd = g.nbrows = 0;
   g.nbnd = (int64_t)bnd.size();
   // rows of the atoms that appear in boundary blocks (all the velocity
   // kernel reads of the eigenvectors)
@@ -734,6 +765,7 @@ int build_boundary_tables(pp_ctx *c) {
     cudaMemcpy(g.d_bndmask, bmask.data(), sizeof(uint16_t) * g.nbnd, cudaMemcpyHostToDevice);
   }
   const cudaError_t e2 = cudaGetLastError();
+  if (e2 == cudaSuccess) c->bnd_blocks = std::move(blocks);
   return e2 == cudaSuccess ? PP_OK : cuda_err(e2);
 }
 
@@ -928,9 +960,7 @@ int pp_ctx_update_fc(pp_ctx *c, const double *fc, int64_t ldfc, int64_t flags, i
   TRY_CUDA(cudaMemcpy2DAsync(c->g.d_fc, sizeof(double) * n, fc, sizeof(double) * ldfc, sizeof(double) * n, n,
                              fc_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s));
   TRY_CUDA(geom_symmetrize_fc(c->g, (flags & PP_FLAG_ENFORCE_ASR) ? 1 : 0, s));
-  // the boundary tables follow Phi's non-zero blocks; a captured graph holds
-  // the old tables' addresses and counts
-  drop_graph(c);
+  // the boundary tables follow Phi's non-zero blocks
   const int r = build_boundary_tables(c);
   if (r) {
     c->broken = 1;
