@@ -66,15 +66,17 @@ PP_D df df_mul(df a, df b) {
   return r;
 }
 // acc += a*b with the low word left unnormalised (call df_norm at the end).
+// TwoSum of acc.hi and p = fl(a.hi b.hi), with the product's own error taken
+// along in one FMA: (p - bb) + (a.hi b.hi - p) = a.hi b.hi - bb.
 PP_D void df_mac(df &acc, df a, df b) {
-  float p = __fmul_rn(a.hi, b.hi);
-  float pe = __fmaf_rn(a.hi, b.hi, -p);
-  pe = __fmaf_rn(a.hi, b.lo, pe);
-  pe = __fmaf_rn(a.lo, b.hi, pe);
-  float s, e;
-  two_sum(acc.hi, p, s, e);
+  const float s = __fadd_rn(acc.hi, __fmul_rn(a.hi, b.hi));
+  const float bb = __fsub_rn(s, acc.hi);
+  float e = __fmaf_rn(a.hi, b.hi, -bb);
+  e = __fmaf_rn(a.hi, b.lo, e);
+  e = __fmaf_rn(a.lo, b.hi, e);
+  e = __fadd_rn(__fsub_rn(acc.hi, __fsub_rn(s, bb)), e);
   acc.hi = s;
-  acc.lo = __fadd_rn(acc.lo, __fadd_rn(e, pe));
+  acc.lo = __fadd_rn(acc.lo, e);
 }
 PP_HD df df_from(double x) {
   df r;

@@ -501,11 +501,12 @@ __global__ void __launch_bounds__(4 * HL_T, HL_BPS * 32 / HL_T) k_hemv_lower(con
 // runs depend on the order of the trailing block, the column of the panel and
 // the number of SMs only.  The first CTAs of the grid form the panel products
 // (panel_dot), 2 per CTA.
-// Bound by instruction issue: 96 double-float lane operations per stored
-// element (two complex multiply-adds), 122 instructions in all where the
+// Bound by instruction issue: 80 double-float lane operations per stored
+// element (two complex multiply-adds), 106 instructions in all where the
 // 32 x 32 tiles of the earlier kernel took 152.  One matrix of order 4764,
-// first columns: 66.5 us -> 53.5 us (3.4 TB/s); four of them 196 us.  Measured
-// and not kept: packed f32x2 arithmetic (30% fewer instructions, but three
+// first columns: 66.5 us -> 53.5 us (3.4 TB/s), with 96 operations; all columns
+// of 8 such matrices, the average: 139 us, with 80 operations (df_mac) 127 us.
+// Measured and not kept: packed f32x2 arithmetic (30% fewer instructions, but three
 // shared-memory reads per vector entry: 57 us); bulk copies by a fetching warp
 // with mbarriers (61 us: 1 KB copies are issued too slowly); tiles of 64 x 64.
 constexpr int HV_R = 64, HV_C = 32, HV_LD = HV_R + 1;
