@@ -70,6 +70,44 @@ __device__ double block_sum(double v, double *sh) {
 // ===========================================================================
 constexpr int TR_NT = 256;   // threads of the column kernels
 
+// The mat-vec and the column steps of a panel are launched as dependent
+// launches: a kernel may start once every block of the one before has called
+// dep_go, does what does not read that kernel's results, and waits in dep_wait
+// until it has completed (every block waits, before any return, so that
+// completion carries over the whole chain; dep_go comes after dep_wait, so that
+// all earlier kernels have completed when a kernel starts).  The mat-vec
+// requests its first tile early, the column step its panel rows, v and the next
+// column.  A pass: n = 1092 (FP64, eigenvalues) 38.6 -> 30.3 ms, n = 2604 with
+// vectors 168 -> 156 ms, n = 1092 x 16 64.8 -> 61.1 ms.  dep_go is called late
+// (a block's last tile, a column's last phase): blocks that wait early hold
+// slots that other streams' kernels need (column step calling it first: 166 and
+// 63.9 ms).
+PP_D void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+PP_D void dep_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <class... P, class... A>
+static cudaError_t launch_dep(void (*kernel)(P...), dim3 grid, int threads, size_t smem, int cluster, bool dep,
+                              cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[2];
+  cfg.attrs = at;
+  if (cluster) {
+    at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    at[cfg.numAttrs].val.clusterDim.x = cluster;
+    at[cfg.numAttrs].val.clusterDim.y = at[cfg.numAttrs].val.clusterDim.z = 1;
+    ++cfg.numAttrs;
+  }
+  if (dep) {
+    at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+    ++cfg.numAttrs;
+  }
+  return cudaLaunchKernelEx(&cfg, kernel, (P)args...);
+}
+
 // Sums over threads.  Double: plain FP64 adds.  Double-float: an unevaluated
 // sum of three floats, whose additions lose nothing above ~2^-70 of the
 // largest term -- no less than an FP64 sum, without the FP64 pipe (a
@@ -399,20 +437,26 @@ __global__ void __launch_bounds__(4 * HL_T, HL_BPS * 32 / HL_T) k_hemv_lower(con
   const int b = blockIdx.z;
   const int n = nvec[b];
   const int r0 = i + 1;
-  if (r0 >= n || hl_tile(n - r0) != HL_T) return;
   const int nd = hl_dots(jj, HL_T);
-  if ((int)blockIdx.x < nd) {
+  if (r0 >= n || hl_tile(n - r0) != HL_T || (int)blockIdx.x < nd) {
+    dep_wait();
+    dep_go();
+    if (r0 >= n || hl_tile(n - r0) != HL_T) return;
     panel_dot_warp(Ab + b * sA, Wb + b * sW, lda, n, i, k0, jj, blockIdx.x * (HL_NT / 32) + threadIdx.x / 32, X + b * ldx);
     return;
   }
   const int bx = blockIdx.x - nd, gx = gridDim.x - nd;  // among the mat-vec's blocks
   const int nt = (n - r0 + HL_T - 1) / HL_T;
   const int npairs = nt * (nt + 1) / 2;
-  if (bx >= npairs) return;
+  if (bx >= npairs) {
+    dep_wait();
+    return;
+  }
   const z64 *A = Ab + b * sA;
   const int tid = threadIdx.x;
-  // copies of tile pair p into buffer buf (zero outside the matrix)
-  auto issue = [&](int p, int buf) {
+  // copies of tile pair p into buffer buf (zero outside the matrix); the first
+  // tile's before the column step has completed, which writes v only
+  auto issue = [&](int p, int buf, bool first = false) {
     int Rt, Ct;
     tile_pair(p, Rt, Ct);
     const int rt0 = r0 + Rt * HL_T, ct0 = r0 + Ct * HL_T;
@@ -427,6 +471,7 @@ __global__ void __launch_bounds__(4 * HL_T, HL_BPS * 32 / HL_T) k_hemv_lower(con
       const bool ok = rr < n && ct0 + cb + CS * j < n;
       cp_async16(dst + CS * j * HL_LD, ok ? (const void *)(src + CS * j * lda) : (const void *)A, ok);
     }
+    if (first) dep_wait();
     if (tid < HL_T) {
       const int rr = rt0 + tid;
       cp_async16(&vR[buf][tid], rr < n ? (const void *)&A[rr + lda * i] : (const void *)A, rr < n);
@@ -441,13 +486,15 @@ __global__ void __launch_bounds__(4 * HL_T, HL_BPS * 32 / HL_T) k_hemv_lower(con
   const int lane = tid & (HL_T - 1), wid = tid / HL_T;
   const int prod = wid >> 1, half = wid & 1;
   constexpr int SPAN = HL_T / 2;
-  issue(bx, 0);
+  issue(bx, 0, true);
   int buf = 0;
   for (int p = bx; p < npairs; p += gx) {
-    if (p + gx < npairs)
+    if (p + gx < npairs) {
       issue(p + gx, buf ^ 1);
-    else
+    } else {
+      dep_go();
       cp_async_commit();  // an empty group keeps "all but the newest" meaning this tile
+    }
     cp_async_wait1();
     __syncthreads();
     int Rt, Ct;
@@ -541,11 +588,13 @@ __global__ void __launch_bounds__(HV_NT, HV_BPS) k_hemv_df(const zdf *Ab, int64_
   const int b = blockIdx.y;
   const int n = nvec[b];
   const int r0 = i + 1;
-  if (r0 >= n) return;
   const zdf *A = Ab + b * sA;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nd = hv_dots(jj);
-  if ((int)blockIdx.x < nd) {
+  if (r0 >= n || (int)blockIdx.x < nd) {
+    dep_wait();
+    dep_go();
+    if (r0 >= n) return;
     const int g = warp >> 2;
     panel_dot(A, Wb + b * sW, lda, n, i, k0, jj, blockIdx.x * 2 + g, tid & 127,
                   (Sum<df>::T(*)[4])hv_smem + 2 * g,
@@ -557,7 +606,10 @@ __global__ void __launch_bounds__(HV_NT, HV_BPS) k_hemv_df(const zdf *Ab, int64_
   const int x = blockIdx.x - nd;
   int t = x * run;
   const int tend = min(t + run, nt * (nt + 1));
-  if (t >= tend) return;
+  if (t >= tend) {
+    dep_wait();
+    return;
+  }
   int R = (int)((sqrtf(4.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
   while ((R + 1) * (R + 2) <= t) ++R;
   while (R * (R + 1) > t) --R;
@@ -566,8 +618,9 @@ __global__ void __launch_bounds__(HV_NT, HV_BPS) k_hemv_df(const zdf *Ab, int64_
   // this thread's part of a tile: row tr, columns tc, tc + 4, ...
   const int tr = tid & (HV_R - 1), tc = tid / HV_R;
   // copies of the next tile and its vector pieces into buffer buf (zero
-  // outside the matrix); an empty group past the run's end
-  auto issue = [&](int buf) {
+  // outside the matrix); an empty group past the run's end.  The first tile is
+  // requested before the column step has completed, which writes v only.
+  auto issue = [&](int buf, bool first = false) {
     if (ti < tend) {
       const int rt0 = r0 + Ri * HV_R, ct0 = r0 + Ci * HV_C;
       const zdf *src = A + rt0 + tr + lda * (ct0 + tc);
@@ -577,6 +630,7 @@ __global__ void __launch_bounds__(HV_NT, HV_BPS) k_hemv_df(const zdf *Ab, int64_
       if (rt0 + HV_R <= n) {  // (every column of a full tile row exists)
 #pragma unroll
         for (int j = 0; j < HV_C / 4; ++j) cp_async16(dst + 4 * j * HV_LD, src + 4 * j * lda);
+        if (first) dep_wait();
         if (tid < HV_R + HV_C) cp_async16(vdst, A + k + lda * i);
       } else {
 #pragma unroll
@@ -584,6 +638,7 @@ __global__ void __launch_bounds__(HV_NT, HV_BPS) k_hemv_df(const zdf *Ab, int64_
           const bool ok = rt0 + tr < n && ct0 + tc + 4 * j < n;
           cp_async16(dst + 4 * j * HV_LD, ok ? (const void *)(src + 4 * j * lda) : (const void *)A, ok);
         }
+        if (first) dep_wait();
         if (tid < HV_R + HV_C) cp_async16(vdst, k < n ? (const void *)(A + k + lda * i) : (const void *)A, k < n);
       }
       ++ti;
@@ -594,13 +649,14 @@ __global__ void __launch_bounds__(HV_NT, HV_BPS) k_hemv_df(const zdf *Ab, int64_
     }
     cp_async_commit();
   };
-  issue(0);
+  issue(0, true);
   zdf y = cz<df>();  // row sum (warps 0-3)
   zdf *Pm = Pb + b * sP;
   for (int buf = 0; t < tend; ++t, buf ^= 1) {
     cp_async_wait0();
     __syncthreads();  // this tile has landed, the other buffer is free
     issue(buf ^ 1);
+    if (t + 1 == tend) dep_go();
     const zdf *tl = tiles + buf * (HV_C * HV_LD);
     const zdf *vl = vecs + buf * (HV_R + HV_C);
     const int off = HV_C * (Cc - 2 * R);  // >= 0 on the diagonal: entry (r, c) is below it for r > c + off
@@ -686,7 +742,8 @@ constexpr int CT_TPR = 8;
 template <class R>
 struct PanelRow {
   C<R> p[4], w[4], v[4], vi, a;
-  __device__ __forceinline__ void load(const PanelCol<R> &c, int r, int sub) {
+  // the mat-vec's results
+  __device__ __forceinline__ void load_p(const PanelCol<R> &c, int r, int sub) {
     const bool in = r < c.n;
     int nseg, skip;
     const int nch = c.slots(in ? r : c.i + 1, nseg, skip);
@@ -694,6 +751,14 @@ struct PanelRow {
     for (int u = 0; u < 4; ++u) {
       const int k = sub + CT_TPR * u;
       p[u] = in && k < nch ? c.P[r + (int64_t)(k + (k >= nseg ? skip : 0)) * c.ldp] : cz<R>();
+    }
+  }
+  // what was there before it
+  __device__ __forceinline__ void load_old(const PanelCol<R> &c, int r, int sub) {
+    const bool in = r < c.n;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int k = sub + CT_TPR * u;
       w[u] = in && k < c.jj ? c.W[r + c.lda * k] : cz<R>();
       v[u] = in && k < c.jj ? c.A[r + c.lda * (c.k0 + k)] : cz<R>();
     }
@@ -738,16 +803,21 @@ struct PanelRow {
     group8_sum(y, nxt);
   }
 };
-// x1 = V^H v, x2 = W^H v and row i + 1 of V and W (conjugated) into shared memory
+// row i + 1 of V and W (conjugated) and, the mat-vec's, x1 = V^H v, x2 = W^H v
+// into shared memory
 template <class R>
-__device__ __forceinline__ void panel_small(const PanelCol<R> &c, const C<R> *X, C<R> *x1, C<R> *x2, C<R> *nv, C<R> *nw) {
-  for (int k = threadIdx.x; k < c.jj; k += blockDim.x) {
-    x1[k] = X[k];
-    x2[k] = X[c.jj + k];
-    if (c.next) {
+__device__ __forceinline__ void panel_next(const PanelCol<R> &c, C<R> *nv, C<R> *nw) {
+  if (c.next)
+    for (int k = threadIdx.x; k < c.jj; k += blockDim.x) {
       nv[k] = cconj(c.A[c.i + 1 + c.lda * (c.k0 + k)]);
       nw[k] = cconj(c.W[c.i + 1 + c.lda * k]);
     }
+}
+template <class R>
+__device__ __forceinline__ void panel_x(const PanelCol<R> &c, const C<R> *X, C<R> *x1, C<R> *x2) {
+  for (int k = threadIdx.x; k < c.jj; k += blockDim.x) {
+    x1[k] = X[k];
+    x2[k] = X[c.jj + k];
   }
 }
 // A complex sum over rows of products rounded to R row by row: the three-float
@@ -800,16 +870,23 @@ __global__ void __launch_bounds__(wp_threads<R>) k_wpart(C<R> *Ab, int64_t lda, 
   const int n = nvec[b];
   const int col = i + 1;
   const int rb = col + blockIdx.x * NW * 4;
-  if (rb >= n) return;
+  if (rb >= n) {
+    dep_wait();
+    return;
+  }
   C<R> *A = Ab + b * sA;
   C<R> *W = Wb + b * sW;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sub = tid % CT_TPR;
   const PanelCol<R> pc(A, W, Pb + b * sP, lda, ldp, n, i, k0, jj, next, sms);
   const int r = rb + tid / CT_TPR;
   PanelRow<R> q;
-  q.load(pc, r, sub);
+  q.load_old(pc, r, sub);
   const C<R> tau = taub[b];
-  panel_small(pc, X + b * ldx, x1, x2, nv, nw);
+  panel_next(pc, nv, nw);
+  dep_wait();
+  q.load_p(pc, r, sub);
+  panel_x(pc, X + b * ldx, x1, x2);
+  dep_go();
   __syncthreads();
   C<R> y, nxt;
   RowSum<R> dot;
@@ -897,6 +974,7 @@ __global__ void __launch_bounds__(TR_NT) k_colstep(C<R> *Ab, int64_t lda, int64_
   const int b = blockIdx.y;
   const int n = nvec[b];
   const int col = i + 1;
+  if (do_w != 1 || col >= n) dep_wait();
   if (col >= n) return;
   cluster_arrive();  // distributed shared memory may be written once every CTA has started
   bool started = false;
@@ -930,9 +1008,12 @@ __global__ void __launch_bounds__(TR_NT) k_colstep(C<R> *Ab, int64_t lda, int64_
     const int sub = lane % CT_TPR;
     PanelRow<R> q;
     int l = warp * 4 + lane / CT_TPR;
-    q.load(pc, row_of(l), sub);
+    q.load_old(pc, row_of(l), sub);
     const C<R> tau = taub[b];
-    panel_small(pc, X + b * ldx, x1, x2, nv, nw);
+    panel_next(pc, nv, nw);
+    dep_wait();
+    q.load_p(pc, row_of(l), sub);
+    panel_x(pc, X + b * ldx, x1, x2);
     __syncthreads();
     RowSum<R> dot;
     dot.zero();
@@ -956,7 +1037,10 @@ __global__ void __launch_bounds__(TR_NT) k_colstep(C<R> *Ab, int64_t lda, int64_
         if (l == 0) wfirst = w;
       }
       l += 4 * CT_NW;
-      if (row_of(l & ~3) < n) q.load(pc, row_of(l), sub);
+      if (row_of(l & ~3) < n) {
+        q.load_old(pc, row_of(l), sub);
+        q.load_p(pc, row_of(l), sub);
+      }
     }
     // w0^H v: lanes 0, 8, 16, 24 of each warp, then all warps of the cluster
     dot.rows4();
@@ -1088,6 +1172,7 @@ __global__ void __launch_bounds__(TR_NT) k_colstep(C<R> *Ab, int64_t lda, int64_
     }
   }
   __syncthreads();
+  dep_go();
   const C<R> sc = s_scale;
   const int skip = s_skip, pe = s_e;
   for (int l = tid; row_of(l) < n; l += TR_NT) {
@@ -1215,31 +1300,23 @@ static cudaError_t launch_colstep(EigWork &w, int i, int k0, int jj, int do_w, i
   const int64_t sW = (int64_t)w.lda * w.nb, sP = (int64_t)w.nchunk * w.lda;
   if (do_w && rows > CT_SPLIT) {
     do_w = 2;
-    PP_KT(KT_COLSTEP, s, (k_wpart<R><<<dim3(cdiv(rows, wp_threads<R> / CT_TPR), w.B), wp_threads<R>, 0, s>>>(
-                             (C<R> *)w.A, w.lda, w.sA, (C<R> *)w.W, sW, (const C<R> *)w.P, sP, w.lda, w.nvec, i, k0, jj,
-                             do_next, device_sms(), (const C<R> *)w.X, 2 * w.nb, (const C<R> *)w.scal,
-                             (RowSum<R> *)w.part, w.spart * ROWSUM_BYTES / (int)sizeof(RowSum<R>))));
+    cudaError_t e = cudaSuccess;
+    PP_KT(KT_COLSTEP, s, (e = launch_dep(k_wpart<R>, dim3(cdiv(rows, wp_threads<R> / CT_TPR), w.B), wp_threads<R>, 0, 0, true,
+                                         s, (C<R> *)w.A, w.lda, w.sA, (C<R> *)w.W, sW, (const C<R> *)w.P, sP, w.lda, w.nvec,
+                                         i, k0, jj, do_next, device_sms(), (const C<R> *)w.X, 2 * w.nb,
+                                         (const C<R> *)w.scal, (RowSum<R> *)w.part,
+                                         w.spart * ROWSUM_BYTES / (int)sizeof(RowSum<R>))));
+    PP_CUDA_TRY(e);
     count_launch(1);
   }
   int cs = 1;
   while (cs < CT_CLUSTER && cs * 8 < rows && cs * std::max(w.batch, w.B) <= device_sms()) cs *= 2;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(cs, w.B);
-  cfg.blockDim = dim3(TR_NT);
-  cfg.stream = s;
-  cudaLaunchAttribute at;
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = cs;
-  at.val.clusterDim.y = at.val.clusterDim.z = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
   cudaError_t e = cudaSuccess;
-  PP_KT(KT_COLSTEP, s, (e = cudaLaunchKernelEx(&cfg, k_colstep<R>, (C<R> *)w.A, w.lda, w.sA, (C<R> *)w.W, sW,
-                                               (const C<R> *)w.P, sP, w.lda, (const int *)w.nvec, i, k0, jj, do_w,
-                                               do_next, device_sms(), (const C<R> *)w.X, 2 * w.nb,
-                                               (const RowSum<R> *)w.part,
-                                               w.spart * ROWSUM_BYTES / (int)sizeof(RowSum<R>), (C<R> *)w.scal, w.d, w.e, w.tau,
-                                               (int64_t)w.nmax)));
+  PP_KT(KT_COLSTEP, s, (e = launch_dep(k_colstep<R>, dim3(cs, w.B), TR_NT, 0, cs, do_w != 0, s, (C<R> *)w.A, w.lda, w.sA,
+                                       (C<R> *)w.W, sW, (const C<R> *)w.P, sP, w.lda, (const int *)w.nvec, i, k0, jj, do_w,
+                                       do_next, device_sms(), (const C<R> *)w.X, 2 * w.nb, (const RowSum<R> *)w.part,
+                                       w.spart * ROWSUM_BYTES / (int)sizeof(RowSum<R>), (C<R> *)w.scal, w.d, w.e, w.tau,
+                                       (int64_t)w.nmax)));
   count_launch(1);
   return e;
 }
@@ -1263,8 +1340,10 @@ cudaError_t tridiagonalize(EigWork &w, cudaStream_t s) {
         // (a smaller matrix of the batch may have more, shorter runs)
         const int nt = cdiv(nmax - i - 1, HV_R);
         const int gx = hv_dots(jj) + std::min(nt * (nt + 1), hv_ctas(jj, device_sms()));
-        PP_KT(KT_HEMV, s, (k_hemv_df<<<dim3(gx, B), HV_NT, HV_SMEM, s>>>(A, lda, sA, w.nvec, i, P, sP, lda, W, sW, k0,
-                                                                        jj, (C<R> *)w.X, 2 * nb, device_sms())));
+        cudaError_t e = cudaSuccess;
+        PP_KT(KT_HEMV, s, (e = launch_dep(k_hemv_df, dim3(gx, B), HV_NT, HV_SMEM, 0, true, s, A, lda, sA, w.nvec, i, P, sP,
+                                          lda, W, sW, k0, jj, (C<R> *)w.X, 2 * nb, device_sms())));
+        PP_CUDA_TRY(e);
         count_launch(1);
       } else {
         // (the tile follows each matrix's own order: a batch that has both kinds runs both kernels)
@@ -1272,15 +1351,19 @@ cudaError_t tridiagonalize(EigWork &w, cudaStream_t s) {
         if (rows > HL_SMALL) {
           const int nt = cdiv(rows, HL_T);
           const int gx = hl_dots(jj, HL_T) + std::min(nt * (nt + 1) / 2, hemv_blocks(w.hemv_bps));
-          PP_KT(KT_HEMV, s, (k_hemv_lower<HL_T><<<dim3(gx, 1, B), 4 * HL_T, 0, s>>>(A, lda, sA, w.nvec, i, P, sP, lda, W,
-                                                                                    sW, k0, jj, (C<R> *)w.X, 2 * nb)));
+          cudaError_t e = cudaSuccess;
+          PP_KT(KT_HEMV, s, (e = launch_dep(k_hemv_lower<HL_T>, dim3(gx, 1, B), 4 * HL_T, 0, 0, true, s, A, lda, sA, w.nvec,
+                                            i, P, sP, lda, W, sW, k0, jj, (C<R> *)w.X, 2 * nb)));
+          PP_CUDA_TRY(e);
           count_launch(1);
         }
         if (w.nmin - i - 1 <= HL_SMALL) {
           const int nt = cdiv(std::min(rows, HL_SMALL), HL_TS);
           const int gx = hl_dots(jj, HL_TS) + nt * (nt + 1) / 2;
-          PP_KT(KT_HEMV, s, (k_hemv_lower<HL_TS><<<dim3(gx, 1, B), 4 * HL_TS, 0, s>>>(A, lda, sA, w.nvec, i, P, sP, lda, W,
-                                                                                      sW, k0, jj, (C<R> *)w.X, 2 * nb)));
+          cudaError_t e = cudaSuccess;
+          PP_KT(KT_HEMV, s, (e = launch_dep(k_hemv_lower<HL_TS>, dim3(gx, 1, B), 4 * HL_TS, 0, 0, true, s, A, lda, sA,
+                                            w.nvec, i, P, sP, lda, W, sW, k0, jj, (C<R> *)w.X, 2 * nb)));
+          PP_CUDA_TRY(e);
           count_launch(1);
         }
       }
