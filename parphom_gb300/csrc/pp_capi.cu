@@ -225,6 +225,20 @@ void free_ws(pp_ctx *c) {
 
 size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 
+// Bytes of a batch's buffers with T threads of inverse iteration (0: the fewest
+// that a large order gets).
+constexpr int64_t IV_T_MIN = 2048;
+size_t ws_bytes_estimate(int64_t n, int B, int mcap, int64_t nbnd, int64_t nbr, int64_t T = 0) {
+  if (T == 0) T = std::min(invit_threads(mcap), IV_T_MIN);
+  size_t per = 16 * (size_t)n * n + 16 * (size_t)n * mcap + (8 * IV_F + 1) * (size_t)n * T +
+               16 * (size_t)n * 64 * 2 + 16 * (size_t)std::max<int64_t>((n + 255) / 256, 8) * 32 * std::max(mcap, 64) +
+               16 * (size_t)n * std::max<int64_t>(3 * ((n + 63) / 64), 8) +  // mat-vec partials
+               16 * (size_t)((n + 63) / 64) * 32 * 32 + her2k_tc_bytes(n) + 8 * (size_t)(n + 128) +
+               8 * 8 * 3 * (size_t)mcap + 16 * 3 * (size_t)nbnd + 16 * (size_t)nbr * (n + mcap) +
+               16 * 1024 * (size_t)std::max<int64_t>(1, (n + 30) / 32);  // compact-WY factors of all panels
+  return per * B;
+}
+
 // Carve every batch buffer out of one allocation.
 int ensure_ws_sized(pp_ctx *c, int B, int mcap, int64_t n, int64_t nbnd_max, int64_t nbr_max) {
   if (c->ws && B <= c->cap_B && mcap <= c->cap_m && n == c->cap_n && nbnd_max <= c->cap_nbnd &&
@@ -235,7 +249,11 @@ int ensure_ws_sized(pp_ctx *c, int B, int mcap, int64_t n, int64_t nbnd_max, int
   const int64_t lda = (n + 7) / 8 * 8;
   // mat-vec partial slots: n/32, n/16 up to 128 rows (FP64 form), 3 ceil(n/64) (double-float form)
   const int nchunk = (int)std::max<int64_t>(3 * ((n + 63) / 64), 8);
-  const int64_t T = std::min<int64_t>(((int64_t)mcap + 63) / 64 * 64, 2048);
+  // inverse iteration: a thread for every eigenvector where memory allows
+  size_t fr = 0, tot = 0;
+  cudaMemGetInfo(&fr, &tot);
+  int64_t T = invit_threads(mcap);
+  if (ws_bytes_estimate(n, B, mcap, nbnd_max, nbr_max, T) > (size_t)(0.6 * (double)fr)) T = std::min(T, IV_T_MIN);
   const int nbr = (int)nbr_max;
   const int ldwp = std::max(std::max(mcap, nbr), 64);
   // split-K partials: 8 chunks of 32 x ldwp, or one per 256 rows
@@ -278,7 +296,7 @@ int ensure_ws_sized(pp_ctx *c, int B, int mcap, int64_t n, int64_t nbnd_max, int
   add((void **)&w.tinfo, 8 * (size_t)B * 8);
   add((void **)&w.cls, 4 * (size_t)B * (n + 1));
   add((void **)&w.ncl, 4 * (size_t)B);
-  add((void **)&w.scratch, 8 * (size_t)B * 5 * n * T);
+  add((void **)&w.scratch, 8 * (size_t)B * IV_F * n * T);
   add((void **)&w.piv, (size_t)B * n * T);
   add((void **)&w.info, 8 * (size_t)B);
   const int64_t npan = std::max<int64_t>(1, (n - 1 + nb - 1) / nb);
@@ -328,17 +346,6 @@ int ensure_ws_sized(pp_ctx *c, int B, int mcap, int64_t n, int64_t nbnd_max, int
 
 int ensure_ws(pp_ctx *c, int B, int mcap) { return ensure_ws_sized(c, B, mcap, c->g.n, c->g.nbnd, c->g.nbrows); }
 
-size_t ws_bytes_estimate(int64_t n, int B, int mcap, int64_t nbnd, int64_t nbr) {
-  const int64_t T = std::min<int64_t>(((int64_t)mcap + 63) / 64 * 64, 2048);
-  size_t per = 16 * (size_t)n * n + 16 * (size_t)n * mcap + 8 * (size_t)5 * n * T + (size_t)n * T +
-               16 * (size_t)n * 64 * 2 + 16 * (size_t)std::max<int64_t>((n + 255) / 256, 8) * 32 * std::max(mcap, 64) +
-               16 * (size_t)n * std::max<int64_t>(3 * ((n + 63) / 64), 8) +  // mat-vec partials
-               16 * (size_t)((n + 63) / 64) * 32 * 32 + her2k_tc_bytes(n) + 8 * (size_t)(n + 128) +
-               8 * 8 * 3 * (size_t)mcap + 16 * 3 * (size_t)nbnd + 16 * (size_t)nbr * (n + mcap) +
-               16 * 1024 * (size_t)std::max<int64_t>(1, (n + 30) / 32);  // compact-WY factors of all panels
-  return per * B;
-}
-
 int check_opts(const pp_ctx *c, const pp_eig_opts *o) {
   if (!o) return -5;
   if (o->jobz != 'N' && o->jobz != 'V') return -5;
@@ -379,7 +386,7 @@ EigWork view_of(const EigWork &w, int off, int cnt) {
   v.tinfo = (double *)sh(w.tinfo, 8 * 8);
   v.cls = (int *)sh(w.cls, 4 * (nmax + 1));
   v.ncl = (int *)sh(w.ncl, 4);
-  v.scratch = (double *)sh(w.scratch, 8 * 5 * nmax * (size_t)T);
+  v.scratch = (double *)sh(w.scratch, 8 * IV_F * nmax * (size_t)T);
   v.piv = (uint8_t *)sh(w.piv, nmax * (size_t)T);
   v.info = (int64_t *)sh(w.info, 8);
   v.Tf = (z64 *)sh(w.Tf, 16 * 1024);  // panel stride sTfp unchanged

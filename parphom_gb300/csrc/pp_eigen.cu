@@ -1835,42 +1835,58 @@ __device__ __forceinline__ uint32_t hash32(uint32_t x) {
   return x;
 }
 
+// 1/x, |x| in the middle of the exponent range: the hardware's estimate and one
+// step of third order (Halley's iteration, r (1 + e + e^2) with e = 1 - x r).
+// Three dependent FP64 operations where a division waits 560 cycles.
+__device__ __forceinline__ double recip(double x) {
+  if ((unsigned)((__double2hiint(x) >> 20 & 0x7ff) - 23) >= 2000u) return 1.0 / x;
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-x, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+
 // One thread per cluster of eigenvalues (clusters cbase .. cbase+T-1).
-// LU of T - lam I with partial pivoting: row k of U holds (u0,u1,u2) at
-// columns (k, k+1, k+2); l is the multiplier, piv marks a row interchange.
-// The factors and the working vector x live in scratch interleaved by thread
-// ([row][field][thread]) so that a warp's accesses coalesce; the finished
-// vector is written to its column of E once.  Every pass over the rows runs
-// in chunks of IV_CH rows whose loads are all issued before the chunk's
-// arithmetic and stores: the recurrences are sequential in the row, and a
-// load behind a store to the same scratch array would otherwise wait out one
-// memory latency per row.  The arithmetic and its order are those of the
-// row-by-row loops.
-constexpr int IV_F = 5;   // u0, u1, u2, l, x
-constexpr int IV_CH = 8;  // rows per chunk
+// LU of T - lam I with partial pivoting: row k of U holds 1/u0, u1 and u2 (u2 =
+// e(k+1) after a row interchange, else 0) at columns (k, k+1, k+2); l is the
+// multiplier, piv marks an interchange.  The factors and the working vector x
+// live in scratch, a block's rows in one piece ([row][field][thread]: a warp's
+// accesses coalesce and have constant offsets in an unrolled loop); the
+// finished vector is written to its column of E once.
+// Bound by latency and the instructions of one warp: everything is a recurrence
+// over the rows, at 64-85 cycles per dependent FP64 operation (and 16 cycles of
+// the SM's FP64 pipe per warp, so a block is one warp).  Hence five passes over
+// the rows -- the first right-hand side is eliminated along with the matrix,
+// norm and largest component are taken in the U solve, the scaling goes with
+// the next pass -- one multiply-add per row on the U solve's chain, reciprocals
+// instead of divisions, and each pass requests IV_CH rows ahead of those it
+// works on.  n = 2604, all vectors of 4 matrices, with the reorthogonalisation:
+// 12.5 ms before (two launches: 2048 threads at most, twelve passes), 4.6 ms
+// now; chunks of 8 rows 5.4 ms (registers); the rows of all threads
+// interleaved, whose addresses took most of 430 instructions per row, 7.5 ms.
+constexpr int IV_CH = 4;  // rows per chunk
+constexpr int IV_NT = 32;
 template <class R>
-__global__ void __launch_bounds__(64) k_invit(const double *__restrict__ dd, const double *__restrict__ ee, int64_t sd,
-                                              const int *nvec, const double *ww, const int64_t *rng,
-                                              const double *tinfo, const int *cls, int64_t scl, const int *ncl,
-                                              int cbase, C<R> *Eb, int64_t lde, int64_t sE, double *scratch,
-                                              uint8_t *pivb, int64_t T, int64_t sS, int64_t sPv, int64_t *info) {
+__global__ void __launch_bounds__(IV_NT) k_invit(const double *__restrict__ dd, const double *__restrict__ ee, int64_t sd,
+                                                 const int *nvec, const double *ww, const int64_t *rng,
+                                                 const double *tinfo, const int *cls, int64_t scl, const int *ncl,
+                                                 int cbase, int nmax, C<R> *Eb, int64_t lde, int64_t sE, double *scratch,
+                                                 uint8_t *pivb, int64_t sS, int64_t sPv, int64_t *info) {
   const int b = blockIdx.y;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int c = cbase + t;
-  if (t >= T || c >= ncl[b]) return;
+  const int c = cbase + blockIdx.x * IV_NT + threadIdx.x;
+  if (c >= ncl[b]) return;
   const int n = nvec[b];
   const double *__restrict__ d = dd + b * sd;
   const double *__restrict__ e = ee + b * sd;
   const double *w = ww + b * sd;
   C<R> *E = Eb + b * sE;
-  double *S = scratch + b * sS;
-  uint8_t *PV = pivb + b * sPv;
-#define SU0(k) S[((int64_t)(k)*IV_F + 0) * T + t]
-#define SU1(k) S[((int64_t)(k)*IV_F + 1) * T + t]
-#define SU2(k) S[((int64_t)(k)*IV_F + 2) * T + t]
-#define SL(k) S[((int64_t)(k)*IV_F + 3) * T + t]
-#define XS(k) S[((int64_t)(k)*IV_F + 4) * T + t]
-#define PIV(k) PV[(int64_t)(k)*T + t]
+  double *S = scratch + b * sS + (int64_t)blockIdx.x * nmax * (IV_F * IV_NT) + threadIdx.x;
+  uint8_t *PV = pivb + b * sPv + (int64_t)blockIdx.x * nmax * IV_NT + threadIdx.x;
+#define SR0(k) S[(int64_t)(k) * (IV_F * IV_NT)]
+#define SU1(k) S[(int64_t)(k) * (IV_F * IV_NT) + IV_NT]
+#define SL(k) S[(int64_t)(k) * (IV_F * IV_NT) + 2 * IV_NT]
+#define XS(k) S[(int64_t)(k) * (IV_F * IV_NT) + 3 * IV_NT]
+#define PIV(k) PV[(int64_t)(k) * IV_NT]
   const double tnorm = tinfo[b * 8 + 2];
   const double eps = DBL_EPSILON * 0.5;
   const double pivtol = fmax(eps * tnorm, DBL_MIN);
@@ -1878,6 +1894,37 @@ __global__ void __launch_bounds__(64) k_invit(const double *__restrict__ dd, con
   const int iters = (j1 - j0 > 1) ? 3 : 2;
   double lam_prev = 0.0;
   int bad = 0;
+  struct Row {
+    double x, a, u;
+    uint8_t pv;
+  };
+  // rows 0, 1, ... of a pass in chunks, the next chunk's loads ahead of this one's work
+  auto pass = [](int rows, auto load, auto work) {
+    Row qa[IV_CH], qb[IV_CH];
+    auto load_chunk = [&](Row(&q)[IV_CH], int kb) {
+#pragma unroll
+      for (int u = 0; u < IV_CH; ++u) load(q[u], kb + u);
+    };
+    auto work_chunk = [&](Row(&q)[IV_CH], int kb) {
+#pragma unroll
+      for (int u = 0; u < IV_CH; ++u) work(q[u], kb + u);
+    };
+    const int full = rows / IV_CH * IV_CH;
+    if (full > 0) load_chunk(qa, 0);
+#pragma unroll 1
+    for (int kb = 0; kb < full; kb += 2 * IV_CH) {
+      if (kb + IV_CH < full) load_chunk(qb, kb + IV_CH);
+      work_chunk(qa, kb);
+      if (kb + IV_CH >= full) break;
+      if (kb + 2 * IV_CH < full) load_chunk(qa, kb + 2 * IV_CH);
+      work_chunk(qb, kb + IV_CH);
+    }
+#pragma unroll 1
+    for (int k = full; k < rows; ++k) {
+      load(qa[0], k);
+      work(qa[0], k);
+    }
+  };
   for (int j = j0; j < j1; ++j) {
     double lam = w[j];
     if (j > j0) {
@@ -1885,218 +1932,148 @@ __global__ void __launch_bounds__(64) k_invit(const double *__restrict__ dd, con
       if (lam <= lam_prev + pert) lam = lam_prev + pert;
     }
     lam_prev = lam;
-    // ---- factor T - lam I
-    double p = d[0] - lam, qv = (n > 1) ? e[0] : 0.0;
-    for (int kb = 0; kb < n - 1; kb += IV_CH) {
-      double ck[IV_CH], dk1[IV_CH], bk[IV_CH];
-#pragma unroll
-      for (int u = 0; u < IV_CH; ++u) {
-        const int k = kb + u;
-        ck[u] = k < n - 1 ? e[k] : 0.0;
-        dk1[u] = k < n - 1 ? d[k + 1] : 0.0;
-        bk[u] = k + 1 < n - 1 ? e[k + 1] : 0.0;
-      }
-#pragma unroll
-      for (int u = 0; u < IV_CH; ++u) {
-        const int k = kb + u;
-        if (k >= n - 1) break;
-        const double ak1 = dk1[u] - lam;
-        double u0, u1, u2, l, pn, qn, r0;
-        uint8_t sw;
-        // one FP64 division per row (FP64 is the scarce pipe): l from the
-        // pivot's reciprocal, and U is stored with 1/u0 so that the U solves
-        // multiply
-        if (fabs(p) >= fabs(ck[u])) {
-          r0 = (p == 0.0) ? 0.0 : 1.0 / p;
-          l = ck[u] * r0;
-          u0 = p;
-          u1 = qv;
-          u2 = 0.0;
-          pn = ak1 - l * qv;
-          qn = bk[u];
-          sw = 0;
-        } else {
-          r0 = 1.0 / ck[u];
-          l = p * r0;
-          u0 = ck[u];
-          u1 = ak1;
-          u2 = bk[u];
-          pn = qv - l * ak1;
-          qn = -l * bk[u];
-          sw = 1;
-        }
-        SU0(k) = (fabs(u0) < pivtol) ? 1.0 / copysign(pivtol, u0) : r0;  // 1 / guarded pivot
-        SU1(k) = u1;
-        SU2(k) = u2;
-        SL(k) = l;
-        PIV(k) = sw;
-        p = pn;
-        qv = qn;
-      }
-    }
-    SU0(n - 1) = 1.0 / ((fabs(p) < pivtol) ? copysign(pivtol, p) : p);
-    SU1(n - 1) = 0.0;
-    SU2(n - 1) = 0.0;
-    // ---- deterministic start vector in (-1, 1)
-    // seeded by the eigenvalue index only: results do not depend on the batch slot
+    // deterministic start vector in (-1, 1), seeded by the eigenvalue index
+    // only: results do not depend on the batch slot.  (1 + 24 bits 2^-24 by its
+    // bits, to (-1, 1))
     const uint32_t seed = hash32((uint32_t)j * 2654435761u ^ 0x9e3779b9u);
-    for (int k = 0; k < n; ++k) {
+    auto start = [&](int k) {
       const uint32_t h = hash32(seed + (uint32_t)k * 0x85ebca6bu);
-      XS(k) = ((double)(h >> 8) * (1.0 / 16777216.0)) * 2.0 - 1.0;
-    }
-    bool ok = true;
+      return fma(__hiloint2double(0x3ff00000 | (int)(h >> 12), (int)((h & 0xf00u) << 20)), 2.0, -3.0);
+    };
+    // ---- factor T - lam I, and L x = (start vector) with the interchanges
+    double p = d[0] - lam, qv = (n > 1) ? e[0] : 0.0, ck = qv, xk = start(0);
+    pass(
+        n - 1,
+        [&](Row &q, int k) {
+          q.x = e[k + 1];  // (row n - 2: not part of T)
+          q.a = d[k + 1];
+        },
+        [&](const Row &q, int k) {
+          const double bk = k + 1 < n - 1 ? q.x : 0.0, ak1 = q.a - lam;
+          const double x1 = start(k + 1);
+          const bool sw = !(fabs(p) >= fabs(ck));
+          const double u0 = sw ? ck : p, r0 = u0 == 0.0 ? 0.0 : recip(u0);
+          const double l = (sw ? p : ck) * r0;
+          SR0(k) = (fabs(u0) < pivtol) ? 1.0 / copysign(pivtol, u0) : r0;  // 1 / guarded pivot
+          SU1(k) = sw ? ak1 : qv;
+          SL(k) = l;
+          PIV(k) = sw;
+          p = sw ? fma(-l, ak1, qv) : fma(-l, qv, ak1);
+          qv = sw ? -l * bk : bk;
+          XS(k) = sw ? x1 : xk;
+          xk = sw ? fma(-l, x1, xk) : fma(-l, xk, x1);
+          ck = bk;
+        });
+    const double rlast = 1.0 / ((fabs(p) < pivtol) ? copysign(pivtol, p) : p);
+    bool ok = true, neg = false;
+    double sc = 1.0;  // the vector is sc x
+#pragma unroll 1
     for (int it = 0; it < iters && ok; ++it) {
-      // L solve with the recorded interchanges (x(k+1) of a chunk is read
-      // before x(k) is overwritten, as in the row-by-row loop)
-      double xk = XS(0);
-      for (int kb = 0; kb < n - 1; kb += IV_CH) {
-        double x1[IV_CH], l[IV_CH];
-        uint8_t pv[IV_CH];
-#pragma unroll
-        for (int u = 0; u < IV_CH; ++u) {
-          const int k = kb + u;
-          const bool in = k < n - 1;
-          x1[u] = in ? XS(k + 1) : 0.0;
-          l[u] = in ? SL(k) : 0.0;
-          pv[u] = in ? PIV(k) : (uint8_t)0;
-        }
-#pragma unroll
-        for (int u = 0; u < IV_CH; ++u) {
-          const int k = kb + u;
-          if (k >= n - 1) break;
-          if (pv[u]) {
-            XS(k) = x1[u];
-            xk = xk - l[u] * x1[u];
-          } else {
-            XS(k) = xk;
-            xk = x1[u] - l[u] * xk;
-          }
-        }
+      if (it > 0) {  // L solve
+        xk = XS(0) * sc;
+        pass(
+            n - 1,
+            [&](Row &q, int k) {
+              q.x = XS(k + 1);
+              q.a = SL(k);
+              q.pv = PIV(k);
+            },
+            [&](const Row &q, int k) {
+              const double x1 = q.x * sc;
+              XS(k) = q.pv ? x1 : xk;
+              xk = q.pv ? fma(-q.a, x1, xk) : fma(-q.a, xk, x1);
+            });
       }
-      XS(n - 1) = xk;
-      // U solve
-      double y1 = 0.0, y2 = 0.0, amax = 0.0;
-      for (int kt = n - 1; kt >= 0; kt -= IV_CH) {
-        double xv[IV_CH], a0[IV_CH], a1[IV_CH], a2[IV_CH];
-#pragma unroll
-        for (int u = 0; u < IV_CH; ++u) {
-          const int k = kt - u;
-          const bool in = k >= 0;
-          xv[u] = in ? XS(k) : 0.0;
-          a0[u] = in ? SU0(k) : 0.0;
-          a1[u] = in ? SU1(k) : 0.0;
-          a2[u] = in ? SU2(k) : 0.0;
-        }
-#pragma unroll
-        for (int u = 0; u < IV_CH; ++u) {
-          const int k = kt - u;
-          if (k < 0) break;
-          const double y = (xv[u] - a1[u] * y1 - a2[u] * y2) * a0[u];
-          XS(k) = y;
-          amax = fmax(amax, fabs(y));
-          y2 = y1;
-          y1 = y;
-        }
-      }
+      // U solve from the last row up: y = x/u0 - (u1/u0) y1 - (u2/u0) y2, its
+      // squares and its largest component (by its bits; the first of equals)
+      double y1 = xk * rlast, y2 = 0.0, nrm2 = y1 * y1;
+      long long big = __double_as_longlong(fabs(y1));
+      neg = y1 < 0.0;
+      XS(n - 1) = y1;
+      pass(
+          n - 1,
+          [&](Row &q, int i) {
+            const int k = n - 2 - i;
+            q.x = XS(k);
+            q.a = SR0(k);
+            q.u = SU1(k);
+            q.pv = PIV(k);
+          },
+          [&](const Row &q, int i) {
+            const int k = n - 2 - i;
+            const double u2 = q.pv && i > 0 ? e[k + 1] : 0.0;
+            const double y = fma(-(q.u * q.a), y1, fma(-(u2 * q.a), y2, q.x * q.a));
+            XS(k) = y;
+            nrm2 = fma(y, y, nrm2);
+            const long long m = __double_as_longlong(fabs(y));
+            if (m >= big) {
+              big = m;
+              neg = __double2hiint(y) < 0;
+            }
+            y2 = y1;
+            y1 = y;
+          });
+      const double amax = __longlong_as_double(big);
       if (!(amax > 0.0) || !isfinite(amax)) {
         ok = false;
         break;
       }
       const double inv = 1.0 / amax;
       // modified Gram-Schmidt against the earlier members of the cluster
-      for (int pass = 0; pass < 2 && j > j0; ++pass) {
+      for (int rep = 0; rep < 2 && j > j0; ++rep) {
         for (int jp = j0; jp < j; ++jp) {
           double dot = 0.0;
-          for (int kb = 0; kb < n; kb += IV_CH) {
-            double ev[IV_CH], xv[IV_CH];
-#pragma unroll
-            for (int u = 0; u < IV_CH; ++u) {
-              const int k = kb + u;
-              const bool in = k < n;
-              ev[u] = in ? RT<R>::to(E[k + lde * jp].re) : 0.0;
-              xv[u] = in ? XS(k) : 0.0;
-            }
-#pragma unroll
-            for (int u = 0; u < IV_CH; ++u)
-              if (kb + u < n) dot += ev[u] * xv[u];
-          }
-          for (int kb = 0; kb < n; kb += IV_CH) {
-            double ev[IV_CH], xv[IV_CH];
-#pragma unroll
-            for (int u = 0; u < IV_CH; ++u) {
-              const int k = kb + u;
-              const bool in = k < n;
-              ev[u] = in ? RT<R>::to(E[k + lde * jp].re) : 0.0;
-              xv[u] = in ? XS(k) : 0.0;
-            }
-#pragma unroll
-            for (int u = 0; u < IV_CH; ++u)
-              if (kb + u < n) XS(kb + u) = xv[u] - dot * ev[u];
-          }
+          auto load = [&](Row &q, int k) {
+            q.a = RT<R>::to(E[k + lde * jp].re);
+            q.x = XS(k);
+          };
+          pass(n, load, [&](const Row &q, int) { dot += q.a * q.x; });
+          pass(n, load, [&](const Row &q, int k) { XS(k) = q.x - dot * q.a; });
         }
       }
-      double nrm2 = 0.0;
-      for (int kb = 0; kb < n; kb += IV_CH) {
-        double xv[IV_CH];
-#pragma unroll
-        for (int u = 0; u < IV_CH; ++u) xv[u] = kb + u < n ? XS(kb + u) : 0.0;
-#pragma unroll
-        for (int u = 0; u < IV_CH; ++u) {
-          if (kb + u < n) {
-            const double v = xv[u] * inv;
-            nrm2 += v * v;
-          }
+      sc = 1.0;
+      if (j > j0 || !(nrm2 > 1e-280 && nrm2 < 1e280)) {
+        // the norm of what is left, scaled (or of squares out of range)
+        sc = inv;
+        nrm2 = 0.0;
+        double left = -1.0;
+        pass(
+            n, [&](Row &q, int k) { q.x = XS(k); },
+            [&](const Row &q, int) {
+              const double v = q.x * inv;
+              nrm2 += v * v;
+              if (fabs(v) > left) {
+                left = fabs(v);
+                neg = v < 0.0;
+              }
+            });
+        if (!(nrm2 > 1e-280)) {
+          ok = false;
+          break;
         }
       }
-      if (!(nrm2 > 1e-280)) {
-        ok = false;
-        break;
-      }
-      const double sc = inv / sqrt(nrm2);
-      for (int kb = 0; kb < n; kb += IV_CH) {
-        double xv[IV_CH];
-#pragma unroll
-        for (int u = 0; u < IV_CH; ++u) xv[u] = kb + u < n ? XS(kb + u) : 0.0;
-#pragma unroll
-        for (int u = 0; u < IV_CH; ++u)
-          if (kb + u < n) XS(kb + u) = xv[u] * sc;
-      }
+      sc = sc / sqrt(nrm2);
     }
     if (!ok) bad = 1;
     // sign convention of dstein: the largest component is positive
-    double big = -1.0;
-    int kbig = 0;
-    for (int kb = 0; kb < n; kb += IV_CH) {
-      double xv[IV_CH];
-#pragma unroll
-      for (int u = 0; u < IV_CH; ++u) xv[u] = kb + u < n ? XS(kb + u) : 0.0;
-#pragma unroll
-      for (int u = 0; u < IV_CH; ++u) {
-        const double v = fabs(xv[u]);
-        if (kb + u < n && v > big) {
-          big = v;
-          kbig = kb + u;
-        }
-      }
-    }
-    const double sgn = XS(kbig) < 0.0 ? -1.0 : 1.0;
-    for (int kb = 0; kb < n; kb += IV_CH) {
-      double xv[IV_CH];
-#pragma unroll
-      for (int u = 0; u < IV_CH; ++u) xv[u] = kb + u < n ? XS(kb + u) : 0.0;
-#pragma unroll
-      for (int u = 0; u < IV_CH; ++u)
-        if (kb + u < n) E[kb + u + lde * j] = cfrom64<R>(xv[u] * sgn, 0.0);
-    }
+    const double ws = neg ? -sc : sc;
+    C<R> *Ej = E + lde * j;
+    pass(
+        n, [&](Row &q, int k) { q.x = XS(k); },
+        [&](const Row &q, int k) { Ej[k] = cfrom64<R>(q.x * ws, 0.0); });
   }
   if (bad) atomicOr((unsigned long long *)&info[b], (unsigned long long)PP_INFO_NOORTH);
-#undef SU0
+#undef SR0
 #undef SU1
-#undef SU2
 #undef SL
 #undef XS
 #undef PIV
 }
+
+// Threads of k_invit with scratch for an eigenvector each, out of mcap: a
+// thread's time is that of the whole recurrence, so a second launch for the
+// rest costs as much as the first (n = 2604: 5.5 ms for 556 of 2604).
+int64_t invit_threads(int64_t mcap) { return std::min<int64_t>((mcap + 63) / 64 * 64, 6144); }
 
 template <class R>
 cudaError_t tridiag_eigenvectors(EigWork &w, cudaStream_t s) {
@@ -2108,10 +2085,10 @@ cudaError_t tridiag_eigenvectors(EigWork &w, cudaStream_t s) {
   const int64_t sS = (int64_t)IV_F * w.nmax * T;
   const int64_t sPv = (int64_t)w.nmax * T;
   for (int64_t cb = 0; cb < w.mcap; cb += T) {
-    dim3 g(cdiv(T, 64), w.B);
-    PP_KT(KT_INVIT, s, (k_invit<R><<<g, 64, 0, s>>>(w.d, w.e, sd, w.nvec, w.w, w.rng, w.tinfo, w.cls, scl, w.ncl,
-                                                    (int)cb, (C<R> *)w.E, w.lde, w.sE, w.scratch, w.piv, T, sS, sPv,
-                                                    w.info)));
+    dim3 g(cdiv(std::min<int64_t>(T, w.mcap - cb), IV_NT), w.B);
+    PP_KT(KT_INVIT, s, (k_invit<R><<<g, IV_NT, 0, s>>>(w.d, w.e, sd, w.nvec, w.w, w.rng, w.tinfo, w.cls, scl, w.ncl,
+                                                    (int)cb, w.nmax, (C<R> *)w.E, w.lde, w.sE, w.scratch, w.piv, sS,
+                                                    sPv, w.info)));
     count_launch(1);
   }
   k_clusters<<<w.B, CL_NT, 0, s>>>(w.w, sd, w.rng, w.tinfo, w.cls, scl, w.ncl, 1e-5);

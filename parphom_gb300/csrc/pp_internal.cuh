@@ -36,6 +36,11 @@ void kt_end(int k, cudaStream_t s);
     if (on__) pp::kt_end((k), (s));                 \
   } while (0)
 
+// Inverse iteration: fields of scratch per row and thread, and the threads that
+// get scratch for mcap eigenvectors.
+constexpr int IV_F = 4;  // 1/u0, u1, l, x
+int64_t invit_threads(int64_t mcap);
+
 // Per-batch state of the eigensolver.  Every matrix b of a batch of `B`
 // Hermitian matrices has its own order nvec[b] <= nmax; all buffers use the
 // leading dimensions of the largest.  Complex buffers hold 16-byte elements:
@@ -72,7 +77,7 @@ struct EigWork {
   double *tinfo = nullptr;// [B][8]  gl, gu, tnorm, pivmin
   int *cls = nullptr;     // [B][nmax+1] cluster starts
   int *ncl = nullptr;     // [B]
-  double *scratch = nullptr; // inverse-iteration LU factors and vector [B][5*nmax*T]
+  double *scratch = nullptr; // inverse-iteration LU factors and vector [B][IV_F*nmax*T]
   uint8_t *piv = nullptr;    // inverse-iteration pivot flags [B][nmax*T]
   int64_t scratch_threads = 0;  // T: clusters handled per launch
   int64_t *info = nullptr;   // [B] info bits
