@@ -2169,14 +2169,17 @@ __global__ void __launch_bounds__(BT_NT) k_vhx(const C<R> *Ab, int64_t lda, int6
 // Y = Tf^H (V^H X); written to Wb.
 // Block of BR_NT threads = 32 columns j x 8 groups of panel rows a (a = g,
 // g + 8, g + 16, g + 24): the partials are summed into shared memory, then
-// every thread forms its four rows of the product with Tf.
+// every thread forms its four rows of the product with Tf.  (Tf is converted to
+// R once per block: with the conversion at each use the FP64 pipe bound the
+// double-float form: n = 2604, 4 matrices 132 -> 38 us a panel, n = 4764, 8
+// matrices 147 -> 51 us.)
 constexpr int BR_NT = 256;
 template <class R>
 __global__ void __launch_bounds__(BR_NT) k_btred(const C<R> *Wp, int64_t ldwp, int64_t sWp, const int *nvec,
                                                  const int64_t *rng, int k0, int jb, int mode, const z64 *Tf,
                                                  C<R> *Wb, int64_t sWb, int ncol_fixed, int rch, int nks_fixed = 0) {
   __shared__ C<R> col[32][33];
-  __shared__ z64 sT[32][33];
+  __shared__ C<R> sT[32][33];
   const int b = blockIdx.y;
   const int n = nvec[b];
   const int ncol = ncol_fixed > 0 ? ncol_fixed : (int)rng[b * 8 + 2];
@@ -2184,7 +2187,7 @@ __global__ void __launch_bounds__(BR_NT) k_btred(const C<R> *Wp, int64_t ldwp, i
   const int nks = nks_fixed > 0 ? (n - k0 - 1 > 0 ? nks_fixed : 0) : (n - k0 - 1 + rch - 1) / rch;
   const int j0 = blockIdx.x * 32;
   if (j0 >= ncol || nks <= 0) return;
-  for (int e = threadIdx.x; e < 32 * 32; e += BR_NT) sT[e / 32][e % 32] = Tf[b * 1024 + e];
+  for (int e = threadIdx.x; e < 32 * 32; e += BR_NT) sT[e / 32][e % 32] = cfrom64<R>(Tf[b * 1024 + e]);
   const int jl = threadIdx.x & 31, g = threadIdx.x >> 5;
   const int j = j0 + jl;
   for (int a = g; a < jb; a += 8) {
@@ -2198,9 +2201,9 @@ __global__ void __launch_bounds__(BR_NT) k_btred(const C<R> *Wp, int64_t ldwp, i
   for (int a = g; a < jb; a += 8) {
     C<R> acc = cz<R>();
     if (mode == 1) {
-      for (int a2 = a; a2 < jb; ++a2) cmac(acc, cfrom64<R>(sT[a][a2]), col[a2][jl]);
+      for (int a2 = a; a2 < jb; ++a2) cmac(acc, sT[a][a2], col[a2][jl]);
     } else {  // mode 2: Tf^H (lower triangular)
-      for (int a2 = 0; a2 <= a; ++a2) cmac(acc, cfrom64<R>(zconj(sT[a2][a])), col[a2][jl]);
+      for (int a2 = 0; a2 <= a; ++a2) cmac(acc, cconj(sT[a2][a]), col[a2][jl]);
     }
     Wb[b * sWb + (int64_t)a * ldwp + j] = cfin(acc);
   }
