@@ -349,10 +349,10 @@ def main():
         torch.distributed.destroy_process_group()
 
 
-# DRAM bytes (read + write) over algorithmic bytes of one k_hemv_lower launch,
-# measured with ncu --set full at N=1588, batch 4, column 300: 695.7 MB for
-# 637.5 MB (reads 1.032x; the partial sums written for the w-completion 5.9%).
-HEMV_TRAFFIC_RATIO = 1.091
+# DRAM bytes (read + write) over algorithmic bytes of one k_hemv_df launch,
+# measured with ncu on one matrix of order 4764, first columns: 191 MB read and
+# 4.5 MB written (the partial sums) for 180.3 MB.
+HEMV_TRAFFIC_RATIO = 1.084
 
 
 def roofline_for(kclass, rec, n, nq):
@@ -370,12 +370,12 @@ def roofline_for(kclass, rec, n, nq):
         # block once: m(m+1)/2 16-byte elements, m = n-i-1
         byts = nq * 16.0 * sum((n - i - 1) * (n - i) / 2 for i in range(n - 1))
         ach = byts / (ms / 1e3) / 1e9
-        return {"bound": "hbm", "kernel": "k_hemv_lower (double-float Hermitian mat-vec, lower triangle)",
+        return {"bound": "hbm", "kernel": "k_hemv_df (double-float Hermitian mat-vec, lower triangle)",
                 "achieved": ach, "peak": hbm,
                 "unit": "GB/s", "frac": ach / hbm, "peak_source": src,
                 "traffic": HEMV_TRAFFIC_RATIO * byts / launches,
-                "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch (column 300, "
-                                  "batch 4) = 1.091 x its algorithmic bytes, scaled to this average launch",
+                "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch (one matrix, "
+                                  "first columns) = 1.084 x its algorithmic bytes, scaled to this average launch",
                 "launches": launches, "avg_launch_ms": ms / launches,
                 "algorithmic_bytes_per_launch": byts / launches}
     # FP32-pipe kernels (double-float arithmetic): count complex MACs
