@@ -24,13 +24,12 @@
 // The tile kernel (k_cupd_tc) takes 128 rows x a few column blocks of 64, one
 // CTA per SM: see there.
 #include <algorithm>
-#include <cfloat>
 #include <cstdint>
 #include <cstdlib>
 #include <mutex>
 #include <cuda_bf16.h>
-#include <cuda_fp16.h>
 
+#include "pp_digits.cuh"
 #include "pp_internal.cuh"
 #include "pp_tc.cuh"
 
@@ -43,11 +42,6 @@ constexpr int TC_KS = 4;                         // k-steps of 16 (K = 64 reals)
 constexpr int TC_TILE = 4096;                    // one (slice, k-step) tile of 128 rows
 constexpr int TC_OP = TC_S * TC_KS * TC_TILE;    // one operand of a 128-row block (114688)
 constexpr int TC_RBLK = 2 * TC_OP;               // V and W operands of a 128-row block
-
-// 2^e as a float (exact for -126 <= e <= 127)
-__device__ __forceinline__ float pow2f(int e) {
-  return (e >= -126 && e <= 127) ? __int_as_float((e + 127) << 23) : ldexpf(1.0f, e);
-}
 
 // Slices of one operand row held by a warp: lane a has the complex value of
 // panel column a; K index a (real part) and 32 + a (imaginary part).
@@ -110,31 +104,6 @@ __global__ void __launch_bounds__(128) k_tc_slices(TcSliceSrc src, const int *nv
   if (lane == 0) E[b * sE + (int64_t)rl * es + eo] = e;
 }
 
-// s += a 2^-8U for one group of the sum over u of a_u 2^-8u, in the order
-// u = 6, 5, 4, 0, 1, 2, 3.  The a_u are integers of at most 2^24 in magnitude.
-// Groups 4-6 add up in float (rounding error below 2^-32 of the unit of group
-// 0).  In groups 1-3 s.hi is a multiple of 2^-8(U-1) and so of ulp(a 2^-8U),
-// which makes the three-operation sum exact without an ordering by magnitude.
-template <int U>
-__device__ __forceinline__ void fold_group(df &s, float a) {
-  constexpr float w = 1.f / (float)((uint64_t)1 << (8 * U));
-  if (U == 6)
-    s.lo = __fmul_rn(a, w);
-  else if (U >= 4)
-    s.lo = __fmaf_rn(a, w, s.lo);
-  else if (U == 0)
-    s.hi = a;
-  else {
-    const float h = __fmaf_rn(a, w, s.hi);
-    s.lo = __fadd_rn(s.lo, __fmaf_rn(a, w, __fsub_rn(s.hi, h)));
-    s.hi = h;
-  }
-}
-__device__ __forceinline__ df fold_done(df s) {
-  df r;
-  two_sum(s.hi, s.lo, r.hi, r.lo);
-  return r;
-}
 // One operand of a product C -= X Y^H: slices in 128-row blocks of TC_OP
 // bytes placed blk bytes apart (matrix b at S + b sS), and the exponent of
 // row r at E[b sE + r es + eo].
@@ -495,73 +464,6 @@ struct LongK {
   int64_t ldo, sO;
 };
 
-// Digits of the long-K operands.  v = x 2^-E, |v| < 1/4, as the 56-bit integer
-// rint(2^56 v) + 0x80...80: byte 6 - s, less 128, is the digit m_s of
-//   v = sum_{s=0..6} 2^-8(s+1) m_s,  |m_s| <= 128,  residual below 2^-57.
-// Three exact extractions (24, 22 and 10 bits) by adding constants; the bits
-// of the three sums are the three integers up to constants.
-struct Fixed56 {
-  uint32_t lo, hi;
-};
-__device__ __forceinline__ Fixed56 to_fixed(float hi, float lo) {
-  constexpr float M0 = 0.75f, M1 = 1.5f * 0x1p-23f, M2 = 1.5f * 0x1p-33f;  // ulps 2^-24, 2^-46, 2^-56
-  constexpr uint64_t off = 0x0080808080808080ull - ((uint64_t)0x3f400000u << 32) - ((uint64_t)0x34400000u << 10) -
-                           0x2f400000u;
-  const float t0 = __fadd_rn(hi, M0);
-  float r = __fsub_rn(hi, __fsub_rn(t0, M0)), e;
-  fast_two_sum(r, lo, r, e);  // |r| >= |lo| or r = 0
-  const float t1 = __fadd_rn(r, M1);
-  r = __fadd_rn(__fsub_rn(r, __fsub_rn(t1, M1)), e);
-  const float t2 = __fadd_rn(r, M2);
-  const uint64_t n = (uint64_t)__float_as_uint(t1) * 1024u +
-                     (((uint64_t)__float_as_uint(t0) << 32) | __float_as_uint(t2)) + off;
-  return Fixed56{(uint32_t)n, (uint32_t)(n >> 32)};
-}
-// digit S of two numbers in half precision (low half: a): 1024 + byte by its
-// bits, less 1152 (exact).  bf16 has no room for an 8-bit byte below its
-// leading bit, and costs five instructions here instead of three.
-template <int S>
-__device__ __forceinline__ uint32_t digit2(Fixed56 a, Fixed56 b) {
-  constexpr uint32_t k = S <= 2 ? 2 - S : 6 - S;  // byte of the word
-  const uint32_t w = __byte_perm(S <= 2 ? a.hi : a.lo, S <= 2 ? b.hi : b.lo, (k + 4) << 8 | k);
-  const uint32_t x = (w & 0x00ff00ffu) | 0x64006400u;
-  const __half2 h = __hsub2(*(const __half2 *)&x, __half2{__ushort_as_half(0x6480), __ushort_as_half(0x6480)});
-  return *(const uint32_t *)&h;
-}
-
-// Exponent E of a row's grid from its largest magnitude (its elements are below
-// 2^(E-2)), and the scaling by 2^-E in up to two exact steps (2^-E exceeds the
-// float range for subnormal rows, e.g. the far tail of a localised
-// eigenvector).  A row with an infinity or NaN gets an exponent that makes every
-// product of it non-finite.
-constexpr int LK_NONFINITE = 1 << 20;
-__device__ __forceinline__ float max_abs(float m, float x) {  // NaN if one is
-  float r;
-  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(m), "f"(fabsf(x)));
-  return r;
-}
-__device__ __forceinline__ int grid_exp(float amax) {
-  if (!(amax <= FLT_MAX)) return LK_NONFINITE;
-  int E = 0;
-  if (amax > 0.f) frexpf(amax, &E);
-  return E + 2;
-}
-__device__ __forceinline__ float grid_scale(int E) { return E == LK_NONFINITE ? 0.f : pow2f(E < -100 ? -E - 100 : -E); }
-// x[0..N) to grid integers (warp-wide call)
-template <int N>
-__device__ __forceinline__ void to_fixed(const df *x, int E, bool neg, Fixed56 *f) {
-  const float sc = neg ? -grid_scale(E) : grid_scale(E);
-  if (__any_sync(0xffffffffu, E < -100)) {
-    const float pre = E < -100 ? 0x1p100f : 1.f;
-#pragma unroll
-    for (int t = 0; t < N; ++t)
-      f[t] = to_fixed(__fmul_rn(__fmul_rn(x[t].hi, pre), sc), __fmul_rn(__fmul_rn(x[t].lo, pre), sc));
-  } else {
-#pragma unroll
-    for (int t = 0; t < N; ++t) f[t] = to_fixed(__fmul_rn(x[t].hi, sc), __fmul_rn(x[t].lo, sc));
-  }
-}
-
 constexpr int LK_BOP = TC_S * TC_KS * 1024;  // 32 rows of one operand (28672 bytes)
 constexpr int LK_LD = 33;                    // staging row stride (16-byte elements)
 constexpr int LK_LDB = 65;                   // and of B in mode 1
@@ -638,25 +540,6 @@ __device__ __forceinline__ void lk_issue(uint32_t d, uint32_t ta, uint64_t b0) {
       tc::mma_bf16_ta(d, ad, br, LK_ID, acc);
       tc::mma_bf16_ta(d + 32, ad, bi, MODE == 0 && j < 2 ? LK_IDN : LK_ID, acc);
     }
-  }
-}
-
-// s += a 2^-8U in the order 6, 5, ..., 0 (see fold_group): here s.hi is a
-// multiple of 2^-8(U+1) below 2^(24-8(U+1)), so that a 2^-8U is a multiple of
-// ulp(s.hi) and the three-operation sum is exact as well.
-template <int U>
-__device__ __forceinline__ void fold_up(df &s, float a) {
-  constexpr float w = 1.f / (float)((uint64_t)1 << (8 * U));
-  if (U == 6)
-    s.lo = __fmul_rn(a, w);
-  else if (U >= 4)
-    s.lo = __fmaf_rn(a, w, s.lo);
-  else if (U == 3)
-    s.hi = __fmul_rn(a, w);
-  else {
-    const float h = __fmaf_rn(a, w, s.hi);
-    s.lo = __fadd_rn(s.lo, __fsub_rn(s.hi, __fmaf_rn(a, -w, h)));
-    s.hi = h;
   }
 }
 
