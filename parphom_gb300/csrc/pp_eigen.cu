@@ -31,6 +31,7 @@
 #include <cstdio>
 
 #include "pp_internal.cuh"
+#include "pp_sums.cuh"
 
 namespace pp {
 
@@ -108,74 +109,6 @@ static cudaError_t launch_dep(void (*kernel)(P...), dim3 grid, int threads, size
   return cudaLaunchKernelEx(&cfg, kernel, (P)args...);
 }
 
-// Sums over threads.  Double: plain FP64 adds.  Double-float: an unevaluated
-// sum of three floats, whose additions lose nothing above ~2^-70 of the
-// largest term -- no less than an FP64 sum, without the FP64 pipe (a
-// dependent FP64 add waits 64-150 cycles on this chip, and a division or a
-// square root 560-690; such chains were most of a column's time).
-struct tf {
-  float a, b, c;
-};
-template <class R>
-struct Sum;
-template <>
-struct Sum<double> {
-  typedef double T;
-  PP_D static T zero() { return 0.0; }
-  PP_D static T from(double x) { return x; }
-  PP_D static T add(T x, T y) { return x + y; }
-  PP_D static T sub(T x, T y) { return x - y; }
-  PP_D static T mul(double x, double y) { return x * y; }
-  PP_D static T shfl_xor(T x, int o) { return __shfl_xor_sync(0xffffffffu, x, o); }
-  PP_D static double to(T x) { return x; }
-  PP_D static double toR(T x) { return x; }
-};
-template <>
-struct Sum<df> {
-  typedef tf T;
-  PP_D static T zero() { return tf{0.f, 0.f, 0.f}; }
-  PP_D static T from(df x) { return tf{x.hi, x.lo, 0.f}; }
-  PP_D static T add(T x, T y) {
-    float s, e0, t, e1, u, e2;
-    two_sum(x.a, y.a, s, e0);
-    two_sum(x.b, y.b, t, e1);
-    two_sum(t, e0, u, e2);
-    return tf{s, u, __fadd_rn(__fadd_rn(x.c, y.c), __fadd_rn(e1, e2))};
-  }
-  PP_D static T sub(T x, T y) { return add(x, tf{-y.a, -y.b, -y.c}); }
-  // the product of two double-floats with every partial product kept
-  PP_D static T mul(df x, df y) {
-    const float p = __fmul_rn(x.hi, y.hi), pe = __fmaf_rn(x.hi, y.hi, -p);
-    const float q = __fmul_rn(x.hi, y.lo), qe = __fmaf_rn(x.hi, y.lo, -q);
-    const float r = __fmul_rn(x.lo, y.hi), re = __fmaf_rn(x.lo, y.hi, -r);
-    float s, e1, u, e2;
-    two_sum(pe, q, s, e1);
-    two_sum(s, r, u, e2);
-    return tf{p, u, __fadd_rn(__fmaf_rn(x.lo, y.lo, __fadd_rn(qe, re)), __fadd_rn(e1, e2))};
-  }
-  PP_D static T shfl_xor(T x, int o) {
-    return tf{__shfl_xor_sync(0xffffffffu, x.a, o), __shfl_xor_sync(0xffffffffu, x.b, o),
-              __shfl_xor_sync(0xffffffffu, x.c, o)};
-  }
-  PP_D static double to(T x) { return (double)x.a + ((double)x.b + (double)x.c); }
-  PP_D static df toR(T x) {
-    float s, e;
-    two_sum(x.a, x.b, s, e);
-    df r;
-    fast_two_sum(s, __fadd_rn(e, x.c), r.hi, r.lo);
-    return r;
-  }
-};
-// complex value of R from another lane
-template <class R>
-__device__ __forceinline__ R shfl_real(R x, int src) {
-  R y;
-  float *dst = (float *)&y;
-  const float *p = (const float *)&x;
-#pragma unroll
-  for (int f = 0; f < (int)(sizeof(R) / sizeof(float)); ++f) dst[f] = __shfl_sync(0xffffffffu, p[f], src);
-  return y;
-}
 template <class R>
 __device__ __forceinline__ R shfl_xor_real(R x, int o) {
   R y;
@@ -820,35 +753,6 @@ __device__ __forceinline__ void panel_x(const PanelCol<R> &c, const C<R> *X, C<R
     x2[k] = X[c.jj + k];
   }
 }
-// A complex sum over rows of products rounded to R row by row: the three-float
-// sums of the double-float form do not depend on how the rows are dealt to
-// lanes and CTAs (beyond ~2^-70), so a matrix gives the same result in a batch
-// of any largest order.
-template <class R>
-struct __align__(16) RowSum {
-  typename Sum<R>::T re, im;
-  __device__ __forceinline__ void zero() { re = im = Sum<R>::zero(); }
-  // += conj(w) v
-  __device__ __forceinline__ void add_product(C<R> w, C<R> v) {
-    C<R> p = cz<R>();
-    cmacc(p, w, v);
-    p = cfin(p);
-    re = Sum<R>::add(re, Sum<R>::from(p.re));
-    im = Sum<R>::add(im, Sum<R>::from(p.im));
-  }
-  __device__ __forceinline__ void add(const RowSum &o) {
-    re = Sum<R>::add(re, o.re);
-    im = Sum<R>::add(im, o.im);
-  }
-  // over lanes 0, 8, 16, 24 (the rows of a warp), in every one of them
-  __device__ __forceinline__ void rows4() {
-#pragma unroll
-    for (int o = 16; o >= 8; o >>= 1) {
-      re = Sum<R>::add(re, Sum<R>::shfl_xor(re, o));
-      im = Sum<R>::add(im, Sum<R>::shfl_xor(im, o));
-    }
-  }
-};
 constexpr int ROWSUM_BYTES = 32;  // the larger of the two forms
 static_assert(sizeof(RowSum<df>) == ROWSUM_BYTES && sizeof(RowSum<double>) <= ROWSUM_BYTES, "partial-sum slots");
 
@@ -985,24 +889,16 @@ __global__ void __launch_bounds__(TR_NT) k_colstep(C<R> *Ab, int64_t lda, int64_
   auto row_of = [&](int l) { return col + ((l >> 2) * CS + rank) * 4 + (l & 3); };
   const bool cached = do_w == 1;  // w0, v and column col are in shared memory
   C<R> alpha = cz<R>(), wn = cz<R>();
-  // alpha from the lanes' parts of w0^H v (summed here over the first warp)
-  auto finish_alpha = [&](const RowSum<R> &part, C<R> w0, C<R> tau) {
-    const T sr = part.re, si = part.im;
-    // lanes 0-15 the real parts, 16-31 the imaginary parts
-    const bool im = lane >= 16;
-    T v = S::add(im ? si : sr, S::shfl_xor(im ? sr : si, 16));
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) v = S::add(v, S::shfl_xor(v, o));
-    const R mine = S::toR(v);
-    const C<R> s{shfl_real(mine, 0), shfl_real(mine, 16)};
-    const C<R> ts = cmul(tau, s);
-    const R h = RT<R>::from(-0.5);
-    const C<R> al{RT<R>::mul(h, ts.re), RT<R>::mul(h, ts.im)};
+  // alpha (over the first warp) and w(i+1): v(i+1) = 1
+  auto finish_alpha = [&](const RowSum<R> &part, C<R> w0, double2 t) {
+    const C<R> al = minus_half_product(part, z64{t.x, t.y});
     if (lane == 0) {
       s_alpha = al;
-      s_wn = cadd(w0, al);  // w(i+1): v(i+1) = 1
+      s_wn = cadd(w0, al);
     }
   };
+  // tau of column i in FP64 (written by the launch that formed its reflector)
+  const double2 *tau_i = (const double2 *)&tau64[b * sd + (i < 0 ? 0 : i)];
   if (do_w == 1) {
     const PanelCol<R> pc(A, W, Pb + b * sP, lda, ldp, n, i, k0, jj, do_next, sms);
     const int sub = lane % CT_TPR;
@@ -1010,6 +906,7 @@ __global__ void __launch_bounds__(TR_NT) k_colstep(C<R> *Ab, int64_t lda, int64_
     int l = warp * 4 + lane / CT_TPR;
     q.load_old(pc, row_of(l), sub);
     const C<R> tau = taub[b];
+    const double2 t64 = __ldcg(tau_i);
     panel_next(pc, nv, nw);
     dep_wait();
     q.load_p(pc, row_of(l), sub);
@@ -1060,18 +957,18 @@ __global__ void __launch_bounds__(TR_NT) k_colstep(C<R> *Ab, int64_t lda, int64_
       RowSum<R> mine;
       mine.zero();
       for (int k = lane; k < CS * CT_NW; k += 32) mine.add(in_wv[k]);
-      finish_alpha(mine, in_w, tau);
+      finish_alpha(mine, in_w, t64);
     }
     __syncthreads();
   } else if (do_w == 2) {
     if (warp == 0) {
       const RowSum<R> *part = partb + b * spart;
-      const C<R> tau = taub[b];
+      const double2 t64 = __ldcg(tau_i);
       const int nparts = cdiv_dev(n - col, wp_threads<R> / CT_TPR);
       RowSum<R> mine;
       mine.zero();
       for (int k = lane; k < nparts; k += 32) mine.add(part[1 + k]);
-      finish_alpha(mine, *(const C<R> *)&part[0], tau);
+      finish_alpha(mine, *(const C<R> *)&part[0], t64);
     }
     __syncthreads();
   }
