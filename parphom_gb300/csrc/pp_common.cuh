@@ -66,9 +66,22 @@ PP_D df df_mul(df a, df b) {
   return r;
 }
 // acc += a*b with the low word left unnormalised (call df_norm at the end).
-// TwoSum of acc.hi and p = fl(a.hi b.hi), with the product's own error taken
-// along in one FMA: (p - bb) + (a.hi b.hi - p) = a.hi b.hi - bb.
 PP_D void df_mac(df &acc, df a, df b) {
+  float p = __fmul_rn(a.hi, b.hi);
+  float pe = __fmaf_rn(a.hi, b.hi, -p);
+  pe = __fmaf_rn(a.hi, b.lo, pe);
+  pe = __fmaf_rn(a.lo, b.hi, pe);
+  float s, e;
+  two_sum(acc.hi, p, s, e);
+  acc.hi = s;
+  acc.lo = __fadd_rn(acc.lo, __fadd_rn(e, pe));
+}
+// The same in ten operations instead of twelve: the product's own error is taken
+// along with TwoSum's correction in one FMA, (p - bb) + (a.hi b.hi - p) = a.hi
+// b.hi - bb.  It rounds once more at the size of the sum (32 terms of random sign:
+// rms 0.22 instead of 0.21 x 2^-46 of sum |a b|), so its sums are kept in two halves
+// (0.13).
+PP_D void df_mac_fused(df &acc, df a, df b) {
   const float s = __fadd_rn(acc.hi, __fmul_rn(a.hi, b.hi));
   const float bb = __fsub_rn(s, acc.hi);
   float e = __fmaf_rn(a.hi, b.hi, -bb);
@@ -161,6 +174,35 @@ PP_D void cmacc(cx<R> &acc, cx<R> a, cx<R> b) {
 template <class R>
 PP_D cx<R> cfin(cx<R> a) {
   return cx<R>{RT<R>::fin(a.re), RT<R>::fin(a.im)};
+}
+// sum += the DF_BLOCK complex products a(k) b(k) (or conj(a(k)) b(k)): those of even
+// and of odd k in a sum each, low words unnormalised
+constexpr int DF_BLOCK = 16;
+PP_D void df_acc(df &sum, df x) {
+  float s, e;
+  two_sum(sum.hi, x.hi, s, e);
+  sum.hi = s;
+  sum.lo = __fadd_rn(sum.lo, __fadd_rn(e, x.lo));
+}
+template <bool CONJ>
+PP_D void cmac_fused(zdf &s, zdf x, zdf y) {
+  df_mac_fused(s.re, x.re, y.re);
+  df_mac_fused(s.re, CONJ ? x.im : df_neg(x.im), y.im);
+  df_mac_fused(s.im, x.re, y.im);
+  df_mac_fused(s.im, CONJ ? df_neg(x.im) : x.im, y.re);
+}
+template <bool CONJ, class A, class B>
+PP_D void df_block(zdf &sum, A a, B b) {
+  zdf s = cz<df>(), t = cz<df>();
+#pragma unroll 2
+  for (int k = 0; k < DF_BLOCK; k += 2) {
+    cmac_fused<CONJ>(s, a(k), b(k));
+    cmac_fused<CONJ>(t, a(k + 1), b(k + 1));
+  }
+  df_acc(s.re, t.re);
+  df_acc(s.im, t.im);
+  df_acc(sum.re, s.re);
+  df_acc(sum.im, s.im);
 }
 template <class R>
 PP_D z64 cto64(cx<R> a) {

@@ -281,7 +281,7 @@ __device__ __forceinline__ void tile_pair(int p, int &Rt, int &Ct) {
 // One of the panel products of column i, by 128 threads (t) of one block of
 // the double-float mat-vec's launch: X[c] = V(:,c)^H v (c < jj), X[jj+c] =
 // W(:,c)^H v over rows [i+1, n).  They need only v, so they run beside the mat-vec instead of in a launch of
-// their own.  Each thread's sum is renormalised every 4 rows.
+// their own.  Each thread adds up 4 rows at a time, the blocks of 4 in three floats.
 __device__ __forceinline__ void panel_dot(const zdf *A, const zdf *W, int64_t lda, int n, int i, int k0, int jj,
                                           int c2, int t, Sum<df>::T (*red)[4], zdf *X) {
   typedef Sum<df> S;
@@ -292,10 +292,15 @@ __device__ __forceinline__ void panel_dot(const zdf *A, const zdf *W, int64_t ld
   const int c = useW ? c2 - jj : c2;
   const zdf *Xc = useW ? (W + lda * c) : (A + lda * (k0 + c));
   const zdf *v = A + lda * i;
-  zdf acc = cz<df>();
+  T sr = S::zero(), si = S::zero();
+  auto flush = [&](zdf acc) {
+    acc = cfin(acc);
+    sr = S::add(sr, S::from(acc.re));
+    si = S::add(si, S::from(acc.im));
+  };
   int r = some ? i + 1 + t : n;
   for (; r + 3 * NT < n; r += 4 * NT) {
-    zdf x[4], y[4];
+    zdf x[4], y[4], acc = cz<df>();
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       x[u] = Xc[r + u * NT];
@@ -303,11 +308,11 @@ __device__ __forceinline__ void panel_dot(const zdf *A, const zdf *W, int64_t ld
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) cmacc(acc, x[u], y[u]);
-    acc = cfin(acc);
+    flush(acc);
   }
-  for (; r < n; r += NT) cmacc(acc, Xc[r], v[r]);
-  acc = cfin(acc);
-  T sr = S::from(acc.re), si = S::from(acc.im);
+  zdf last = cz<df>();
+  for (; r < n; r += NT) cmacc(last, Xc[r], v[r]);
+  flush(last);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     sr = S::add(sr, S::shfl_xor(sr, o));
@@ -481,11 +486,15 @@ __global__ void __launch_bounds__(4 * HL_T, HL_BPS * 32 / HL_T) k_hemv_lower(con
 // runs depend on the order of the trailing block, the column of the panel and
 // the number of SMs only.  The first CTAs of the grid form the panel products
 // (panel_dot), 2 per CTA.
+// A lane's 16 products of a tile are summed on their own (df_block) and added to
+// the row's sum.
 // Bound by instruction issue: 80 double-float lane operations per stored
-// element (two complex multiply-adds), 106 instructions in all where the
-// 32 x 32 tiles of the earlier kernel took 152.  One matrix of order 4764,
-// first columns: 66.5 us -> 53.5 us (3.4 TB/s), with 96 operations; all columns
-// of 8 such matrices, the average: 139 us, with 80 operations (df_mac) 127 us.
+// element (two complex multiply-adds of ten operations each), about 110 instructions
+// in all where the 32 x 32 tiles of the earlier kernel took 152.  One matrix of order
+// 4764, first columns: 66.5 us -> 53.5 us (3.4 TB/s), with twelve operations; all columns
+// of 8 such matrices, the average: 139 us with twelve operations, 131 us with ten in
+// two sums per tile (127 us with one sum along the row, whose rounding errors are
+// larger than those of the twelve).
 // Measured and not kept: packed f32x2 arithmetic (30% fewer instructions, but three
 // shared-memory reads per vector entry: 57 us); bulk copies by a fetching warp
 // with mbarriers (61 us: 1 KB copies are issued too slowly); tiles of 64 x 64.
@@ -596,12 +605,11 @@ __global__ void __launch_bounds__(HV_NT, HV_BPS) k_hemv_df(const zdf *Ab, int64_
     if (warp < 4) {
       const int r = warp * 16 + (lane & 15), cb = lane & 16;
       const zdf *vc = vl + HV_R + cb, *ta = tl + cb * HV_LD + r;
-      if (off < 0) {
-#pragma unroll 4
-        for (int k = 0; k < 16; ++k) cmac(y, ta[k * HV_LD], vc[k]);
-      } else {
-        for (int k = 0; k < 16; ++k) cmac(y, r >= cb + k + off ? ta[k * HV_LD] : cz<df>(), vc[k]);
-      }
+      auto vec = [&](int k) { return vc[k]; };
+      if (off < 0)
+        df_block<false>(y, [&](int k) { return ta[k * HV_LD]; }, vec);
+      else
+        df_block<false>(y, [&](int k) { return r >= cb + k + off ? ta[k * HV_LD] : cz<df>(); }, vec);
       y = cfin(y);
       if (off == HV_C || t + 1 == tend) {  // the row sums end here
         y = cadd(y, zdf{shfl_xor_real(y.re, 16), shfl_xor_real(y.im, 16)});
@@ -615,12 +623,11 @@ __global__ void __launch_bounds__(HV_NT, HV_BPS) k_hemv_df(const zdf *Ab, int64_
       const int c = (warp - 4) * 8 + (lane & 7), rb = (lane >> 3) * 16;
       const zdf *vr = vl + rb, *ta = tl + c * HV_LD + rb;
       zdf s = cz<df>();
-      if (off < 0) {
-#pragma unroll 4
-        for (int k = 0; k < 16; ++k) cmacc(s, ta[k], vr[k]);
-      } else {
-        for (int k = 0; k < 16; ++k) cmacc(s, rb + k > c + off ? ta[k] : cz<df>(), vr[k]);
-      }
+      auto vec = [&](int k) { return vr[k]; };
+      if (off < 0)
+        df_block<true>(s, [&](int k) { return ta[k]; }, vec);
+      else
+        df_block<true>(s, [&](int k) { return rb + k > c + off ? ta[k] : cz<df>(); }, vec);
       s = cfin(s);
       // over the four row groups: lanes below 16 end up with the real part, the others with the imaginary part
       const bool im = lane >= 16;
