@@ -202,7 +202,9 @@ PP_API int pp_dos_smearing(int32_t method, const double *freq, int64_t ldf, int6
  * weights_dev and the outputs (ne doubles each) all device memory.  Results
  * as pp_dos_triangulation / pp_dos_smearing; the bands are summed in a
  * different order (last-bit differences).  Enqueued on `stream`; nothing is
- * allocated.  Replaces the same routines as the host forms
+ * allocated (the triangulation keeps partial sums in arrays of 2.6 MB compiled
+ * into the library; a call that finds them in use by two other streams waits for
+ * one on the device, and inside a stream capture it goes without).  Replaces the same routines as the host forms
  * (bz_integration.f90:12-199 as called from pyphutil.py:214-359). */
 PP_API int pp_dos_triangulation_device(const double *freq_dev, int64_t ldf, int64_t nk, int64_t nbands,
                                        const double *func_dev, int64_t ldfunc, const int64_t *tri_dev, int64_t ntri,

@@ -13,6 +13,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <mutex>
 #include <vector>
 
 #include "../../include/parphom_gpu.h"
@@ -84,8 +85,10 @@ __device__ __noinline__ void triangle_by_sort(const double *freq, int64_t ldf, c
 // Most energies lie above all 32 triangles (they add the warp's weights to nd)
 // or below (nothing): lanes then stand for energies, 32 at a time.  For the few
 // in between, lanes stand for triangles.  Each warp adds to sums of its own in
-// shared memory (DT_E energies); a block's are added at the end, to pdos / pnd
-// ([energy][block], a sum of fixed order follows) or to dos / nd.
+// shared memory (DT_E energies); a block's go to part ([dos, nd][energy][block]) at
+// the end, which k_dos_sum adds up, or without part are added to dos / nd one after
+// the other (32 x 32 grid, 444 bands, rms: dos off by 2.4e-16 and nd by 2.3e-16 that
+// way, by 1.0e-16 both with part).
 //
 // Bound by the FP64 pipe (16 cycles per instruction of a warp): two comparisons
 // per 32 energies and about 40 instructions per energy in between, no division.
@@ -97,7 +100,7 @@ constexpr int DT_SMEM = (2 * DT_W + 1) * DT_E * 8;
 __global__ void __launch_bounds__(32 * DT_W, 1) k_dos_tri(const double *freq, int64_t ldf, const double *func,
                                                           int64_t ldfunc, int64_t nbands, const int64_t *tri,
                                                           int64_t ntri, const double *E, int64_t ne, double *dos,
-                                                          double *nd, double *pdos, double *pnd) {
+                                                          double *nd, double *part) {
   extern __shared__ double sm[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double *sE = sm, *sd = sm + DT_E + 2 * DT_E * warp, *sn = sd + DT_E;
@@ -189,9 +192,9 @@ __global__ void __launch_bounds__(32 * DT_W, 1) k_dos_tri(const double *freq, in
       d += sm[DT_E + 2 * DT_E * w + i];
       n += sm[DT_E + 2 * DT_E * w + DT_E + i];
     }
-    if (pdos) {
-      pdos[(i0 + i) * gridDim.x + blockIdx.x] = d;
-      pnd[(i0 + i) * gridDim.x + blockIdx.x] = n;
+    if (part) {
+      part[(i0 + i) * gridDim.x + blockIdx.x] = d;
+      part[(ne + i0 + i) * gridDim.x + blockIdx.x] = n;
     } else {
       atomicAdd(&dos[i0 + i], d);
       atomicAdd(&nd[i0 + i], n);
@@ -204,15 +207,89 @@ unsigned dos_tri_blocks(int64_t ntri, int64_t nbands, int64_t ne) {
   const int64_t per = std::max<int64_t>(1, pp::device_sms() / std::min<int64_t>(slices, pp::device_sms()));
   return (unsigned)std::max<int64_t>(1, std::min<int64_t>((items + DT_W - 1) / DT_W, per));
 }
+// The blocks' parts of dos and nd added up: a warp per sum, its lanes' parts by a
+// tree, so that few additions round at the size of the total (carrying their
+// rounding errors along as well: 0.88e-16 instead of 0.95e-16, 2 us more a call).
+__global__ void __launch_bounds__(128) k_dos_sum(const double *part, int nblk, int64_t ne, double *dos, double *nd) {
+  const int64_t i = (int64_t)blockIdx.x * 4 + threadIdx.x / 32;
+  const int lane = threadIdx.x & 31;
+  if (i >= 2 * ne) return;
+  double s = 0.0;
+  for (int k = lane; k < nblk; k += 32) s += part[i * nblk + k];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) (i < ne ? dos : nd)[i < ne ? i : i - ne] = s;
+}
+
+// dos and nd with the blocks' parts in `part` (2 ne dos_tri_blocks doubles), or
+// without.
 cudaError_t dos_tri(const double *freq, int64_t ldf, const double *func, int64_t ldfunc, int64_t nbands,
                     const int64_t *tri, int64_t ntri, const double *E, int64_t ne, double *dos, double *nd,
-                    double *pdos, double *pnd, cudaStream_t s) {
+                    double *part, cudaStream_t s) {
   cudaError_t e = cudaFuncSetAttribute(k_dos_tri, cudaFuncAttributeMaxDynamicSharedMemorySize, DT_SMEM);
+  if (e == cudaSuccess && !part) e = cudaMemsetAsync(dos, 0, sizeof(double) * ne, s);
+  if (e == cudaSuccess && !part) e = cudaMemsetAsync(nd, 0, sizeof(double) * ne, s);
   if (e != cudaSuccess) return e;
-  k_dos_tri<<<dim3(dos_tri_blocks(ntri, nbands, ne), (unsigned)((ne + DT_E - 1) / DT_E)), 32 * DT_W, DT_SMEM, s>>>(
-      freq, ldf, func, ldfunc, nbands, tri, ntri, E, ne, dos, nd, pdos, pnd);
-  pp::count_launch(1);
+  const unsigned nblk = dos_tri_blocks(ntri, nbands, ne);
+  k_dos_tri<<<dim3(nblk, (unsigned)((ne + DT_E - 1) / DT_E)), 32 * DT_W, DT_SMEM, s>>>(
+      freq, ldf, func, ldfunc, nbands, tri, ntri, E, ne, dos, nd, part);
+  if (part) k_dos_sum<<<(unsigned)((2 * ne + 3) / 4), 128, 0, s>>>(part, (int)nblk, ne, dos, nd);
+  pp::count_launch(part ? 2 : 1);
   return cudaGetLastError();
+}
+
+// Room for the parts of the device-resident form, which allocates nothing: fixed
+// arrays of the library, one for each of up to DS_SLOTS calls in flight on a
+// device.  A call takes the array that its stream used last, or one whose last
+// call has ended, or waits on the device for one; inside a stream capture (a graph
+// may run at any time) and past DS_CAP it goes without.
+constexpr int DS_SLOTS = 2;
+constexpr int64_t DS_CAP = 2 * 160 * DT_E;  // doubles: 160 SMs with DT_E energies each
+__device__ double dos_parts[DS_SLOTS][DS_CAP];
+struct DosSlots {
+  double *base = nullptr;
+  cudaStream_t stream[DS_SLOTS] = {};
+  cudaEvent_t done[DS_SLOTS] = {};
+  bool used[DS_SLOTS] = {};
+};
+std::mutex ds_mu;
+DosSlots ds_slots[pp::PP_MAX_DEVICES];
+
+// launch(part) with a slot's array or with nullptr
+template <class F>
+cudaError_t with_parts(int64_t need, cudaStream_t s, F launch) {
+  const int dev = pp::device_index();
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {  // (the legacy stream while another is captured)
+    cudaGetLastError();
+    cs = cudaStreamCaptureStatusActive;
+  }
+  if (dev < 0 || need > DS_CAP || cs != cudaStreamCaptureStatusNone) return launch(nullptr);
+  std::lock_guard<std::mutex> g(ds_mu);
+  DosSlots &d = ds_slots[dev];
+  if (!d.base) {
+    void *p = nullptr;
+    cudaError_t e = cudaGetSymbolAddress(&p, dos_parts);
+    for (int k = 0; k < DS_SLOTS && e == cudaSuccess; ++k)
+      if (!d.done[k]) e = cudaEventCreateWithFlags(&d.done[k], cudaEventDisableTiming);
+    if (e != cudaSuccess) return e;
+    d.base = (double *)p;
+  }
+  int k = -1;
+  for (int t = 0; t < DS_SLOTS; ++t)
+    if (d.used[t] && d.stream[t] == s) k = t;
+  for (int t = 0; t < DS_SLOTS && k < 0; ++t)
+    if (!d.used[t] || cudaEventQuery(d.done[t]) == cudaSuccess) k = t;
+  if (k < 0) {
+    cudaGetLastError();  // (not ready)
+    k = 0;
+  }
+  cudaError_t e = d.used[k] ? cudaStreamWaitEvent(s, d.done[k], 0) : cudaSuccess;
+  if (e != cudaSuccess) return e;
+  e = launch(d.base + k * DS_CAP);
+  d.used[k] = true;
+  d.stream[k] = s;
+  const cudaError_t r = cudaEventRecord(d.done[k], s);
+  return e != cudaSuccess ? e : r;
 }
 
 __global__ void k_dos_smear(int method, const double *freq, int64_t ldf, int64_t nq, int64_t nbands,
@@ -319,7 +396,7 @@ extern "C" PP_API int pp_dos_triangulation(const double *freq, int64_t ldf, int6
   for (int64_t j = 0; j < 3 * ntri; ++j)
     if (tri[j] < 0 || tri[j] >= nk) return -6;
   if (ne == 0) return PP_OK;
-  double *dfreq = nullptr, *dfunc = nullptr, *dE = nullptr, *pd = nullptr, *pn = nullptr, *od = nullptr, *on = nullptr;
+  double *dfreq = nullptr, *dfunc = nullptr, *dE = nullptr, *part = nullptr, *od = nullptr, *on = nullptr;
   int64_t *dtri = nullptr;
   cudaError_t e = cudaSuccess;
   auto al = [&](void **p, size_t b) {
@@ -329,25 +406,17 @@ extern "C" PP_API int pp_dos_triangulation(const double *freq, int64_t ldf, int6
   if (func) al((void **)&dfunc, sizeof(double) * nk * ldf);
   al((void **)&dtri, sizeof(int64_t) * 3 * ntri);
   al((void **)&dE, sizeof(double) * ne);
-  const unsigned nblk = dos_tri_blocks(ntri, nbands, ne);
-  al((void **)&pd, sizeof(double) * ne * nblk);
-  al((void **)&pn, sizeof(double) * ne * nblk);
+  al((void **)&part, sizeof(double) * 2 * ne * dos_tri_blocks(ntri, nbands, ne));
   al((void **)&od, sizeof(double) * ne);
   al((void **)&on, sizeof(double) * ne);
   if (e == cudaSuccess) e = cudaMemcpy(dfreq, freq, sizeof(double) * nk * ldf, cudaMemcpyHostToDevice);
   if (e == cudaSuccess && func) e = cudaMemcpy(dfunc, func, sizeof(double) * nk * ldf, cudaMemcpyHostToDevice);
   if (e == cudaSuccess && ntri) e = cudaMemcpy(dtri, tri, sizeof(int64_t) * 3 * ntri, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(dE, energy, sizeof(double) * ne, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = dos_tri(dfreq, ldf, dfunc, ldf, nbands, dtri, ntri, dE, ne, od, on, pd, pn, 0);
-  if (e == cudaSuccess) {
-    k_sum_rows<<<(unsigned)((ne + 127) / 128), 128>>>(pd, ne, nblk, 1.0, od);
-    k_sum_rows<<<(unsigned)((ne + 127) / 128), 128>>>(pn, ne, nblk, 1.0, on);
-    pp::count_launch(2);
-    e = cudaGetLastError();
-  }
+  if (e == cudaSuccess) e = dos_tri(dfreq, ldf, dfunc, ldf, nbands, dtri, ntri, dE, ne, od, on, part, 0);
   if (e == cudaSuccess) e = cudaMemcpy(dos, od, sizeof(double) * ne, cudaMemcpyDeviceToHost);
   if (e == cudaSuccess) e = cudaMemcpy(nd, on, sizeof(double) * ne, cudaMemcpyDeviceToHost);
-  for (void *p : {(void *)dfreq, (void *)dfunc, (void *)dtri, (void *)dE, (void *)pd, (void *)pn, (void *)od, (void *)on})
+  for (void *p : {(void *)dfreq, (void *)dfunc, (void *)dtri, (void *)dE, (void *)part, (void *)od, (void *)on})
     if (p) cudaFree(p);
   return cerr(e);
 }
@@ -410,11 +479,9 @@ extern "C" PP_API int pp_dos_triangulation_device(const double *freq_dev, int64_
   if (!nd_dev) return -12;
   if (ne == 0) return PP_OK;
   cudaStream_t s = (cudaStream_t)stream;
-  cudaError_t e = cudaMemsetAsync(dos_dev, 0, sizeof(double) * ne, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(nd_dev, 0, sizeof(double) * ne, s);
-  if (e == cudaSuccess)
-    e = dos_tri(freq_dev, ldf, func_dev, ldfunc, nbands, tri_dev, ntri, energy_dev, ne, dos_dev, nd_dev, nullptr,
-                nullptr, s);
+  const cudaError_t e = with_parts(2 * ne * dos_tri_blocks(ntri, nbands, ne), s, [&](double *part) {
+    return dos_tri(freq_dev, ldf, func_dev, ldfunc, nbands, tri_dev, ntri, energy_dev, ne, dos_dev, nd_dev, part, s);
+  });
   return cerr(e);
 }
 
