@@ -137,6 +137,9 @@ __global__ void __launch_bounds__(32 * DT_W, 1) k_dos_tri(const double *freq, in
       order(e0, f0, e1, f1);
     }
     const double r10 = 1.0 / (e1 - e0), r20 = 1.0 / (e2 - e0), r21 = 1.0 / (e2 - e1);
+    // (values so close that a reciprocal overflows: by quotients as well)
+    auto inf = [](double x) { return (__double2hiint(x) & 0x7fffffff) == 0x7ff00000; };
+    odd = odd || (inf(r10) && e1 > e0) || (inf(r21) && e2 > e1);
     const double fs = f0 + f1 + f2;
     double lo = odd ? -INFINITY : e0, hi = odd ? INFINITY : have ? e2 : -INFINITY, all = fs;
     for (int o = 16; o > 0; o >>= 1) {

@@ -94,3 +94,21 @@ def test_captured_call():
         torch.cuda.synchronize()
         for a, b in ((dc, d), (nc, n)):
             assert float((a - b).abs().max()) <= 1e-13 * float(b.abs().max())
+
+
+@pytest.mark.parametrize("vals", [(0.0, 1e-310, 1.0), (-1.0, 0.0, 3e-309), (0.0, 4e-310, 9e-310)])
+def test_values_a_subnormal_apart(vals):
+    """nd of a triangle whose frequencies lie so close that 1 / difference overflows: finite, as the quotients give it."""
+    freq = np.array(vals)[:, None]
+    gap = [k for k in range(2) if vals[k + 1] - vals[k] < 1e-308]
+    E = np.array([vals[k] + f * (vals[k + 1] - vals[k]) for k in gap for f in (0.25, 0.5, 0.75)])
+    _, nd = dos.linear_triangulation(freq, np.array([[0, 1, 2]]), E)
+    for x, n in zip(E, nd):
+        e0, e1, e2 = vals
+        if x < e1:
+            a, b = (x - e0) / (e1 - e0), (x - e0) / (e2 - e0)
+            want = (3 - a - b + a + b) * a * b
+        else:
+            c, d = (e2 - x) / (e2 - e0), (e2 - x) / (e2 - e1)
+            want = (1 - d * c * c) + (1 - c * d * d) + (1 - 3 * c * d + d * c * c + c * d * d)
+        assert abs(n - want) <= 1e-12 * want
