@@ -76,15 +76,23 @@ constexpr int TR_NT = 256;   // threads of the column kernels
 // dep_go, does what does not read that kernel's results, and waits in dep_wait
 // until it has completed (every block waits, before any return, so that
 // completion carries over the whole chain; dep_go comes after dep_wait, so that
-// all earlier kernels have completed when a kernel starts).  The mat-vec
-// requests its first tile early, the column step its panel rows, v and the next
-// column.  A pass: n = 1092 (FP64, eigenvalues) 38.6 -> 30.3 ms, n = 2604 with
+// all earlier kernels but the one before have completed when a kernel starts).
+// What is loaded before dep_wait may be what a completed kernel wrote to lines that
+// this SM's L1 has held before, and no rule says that the early start clears it: those
+// loads go past L1 (load_l2, cp.async.cg).  The mat-vec requests its first tile early,
+// the column step its panel rows, v and the next column.  A pass: n = 1092 (FP64,
+// eigenvalues) 38.6 -> 30.3 ms, n = 2604 with
 // vectors 168 -> 156 ms, n = 1092 x 16 64.8 -> 61.1 ms.  dep_go is called late
 // (a block's last tile, a column's last phase): blocks that wait early hold
 // slots that other streams' kernels need (column step calling it first: 166 and
 // 63.9 ms).
 PP_D void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 PP_D void dep_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <class R>
+PP_D cx<R> load_l2(const cx<R> *p) {
+  const float4 v = __ldcg((const float4 *)p);
+  return *(const cx<R> *)&v;
+}
 template <class... P, class... A>
 static cudaError_t launch_dep(void (*kernel)(P...), dim3 grid, int threads, size_t smem, int cluster, bool dep,
                               cudaStream_t s, A... args) {
@@ -693,18 +701,18 @@ struct PanelRow {
       p[u] = in && k < nch ? c.P[r + (int64_t)(k + (k >= nseg ? skip : 0)) * c.ldp] : cz<R>();
     }
   }
-  // what was there before it
+  // what was there before it (loaded before dep_wait, too)
   __device__ __forceinline__ void load_old(const PanelCol<R> &c, int r, int sub) {
     const bool in = r < c.n;
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int k = sub + CT_TPR * u;
-      w[u] = in && k < c.jj ? c.W[r + c.lda * k] : cz<R>();
-      v[u] = in && k < c.jj ? c.A[r + c.lda * (c.k0 + k)] : cz<R>();
+      w[u] = in && k < c.jj ? load_l2(&c.W[r + c.lda * k]) : cz<R>();
+      v[u] = in && k < c.jj ? load_l2(&c.A[r + c.lda * (c.k0 + k)]) : cz<R>();
     }
     const bool own = in && sub == 0;
-    vi = own ? c.A[r + c.lda * c.i] : cz<R>();
-    a = own && c.next ? c.A[r + c.lda * (c.i + 1)] : cz<R>();
+    vi = own ? load_l2(&c.A[r + c.lda * c.i]) : cz<R>();
+    a = own && c.next ? load_l2(&c.A[r + c.lda * (c.i + 1)]) : cz<R>();
   }
   // y = (mat-vec) - W x1 - V x2 and nxt = the panel columns' part of column
   // i + 1's update (x1, x2, row i + 1 of V and W conjugated in shared memory),
@@ -749,8 +757,8 @@ template <class R>
 __device__ __forceinline__ void panel_next(const PanelCol<R> &c, C<R> *nv, C<R> *nw) {
   if (c.next)
     for (int k = threadIdx.x; k < c.jj; k += blockDim.x) {
-      nv[k] = cconj(c.A[c.i + 1 + c.lda * (c.k0 + k)]);
-      nw[k] = cconj(c.W[c.i + 1 + c.lda * k]);
+      nv[k] = cconj(load_l2(&c.A[c.i + 1 + c.lda * (c.k0 + k)]));
+      nw[k] = cconj(load_l2(&c.W[c.i + 1 + c.lda * k]));
     }
 }
 template <class R>
@@ -792,7 +800,7 @@ __global__ void __launch_bounds__(wp_threads<R>) k_wpart(C<R> *Ab, int64_t lda, 
   const int r = rb + tid / CT_TPR;
   PanelRow<R> q;
   q.load_old(pc, r, sub);
-  const C<R> tau = taub[b];
+  const C<R> tau = load_l2(&taub[b]);
   panel_next(pc, nv, nw);
   dep_wait();
   q.load_p(pc, r, sub);
@@ -912,7 +920,7 @@ __global__ void __launch_bounds__(TR_NT) k_colstep(C<R> *Ab, int64_t lda, int64_
     PanelRow<R> q;
     int l = warp * 4 + lane / CT_TPR;
     q.load_old(pc, row_of(l), sub);
-    const C<R> tau = taub[b];
+    const C<R> tau = load_l2(&taub[b]);
     const double2 t64 = __ldcg(tau_i);
     panel_next(pc, nv, nw);
     dep_wait();
