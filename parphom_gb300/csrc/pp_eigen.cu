@@ -29,6 +29,7 @@
 #include <cfloat>
 #include <type_traits>
 #include <cstdio>
+#include <cstdlib>
 
 #include "pp_internal.cuh"
 #include "pp_sums.cuh"
@@ -852,7 +853,7 @@ __global__ void __launch_bounds__(wp_threads<R>) k_wpart(C<R> *Ab, int64_t lda, 
 // corrections; 7-12 us each, mostly FP64 reductions, divisions and square
 // roots), now 9.3 us at n = 84 (one launch), 11.5 us at n = 1092 and 13.3 us at
 // n = 4764 (with k_wpart).
-constexpr int CT_CLUSTER = 16;           // largest cluster (non-portable size)
+constexpr int CT_CLUSTER = 16;           // largest cluster (non-portable size, where it can be placed)
 constexpr int CT_CAP = 512;              // rows of a CTA kept in shared memory
 constexpr int CT_NW = TR_NT / 32;        // warps
 __device__ __forceinline__ void cluster_arrive() {
@@ -1182,19 +1183,39 @@ __global__ void __launch_bounds__(256) k_her2k(C<R> *Ab, int64_t lda, int64_t sA
 static int hemv_blocks(int bps) { return device_sms() * std::max(1, std::min(bps, HL_BPS)); }
 
 // Clusters of 16 CTAs are beyond the portable size, the mat-vec's tiles beyond
-// 48 KB of shared memory: opted in once per device.
+// 48 KB of shared memory: opted in once per device.  *cluster: the column step's
+// largest cluster there, 16 or what the device (a partition of it) can place, at
+// least the portable 8; PARPHOM_GPU_CLUSTER caps it.
 template <class R>
-static cudaError_t prepare_colstep() {
+static cudaError_t prepare_colstep(int *cluster) {
   static std::mutex mu;
-  static bool done[PP_MAX_DEVICES] = {};
+  static int largest[PP_MAX_DEVICES] = {};
   const int dev = device_index();
-  std::lock_guard<std::mutex> g(mu);
-  if (dev >= 0 && done[dev]) return cudaSuccess;
-  cudaError_t e = cudaFuncSetAttribute(k_colstep<R>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  if (std::is_same<R, df>::value && e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_hemv_df, cudaFuncAttributeMaxDynamicSharedMemorySize, HV_SMEM);
-  if (e == cudaSuccess && dev >= 0) done[dev] = true;
-  return e;
+  {
+    std::lock_guard<std::mutex> g(mu);
+    int c = dev >= 0 ? largest[dev] : 0;
+    if (c == 0) {
+      c = 8;
+      if (cudaFuncSetAttribute(k_colstep<R>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(CT_CLUSTER);
+        cfg.blockDim = dim3(TR_NT);
+        int most = 0;
+        if (cudaOccupancyMaxPotentialClusterSize(&most, k_colstep<R>, &cfg) == cudaSuccess)
+          while (c < CT_CLUSTER && 2 * c <= most) c *= 2;
+      }
+      cudaGetLastError();
+      if (std::is_same<R, df>::value)
+        PP_CUDA_TRY(cudaFuncSetAttribute(k_hemv_df, cudaFuncAttributeMaxDynamicSharedMemorySize, HV_SMEM));
+      if (dev >= 0) largest[dev] = c;
+    }
+    *cluster = c;
+  }
+  if (const char *v = getenv("PARPHOM_GPU_CLUSTER")) {
+    const int cap = atoi(v);
+    while (*cluster > 1 && *cluster > cap) *cluster /= 2;
+  }
+  return cudaSuccess;
 }
 
 // One column step; the cluster has a CTA per 8 rows, at most CT_CLUSTER, and
@@ -1207,7 +1228,7 @@ static cudaError_t prepare_colstep() {
 // n = 4764; FP64 form 12.4 us / 22.4 us at n = 1092).
 constexpr int CT_SPLIT = CT_CLUSTER * CT_NW * 4;
 template <class R>
-static cudaError_t launch_colstep(EigWork &w, int i, int k0, int jj, int do_w, int do_next, cudaStream_t s) {
+static cudaError_t launch_colstep(EigWork &w, int i, int k0, int jj, int do_w, int do_next, int cluster, cudaStream_t s) {
   const int rows = w.nmax - i - 1;
   const int64_t sW = (int64_t)w.lda * w.nb, sP = (int64_t)w.nchunk * w.lda;
   if (do_w && rows > CT_SPLIT) {
@@ -1222,7 +1243,7 @@ static cudaError_t launch_colstep(EigWork &w, int i, int k0, int jj, int do_w, i
     count_launch(1);
   }
   int cs = 1;
-  while (cs < CT_CLUSTER && cs * 8 < rows && cs * std::max(w.batch, w.B) <= device_sms()) cs *= 2;
+  while (cs < cluster && cs * 8 < rows && cs * std::max(w.batch, w.B) <= device_sms()) cs *= 2;
   cudaError_t e = cudaSuccess;
   PP_KT(KT_COLSTEP, s, (e = launch_dep(k_colstep<R>, dim3(cs, w.B), TR_NT, 0, cs, do_w != 0, s, (C<R> *)w.A, w.lda, w.sA,
                                        (C<R> *)w.W, sW, (const C<R> *)w.P, sP, w.lda, (const int *)w.nvec, i, k0, jj, do_w,
@@ -1240,11 +1261,12 @@ cudaError_t tridiagonalize(EigWork &w, cudaStream_t s) {
   C<R> *P = (C<R> *)w.P;
   const int B = w.B, nmax = w.nmax, nb = w.nb;
   const int64_t lda = w.lda, sA = w.sA, sW = (int64_t)w.lda * nb, sP = (int64_t)w.nchunk * w.lda;
-  PP_CUDA_TRY(prepare_colstep<R>());
+  int cluster = 1;
+  PP_CUDA_TRY(prepare_colstep<R>(&cluster));
   if (w.tcErr) PP_CUDA_TRY(cudaMemsetAsync(w.tcErr, 0, sizeof(int) * B, s));
   for (int k0 = 0; k0 < nmax; k0 += nb) {
     const int jb = min(nb, nmax - k0);
-    PP_CUDA_TRY(launch_colstep<R>(w, k0 - 1, k0, 0, 0, 1, s));  // the panel's first column
+    PP_CUDA_TRY(launch_colstep<R>(w, k0 - 1, k0, 0, 0, 1, cluster, s));  // the panel's first column
     for (int jj = 0; jj < jb; ++jj) {
       const int i = k0 + jj;
       if (i >= nmax - 1) break;
@@ -1279,7 +1301,7 @@ cudaError_t tridiagonalize(EigWork &w, cudaStream_t s) {
           count_launch(1);
         }
       }
-      PP_CUDA_TRY(launch_colstep<R>(w, i, k0, jj, 1, jj + 1 < jb ? 1 : 0, s));
+      PP_CUDA_TRY(launch_colstep<R>(w, i, k0, jj, 1, jj + 1 < jb ? 1 : 0, cluster, s));
     }
     const int k1 = k0 + jb;
     if (k1 < nmax) {
