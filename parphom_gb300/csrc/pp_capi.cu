@@ -263,7 +263,7 @@ int ensure_ws_sized(pp_ctx *c, int B, int mcap, int64_t n, int64_t nbnd_max, int
   EigWork &w = c->w;
   w = EigWork();
   w.B = B;
-  w.nmax = w.nmin = (int)n;
+  w.nmax = (int)n;
   w.mcap = mcap;
   w.nb = nb;
   w.lda = lda;
@@ -371,6 +371,7 @@ EigWork view_of(const EigWork &w, int off, int cnt) {
   const size_t nmax = (size_t)w.nmax;
   const int64_t T = w.scratch_threads;
   v.nvec = w.nvec + off;
+  v.orders = w.orders ? w.orders + off : nullptr;
   v.A = sh(w.A, 16 * (size_t)w.sA);
   v.E = sh(w.E, 16 * (size_t)w.sE);
   v.W = sh(w.W, 16 * (size_t)w.lda * w.nb);
@@ -1290,15 +1291,14 @@ int pp_solve_multi(pp_ctx *const *ctxs, int64_t nctx, const int64_t *cell, const
     TRY_CUDA(cudaMemcpyAsync(h->d_q, qh.data(), sizeof(double) * 3 * Bb, cudaMemcpyHostToDevice, s));
     TRY_CUDA(cudaMemcpyAsync(w.nvec, nv.data(), sizeof(int) * Bb, cudaMemcpyHostToDevice, s));
     w.B = w.batch = Bb;
-    w.nmin = *std::min_element(nv.begin(), nv.begin() + Bb);
     for (auto &g : segs) {
       EigWork v = view_of(w, g.off, g.cnt);
       TRY_CUDA(assemble_batch(g.c->g, h->d_q + 3 * g.off, g.cnt, v.A, w.lda, w.sA, fmt, s));
     }
-    if (prec == PP_PREC_MIXED)
-      TRY_CUDA(tridiagonalize<df>(w, s));
-    else
-      TRY_CUDA(tridiagonalize<double>(w, s));
+    w.orders = nv.data();
+    const cudaError_t et = prec == PP_PREC_MIXED ? tridiagonalize<df>(w, s) : tridiagonalize<double>(w, s);
+    w.orders = nullptr;
+    TRY_CUDA(et);
     TRY_CUDA(tridiag_eigenvalues(w, o->range, o->vl / C_RANGE, o->vu / C_RANGE, o->il, o->iu, o->abstol, s,
                                  prec == PP_PREC_MIXED));
     if (needs_vectors(o)) {

@@ -1254,6 +1254,13 @@ static cudaError_t launch_colstep(EigWork &w, int i, int k0, int jj, int do_w, i
   return e;
 }
 
+// Whether a matrix of the batch has a trailing block of 1 .. HL_SMALL rows past
+// column i (one that has ended has none: the larger ones carry no empty launch).
+static bool any_small(const EigWork &w, int i) {
+  auto small = [&](int n) { return n - i - 1 > 0 && n - i - 1 <= HL_SMALL; };
+  return w.orders ? std::any_of(w.orders, w.orders + w.B, small) : small(w.nmax);
+}
+
 template <class R>
 cudaError_t tridiagonalize(EigWork &w, cudaStream_t s) {
   C<R> *A = (C<R> *)w.A;
@@ -1291,7 +1298,7 @@ cudaError_t tridiagonalize(EigWork &w, cudaStream_t s) {
           PP_CUDA_TRY(e);
           count_launch(1);
         }
-        if (w.nmin - i - 1 <= HL_SMALL) {
+        if (any_small(w, i)) {
           const int nt = cdiv(std::min(rows, HL_SMALL), HL_TS);
           const int gx = hl_dots(jj, HL_TS) + nt * (nt + 1) / 2;
           cudaError_t e = cudaSuccess;

@@ -49,7 +49,7 @@ struct EigWork {
   int B = 0;           // matrices in the batch
   int boff = 0;        // index of the first matrix in the whole batch (views)
   int nmax = 0;        // largest order
-  int nmin = 0;        // smallest order
+  const int *orders = nullptr;  // the orders on the host (null: all nmax)
   int batch = 0;       // matrices in the whole batch (views)
   int mcap = 0;        // eigenvector columns allocated per matrix
   int nb = 32;         // panel width

@@ -140,7 +140,7 @@ extern "C" PP_API int pp_heevx_values_noalloc(double *a_dev, int64_t lda, int64_
   cudaStream_t s = (cudaStream_t)stream;
   pp::EigWork w;
   w.B = 1;
-  w.nmax = w.nmin = (int)n;
+  w.nmax = (int)n;
   w.batch = 1;
   w.mcap = 0;
   w.nb = (int)NB;
