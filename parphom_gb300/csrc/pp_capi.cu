@@ -227,9 +227,8 @@ size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // Bytes of a batch's buffers with T threads of inverse iteration (0: the fewest
 // that a large order gets).
-constexpr int64_t IV_T_MIN = 2048;
 size_t ws_bytes_estimate(int64_t n, int B, int mcap, int64_t nbnd, int64_t nbr, int64_t T = 0) {
-  if (T == 0) T = std::min(invit_threads(mcap), IV_T_MIN);
+  if (T == 0) T = invit_threads(mcap, 0);
   size_t per = 16 * (size_t)n * n + 16 * (size_t)n * mcap + (8 * IV_F + 1) * (size_t)n * T +
                16 * (size_t)n * 64 * 2 + 16 * (size_t)std::max<int64_t>((n + 255) / 256, 8) * 32 * std::max(mcap, 64) +
                16 * (size_t)n * std::max<int64_t>(3 * ((n + 63) / 64), 8) +  // mat-vec partials
@@ -249,11 +248,15 @@ int ensure_ws_sized(pp_ctx *c, int B, int mcap, int64_t n, int64_t nbnd_max, int
   const int64_t lda = (n + 7) / 8 * 8;
   // mat-vec partial slots: n/32, n/16 up to 128 rows (FP64 form), 3 ceil(n/64) (double-float form)
   const int nchunk = (int)std::max<int64_t>(3 * ((n + 63) / 64), 8);
-  // inverse iteration: a thread for every eigenvector where memory allows
+  // inverse iteration: a thread for every eigenvector of a small batch, where memory allows
   size_t fr = 0, tot = 0;
   cudaMemGetInfo(&fr, &tot);
-  int64_t T = invit_threads(mcap);
-  if (ws_bytes_estimate(n, B, mcap, nbnd_max, nbr_max, T) > (size_t)(0.6 * (double)fr)) T = std::min(T, IV_T_MIN);
+  int64_t T = invit_threads(mcap, B);
+  if (ws_bytes_estimate(n, B, mcap, nbnd_max, nbr_max, T) > (size_t)(0.6 * (double)fr)) T = invit_threads(mcap, 0);
+  if (const char *env = getenv("PARPHOM_GPU_INVIT_THREADS")) {
+    const int64_t cap = atoll(env);
+    if (cap > 0) T = std::min(T, (cap + 31) / 32 * 32);
+  }
   const int nbr = (int)nbr_max;
   const int ldwp = std::max(std::max(mcap, nbr), 64);
   // split-K partials: 8 chunks of 32 x ldwp, or one per 256 rows

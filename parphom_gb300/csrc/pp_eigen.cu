@@ -2011,10 +2011,19 @@ __global__ void __launch_bounds__(IV_NT) k_invit(const double *__restrict__ dd, 
 #undef PIV
 }
 
-// Threads of k_invit with scratch for an eigenvector each, out of mcap: a
-// thread's time is that of the whole recurrence, so a second launch for the
-// rest costs as much as the first (n = 2604: 5.5 ms for 556 of 2604).
-int64_t invit_threads(int64_t mcap) { return std::min<int64_t>((mcap + 63) / 64 * 64, 6144); }
+// Threads of k_invit with scratch for an eigenvector each, out of mcap: 2048, or
+// all (up to 6144: beyond, the reduction takes seconds) in batches of up to IV_BUSY
+// threads.  A thread's time is that of the whole recurrence, so while a launch
+// leaves the FP64 pipes idle a second one for the rest costs as much as the first:
+// n = 2604, 4 matrices 8.8 -> 4.6 ms, n = 4764, 8 matrices 50 -> 37 ms (969 instead
+// of 983 ms a pass).  Past that the pipes are busy either way and the scratch (33 n
+// bytes a thread) is not worth it: n = 4764, 24 matrices 53 -> 38 ms of a pass of
+// 2696 and 2699 ms for 10 GB more, n = 2604, 48 matrices 26 -> 27 ms for 3 GB.
+constexpr int64_t IV_BUSY = 40960;
+int64_t invit_threads(int64_t mcap, int B) {
+  const int64_t all = std::min<int64_t>((mcap + 63) / 64 * 64, 6144);
+  return B > 0 && all * B <= IV_BUSY ? all : std::min<int64_t>(all, 2048);
+}
 
 template <class R>
 cudaError_t tridiag_eigenvectors(EigWork &w, cudaStream_t s) {

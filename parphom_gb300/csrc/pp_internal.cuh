@@ -37,9 +37,9 @@ void kt_end(int k, cudaStream_t s);
   } while (0)
 
 // Inverse iteration: fields of scratch per row and thread, and the threads that
-// get scratch for mcap eigenvectors.
+// get scratch for mcap eigenvectors of each of B matrices (B = 0: the fewest).
 constexpr int IV_F = 4;  // 1/u0, u1, l, x
-int64_t invit_threads(int64_t mcap);
+int64_t invit_threads(int64_t mcap, int B);
 
 // Per-batch state of the eigensolver.  Every matrix b of a batch of `B`
 // Hermitian matrices has its own order nvec[b] <= nmax; all buffers use the
