@@ -126,7 +126,9 @@ struct pp_ctx {
   // captured CUDA graphs of the last batch configurations: a pass that
   // alternates between configurations (forward and backward of a fit, the full
   // and the last batch of a long list) replays them instead of capturing each
-  // anew
+  // anew.  A kernel in a graph takes about 5 KB of host memory and 2 KB on the
+  // device (n = 4764, 4 streams: 61097 kernels), so all but the newest are kept
+  // up to GRAPH_KERNELS in all.
   struct Graph {
     cudaGraphExec_t exec = nullptr;
     char key[192] = {0};
@@ -134,8 +136,8 @@ struct pp_ctx {
     uint64_t used = 0;
   };
   static constexpr int MAX_GRAPHS = 4;
+  static constexpr int64_t GRAPH_KERNELS = 250000;
   Graph graphs[MAX_GRAPHS];
-  Graph *graph = nullptr;  // of the current configuration
   std::vector<int64_t> bnd_blocks;  // boundary blocks (I + N J) of the tables in g
   uint64_t graph_uses = 0;
 };
@@ -210,7 +212,6 @@ void drop_graph(pp_ctx::Graph &g) {
 }
 void drop_graphs(pp_ctx *c) {
   for (auto &g : c->graphs) drop_graph(g);
-  c->graph = nullptr;
 }
 
 void free_ws(pp_ctx *c) {
@@ -547,20 +548,71 @@ bool graphs_enabled() {
   return !(e && e[0] == '0');
 }
 
-// run_batch through a captured CUDA graph: the launch sequence depends only on
-// the batch size, the options and the workspace, so it is captured once and
-// replayed (one graph launch instead of ~6 launches per matrix column).
-int run_batch_graph_cfg(pp_ctx *c, int B, const pp_eig_opts *o, int mcap, bool want_z, bool launch = true);
+// Capture the launch sequence of a batch in the current launch configuration (it
+// depends only on the batch size, the options and the workspace) and
+// instantiate it.  PP_OK, or the graph path is not available.
+int capture_graph(pp_ctx *c, int B, const pp_eig_opts *o, int mcap, bool want_z, pp_ctx::Graph &out) {
+  cudaStream_t s = c->stream;
+  TRY_CUDA(prepare_bisect(bisect_smem(c->w.nmax, o->precision == PP_PREC_MIXED)));
+  if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+    cudaGetLastError();
+    return 1;
+  }
+  const int64_t l0 = pp::g_launches.load();
+  const int r = run_batch(c, B, o, mcap, want_z);
+  out.launches = pp::g_launches.load() - l0;
+  pp::g_launches.fetch_sub(out.launches);  // captured, not launched
+  cudaGraph_t g = nullptr;
+  cudaError_t e = cudaStreamEndCapture(s, &g);
+  if (r == PP_OK && e == cudaSuccess && g) e = cudaGraphInstantiate(&out.exec, g, 0);
+  if (g) cudaGraphDestroy(g);
+  if (r == PP_OK && e == cudaSuccess && g) return PP_OK;
+  out = pp_ctx::Graph();
+  cudaGetLastError();
+  return 1;
+}
+
+// The key of a batch's graph in the current launch configuration.
+void graph_key(const pp_ctx *c, int B, const pp_eig_opts *o, bool want_z, char (&key)[192]) {
+  snprintf(key, sizeof(key), "%p|%d|%d|%c%c%c|%d|%lld|%lld|%.17g|%.17g|%.17g|%d|%d|%d|%d", c->ws, B, o->precision,
+           o->jobz, o->range, o->vel_method, o->vel, (long long)o->il, (long long)o->iu, o->vl, o->vu, o->abstol,
+           want_z ? 1 : 0, c->cur_split, c->cur_bps, o->want_resid ? 1 : 0);
+}
+
+// Keep a graph under a key, in the place of the one unused for longest; further
+// ones go while there are too many kernels in all.
+pp_ctx::Graph &keep_graph(pp_ctx *c, pp_ctx::Graph &g, const char *key) {
+  pp_ctx::Graph *slot = &c->graphs[0];
+  for (auto &x : c->graphs)
+    if (x.used < slot->used) slot = &x;
+  drop_graph(*slot);
+  std::swap(*slot, g);
+  snprintf(slot->key, sizeof(slot->key), "%s", key);
+  slot->used = ++c->graph_uses;
+  for (;;) {
+    int64_t kernels = 0, others = 0;
+    for (auto &x : c->graphs) {
+      kernels += x.launches;
+      if (&x != slot) others += x.launches;
+    }
+    if (kernels <= pp_ctx::GRAPH_KERNELS || others == 0) return *slot;
+    pp_ctx::Graph *p = nullptr;
+    for (auto &x : c->graphs)
+      if (&x != slot && x.exec && (!p || x.used < p->used)) p = &x;
+    drop_graph(*p);
+  }
+}
 
 // Time one launch configuration: capture and instantiate its graph (host
 // work, not timed), then time one launch of it on the stream with events.
 // Returns the milliseconds, or a negative value if the graph path is not
 // available.
-float time_config(pp_ctx *c, int B, const pp_eig_opts *o, int mcap, bool want_z, int split, int bps) {
+float time_config(pp_ctx *c, int B, const pp_eig_opts *o, int mcap, bool want_z, int split, int bps,
+                  pp_ctx::Graph &g) {
   c->cur_split = split;
   c->cur_bps = bps;
   cudaStream_t s = c->stream;
-  if (run_batch_graph_cfg(c, B, o, mcap, want_z, false) != PP_OK || !c->graph) return -1.f;
+  if (capture_graph(c, B, o, mcap, want_z, g) != PP_OK) return -1.f;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) {
     cudaGetLastError();
@@ -569,8 +621,8 @@ float time_config(pp_ctx *c, int B, const pp_eig_opts *o, int mcap, bool want_z,
   }
   float ms = -1.f;
   cudaEventRecord(e0, s);
-  const cudaError_t r = cudaGraphLaunch(c->graph->exec, s);
-  pp::count_launch(c->graph->launches);
+  const cudaError_t r = cudaGraphLaunch(g.exec, s);
+  pp::count_launch(g.launches);
   cudaEventRecord(e1, s);
   if (r == cudaSuccess && cudaEventSynchronize(e1) == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
   cudaGetLastError();
@@ -578,6 +630,8 @@ float time_config(pp_ctx *c, int B, const pp_eig_opts *o, int mcap, bool want_z,
   cudaEventDestroy(e1);
   return ms;
 }
+
+int run_batch_graph_cfg(pp_ctx *c, int B, const pp_eig_opts *o, int mcap, bool want_z);
 
 int run_batch_graph(pp_ctx *c, int B, const pp_eig_opts *o, int mcap, bool want_z) {
   c->cur_split = split_ways();
@@ -600,21 +654,37 @@ int run_batch_graph(pp_ctx *c, int B, const pp_eig_opts *o, int mcap, bool want_
     const bool can_tune = graphs_enabled() && !pp::kt_mask && !tc_stall_armed() && cs == cudaStreamCaptureStatusNone;
     if (t.split < 0 && !can_tune) t = Tuned{split_ways(), 6, 0.f};
     if (t.split < 0) {
-      // greedy: split over {4, 8, 16, 32} (at most B) with 6 mat-vec blocks per SM
+      // greedy: split over {4, 8, 16, 32} (at most B) with 6 mat-vec blocks per SM.  Only the
+      // fastest candidate's graph is kept, and none of the other configurations' goes for the rest
       Tuned best{std::min(B, 8), 6, 1e30f};
+      pp_ctx::Graph best_graph;
+      auto timed = [&](int split, int bps) {
+        pp_ctx::Graph g;
+        const float ms = time_config(c, B, o, mcap, want_z, split, bps, g);
+        const bool better = ms > 0.f && ms < best.ms;
+        if (better) {
+          best = Tuned{split, bps, ms};
+          std::swap(g, best_graph);
+        }
+        drop_graph(g);
+        return better;
+      };
       for (int sp : {4, 8, 16, 32}) {
         if (sp > B && sp != 4) continue;
-        const int spc = std::min(sp, B);
-        const float ms = time_config(c, B, o, mcap, want_z, spc, 6);
-        if (ms > 0.f && ms < best.ms) best = Tuned{spc, 6, ms};
+        timed(std::min(sp, B), 6);
       }
       // then, FP64 form, fewer persistent mat-vec blocks per SM (6 -> 4 -> 3 -> 2) while that helps:
       // with several streams the mat-vecs of different parts share the SMs
       for (int bps : {4, 3, 2}) {
         if (best.ms > 1e29f || o->precision == PP_PREC_MIXED) break;
-        const float ms = time_config(c, B, o, mcap, want_z, best.split, bps);
-        if (!(ms > 0.f && ms < best.ms)) break;
-        best = Tuned{best.split, bps, ms};
+        if (!timed(best.split, bps)) break;
+      }
+      if (best_graph.exec) {
+        char gkey[192];
+        c->cur_split = best.split;
+        c->cur_bps = best.bps;
+        graph_key(c, B, o, want_z, gkey);
+        keep_graph(c, best_graph, gkey);
       }
       if (best.ms > 1e29f) best.ms = 0.f;
       t = best;
@@ -628,61 +698,24 @@ int run_batch_graph(pp_ctx *c, int B, const pp_eig_opts *o, int mcap, bool want_
 }
 
 // The batch through its captured graph (captured on the first use of a
-// configuration); with launch = false the graph is only captured and
-// instantiated (used by the autotuner, which then times the launch).
-int run_batch_graph_cfg(pp_ctx *c, int B, const pp_eig_opts *o, int mcap, bool want_z, bool launch) {
+// configuration; one graph launch instead of 2 to 3 launches per matrix column).
+int run_batch_graph_cfg(pp_ctx *c, int B, const pp_eig_opts *o, int mcap, bool want_z) {
   // (an armed test stall is a one-shot launch parameter: never captured)
-  if (!graphs_enabled() || pp::kt_mask || tc_stall_armed()) return launch ? run_batch(c, B, o, mcap, want_z) : 1;
+  if (!graphs_enabled() || pp::kt_mask || tc_stall_armed()) return run_batch(c, B, o, mcap, want_z);
   char key[192];
-  snprintf(key, sizeof(key), "%p|%d|%d|%c%c%c|%d|%lld|%lld|%.17g|%.17g|%.17g|%d|%d|%d|%d", c->ws, B, o->precision,
-           o->jobz, o->range, o->vel_method, o->vel, (long long)o->il, (long long)o->iu, o->vl, o->vu, o->abstol,
-           want_z ? 1 : 0, c->cur_split, c->cur_bps, o->want_resid ? 1 : 0);
-  cudaStream_t s = c->stream;
+  graph_key(c, B, o, want_z, key);
   c->w.B = c->w.batch = B;  // (what follows the graph reads it)
-  c->graph = nullptr;
-  pp_ctx::Graph *slot = &c->graphs[0];  // this configuration's, or the one unused for longest
-  for (auto &g : c->graphs) {
-    if (g.exec && strcmp(key, g.key) == 0) {
-      g.used = ++c->graph_uses;
-      c->graph = &g;
-      if (!launch) return PP_OK;
-      TRY_CUDA(cudaGraphLaunch(g.exec, s));
-      pp::count_launch(g.launches);
-      return PP_OK;
-    }
-    if (g.used < slot->used) slot = &g;
+  pp_ctx::Graph *graph = nullptr;
+  for (auto &g : c->graphs)
+    if (g.exec && strcmp(key, g.key) == 0) graph = &g;
+  if (!graph) {
+    pp_ctx::Graph g;
+    if (capture_graph(c, B, o, mcap, want_z, g) != PP_OK) return run_batch(c, B, o, mcap, want_z);
+    graph = &keep_graph(c, g, key);
   }
-  drop_graph(*slot);
-  TRY_CUDA(prepare_bisect(bisect_smem(c->w.nmax, o->precision == PP_PREC_MIXED)));
-  if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-    cudaGetLastError();
-    return launch ? run_batch(c, B, o, mcap, want_z) : 1;
-  }
-  const int64_t l0 = pp::g_launches.load();
-  const int r = run_batch(c, B, o, mcap, want_z);
-  slot->launches = pp::g_launches.load() - l0;
-  cudaGraph_t g = nullptr;
-  cudaError_t e = cudaStreamEndCapture(s, &g);
-  if (r != PP_OK || e != cudaSuccess || !g) {
-    if (g) cudaGraphDestroy(g);
-    cudaGetLastError();
-    return launch ? run_batch(c, B, o, mcap, want_z) : 1;
-  }
-  e = cudaGraphInstantiate(&slot->exec, g, 0);
-  cudaGraphDestroy(g);
-  if (e != cudaSuccess) {
-    slot->exec = nullptr;
-    cudaGetLastError();
-    return launch ? run_batch(c, B, o, mcap, want_z) : 1;
-  }
-  snprintf(slot->key, sizeof(slot->key), "%s", key);
-  slot->used = ++c->graph_uses;
-  c->graph = slot;
-  if (!launch) {
-    pp::g_launches.fetch_sub(slot->launches);  // captured, not launched
-    return PP_OK;
-  }
-  TRY_CUDA(cudaGraphLaunch(slot->exec, s));
+  graph->used = ++c->graph_uses;
+  TRY_CUDA(cudaGraphLaunch(graph->exec, c->stream));
+  pp::count_launch(graph->launches);
   return PP_OK;
 }
 
