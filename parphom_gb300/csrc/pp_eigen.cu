@@ -1776,17 +1776,6 @@ __device__ __forceinline__ uint32_t hash32(uint32_t x) {
   return x;
 }
 
-// 1/x, |x| in the middle of the exponent range: the hardware's estimate and one
-// step of third order (Halley's iteration, r (1 + e + e^2) with e = 1 - x r).
-// Three dependent FP64 operations where a division waits 560 cycles.
-__device__ __forceinline__ double recip(double x) {
-  if ((unsigned)((__double2hiint(x) >> 20 & 0x7ff) - 23) >= 2000u) return 1.0 / x;
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  const double e = fma(-x, r, 1.0);
-  return fma(r, fma(e, e, e), r);
-}
-
 // One thread per cluster of eigenvalues (clusters cbase .. cbase+T-1).
 // LU of T - lam I with partial pivoting: row k of U holds 1/u0, u1 and u2 (u2 =
 // e(k+1) after a row interchange, else 0) at columns (k, k+1, k+2); l is the

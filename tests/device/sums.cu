@@ -20,6 +20,17 @@ __global__ void k_sums(int n, const float4 *w, const float4 *v, const double2 *t
   if (lane == 0) out[c] = make_float4(r.re.hi, r.re.lo, r.im.hi, r.im.lo);
 }
 
+__global__ void k_recip(int n, const double *x, double *r, double *q) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  r[i] = recip(x[i]);
+  q[i] = 1.0 / x[i];
+}
+
+EXPORT int reciprocals(int n, const double *x, double *r, double *q) {
+  k_recip<<<(n + 127) / 128, 128>>>(n, x, r, q);
+  return (int)cudaDeviceSynchronize();
+}
 EXPORT int sums(int cases, int n, const float *w, const float *v, const double *t, float *own, float *out) {
   k_sums<<<cases, 32>>>(n, (const float4 *)w, (const float4 *)v, (const double2 *)t, own, (float4 *)out);
   return (int)cudaDeviceSynchronize();
