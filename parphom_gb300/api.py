@@ -356,7 +356,7 @@ def heevx_values_noalloc(a_ptr: int, lda: int, n: int, w_ptr: int, m_ptr: int, i
 
 def kernel_timer(names: str) -> None:
     """Record CUDA events around every launch of the named kernel classes
-    (comma separated: hemv, colstep, her2k, vhx, applyV, xhz, invit, bisect, assemble, vel);
+    (comma separated: hemv, colstep, her2k, vhx, btred, applyV, xhz, invit, bisect, assemble, vel);
     empty string disables."""
     load().pp_ktimer_enable(names.encode())
 

@@ -13,7 +13,8 @@
 //     A = Q T Q^H with Q = H(0) H(1) ... H(n-2), H(i) = I - tau_i v_i v_i^H.
 //  2. Eigenvalues of T by Sturm-count bisection, one thread per eigenvalue
 //     index, with the dstebz tolerance rule max(abstol, pivmin,
-//     2 ulp max(|lo|,|hi|)).  Always FP64.
+//     2 ulp max(|lo|,|hi|)): FP32 counts first, then FP64 ones (mixed form:
+//     double-float ones, down to 4 x 2^-44 ||T||).
 //  3. Eigenvectors of T by inverse iteration with partial-pivoting LU of
 //     T - lambda I, one thread per eigenvalue cluster, modified Gram-Schmidt
 //     inside clusters (consecutive eigenvalues closer than 1e-7 ||T||), then
@@ -255,18 +256,18 @@ __device__ __forceinline__ C<df> prescale(C<df> x, int e) {
 __device__ __forceinline__ float magnitude(C<double>) { return 0.f; }
 __device__ __forceinline__ float magnitude(C<df> x) { return fmaxf(fabsf(x.re.hi), fabsf(x.im.hi)); }
 
+// ---- the mat-vec of the FP64 form
 // Lower-triangle Hermitian mat-vec y = A v on the trailing block [i+1, n),
 // over the lower tile pairs (R >= C) of HL_T x HL_T: a tile is read once and
 // gives both A_RC v_C (into slot C of the rows of R) and A_RC^H v_R (into
 // slot R of the rows of C).  Every row receives exactly one partial per slot
-// 0 .. ntiles-1, summed later by k_wcorr.  Blocks are persistent over a
-// strided set of tile pairs with two shared-memory buffers: the next tile
-// (and its two vector pieces) is copied by cp.async while the double-float
+// 0 .. ntiles-1, summed by the column step (k_wpart, k_colstep).  Blocks are
+// persistent over a strided set of tile pairs with two shared-memory buffers: the
+// next tile (and its two vector pieces) is copied by cp.async while the FP64
 // arithmetic of the current one runs.
 constexpr int HL_T = 32;         // tile of large trailing blocks
 constexpr int HL_TS = 16;        // tile of trailing blocks up to HL_SMALL rows: four times the tiles, so that
 constexpr int HL_SMALL = 128;    // more SMs' FP64 pipes take part (n = 84: 9.1 -> 7.9 us between events)
-constexpr int HL_NT = 128;       // threads for a tile of 32 (4 T)
 constexpr int HL_BPS = 6;        // resident blocks per SM
 constexpr int HL_UNROLL = 4;     // inner-loop unrolling (keeps the kernel's code small)
 __host__ __device__ __forceinline__ int hl_tile(int rows) { return rows <= HL_SMALL ? HL_TS : HL_T; }

@@ -130,8 +130,7 @@ cudaError_t geom_build_masks(Geometry &g, cudaStream_t s);
 cudaError_t geom_symmetrize_fc(Geometry &g, int enforce_asr, cudaStream_t s);
 cudaError_t geom_block_nonzero(const Geometry &g, uint8_t *d_flags, cudaStream_t s);
 
-// D(q) for B q-points into 16-byte complex storage (z64 if dfmt==0, double-float
-// in the trailing matrix's order zpk if 1).
+// D(q) for B q-points into 16-byte complex storage (z64 if dfmt==0, zdf if 1).
 cudaError_t assemble_batch(const Geometry &g, const double *d_q, int B, void *A, int64_t lda, int64_t sA,
                            int dfmt, cudaStream_t s);
 // dD/dq_k (derivative 1..3, method 'A' or 'C') or D (derivative 0), FP64.

@@ -1033,7 +1033,7 @@ cudaError_t applyV_tc(EigWork &w, int k0, int jb, zdf *X, int64_t ldx, int64_t s
 }
 
 // Wp(a, c) = (V^H X)(a, c) over the rows r > k0 (V: panel k0 of width jb),
-// c < ncols; written to the first split-K slot of Wp.
+// c < ncols; the rows in vhx_tc_splits(w) ranges, a split-K slot of Wp each.
 int vhx_tc_splits(const EigWork &w) { return std::max(1, std::min(4, w.ksplit)); }
 
 cudaError_t vhx_tc(EigWork &w, int k0, int jb, const zdf *X, int64_t ldx, int64_t sX, int ncols, zdf *Wp,
