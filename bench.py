@@ -355,8 +355,8 @@ def main():
 HEMV_TRAFFIC_RATIO = 1.084
 
 
-def roofline_for(kclass, rec, n, nq):
-    """Algorithmic work of the dominant kernel class over the timed region."""
+def roofline_for(kclass, rec, n, nq, fp64=False):
+    """Algorithmic work of the dominant kernel class over the timed region (fp64: of the plain FP64 form)."""
     launches, ms = rec
     peaks = {}
     try:
@@ -365,7 +365,7 @@ def roofline_for(kclass, rec, n, nq):
         pass
     hbm = peaks.get("hbm_gbs", 6800.0)
     src = "of measured" if "hbm_gbs" in peaks else "of fallback"
-    if kclass == "hemv":
+    if kclass == "hemv" and not fp64:
         # each column i reads the lower triangle of the trailing (n-i-1)^2
         # block once: m(m+1)/2 16-byte elements, m = n-i-1
         byts = nq * 16.0 * sum((n - i - 1) * (n - i) / 2 for i in range(n - 1))
@@ -378,23 +378,31 @@ def roofline_for(kclass, rec, n, nq):
                                   "first columns) = 1.084 x its algorithmic bytes, scaled to this average launch",
                 "launches": launches, "avg_launch_ms": ms / launches,
                 "algorithmic_bytes_per_launch": byts / launches}
-    # FP32-pipe kernels (double-float arithmetic): count complex MACs
-    macs = {"her2k": 2.0 * sum((n - k) ** 2 * 32 for k in range(32, n, 32)),
+    # count complex MACs (a stored element of the mat-vec's lower triangle takes part in two)
+    macs = {"hemv": sum(float(n - i - 1) * (n - i) for i in range(n - 1)),
+            "her2k": sum((n - k) ** 2 * 32.0 for k in range(32, n, 32)),  # lower triangle
             "vhx": sum(n * (n - k) * 32.0 for k in range(0, n, 32)),
             "applyV": sum(n * (n - k) * 32.0 for k in range(0, n, 32))}.get(kclass)
     if macs is None:
-        return {"bound": "hbm", "kernel": kclass, "achieved": None, "peak": hbm, "unit": "GB/s", "frac": None,
+        return {"bound": None, "kernel": kclass, "achieved": None, "peak": None, "unit": None, "frac": None,
                 "launches": launches, "avg_launch_ms": ms / launches}
     flops = 8.0 * macs * nq
     ach = flops / (ms / 1e3) / 1e12
-    return {"bound": "fp32-simt (double-float)", "kernel": kclass, "achieved": ach, "peak": None, "unit": "TFLOP/s",
-            "frac": None, "launches": launches, "avg_launch_ms": ms / launches}
+    kernel = {"hemv": "k_hemv_lower", "her2k": "k_her2k", "vhx": "k_vhx", "applyV": "k_applyV"} if fp64 else \
+        {"her2k": "k_cupd_tc (trailing update)", "vhx": "k_longk_tc (V^H X)", "applyV": "k_cupd_tc (X -= V Y)"}
+    peak = FP64_TFLOPS if fp64 else None
+    return {"bound": "fp64 pipe" if fp64 else "tensor cores (28 slice products per real one)", "kernel": kernel[kclass],
+            "achieved": ach, "peak": peak, "unit": "TFLOP/s", "frac": ach / peak if peak else None,
+            "peak_source": "torch float64 GEMM" if fp64 else None, "launches": launches, "avg_launch_ms": ms / launches}
+
+
+FP64_TFLOPS = 1.10  # torch float64 and complex128 GEMM on a GB300
 
 
 ALL_KERNELS = "assemble,hemv,colstep,her2k,bisect,invit,vhx,btred,applyV,vel,xhz"
 
 
-def timed(fn, nq, n, kclasses=ALL_KERNELS):
+def timed(fn, nq, n, kclasses=ALL_KERNELS, fp64=False):
     """q-points/s of one call of fn through the host C ABI (host buffers in and
     out, copies included), after one untimed call of the same batch (which
     tunes and captures its launch configuration), then the same call again
@@ -416,13 +424,13 @@ def timed(fn, nq, n, kclasses=ALL_KERNELS):
     if kt:
         dom = max(kt, key=lambda k: kt[k][1])
         if isinstance(n, (list, tuple)):   # cells of several orders: (order, q-points) pairs
-            parts = [roofline_for(dom, kt[dom], ni, qi) for ni, qi in n]
+            parts = [roofline_for(dom, kt[dom], ni, qi, fp64) for ni, qi in n]
             roof = dict(parts[0])
             if roof.get("achieved") is not None:
                 roof["achieved"] = sum(pp["achieved"] for pp in parts)
                 roof["frac"] = roof["achieved"] / roof["peak"] if roof.get("peak") else None
         else:
-            roof = roofline_for(dom, kt[dom], n, nq)
+            roof = roofline_for(dom, kt[dom], n, nq, fp64)
         roof = {k: roof.get(k) for k in ("kernel", "bound", "achieved", "unit", "frac", "peak")}
         roof["share_of_kernel_time"] = round(kt[dom][1] / sum(v[1] for v in kt.values()), 3)
     return out, {"value": nq / dt, "unit": UNIT, "s": dt, "n_q": nq, "roofline": roof}
@@ -458,7 +466,7 @@ def other_configs(dev):
     with api.PhononContext.from_cell(c, phi) as ctx:
         q = synth.band_path(64)
         o = api.EigOpts(jobz="N", precision=api.PP_PREC_FP64)
-        r, e = timed(lambda: ctx.solve(q, o, want_z=False), 64, c.n)
+        r, e = timed(lambda: ctx.solve(q, o, want_z=False), 64, c.n, fp64=True)
         e.update({"workload": "N=148 (3N=444), FP64, 64 q band path, range A, no vectors", "sample": "all 64 q",
                   "vs_oracle": oracle_check(S, q[5], r.w[5], None)})
         res["1_n148_fp64"] = e
@@ -473,7 +481,7 @@ def other_configs(dev):
         outs = {}
         for name, prec in (("fp64", api.PP_PREC_FP64), ("mixed", api.PP_PREC_MIXED)):
             o = api.EigOpts(jobz="V", vel=True, precision=prec)
-            outs[name], ent[name] = timed(lambda: ctx.solve(q, o), len(q), c.n)
+            outs[name], ent[name] = timed(lambda: ctx.solve(q, o), len(q), c.n, fp64=prec == api.PP_PREC_FP64)
         ent["mixed_over_fp64"] = ent["mixed"]["value"] / ent["fp64"]["value"]
         big = np.abs(outs["fp64"].w) >= 1.0
         ent["mixed_vs_fp64"] = {
