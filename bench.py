@@ -393,10 +393,10 @@ def roofline_for(kclass, rec, n, nq, fp64=False):
     peak = FP64_TFLOPS if fp64 else None
     return {"bound": "fp64 pipe" if fp64 else "tensor cores (28 slice products per real one)", "kernel": kernel[kclass],
             "achieved": ach, "peak": peak, "unit": "TFLOP/s", "frac": ach / peak if peak else None,
-            "peak_source": "torch float64 GEMM" if fp64 else None, "launches": launches, "avg_launch_ms": ms / launches}
+            "peak_source": "2 multiply-adds per SM and clock" if fp64 else None, "launches": launches, "avg_launch_ms": ms / launches}
 
 
-FP64_TFLOPS = 1.10  # torch float64 and complex128 GEMM on a GB300
+FP64_TFLOPS = 4 * 152 * 2.07e-3  # 2 multiply-adds per SM and clock, 152 SMs, 2070 MHz (a float64 GEMM: 1.10)
 
 
 ALL_KERNELS = "assemble,hemv,colstep,her2k,bisect,invit,vhx,btred,applyV,vel,xhz"
