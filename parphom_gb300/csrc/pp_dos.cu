@@ -241,10 +241,10 @@ cudaError_t dos_tri(const double *freq, int64_t ldf, const double *func, int64_t
 }
 
 // Room for the parts of the device-resident form, which allocates nothing: fixed
-// arrays of the library, one for each of up to DS_SLOTS calls in flight on a
-// device.  A call takes the array that its stream used last, or one whose last
-// call has ended, or waits on the device for one; inside a stream capture (a graph
-// may run at any time) and past DS_CAP it goes without.
+// arrays of the library, one for each of up to DS_SLOTS streams with calls in flight
+// on a device.  A call takes the array that its stream used last, or the one unused
+// for longest, whose last call it waits for on the device; inside a stream capture (a
+// graph may run at any time) and past DS_CAP it goes without.
 constexpr int DS_SLOTS = 2;
 constexpr int64_t DS_CAP = 2 * 160 * DT_E;  // doubles: 160 SMs with DT_E energies each
 __device__ double dos_parts[DS_SLOTS][DS_CAP];
@@ -252,7 +252,7 @@ struct DosSlots {
   double *base = nullptr;
   cudaStream_t stream[DS_SLOTS] = {};
   cudaEvent_t done[DS_SLOTS] = {};
-  bool used[DS_SLOTS] = {};
+  uint64_t used[DS_SLOTS] = {}, uses = 0;  // 0: never
 };
 std::mutex ds_mu;
 DosSlots ds_slots[pp::PP_MAX_DEVICES];
@@ -270,26 +270,26 @@ cudaError_t with_parts(int64_t need, cudaStream_t s, F launch) {
   std::lock_guard<std::mutex> g(ds_mu);
   DosSlots &d = ds_slots[dev];
   if (!d.base) {
+    // (another thread may be capturing: neither call touches its stream)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
     void *p = nullptr;
     cudaError_t e = cudaGetSymbolAddress(&p, dos_parts);
     for (int k = 0; k < DS_SLOTS && e == cudaSuccess; ++k)
       if (!d.done[k]) e = cudaEventCreateWithFlags(&d.done[k], cudaEventDisableTiming);
+    cudaThreadExchangeStreamCaptureMode(&mode);
     if (e != cudaSuccess) return e;
     d.base = (double *)p;
   }
-  int k = -1;
+  int k = 0;
+  for (int t = 1; t < DS_SLOTS; ++t)
+    if (d.used[t] < d.used[k]) k = t;
   for (int t = 0; t < DS_SLOTS; ++t)
     if (d.used[t] && d.stream[t] == s) k = t;
-  for (int t = 0; t < DS_SLOTS && k < 0; ++t)
-    if (!d.used[t] || cudaEventQuery(d.done[t]) == cudaSuccess) k = t;
-  if (k < 0) {
-    cudaGetLastError();  // (not ready)
-    k = 0;
-  }
   cudaError_t e = d.used[k] ? cudaStreamWaitEvent(s, d.done[k], 0) : cudaSuccess;
   if (e != cudaSuccess) return e;
   e = launch(d.base + k * DS_CAP);
-  d.used[k] = true;
+  d.used[k] = ++d.uses;
   d.stream[k] = s;
   const cudaError_t r = cudaEventRecord(d.done[k], s);
   return e != cudaSuccess ? e : r;

@@ -112,3 +112,51 @@ def test_values_a_subnormal_apart(vals):
             c, d = (e2 - x) / (e2 - e0), (e2 - x) / (e2 - e1)
             want = (1 - d * c * c) + (1 - c * d * d) + (1 - 3 * c * d + d * c * c + c * d * d)
         assert abs(n - want) <= 1e-12 * want
+
+
+def test_call_while_another_thread_captures():
+    """A call on an ordinary stream while another thread captures its own in the global mode: neither disturbs the other."""
+    import threading
+    import torch
+    dev = torch.device("cuda")
+    freq, w, tri = _bands(8, 50, 4)
+    E = np.linspace(0.0, 1650.0, 300)
+    F, T, X = (torch.tensor(a, device=dev) for a in (freq, tri, E))
+    d, n = dos.linear_triangulation_device(F, T, X)
+    outs = [(torch.zeros_like(d), torch.zeros_like(n)) for _ in range(4)]
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    begun, called, err = threading.Event(), threading.Event(), []
+    y = torch.zeros(16, device=dev)
+    g = torch.cuda.CUDAGraph()
+
+    def capture():
+        try:
+            s = torch.cuda.Stream()
+            with torch.cuda.stream(s):
+                g.capture_begin(capture_error_mode="global")
+                y.add_(1.0)
+                begun.set()
+                called.wait(20)
+                y.add_(1.0)
+                g.capture_end()
+        except Exception as ex:   # noqa: BLE001
+            err.append(ex)
+            begun.set()
+
+    t = threading.Thread(target=capture)
+    t.start()
+    begun.wait(20)
+    L, p = dos._lib(), dos._ptr
+    import ctypes
+    rcs = [L.pp_dos_triangulation_device(p(F), F.shape[1], F.shape[0], F.shape[1], None, F.shape[1], p(T), len(T),
+                                         p(X), len(X), p(a), p(b), ctypes.c_void_p(side.cuda_stream)) for a, b in outs]
+    called.set()
+    t.join()
+    torch.cuda.synchronize()
+    assert not err and rcs == [0] * 4, (err, rcs)
+    for a, b in outs:
+        assert torch.equal(a, d) and torch.equal(b, n)
+    g.replay()
+    torch.cuda.synchronize()
+    assert float(y[0]) == 2.0
