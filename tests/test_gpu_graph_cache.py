@@ -82,7 +82,9 @@ def test_tuning_leaves_other_configurations_captured():
         ctx.solve(q, api.EigOpts(jobz="N", precision=api.PP_PREC_MIXED))    # (sizes the workspace)
         once(ctx, 1, 16)
         before = min(once(ctx, 1, 16) for _ in range(3))
-        once(ctx, 1, 15)
-        once(ctx, 1, 14)
-        after = once(ctx, 1, 16)
-    assert after <= 1.3 * before, (before, after)
+        after = []
+        for nq in (15, 13, 11):                # (the best of three: a host may be busy once)
+            once(ctx, 1, nq)
+            once(ctx, 1, nq - 1)
+            after.append(once(ctx, 1, 16))
+    assert min(after) <= 1.3 * before, (before, after)
