@@ -1215,7 +1215,7 @@ static cudaError_t prepare_colstep(int *cluster) {
   }
   if (const char *v = getenv("PARPHOM_GPU_CLUSTER")) {
     const int cap = atoi(v);
-    while (*cluster > 1 && *cluster > cap) *cluster /= 2;
+    while (cap > 0 && *cluster > cap) *cluster /= 2;
   }
   return cudaSuccess;
 }
